@@ -299,6 +299,69 @@ __global__ void __launch_bounds__(256) outer_kernel(P p) {
   }
 }
 
+// One warp per (sample, output row), C2 / 4 a power of two up to 32: a lane keeps its four columns of y for all rows a
+// it serves, so an entry costs one 4-wide load of y, one broadcast load of x and four FMAs per four outputs, and the
+// row leaves as 128-bit stores of consecutive lanes.  Bound: the C1 * C2 values written per row.  The form above spends
+// several 64-bit divisions per output element; 2000 samples x 35 rows x 32 x 32 float32: 929 -> 78 us (3.7 TB/s).
+template <typename T> struct alignas(4 * sizeof(T)) Quad { T v[4]; };
+template <typename T>
+__global__ void __launch_bounds__(256) outer_rows_kernel(P p) {
+  using A = typename Acc<T>::type;
+  constexpr int U = 8;                               // rows a per lane and pass
+  const T* x = static_cast<const T*>(p.in1);
+  const T* y = static_cast<const T*>(p.in2);
+  T* out = static_cast<T*>(p.out);
+  const int C1 = (int)p.c1, C2 = (int)p.c2, lanes_b = C2 / 4;
+  const int lane = threadIdx.x & 31, b = (lane % lanes_b) * 4, a_first = lane / lanes_b, a_step = 32 / lanes_b;
+  const int num_out = (int)p.num_out;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5), total = p.n * p.num_out;
+  int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  int64_t n = w / num_out;
+  int o = (int)(w - n * num_out);
+  const int64_t step_n = warps / num_out;
+  const int step_o = (int)(warps - step_n * num_out);
+  for (; w < total; w += warps) {
+    int64_t t0, t1;
+    seg_range(p, o, t0, t1);
+    T* orow = out + (n * p.out_size + out_row(p, o)) * C1 * C2 + b;
+    for (int a0 = a_first; a0 < C1; a0 += U * a_step) {
+      A acc[U][4];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[u][k] = A(0);
+      for (int64_t t = t0; t < t1; ++t) {
+        const Entry e = entry(p, t);
+        const Quad<T> yq = *reinterpret_cast<const Quad<T>*>(y + n * p.bs2 + e.r2 * C2 + b);
+        const A s = scale_of<T>(p, e.tt);
+        A yv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) yv[k] = static_cast<A>(yq.v[k]) * s;
+        const T* xr = x + n * p.bs1 + e.r1 * C1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int a = a0 + u * a_step;
+          const A xv = a < C1 ? ld(xr + a) : A(0);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[u][k] = fma(xv, yv[k], acc[u][k]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int a = a0 + u * a_step;
+        if (a >= C1) break;
+        Quad<T> q;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q.v[k] = static_cast<T>(acc[u][k]);
+        *reinterpret_cast<Quad<T>*>(orow + (int64_t)a * C2) = q;
+      }
+    }
+    n += step_n;
+    o += step_o;
+    if (o >= num_out) { o -= num_out; ++n; }
+  }
+}
+
 // Batch-summed outer product = a GEMM whose reduction runs over (sample, table entry) pairs:
 //   out[o, a, b] = sum_{n, t in seg[o]} s_t x[n, i1_t, a] y[n, i2_t, b].
 // 64x64 output tile per block, 4x4 per thread, 8 pairs staged in shared memory per step.
@@ -566,6 +629,13 @@ int launch(const eqt_product_args& a, P p, cudaStream_t s) {
       dim3 grid((unsigned)tiles, (unsigned)p.num_out, (unsigned)ceil_div(p.n, chunk));
       outer_acc_kernel<T><<<grid, 256, 0, s>>>(p, chunk);
       return check_launch("outer_acc_kernel");
+    }
+    // lanes own four columns each: 4, 8, ... 128 columns and operands whose rows allow 4-wide accesses
+    const int64_t q = p.c2 / 4;
+    if (p.c2 % 4 == 0 && q <= 32 && (q & (q - 1)) == 0 && p.c1 <= 0x7fffff && p.num_out <= 0x7fffffff &&
+        ((reinterpret_cast<uintptr_t>(p.in2) | reinterpret_cast<uintptr_t>(p.out)) & (4 * sizeof(T) - 1)) == 0) {
+      outer_rows_kernel<T><<<flat_grid(p.n * p.num_out, 8, 8), 256, 0, s>>>(p);
+      return check_launch("outer_rows_kernel");
     }
     outer_kernel<T><<<flat_grid(p.n * p.num_out * p.c1 * p.c2, 256), 256, 0, s>>>(p);
     return check_launch("outer_kernel");
