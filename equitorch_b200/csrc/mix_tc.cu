@@ -375,10 +375,12 @@ extern "C" int eqt_vecmat_tc(const float* x, const float* w, const int64_t* inde
   L.out = out; L.kb_begin = kb_begin; L.a_col = a_col; L.n = n; L.num_out = num_out; L.n_cols = cout; L.status = status;
   L.total_items = (int64_t)num_out * ceil_div(n, TILE_M);
   const uint32_t stage_bytes = TILE_M * KB * 4 + 2u * (uint32_t)cout * KB * 4;
-  L.stages = (int)std::min<size_t>(std::min<size_t>(8, (220 * 1024 - 1024 - EPI_PATCH_BYTES) / stage_bytes), (512 - 2 * cout) / 64);
+  L.acc_sets = cout <= 64 ? 2 : 1;               // a pair of accumulators each: at least four A slots stay free
+  const int acc_cols = 2 * L.acc_sets * cout;
+  L.stages = (int)std::min<size_t>(std::min<size_t>(8, (220 * 1024 - 1024 - EPI_PATCH_BYTES) / stage_bytes), (512 - acc_cols) / 64);
   if (L.stages < 2) return fail(EQT_ERR_UNSUPPORTED, "tile too wide for the shared-memory ring");
   L.tmem_cols = 32;
-  while (L.tmem_cols < 2 * cout + 64 * L.stages) L.tmem_cols <<= 1;
+  while (L.tmem_cols < acc_cols + 64 * L.stages) L.tmem_cols <<= 1;
   {
     cuuint64_t dims[3] = {(cuuint64_t)rows1 * cin, 1, (cuuint64_t)n};
     cuuint64_t strides[2] = {(cuuint64_t)rows1 * cin * 4, (cuuint64_t)rows1 * cin * 4};

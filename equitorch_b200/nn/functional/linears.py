@@ -324,14 +324,16 @@ class IrrepsLinear(Function):
     """Channel mixing between every pair of equal irreps of the input and the output
     (``equitorch/nn/functional/linears.py:532-574``).  The reference scatters the per-row results
     to their output components with a third-party ``scatter``; the rows are already unique and
-    sorted, so here ``M_out`` is handed to the kernel as its output-row table."""
+    sorted, so here ``M_out`` is handed to the kernel as its output-row table - or nothing, where every output
+    component receives a path and the table is the identity."""
 
     @staticmethod
     def forward(ctx, input: Tensor, weight: Tensor, info_forward: IrrepsLinearInfo, info_backward: IrrepsLinearInfo):
         from ...ops.batched_sparse_dense_op import indexed_vecmat_scale_gather
         f = info_forward
         out = indexed_vecmat_scale_gather(input, weight, scale=f.scale_MM0, index1=f.M0_MM0, index2=f.ii0_MM0,
-                                          seg=f.M_seg_MM0, index_out=f.M_out, out_size=f.out_size)
+                                          seg=f.M_seg_MM0, index_out=None if f.M_out.shape[0] == f.out_size else f.M_out,
+                                          out_size=f.out_size)
         ctx.save_for_backward(input, weight)
         ctx.infos = (info_forward, info_backward)
         return out
