@@ -70,6 +70,12 @@ class MixBlockStruct(C.Structure):
                 ("w_offset", C.c_int64)]
 
 
+class PathTableStruct(C.Structure):
+    _fields_ = [("fwd_blocks", C.c_void_p), ("bwd_blocks", C.c_void_p), ("fwd_paths", C.c_void_p), ("bwd_paths", C.c_void_p),
+                ("d1", C.c_int32), ("d2", C.c_int32), ("d_out", C.c_int32), ("num_weights", C.c_int32), ("num_paths", C.c_int32),
+                ("num_fwd_blocks", C.c_int32), ("num_bwd_blocks", C.c_int32)]
+
+
 # name -> (restype, argtypes); every symbol declared in include/eqt_b200.h appears here
 SIGNATURES = {
     "eqt_sparse_product": (C.c_int, [C.POINTER(ProductArgs), C.c_void_p]),
@@ -113,6 +119,12 @@ SIGNATURES = {
                                    C.c_void_p, C.c_void_p, C.c_void_p]),
     "eqt_radius_edges": (C.c_int, [C.POINTER(RadiusGridStruct), C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_int32, C.c_int32,
                                    C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(EdgeFeaturesStruct), C.c_void_p, C.c_void_p]),
+    "eqt_so3_uu_scratch_floats": (C.c_int64, [C.POINTER(PathTableStruct), C.c_int64, C.c_int32, C.c_int32, C.c_int32]),
+    "eqt_so3_uu_forward": (C.c_int, [C.POINTER(PathTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
+                                     C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
+    "eqt_so3_uu_backward": (C.c_int, [C.POINTER(PathTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                      C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_int32, C.c_int32,
+                                      C.c_void_p]),
     "eqt_pack_weights": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_int32, C.c_int32,
                                    C.c_void_p, C.c_void_p, C.c_void_p]),
     "eqt_irrep_scale": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,

@@ -1,0 +1,75 @@
+"""Generate ``generated/path_specs.inc``: one Clebsch-Gordan block per (l_out, l_1, l_2) as straight-line code.
+
+A layer's table is a list of paths (k, i, j) between irreps; what a path does depends on its three degrees only.  For
+degrees up to ``MAX_L`` the block's multiply-adds are emitted with the CG values as immediates, on register blocks of V
+channels: products of several y components with the same (M, m1) are summed before they meet the channels.
+
+    python -m equitorch_b200.csrc.gen_path_specs        # rewrites generated/path_specs.inc
+"""
+from __future__ import annotations
+
+import os
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+OUT = os.path.join(HERE, "generated", "path_specs.inc")
+MAX_L = 3
+
+
+def triples():
+    return [(lo, l1, l2) for lo in range(MAX_L + 1) for l1 in range(MAX_L + 1) for l2 in range(MAX_L + 1)
+            if abs(l1 - l2) <= lo <= l1 + l2]
+
+
+def _lit(v: float) -> str:
+    return f"{v:.9g}f" if "." in f"{v:.9g}" or "e" in f"{v:.9g}" else f"{v:.9g}.f"
+
+
+def _emit(lo: int, l1: int, l2: int) -> str:
+    from ..constants import so3_clebsch_gordan
+    cg = so3_clebsch_gordan(lo, l1, l2)
+    pairs = {}                                          # (M, m1) -> [(m2, value)]
+    for M, m1, m2 in zip(*cg.nonzero()):
+        pairs.setdefault((int(M), int(m1)), []).append((int(m2), float(cg[M, m1, m2])))
+
+    def coef(ts):
+        expr = f"{_lit(ts[0][1])} * y[{ts[0][0]}]"
+        for m2, v in ts[1:]:
+            expr = f"fmaf({_lit(v)}, y[{m2}], {expr})"
+        return expr
+    no, n1, n2 = 2 * lo + 1, 2 * l1 + 1, 2 * l2 + 1
+    out = [f"template <> struct CgPath<{lo}, {l1}, {l2}> {{",
+           f"  // o[M] += sum_m1 (sum_m2 cg y[m2]) x[m1]",
+           f"  template <int V> __device__ __forceinline__ static void forward(float (&o)[{no}][V], const float (&x)[{n1}][V], const float (&y)[{n2}]) {{"]
+    for (M, m1), ts in pairs.items():
+        out.append(f"    axpy<V>(o[{M}], {coef(ts)}, x[{m1}]);")
+    out += ["  }",
+            f"  // r[m1] += sum_M (sum_m2 cg y[m2]) g[M]",
+            f"  template <int V> __device__ __forceinline__ static void adjoint(float (&r)[{n1}][V], const float (&g)[{no}][V], const float (&y)[{n2}]) {{"]
+    for (M, m1), ts in pairs.items():
+        out.append(f"    axpy<V>(r[{m1}], {coef(ts)}, g[{M}]);")
+    out += ["  }",
+            f"  // gy[m2] += sum_(M, m1) cg <g[M], x[m1]> over the V channels",
+            f"  template <int V> __device__ __forceinline__ static void inner(float (&gy)[{n2}], const float (&g)[{no}][V], const float (&x)[{n1}][V]) {{",
+            "    float d;"]
+    for (M, m1), ts in pairs.items():
+        out.append(f"    d = dot<V>(g[{M}], x[{m1}]);")
+        out += [f"    gy[{m2}] = fmaf({_lit(v)}, d, gy[{m2}]);" for m2, v in ts]
+    out += ["  }", "};"]
+    return "\n".join(out)
+
+
+def generate(path: str = OUT) -> str:
+    body = ["// AUTO-GENERATED by equitorch_b200/csrc/gen_path_specs.py - do not edit.", "#pragma once",
+            "template <int LO, int L1, int L2> struct CgPath;", ""]
+    body += [_emit(*t) for t in triples()]
+    body.append(f"constexpr int PATH_MAX_L = {MAX_L};")
+    text = "\n".join(body) + "\n"
+    os.makedirs(os.path.dirname(path), exist_ok=True)
+    if not os.path.exists(path) or open(path).read() != text:
+        with open(path, "w") as fh:
+            fh.write(text)
+    return path
+
+
+if __name__ == "__main__":
+    print(generate())

@@ -18,6 +18,7 @@ import torch
 from torch import Tensor
 from torch.autograd import Function
 
+from ...ops import so3_uu_op as _uu
 from ...ops.graph_ops import segment_sum  # noqa: F401  (re-exported for users of the functional API)
 from ...ops.indexed_product_scale_segment_op import indexed_vecmat_scale_segment
 from ...ops.indexed_product_segment_op import indexed_outer_segment
@@ -160,6 +161,35 @@ def tensor_product_uu1(input1, input2, weight, tp_info_forward, tp_info_backward
 
 
 so3_linear_uu = tensor_product_u1u
+
+
+class SO3LinearUU(Function):
+    """:func:`tensor_product_u1u` in one kernel per direction (``plan``: the layer's tables on the device).  A backward
+    pass that is itself differentiated is composed of the differentiable products instead."""
+
+    @staticmethod
+    def forward(ctx, input1, input2, weight, plan, infos):
+        input1, input2, weight = input1.contiguous(), input2.contiguous(), weight.contiguous()
+        ctx.save_for_backward(input1, input2, weight)
+        ctx.plan, ctx.infos = plan, infos
+        return _uu.so3_uu_forward(plan, input1, input2, weight)
+
+    @staticmethod
+    def backward(ctx, grad):
+        input1, input2, weight = ctx.saved_tensors
+        need = ctx.needs_input_grad[:3]
+        grad = grad.contiguous()
+        if not torch.is_grad_enabled() and grad.dtype == input1.dtype and grad.data_ptr() % 16 == 0:
+            return (*_uu.so3_uu_backward(ctx.plan, input1, input2, weight, grad, need), None, None)
+        f = ctx.infos[0]
+        r1, r2 = _rot(ctx.infos)
+        g1 = tensor_product_1uu(input2, grad, weight, *r1) if need[0] else None
+        g2 = tensor_product_uu1(grad, input1, weight, *r2) if need[1] else None
+        gw = None
+        if need[2]:
+            inter = sparse_vecsca(input1, input2, *_mij(f, 0))
+            gw = sparse_mul(grad, inter, *_m(f, 2), out_accumulated=weight.ndim == 2)
+        return g1, g2, gw, None, None
 
 
 # ------------------------------------------------------------------------------------------

@@ -12,9 +12,11 @@ import torch
 from torch import Tensor
 
 from ..irreps import check_irreps
-from ..tables import irreps_info, irreps_linear_infos, so2_linear_infos, tp_infos
+from ..ops.so3_uu_op import PathPlan
+from ..tables import (generate_fully_connected_tp_paths, irreps_info, irreps_linear_infos, so2_linear_infos, so3_path_norms,
+                      tp_infos)
 from ._base import _WeightedTableModule
-from .functional.linears import irrep_wise_linear, irreps_linear, so3_linear_uu, so3_linear_uv
+from .functional.linears import SO3LinearUU, irrep_wise_linear, irreps_linear, so3_linear_uu, so3_linear_uv
 from .functional.sparse_product import sparse_mul, sparse_vecmat
 from .init import initialize_linear, initialize_so3_so2_linear
 
@@ -51,9 +53,33 @@ class SO3Linear(_WeightedTableModule):
         (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2, self.num_paths) = tp_infos(
             self.irreps_out, self.irreps_in1, self.irreps_in2, path=path, path_norm=path_norm,
             channel_norm=self.channel_norm, channel_scale=fan_in ** (-0.5) if fan_in else 1.0)
+        paths = path or generate_fully_connected_tp_paths(self.irreps_out, self.irreps_in1, self.irreps_in2)
+        self._paths = (list(paths), so3_path_norms(paths, path_norm, self.channel_norm, fan_in ** (-0.5) if fan_in else 1.0))
+        self._own_info, self._path_plans = self.tp_info_forward, {}
         shape = (self.num_paths, channels_in, channels_out) if feature_mode == "uv" else (self.num_paths, channels_out)
         self._setup_weight(shape, internal_weights,
                            lambda w: initialize_so3_so2_linear(w, feature_mode, channel_normed=self.channel_norm))
+
+    def _path_plan(self, device) -> Optional[PathPlan]:
+        """The tables of the one-pass kernels on ``device``, built at the first call there; ``None`` when the layer's
+        own tables have been exchanged."""
+        if self.tp_info_forward is not self._own_info:
+            return None
+        plan = self._path_plans.get(device)
+        if plan is None:
+            plan = self._path_plans[device] = PathPlan(*self._paths, self.irreps_out, self.irreps_in1, self.irreps_in2, device)
+        return plan
+
+    def _apply(self, fn, *args, **kwargs):
+        own = self.tp_info_forward is self._own_info
+        module = super()._apply(fn, *args, **kwargs)
+        module._path_plans = {}
+        if own:
+            module._own_info = module.tp_info_forward
+        return module
+
+    def __getstate__(self):
+        return {k: ({} if k in ("_path_plans", "_plans") else v) for k, v in self.__dict__.items()}   # device tables are rebuilt
 
     def forward(self, input1: Tensor, input2: Tensor, weight: Optional[Tensor] = None) -> Tensor:
         assert input1.shape[-2] == self.irreps_in1_dim, \
@@ -65,6 +91,11 @@ class SO3Linear(_WeightedTableModule):
         assert self.channels_in is None or input1.shape[-1] == self.channels_in, \
             f"Input1 channel dim mismatch: expected {self.channels_in}, got {input1.shape[-1]}"
         weight = self._resolve_weight(weight)
+        if self.feature_mode == "uu" and input1.is_cuda:
+            plan = self._path_plan(input1.device)
+            if plan is not None and plan.supported(input1, input2, weight):
+                return SO3LinearUU.apply(input1, input2, weight, plan,
+                                         (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2))
         fn = so3_linear_uu if self.feature_mode == "uu" else so3_linear_uv
         return fn(input1, input2, weight, self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2)
 

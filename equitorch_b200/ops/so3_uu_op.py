@@ -1,0 +1,88 @@
+"""Channel-wise ``SO3Linear`` in one kernel per direction (operator layer over ``eqt_so3_uu_*``)."""
+from __future__ import annotations
+
+import ctypes as C
+from typing import Optional, Sequence, Tuple
+
+import numpy as np
+import torch
+from torch import Tensor
+
+from .. import _lib
+from ..csrc.gen_path_specs import MAX_L as PATH_MAX_L
+
+_PATH = np.dtype([("code", "<i4"), ("offset", "<i4"), ("offset_y", "<i4"), ("weight", "<i4"), ("scale", "<f4")])
+_BLOCK = np.dtype([("l", "<i4"), ("offset", "<i4"), ("first", "<i4"), ("count", "<i4")])
+
+
+class PathPlan:
+    """Device tables of one layer for the one-pass kernels.  ``paths``: (k, i, j) of every weight - output, first and
+    second operand irrep - and ``scales`` the factors on their Clebsch-Gordan blocks."""
+
+    def __init__(self, paths: Sequence[Tuple[int, int, int]], scales: Sequence[float], irreps_out, irreps1, irreps2, device):
+        self.device, self._fits = torch.device(device), {}
+        ls = [[ir.l for ir in irs] for irs in (irreps_out, irreps1, irreps2)]
+        self.usable = len(paths) > 0 and all(0 <= l <= PATH_MAX_L for degrees in ls for l in degrees)
+        if not self.usable:
+            return
+        start = [np.cumsum([0] + [2 * l + 1 for l in degrees]).tolist() for degrees in ls]
+        parts = []
+        for key, other in ((0, 1), (1, 0)):
+            order = sorted(range(len(paths)), key=lambda w: paths[w][key])
+            parts.append(np.array([(4 * ls[other][paths[w][other]] + ls[2][paths[w][2]], start[other][paths[w][other]],
+                                    start[2][paths[w][2]], w, scales[w]) for w in order], dtype=_PATH))
+            first = np.searchsorted([paths[w][key] for w in order], np.arange(len(ls[key]) + 1)).tolist()
+            parts.append(np.array([(l, start[key][n], first[n], first[n + 1] - first[n]) for n, l in enumerate(ls[key])], dtype=_BLOCK))
+        # one upload: the parts back to back, each on a 16-byte boundary
+        blob, at, size = [], [], 0
+        for part in parts:
+            at.append(size)
+            raw = part.tobytes()
+            blob.append(raw + b"\0" * (-len(raw) % 16))
+            size += len(blob[-1])
+        self.blob = torch.frombuffer(bytearray(b"".join(blob)), dtype=torch.uint8).to(device)
+        base = self.blob.data_ptr()
+        self.sizes = (start[1][-1], start[2][-1], start[0][-1], len(paths))
+        self.struct = _lib.PathTableStruct(base + at[1], base + at[3], base + at[0], base + at[2], *self.sizes, len(paths),
+                                           len(ls[0]), len(ls[1]))
+        self.ref = C.byref(self.struct)
+
+    def supported(self, x: Tensor, y: Tensor, w: Tensor) -> bool:
+        if not (self.usable and x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and x.dtype == y.dtype == w.dtype
+                and x.ndim == 3 and y.ndim == 2 and x.shape[0] == y.shape[0] and x.shape[0] > 0 and w.ndim in (2, 3)
+                and x.shape[2] == w.shape[-1] and x.shape[1] == self.sizes[0] and y.shape[1] == self.sizes[1]
+                and w.shape[-2] == self.sizes[3] and (w.ndim == 2 or w.shape[0] == x.shape[0])
+                and y.device == x.device == w.device == self.device):
+            return False
+        key = (x.shape[2], w.ndim, x.dtype)
+        if key not in self._fits:
+            self._fits[key] = all(_lib.lib().eqt_so3_uu_scratch_floats(self.ref, n, x.shape[2], int(w.ndim == 3),
+                                                                       _lib.DTYPE_CODE[x.dtype]) >= 0 for n in (1, 1 << 30))
+        return self._fits[key] and (x.data_ptr() | w.data_ptr()) % 16 == 0
+
+
+def so3_uu_forward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor) -> Tensor:
+    """``out[n, M, c] = sum_t s_t x[n, M1_t, c] y[n, M2_t] w[(n,) p_t, c]``; contiguous operands of one dtype."""
+    n, _, c = x.shape
+    out = torch.empty(n, plan.sizes[2], c, dtype=x.dtype, device=x.device)
+    with torch.cuda.device(x.device):
+        _lib.check(_lib.lib().eqt_so3_uu_forward(plan.ref, x.data_ptr(), y.data_ptr(), w.data_ptr(), out.data_ptr(), n, c,
+                                                 int(w.ndim == 3), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(x.device)),
+                   "eqt_so3_uu_forward")
+    return out
+
+
+def so3_uu_backward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor, g: Tensor,
+                    need: Tuple[bool, bool, bool]) -> Tuple[Optional[Tensor], Optional[Tensor], Optional[Tensor]]:
+    """Gradients with respect to x, y and w (``None`` where not needed), all from one launch."""
+    n, _, c = x.shape
+    gx, gy, gw = (torch.empty_like(t) if wanted else None for t, wanted in zip((x, y, w), need))
+    lib, scratch, floats = _lib.lib(), None, 0
+    with torch.cuda.device(x.device):
+        if need[2] and w.ndim == 2:
+            floats = int(lib.eqt_so3_uu_scratch_floats(plan.ref, n, c, 0, _lib.DTYPE_CODE[x.dtype]))
+            scratch = torch.empty(floats, dtype=torch.float32, device=x.device)
+        _lib.check(lib.eqt_so3_uu_backward(plan.ref, x.data_ptr(), y.data_ptr(), w.data_ptr(), g.data_ptr(), _lib.ptr(gx),
+                                           _lib.ptr(gy), _lib.ptr(gw), _lib.ptr(scratch), floats, n, c, int(w.ndim == 3),
+                                           _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(x.device)), "eqt_so3_uu_backward")
+    return gx, gy, gw

@@ -182,6 +182,16 @@ def generate_fully_connected_tp_paths(irreps_out: Irreps, irreps1: Irreps, irrep
             for j, b in enumerate(in2) if has_path(ko, a, b)]
 
 
+def so3_path_norms(path, path_norm: bool = True, channel_norm: bool = False, channel_scale: float = 1.0):
+    """Factor on the CG block of every path (see :func:`prepare_so3`)."""
+    fan: Dict[int, int] = {}
+    prev = None
+    for k, _, _ in path:
+        fan[k] = fan[k] + 1 if k == prev else 1
+        prev = k
+    return [(fan[k] ** (-0.5) if path_norm else 1.0) * (channel_scale if channel_norm else 1.0) for k, _, _ in path]
+
+
 def prepare_so3(irreps_out: Irreps, irreps1: Irreps, irreps2: Irreps, path=None,
                 path_norm: bool = True, channel_norm: bool = False, channel_scale: float = 1.0):
     """Flat list of the non-zero, normalised CG entries of every path.
@@ -195,17 +205,11 @@ def prepare_so3(irreps_out: Irreps, irreps1: Irreps, irreps2: Irreps, path=None,
     out, in1, in2 = list(irreps_out), list(irreps1), list(irreps2)
     off_out, off1, off2 = irrep_segments(irreps_out), irrep_segments(irreps1), irrep_segments(irreps2)
 
-    fan: Dict[int, int] = {}
-    prev = None
-    for k, _, _ in path:
-        fan[k] = fan[k] + 1 if k == prev else 1
-        prev = k
-
     cols = [[] for _ in range(8)]
+    norms = so3_path_norms(path, path_norm, channel_norm, channel_scale)
     for w, (k, i, j) in enumerate(path):
         cg = so3_clebsch_gordan(out[k].l, in1[i].l, in2[j].l)
-        norm = (fan[k] ** (-0.5) if path_norm else 1.0) * (channel_scale if channel_norm else 1.0)
-        vals = cg * norm
+        vals = cg * norms[w]
         mo, m1, m2 = np.nonzero(vals)          # C order == (m_out, m1, m2) nested loops
         cols[0].append(vals[mo, m1, m2])
         cols[1].append(mo + off_out[k])

@@ -303,6 +303,46 @@ int eqt_wgrad_tc_static(const float* s, const float* g, float* gw_packed, int64_
 int64_t eqt_wgrad_tc_static_capacity(void);
 
 /*
+ * Channel-wise tensor product with a channel-less second operand ('uu' SO3Linear) over irreps of degree up to 3, one
+ * launch per direction and one small reduction for weights shared by the batch:
+ *   out[n, M, c] = sum_{t: M_t = M} s_t x[n, M1_t, c] y[n, M2_t] w[(n,) p_t, c]      and the three gradients.
+ * x (n, d1, c), y (n, d2), w (num_weights, c) or (n, num_weights, c) with `per_sample_weight`, out / g (n, d_out, c);
+ * float32 or bfloat16 storage, float32 arithmetic.  The table lists the paths (output irrep, x irrep, y irrep, weight)
+ * with the factor of their Clebsch-Gordan block, once in blocks of one output irrep each (every output irrep has a
+ * block, of zero paths if nothing reaches it) and once in blocks of one x irrep each; device memory.  Every weight
+ * belongs to exactly one path.  Gradients that are NULL are not written.  Shared weights need
+ * eqt_so3_uu_scratch_floats() floats of scratch (the sums of the thread blocks, added in a fixed order); -1 means that
+ * this many channels are not supported (a multiple of 4 up to 512 whose columns fit shared memory).  Operands with a
+ * channel axis must be aligned to four elements.
+ * replaces: SO3Linear 'uu' = TensorProductU1U (equitorch/nn/functional/linears.py:16-93) and its adjoints.
+ */
+typedef struct eqt_path {
+  int32_t code;        /* forward order: 4 l_1 + l_2; backward order: 4 l_out + l_2        */
+  int32_t offset;      /* first component of the path's x (forward) or output (backward) irrep */
+  int32_t offset_y;    /* first component of its y irrep                                    */
+  int32_t weight;
+  float scale;         /* factor on the Clebsch-Gordan values                               */
+} eqt_path;
+typedef struct eqt_path_block {
+  int32_t l, offset;   /* degree and first component of the block's irrep                   */
+  int32_t first, count; /* its paths                                                        */
+} eqt_path_block;
+typedef struct eqt_path_table {
+  const eqt_path_block* fwd_blocks;
+  const eqt_path_block* bwd_blocks;
+  const eqt_path* fwd_paths;
+  const eqt_path* bwd_paths;
+  int32_t d1, d2, d_out, num_weights, num_paths, num_fwd_blocks, num_bwd_blocks;
+} eqt_path_table;
+int64_t eqt_so3_uu_scratch_floats(const eqt_path_table* table, int64_t n, int32_t channels, int32_t per_sample_weight,
+                                  int32_t dtype);
+int eqt_so3_uu_forward(const eqt_path_table* table, const void* x, const void* y, const void* w, void* out, int64_t n,
+                       int32_t channels, int32_t per_sample_weight, int32_t dtype, void* stream);
+int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, const void* y, const void* w, const void* g, void* gx,
+                        void* gy, void* gw, float* scratch, int64_t scratch_floats, int64_t n, int32_t channels,
+                        int32_t per_sample_weight, int32_t dtype, void* stream);
+
+/*
  * Gather, lay out and split shared weights w (num_paths, cin, cout) for the tensor-core entry points:
  * path_gather (device, int64) lists the paths of all blocks back to back (w_offset of a block =
  * first gathered path * cin * cout).  k_major != 0 writes the per-block (cout, paths*cin) matrices that

@@ -1,0 +1,65 @@
+"""``SO3Linear`` 'uu' through the one-pass kernels against the dense float64 oracle: channel counts that give 1 to 64
+threads per sample (powers of two and not), batches from one sample (output irreps spread over the grid, smaller
+blocks) to several waves, degrees 0 to 3 with even and odd degree sums, shared and per-sample weights, float32 and bfloat16; and a differentiated
+backward pass against the composed products."""
+import copy
+
+import pytest
+import torch
+
+from equitorch_b200 import _lib
+from equitorch_b200 import nn as enn
+from equitorch_b200.nn.functional.linears import tensor_product_u1u
+from oracle import tensor_products as otp
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+# float32: an element is a sum of up to 40 terms of random sign, a weight gradient of 40 n; bfloat16: one rounding of the result
+BOUND = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -7}
+
+
+def _rel(a, b):
+    return float((a.detach().double().cpu() - b.detach().double()).abs().max() / b.detach().double().abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("per_sample", [False, True])
+@pytest.mark.parametrize("ir,ir_y,n,c", [("0e+1o", "0e+1o", 1, 4), ("0e+1o+2e", "0e+1o+2e", 7, 12), ("0e+1o+2e+3o", "0e+1o+2e+3o", 129, 64),
+                                         ("4x0e+2x1o+2e", "0e+1o+2e", 3001, 32), ("0e+1o+2e", "0e+1o+2e", 5003, 48),
+                                         ("0e+1o", "0e+1o", 300, 512), ("0o+1e+2e+3e", "0e+1e+2o+3e", 1000, 20), ("0e+1o+2e", "0e+1o+2e", 20001, 16)])
+def test_one_pass_kernels(ir, ir_y, n, c, per_sample, dtype):
+    g = torch.Generator().manual_seed(n + c)
+    layer = enn.SO3Linear(ir, ir_y, ir, c, c, internal_weights=False, feature_mode="uu").to(DEV)
+    dim, dim_y, p = layer.irreps_in1_dim, layer.irreps_in2_dim, layer.num_paths
+    x, y = torch.randn(n, dim, c, generator=g).to(dtype), torch.randn(n, dim_y, generator=g).to(dtype)
+    w = torch.randn(*((n,) if per_sample else ()), p, c, generator=g).to(dtype)
+    cot = torch.randn(n, dim, c, generator=g).to(dtype)
+    xo, yo, wo = (t.double().requires_grad_(True) for t in (x, y, w))
+    want = otp.so3_linear_dense(xo, yo, wo, ir, ir_y, ir, feature_mode="uu")
+    want = [want, *torch.autograd.grad(want, [xo, yo, wo], cot.double())]
+    xg, yg, wg = (t.to(DEV).requires_grad_(True) for t in (x, y, w))
+    before = _lib.launch_count()
+    got = layer(xg, yg, wg)
+    got = [got, *torch.autograd.grad(got, [xg, yg, wg], cot.to(DEV))]
+    assert _lib.launch_count() - before == (2 if per_sample and n > 1 else 3)       # one sample's weights are shared ones
+    for a, b in zip(got, want):
+        assert a.dtype == dtype and a.shape == b.shape and _rel(a, b) < BOUND[dtype]
+    # a gradient for one operand alone, from a copy of the layer
+    (gy,) = torch.autograd.grad(copy.deepcopy(layer)(xg.detach(), yg, wg.detach()), [yg], cot.to(DEV))
+    assert torch.equal(gy, got[2])
+
+
+def test_differentiated_backward_pass():
+    g = torch.Generator().manual_seed(0)
+    ir, n, c = "0e+1o+2e", 33, 8
+    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode="uu").to(DEV)
+    leaves = [t.to(DEV).requires_grad_(True) for t in (torch.randn(n, 9, c, generator=g), torch.randn(n, 9, generator=g),
+                                                       torch.randn(11, c, generator=g), torch.randn(n, 9, c, generator=g))]
+    infos = (layer.tp_info_forward, layer.tp_info_backward1, layer.tp_info_backward2)
+
+    def second(fn):
+        x, y, w, cot = leaves
+        first = torch.autograd.grad(fn(x, y, w), [x, y, w], cot, create_graph=True)
+        return torch.autograd.grad(sum((t * t).sum() for t in first), leaves)
+    for a, b in zip(second(layer), second(lambda x, y, w: tensor_product_u1u(x, y, w, *infos))):
+        assert _rel(a, b.cpu()) < 1e-5
