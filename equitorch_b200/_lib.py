@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import threading
+from contextlib import nullcontext
 from typing import Optional
 
 import torch
@@ -86,6 +87,8 @@ SIGNATURES = {
     "eqt_segment_sum": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                   C.c_int64, C.c_void_p]),
     "eqt_gather_rows": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]),
+    "eqt_expand_segments": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p]),
+    "eqt_scatter_add_rows": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p]),
     "eqt_tp_cg_segment_sum": (C.c_int, [C.POINTER(TpTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                         C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]),
     "eqt_tp_cg_inner": (C.c_int, [C.POINTER(TpTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
@@ -170,7 +173,17 @@ def check(rc: int, what: str) -> None:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Raw handle of the current stream (without building a ``torch.cuda.Stream`` per call)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+_NO_SWITCH = nullcontext()
+
+
+def on_device(device: torch.device):
+    """Context in which ``device`` is current; costs nothing when it already is (the usual case of one device)."""
+    return _NO_SWITCH if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def ptr(t: Optional[torch.Tensor]) -> Optional[int]:

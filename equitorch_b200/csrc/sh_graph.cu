@@ -212,31 +212,172 @@ int sh_launch_unrolled(bool backward, const void* xyz, const void* gout, void* o
   return check_launch("sh_forward_unrolled_kernel");
 }
 
-template <typename T>
+// ---- rows of nodes and edges ----------------------------------------------------------------------------------------
+// All of these move whole rows, so they work on 16-byte units where rows and pointers allow it (U = units' element
+// count) and on elements otherwise, with a 32-bit flat index (the launchers check that it fits).  Bound: HBM / L2.
+// 20,480 rows of 480: gather of bfloat16 24 -> 6 us, sum of float32 into 960 segments 18 -> 8.5 us.
+template <typename T, int U> struct alignas(sizeof(T) * U) Unit { T v[U]; };
+
+template <typename T, int U>
 __global__ void __launch_bounds__(256) segment_sum_kernel(const T* __restrict__ in, const int64_t* __restrict__ ptr,
                                                           const int64_t* __restrict__ perm, T* __restrict__ out,
-                                                          int64_t segments, int64_t width) {
+                                                          uint32_t segments, uint32_t units) {
   using A = typename Acc<T>::type;
-  const int64_t total = segments * width;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t d = idx / width, c = idx % width;
-    A acc = 0;
-    for (int64_t e = __ldg(ptr + d); e < __ldg(ptr + d + 1); ++e) {
-      const int64_t row = perm ? __ldg(perm + e) : e;
-      acc += ld(in + row * width + c);
+  using Q = Unit<T, U>;
+  const Q* src = reinterpret_cast<const Q*>(in);
+  Q* dst = reinterpret_cast<Q*>(out);
+  const uint32_t total = segments * units;
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const uint32_t d = idx / units, c = idx - d * units;
+    A acc[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) acc[i] = A(0);
+    const int64_t e1 = __ldg(ptr + d + 1);
+    int64_t e = __ldg(ptr + d);
+    for (; e + 4 <= e1; e += 4) {                      // four rows in flight, added in ascending order
+      Q q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = src[(perm ? __ldg(perm + e + k) : e + k) * units + c];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int i = 0; i < U; ++i) acc[i] += static_cast<A>(q[k].v[i]);
     }
-    st(out + idx, acc);
+    for (; e < e1; ++e) {
+      const Q q = src[(perm ? __ldg(perm + e) : e) * units + c];
+#pragma unroll
+      for (int i = 0; i < U; ++i) acc[i] += static_cast<A>(q.v[i]);
+    }
+    Q o;
+#pragma unroll
+    for (int i = 0; i < U; ++i) o.v[i] = static_cast<T>(acc[i]);
+    dst[idx] = o;
   }
 }
 
-template <typename T>
+template <typename T, int U>
 __global__ void __launch_bounds__(256) gather_rows_kernel(const T* __restrict__ in, const int64_t* __restrict__ index,
-                                                          T* __restrict__ out, int64_t rows, int64_t width) {
-  const int64_t total = rows * width;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x)
-    out[idx] = in[__ldg(index + idx / width) * width + idx % width];
+                                                          T* __restrict__ out, uint32_t rows, uint32_t units) {
+  using Q = Unit<T, U>;
+  const Q* src = reinterpret_cast<const Q*>(in);
+  Q* dst = reinterpret_cast<Q*>(out);
+  const uint32_t total = rows * units;
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const uint32_t r = idx / units, c = idx - r * units;
+    dst[idx] = src[__ldg(index + r) * units + c];
+  }
+}
+
+// Adjoint of the segment sum: every row of segment d becomes row d of `in`; rows outside all segments become zero.
+// A warp holds 32 units of one segment's row and writes them to its edges.
+template <typename T, int U>
+__global__ void __launch_bounds__(256) expand_segments_kernel(const T* __restrict__ in, const int64_t* __restrict__ ptr,
+                                                              T* __restrict__ out, int64_t segments, int64_t rows, uint32_t units) {
+  using Q = Unit<T, U>;
+  const Q* src = reinterpret_cast<const Q*>(in);
+  Q* dst = reinterpret_cast<Q*>(out);
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5), warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const uint32_t c = blockIdx.y * 32 + lane;
+  if (c >= units) return;
+  for (int64_t d = warp; d < segments; d += warps) {
+    const int64_t e0 = max(__ldg(ptr + d), (int64_t)0), e1 = min(__ldg(ptr + d + 1), rows);
+    if (e0 >= e1) continue;
+    const Q q = src[d * units + c];
+    for (int64_t e = e0; e < e1; ++e) dst[e * units + c] = q;
+  }
+  Q zero;
+#pragma unroll
+  for (int i = 0; i < U; ++i) zero.v[i] = static_cast<T>(0.f);
+  const int64_t first = min(segments ? __ldg(ptr) : rows, rows), last = segments ? __ldg(ptr + segments) : rows;
+  for (int64_t e = warp; e < first; e += warps) dst[e * units + c] = zero;
+  for (int64_t e = max(last, (int64_t)0) + warp; e < rows; e += warps) dst[e * units + c] = zero;
+}
+
+// Adjoint of the gather: out[index[e]] += in[e] in float32 whatever the storage type, with 16-byte reductions at L2
+// where the row width allows.  Replaces element-wise atomics in the storage type (73 us for 20,480 rows of 480
+// bfloat16, 12 us here) and their bfloat16 sums.
+template <typename T, int U>
+__global__ void __launch_bounds__(256) scatter_add_rows_kernel(const T* __restrict__ in, const int64_t* __restrict__ index,
+                                                               float* __restrict__ out, uint32_t rows, uint32_t units, int64_t out_rows) {
+  using Q = Unit<T, U>;
+  const Q* src = reinterpret_cast<const Q*>(in);
+  const uint32_t total = rows * units;
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const uint32_t r = idx / units, c = idx - r * units;
+    const int64_t to = __ldg(index + r);
+    if (to < 0 || to >= out_rows) continue;
+    const Q q = src[idx];
+    float* o = out + (to * units + c) * U;
+    if constexpr (U == 4)
+      atomicAdd(reinterpret_cast<float4*>(o), make_float4(static_cast<float>(q.v[0]), static_cast<float>(q.v[1]),
+                                                          static_cast<float>(q.v[2]), static_cast<float>(q.v[3])));
+    else
+      atomicAdd(o, static_cast<float>(q.v[0]));
+  }
+}
+
+inline bool unit_ok(int64_t width, size_t elem, size_t bytes, const void* a, const void* b) {
+  return (width * elem) % bytes == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & (bytes - 1)) == 0;
+}
+
+// rows are processed in pieces whose flat unit index (grid stride included) fits 32 bits
+template <typename F> int row_pieces(int64_t rows, int64_t units, F launch) {
+  const int64_t cap = std::max<int64_t>(1, (int64_t(1) << 31) / std::max<int64_t>(1, units));
+  if (units >= (int64_t(1) << 31)) return fail(EQT_ERR_UNSUPPORTED, "rows of more than 2^31 elements");
+  for (int64_t r = 0; r < rows; r += cap)
+    if (int rc = launch(r, std::min(cap, rows - r))) return rc;
+  return EQT_OK;
+}
+
+template <typename T>
+int run_segment_sum(const T* in, const int64_t* ptr, const int64_t* perm, T* out, int64_t segments, int64_t width, cudaStream_t s) {
+  constexpr int U = 16 / sizeof(T);
+  const bool wide = unit_ok(width, sizeof(T), 16, in, out);
+  const int64_t units = wide ? width / U : width;
+  return row_pieces(segments, units, [&](int64_t r, int64_t n) {
+    const unsigned grid = flat_grid(n * units, 256);
+    if (wide) segment_sum_kernel<T, U><<<grid, 256, 0, s>>>(in, ptr + r, perm, out + r * width, (uint32_t)n, (uint32_t)units);
+    else segment_sum_kernel<T, 1><<<grid, 256, 0, s>>>(in, ptr + r, perm, out + r * width, (uint32_t)n, (uint32_t)units);
+    return check_launch("segment_sum_kernel");
+  });
+}
+
+template <typename T>
+int run_gather_rows(const T* in, const int64_t* index, T* out, int64_t rows, int64_t width, cudaStream_t s) {
+  constexpr int U = 16 / sizeof(T);
+  const bool wide = unit_ok(width, sizeof(T), 16, in, out);
+  const int64_t units = wide ? width / U : width;
+  return row_pieces(rows, units, [&](int64_t r, int64_t n) {
+    const unsigned grid = flat_grid(n * units, 256);
+    if (wide) gather_rows_kernel<T, U><<<grid, 256, 0, s>>>(in, index + r, out + r * width, (uint32_t)n, (uint32_t)units);
+    else gather_rows_kernel<T, 1><<<grid, 256, 0, s>>>(in, index + r, out + r * width, (uint32_t)n, (uint32_t)units);
+    return check_launch("gather_rows_kernel");
+  });
+}
+
+template <typename T>
+int run_expand_segments(const T* in, const int64_t* ptr, T* out, int64_t segments, int64_t rows, int64_t width, cudaStream_t s) {
+  constexpr int U = 16 / sizeof(T);
+  const bool wide = unit_ok(width, sizeof(T), 16, in, out);
+  const int64_t units = wide ? width / U : width;
+  if (ceil_div(units, 32) > 65535) return fail(EQT_ERR_UNSUPPORTED, "rows of more than 2^21 units");
+  const dim3 grid(flat_grid(std::max(segments, int64_t(1)) * 32, 256, 16), (unsigned)ceil_div(units, 32));
+  if (wide) expand_segments_kernel<T, U><<<grid, 256, 0, s>>>(in, ptr, out, segments, rows, (uint32_t)units);
+  else expand_segments_kernel<T, 1><<<grid, 256, 0, s>>>(in, ptr, out, segments, rows, (uint32_t)units);
+  return check_launch("expand_segments_kernel");
+}
+
+template <typename T>
+int run_scatter_add(const T* in, const int64_t* index, float* out, int64_t rows, int64_t width, int64_t out_rows, cudaStream_t s) {
+  const bool wide = width % 4 == 0 && unit_ok(width, sizeof(T), 4 * sizeof(T), in, in) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  const int64_t units = wide ? width / 4 : width;
+  return row_pieces(rows, units, [&](int64_t r, int64_t n) {
+    const unsigned grid = flat_grid(n * units, 256);
+    if (wide) scatter_add_rows_kernel<T, 4><<<grid, 256, 0, s>>>(in + r * width, index + r, out, (uint32_t)n, (uint32_t)units, out_rows);
+    else scatter_add_rows_kernel<T, 1><<<grid, 256, 0, s>>>(in + r * width, index + r, out, (uint32_t)n, (uint32_t)units, out_rows);
+    return check_launch("scatter_add_rows_kernel");
+  });
 }
 
 int check_table(const eqt_sh_table* t) {
@@ -310,14 +451,12 @@ extern "C" int eqt_segment_sum(int32_t dtype, const void* in, const int64_t* ptr
   if (num_segments == 0 || width == 0) return EQT_OK;
   if (!in || !ptr || !out) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const unsigned grid = flat_grid(num_segments * width, 256);
   switch (dtype) {
-    case EQT_F32: segment_sum_kernel<float><<<grid, 256, 0, s>>>((const float*)in, ptr, perm, (float*)out, num_segments, width); break;
-    case EQT_F64: segment_sum_kernel<double><<<grid, 256, 0, s>>>((const double*)in, ptr, perm, (double*)out, num_segments, width); break;
-    case EQT_BF16: segment_sum_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)in, ptr, perm, (__nv_bfloat16*)out, num_segments, width); break;
+    case EQT_F32: return run_segment_sum((const float*)in, ptr, perm, (float*)out, num_segments, width, s);
+    case EQT_F64: return run_segment_sum((const double*)in, ptr, perm, (double*)out, num_segments, width, s);
+    case EQT_BF16: return run_segment_sum((const __nv_bfloat16*)in, ptr, perm, (__nv_bfloat16*)out, num_segments, width, s);
     default: return fail(EQT_ERR_BAD_ARGUMENT, "unknown dtype %d", dtype);
   }
-  return check_launch("segment_sum_kernel");
 }
 
 extern "C" int eqt_gather_rows(int32_t dtype, const void* in, const int64_t* index, void* out, int64_t num_rows,
@@ -327,12 +466,39 @@ extern "C" int eqt_gather_rows(int32_t dtype, const void* in, const int64_t* ind
   if (num_rows == 0 || width == 0) return EQT_OK;
   if (!in || !index || !out) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const unsigned grid = flat_grid(num_rows * width, 256);
   switch (dtype) {
-    case EQT_F32: gather_rows_kernel<float><<<grid, 256, 0, s>>>((const float*)in, index, (float*)out, num_rows, width); break;
-    case EQT_F64: gather_rows_kernel<double><<<grid, 256, 0, s>>>((const double*)in, index, (double*)out, num_rows, width); break;
-    case EQT_BF16: gather_rows_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)in, index, (__nv_bfloat16*)out, num_rows, width); break;
+    case EQT_F32: return run_gather_rows((const float*)in, index, (float*)out, num_rows, width, s);
+    case EQT_F64: return run_gather_rows((const double*)in, index, (double*)out, num_rows, width, s);
+    case EQT_BF16: return run_gather_rows((const __nv_bfloat16*)in, index, (__nv_bfloat16*)out, num_rows, width, s);
     default: return fail(EQT_ERR_BAD_ARGUMENT, "unknown dtype %d", dtype);
   }
-  return check_launch("gather_rows_kernel");
+}
+
+extern "C" int eqt_expand_segments(int32_t dtype, const void* in, const int64_t* ptr, void* out, int64_t num_segments,
+                                   int64_t num_rows, int64_t width, void* stream) {
+  using namespace eqt;
+  if (num_segments < 0 || num_rows < 0 || width < 0) return fail(EQT_ERR_BAD_ARGUMENT, "negative size");
+  if (num_rows == 0 || width == 0) return EQT_OK;
+  if ((num_segments > 0 && (!in || !ptr)) || !out) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case EQT_F32: return run_expand_segments((const float*)in, ptr, (float*)out, num_segments, num_rows, width, s);
+    case EQT_F64: return run_expand_segments((const double*)in, ptr, (double*)out, num_segments, num_rows, width, s);
+    case EQT_BF16: return run_expand_segments((const __nv_bfloat16*)in, ptr, (__nv_bfloat16*)out, num_segments, num_rows, width, s);
+    default: return fail(EQT_ERR_BAD_ARGUMENT, "unknown dtype %d", dtype);
+  }
+}
+
+extern "C" int eqt_scatter_add_rows(int32_t dtype, const void* in, const int64_t* index, float* out, int64_t num_rows, int64_t width,
+                                    int64_t out_rows, void* stream) {
+  using namespace eqt;
+  if (num_rows < 0 || width < 0 || out_rows < 0) return fail(EQT_ERR_BAD_ARGUMENT, "negative size");
+  if (num_rows == 0 || width == 0) return EQT_OK;
+  if (!in || !index || !out) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case EQT_F32: return run_scatter_add((const float*)in, index, out, num_rows, width, out_rows, s);
+    case EQT_BF16: return run_scatter_add((const __nv_bfloat16*)in, index, out, num_rows, width, out_rows, s);
+    default: return fail(EQT_ERR_UNSUPPORTED, "row scatter sums float32 or bfloat16 rows");
+  }
 }

@@ -128,6 +128,19 @@ int eqt_gather_rows(int32_t dtype, const void* in, const int64_t* index, void* o
                     int64_t width, void* stream);
 
 /*
+ * Their adjoints:
+ *   eqt_expand_segments:  out[e, :] = in[d, :] for e in [ptr[d], ptr[d+1]), zero for rows of no segment (ptr ascending)
+ *   eqt_scatter_add_rows: out[index[e], :] += in[e, :] in float32 (EQT_F32 / EQT_BF16 rows), out zero-filled by the
+ *                         caller; the order of the additions is not fixed; rows with index outside [0, out_rows) are
+ *                         skipped.
+ */
+int eqt_expand_segments(int32_t dtype, const void* in, const int64_t* ptr, void* out, int64_t num_segments,
+                        int64_t num_rows, int64_t width, void* stream);
+int eqt_scatter_add_rows(int32_t dtype, const void* in, const int64_t* index, float* out, int64_t num_rows,
+                         int64_t width, int64_t out_rows, void* stream);
+
+
+/*
  * CG step of a tensor-product layer whose second operand has no channel axis, for one role
  * assignment: table entry t adds  scale[t] * feat[.., m_feat[t], c] * y[.., m_y[t]]  to intermediate
  * row r, where the entries of row r are [row_ptr[r], row_ptr[r+1]).  These are the fields of the
