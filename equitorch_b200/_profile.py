@@ -8,7 +8,7 @@ kernels inside the timed region itself.
 from __future__ import annotations
 
 from collections import defaultdict
-from contextlib import contextmanager
+from contextlib import contextmanager, nullcontext
 from typing import Dict, List, Tuple
 
 import torch
@@ -24,11 +24,15 @@ def enable(flag: bool = True) -> None:
         _pending.clear()
 
 
-@contextmanager
+_OFF = nullcontext()
+
+
 def timed(name: str):
-    if not _enabled:
-        yield
-        return
+    return _record(name) if _enabled else _OFF
+
+
+@contextmanager
+def _record(name: str):
     start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     start.record()
     try:

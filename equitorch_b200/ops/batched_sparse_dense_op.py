@@ -147,7 +147,7 @@ def sparse_product(op: int, input1: Tensor, input2: Optional[Tensor], scale=None
         index1=_lib.ptr(index1), index2=_lib.ptr(index2), seg=_lib.ptr(seg),
         gather_index=_lib.ptr(gather_index), index_out=_lib.ptr(index_out),
         n=n, rows1=rows1, rows2=rows2, num_out=num_out, out_size=out_size, c1=c1, c2=c2)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_sparse_product(C.byref(args), _lib.stream_ptr(dev)), "eqt_sparse_product")
     if out is not None and buf is not out:
         out.copy_(buf)

@@ -84,7 +84,7 @@ def radius_graph_features(pos: Tensor, r: float, batch: Optional[Tensor] = None,
     degree = torch.empty(n, dtype=torch.int32, device=dev)
     flag = _flag(dev)
     lib = _lib.lib()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.eqt_radius_count(C.byref(cells.struct), pos.data_ptr(), _lib.ptr(batch), n, float(r), int(loop),
                                         int(max_num_neighbors), degree.data_ptr(), flag.data_ptr(), _lib.stream_ptr(dev)),
                    "eqt_radius_count")
@@ -111,7 +111,7 @@ def radius_graph_features(pos: Tensor, r: float, batch: Optional[Tensor] = None,
                                     l_max or 0, int(integral_normalize), 0 if bw is None else bw.numel(),
                                     CUTOFF_KINDS[cutoff] if cutoff is not None else 0, float(bessel_r_max or 1.0),
                                     float(cutoff_r_min), float(cutoff_r_max or 1.0), float(cutoff_p), float(cutoff_eps))
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.eqt_radius_edges(C.byref(cells.struct), pos.data_ptr(), _lib.ptr(batch), n, float(r), int(loop),
                                         int(max_num_neighbors), ptr.data_ptr(), src.data_ptr(), dst.data_ptr(), C.byref(feats),
                                         flag.data_ptr(), _lib.stream_ptr(dev)), "eqt_radius_edges")

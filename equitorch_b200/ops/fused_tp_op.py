@@ -73,7 +73,7 @@ def cg_segment_sum(table: TpTable, feat: Tensor, y: Tensor, feat_index: Optional
     if seg_ptr is None:
         num_out = n_edges
     out = torch.empty(num_out, table.num_rows, c, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_tp_cg_segment_sum(
             C.byref(table.struct), feat.data_ptr(), _lib.ptr(feat_index), y.data_ptr(), _lib.ptr(y_index),
             _lib.ptr(seg_ptr), out.data_ptr(), num_out, n_edges, c, status_flag(dev).data_ptr(),
@@ -89,7 +89,7 @@ def cg_inner(table: TpTable, feat: Tensor, g: Tensor, feat_index: Optional[Tenso
     assert g.ndim == 3 and g.shape[1] == table.num_rows and g.shape[2] == feat.shape[2]
     n_edges = edge_node.numel()
     out = (torch.empty if num_y_rows == n_edges else torch.zeros)(num_y_rows, table.d_y, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_tp_cg_inner(
             C.byref(table.struct), feat.data_ptr(), _lib.ptr(feat_index), g.data_ptr(), seg_ptr.data_ptr(),
             edge_node.data_ptr(), _lib.ptr(y_index), out.data_ptr(), g.shape[0], n_edges, feat.shape[2],

@@ -83,7 +83,7 @@ def vecmat_tc(x: Tensor, w: Tensor, scale, index1, index2, seg, num_out: int) ->
                    lambda: VecmatPlan(index1, seg, entries, num_out, cin, dev))
     packed = torch.empty(2, max(entries, 1) * cin * cout, dtype=torch.float32, device=dev)
     out = torch.empty(n, num_out, cout, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_vecmat_tc(x.data_ptr(), w.data_ptr(), _lib.ptr(index2), _lib.ptr(scale), packed[0].data_ptr(),
                                             packed[1].data_ptr(), out.data_ptr(), n, rows1, cin, cout, num_out, entries,
                                             plan.kb_begin.data_ptr(), plan.a_col.data_ptr(), status_flag(dev).data_ptr(),
@@ -146,7 +146,7 @@ def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Te
     plan = _cached("outer", dev, (scale, index1, index2, seg), (entries, num_w, c1, c2),
                    lambda: OuterPlan(scale, index1, index2, seg, entries, num_w, c1, c2, dev))
     out = torch.empty(num_w, c1, c2, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         need = int(_lib.lib().eqt_outer_tc_scratch_floats(n, c2, max(plan.m_tiles, 1)))
         scratch = _buffer(dev, max(need, 1))
         _lib.check(_lib.lib().eqt_outer_tc(a.data_ptr(), b.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(), n,

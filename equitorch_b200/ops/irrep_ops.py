@@ -29,7 +29,7 @@ def irrep_scale(x: Tensor, s: Tensor, irrep_index: Tensor, mode: int) -> Tensor:
     if tuple(s.shape) != want:
         raise ValueError(f"scale operand of mode {mode} must be {want}, got {tuple(s.shape)}")
     out = torch.empty_like(x)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_irrep_scale(x.data_ptr(), s.data_ptr(), out.data_ptr(), irrep_index.data_ptr(), n, d, k, c,
                                               mode, _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)), "eqt_irrep_scale")
     return out
@@ -47,7 +47,7 @@ def irrep_dot(a: Tensor, b: Tensor, irrep_seg: Tensor) -> Tensor:
     n, d, c = a.shape
     k = irrep_seg.numel() - 1
     out = torch.empty(n, k, c, dtype=a.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_irrep_dot(a.data_ptr(), b.data_ptr(), out.data_ptr(), irrep_seg.data_ptr(), n, d, k, c,
                                             _lib.DTYPE_CODE[a.dtype], _lib.stream_ptr(dev)), "eqt_irrep_dot")
     return out
@@ -71,7 +71,7 @@ def layer_rms_forward(x: Tensor, weight, irrep_seg: Tensor, scaled: bool, eps: f
     k = irrep_seg.numel() - 1
     out = torch.empty_like(x)
     rsigma = torch.empty(n, k, dtype=x.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_layer_rms_forward(x.data_ptr(), _lib.ptr(w), out.data_ptr(), rsigma.data_ptr(),
                                                     irrep_seg.data_ptr(), n, d, k, c, int(scaled), float(eps),
                                                     _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)), "eqt_layer_rms_forward")
@@ -90,7 +90,7 @@ def layer_rms_backward(x: Tensor, grad_out: Tensor, weight, rsigma: Tensor, irre
     partial = None
     if need_weight_grad:
         partial = torch.empty(_lib.lib().eqt_layer_rms_num_partials(n), k, c, dtype=x.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_layer_rms_backward(x.data_ptr(), grad_out.data_ptr(), _lib.ptr(w), rsigma.data_ptr(),
                                                      gx.data_ptr(), _lib.ptr(partial), irrep_seg.data_ptr(), n, d, k, c,
                                                      int(scaled), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)),

@@ -69,7 +69,7 @@ class MixPlan:
         big = torch.empty(n, dtype=torch.float32, device=w.device)
         small = torch.empty(n, dtype=torch.float32, device=w.device)
         blocks = self.structs(cin, cout)
-        with torch.cuda.device(w.device):
+        with _lib.on_device(w.device):
             _lib.check(_lib.lib().eqt_pack_weights(w.data_ptr(), self.path_gather.data_ptr(), cin, cout, blocks,
                                                    len(blocks), int(k_major), big.data_ptr(), small.data_ptr(),
                                                    _lib.stream_ptr(w.device)), "eqt_pack_weights")
@@ -87,7 +87,7 @@ def mix_tc_transposed(g: Tensor, weight: Tensor, plan: MixPlan) -> Tensor:
     big, small = plan.pack(weight, k_major=False)
     out = torch.empty(n, plan.rows, cin, dtype=torch.float32, device=dev)
     blocks = plan.structs(cin, cout)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_mix_tc_transposed(g.data_ptr(), big.data_ptr(), small.data_ptr(), out.data_ptr(), n,
                                                     plan.rows, comps, cin, cout, blocks, len(blocks),
                                                     status_flag(dev).data_ptr(), _lib.stream_ptr(dev)),
@@ -119,7 +119,7 @@ def wgrad_tc(s: Tensor, g: Tensor, plan: MixPlan, num_paths: int) -> Tensor:
     cout = g.shape[-1]
     packed = torch.empty(plan.path_gather.numel(), cin, cout, dtype=torch.float32, device=dev)
     blocks = plan.structs(cin, cout)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         need = int(_lib.lib().eqt_wgrad_tc_scratch_floats(n, cin, cout, blocks, len(blocks)))
         if need < 0:
             raise _lib.EqtError("eqt_wgrad_tc refuses these blocks")
@@ -156,7 +156,7 @@ def mix_tc(s: Tensor, weight: Tensor, plan: MixPlan) -> Tensor:
     out = torch.zeros(n, plan.comps, cout, dtype=torch.float32, device=dev) if _has_empty(plan) else \
         torch.empty(n, plan.comps, cout, dtype=torch.float32, device=dev)
     blocks = plan.structs(cin, cout)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_mix_tc(s.data_ptr(), big.data_ptr(), small.data_ptr(), out.data_ptr(), n, rows,
                                          plan.comps, cin, cout, blocks, len(blocks), status_flag(dev).data_ptr(),
                                          _lib.stream_ptr(dev)), "eqt_mix_tc")

@@ -65,7 +65,7 @@ def so3_uu_forward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor) -> Tensor:
     """``out[n, M, c] = sum_t s_t x[n, M1_t, c] y[n, M2_t] w[(n,) p_t, c]``; contiguous operands of one dtype."""
     n, _, c = x.shape
     out = torch.empty(n, plan.sizes[2], c, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(_lib.lib().eqt_so3_uu_forward(plan.ref, x.data_ptr(), y.data_ptr(), w.data_ptr(), out.data_ptr(), n, c,
                                                  int(w.ndim == 3), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(x.device)),
                    "eqt_so3_uu_forward")
@@ -78,7 +78,7 @@ def so3_uu_backward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor, g: Tensor,
     n, _, c = x.shape
     gx, gy, gw = (torch.empty_like(t) if wanted else None for t, wanted in zip((x, y, w), need))
     lib, scratch, floats = _lib.lib(), None, 0
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         if need[2] and w.ndim == 2:
             floats = int(lib.eqt_so3_uu_scratch_floats(plan.ref, n, c, 0, _lib.DTYPE_CODE[x.dtype]))
             scratch = torch.empty(floats, dtype=torch.float32, device=x.device)

@@ -33,7 +33,7 @@ def sh_forward(xyz: Tensor, l_max: int, normalize: bool, out_scale: float) -> Te
         raise TypeError("spherical harmonics take float32 or float64 input")
     flat = xyz.reshape(-1, 3).contiguous()
     out = torch.empty(flat.shape[0], (l_max + 1) ** 2, dtype=xyz.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_sh_forward(_lib.DTYPE_CODE[xyz.dtype], flat.data_ptr(), out.data_ptr(), flat.shape[0],
                                              C.byref(device_table(l_max, dev)), int(normalize), float(out_scale),
                                              _lib.stream_ptr(dev)), "eqt_sh_forward")
@@ -45,7 +45,7 @@ def sh_backward(xyz: Tensor, grad_out: Tensor, l_max: int, normalize: bool, out_
     flat = xyz.reshape(-1, 3).contiguous()
     g = grad_out.to(xyz.dtype).reshape(-1, (l_max + 1) ** 2).contiguous()
     gx = torch.empty_like(flat)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_sh_backward(_lib.DTYPE_CODE[xyz.dtype], flat.data_ptr(), g.data_ptr(), gx.data_ptr(),
                                               flat.shape[0], C.byref(device_table(l_max, dev)), int(normalize),
                                               float(out_scale), _lib.stream_ptr(dev)), "eqt_sh_backward")

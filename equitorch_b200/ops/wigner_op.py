@@ -78,7 +78,7 @@ def wigner_d_forward(table: WignerTable, alpha: Tensor, beta: Tensor, gamma: Ten
     alpha, beta, gamma = alpha.contiguous(), beta.contiguous(), gamma.contiguous()
     n = alpha.shape[0]
     out = torch.empty(n, table.dim, table.dim, dtype=alpha.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_wigner_d_forward(C.byref(table.struct), alpha.data_ptr(), beta.data_ptr(), gamma.data_ptr(),
                                                    out.data_ptr(), n, _lib.DTYPE_CODE[alpha.dtype], _lib.stream_ptr(dev)),
                    "eqt_wigner_d_forward")
@@ -90,7 +90,7 @@ def wigner_d_backward(table: WignerTable, alpha: Tensor, beta: Tensor, gamma: Te
     alpha, beta, gamma, grad_d = alpha.contiguous(), beta.contiguous(), gamma.contiguous(), grad_d.contiguous()
     n = alpha.shape[0]
     grads = torch.empty(3, n, dtype=alpha.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_wigner_d_backward(C.byref(table.struct), alpha.data_ptr(), beta.data_ptr(), gamma.data_ptr(),
                                                     grad_d.data_ptr(), grads[0].data_ptr(), grads[1].data_ptr(),
                                                     grads[2].data_ptr(), n, _lib.DTYPE_CODE[alpha.dtype], _lib.stream_ptr(dev)),
@@ -120,7 +120,7 @@ def dense_rotation(matrix: Tensor, x: Tensor, transposed: bool = False, row_rang
     dev = _lib.require_cuda(matrix, x)
     n, d, c = x.shape
     out = torch.empty_like(x)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_dense_rotation(matrix.data_ptr(), x.data_ptr(), out.data_ptr(), n, d, c, int(transposed),
                                                  _lib.ptr(row_range), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)),
                    "eqt_dense_rotation")
@@ -132,7 +132,7 @@ def dense_rotation_grad_matrix(grad_out: Tensor, x: Tensor, row_range: Tensor = 
     dev = _lib.require_cuda(grad_out, x)
     n, d, c = x.shape
     gm = torch.empty(n, d, d, dtype=x.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_dense_rotation_grad_matrix(grad_out.data_ptr(), x.data_ptr(), gm.data_ptr(), n, d, c,
                                                              _lib.ptr(row_range), _lib.DTYPE_CODE[x.dtype],
                                                              _lib.stream_ptr(dev)),
