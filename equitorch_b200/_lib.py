@@ -73,8 +73,9 @@ class MixBlockStruct(C.Structure):
 
 class PathTableStruct(C.Structure):
     _fields_ = [("fwd_blocks", C.c_void_p), ("bwd_blocks", C.c_void_p), ("fwd_paths", C.c_void_p), ("bwd_paths", C.c_void_p),
+                ("bwd_rows", C.c_void_p),
                 ("d1", C.c_int32), ("d2", C.c_int32), ("d_out", C.c_int32), ("num_weights", C.c_int32), ("num_paths", C.c_int32),
-                ("num_fwd_blocks", C.c_int32), ("num_bwd_blocks", C.c_int32)]
+                ("num_fwd_blocks", C.c_int32), ("num_bwd_blocks", C.c_int32), ("num_rows", C.c_int32)]
 
 
 # name -> (restype, argtypes); every symbol declared in include/eqt_b200.h appears here
@@ -128,6 +129,10 @@ SIGNATURES = {
     "eqt_so3_uu_backward": (C.c_int, [C.POINTER(PathTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                       C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_int32, C.c_int32,
                                       C.c_void_p]),
+    "eqt_so3_uv_supported": (C.c_int, [C.POINTER(PathTableStruct), C.c_int32]),
+    "eqt_so3_uv_expand": (C.c_int, [C.POINTER(PathTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p]),
+    "eqt_so3_uv_backward": (C.c_int, [C.POINTER(PathTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                      C.c_int64, C.c_int32, C.c_void_p]),
     "eqt_pack_weights": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_int32, C.c_int32,
                                    C.c_void_p, C.c_void_p, C.c_void_p]),
     "eqt_irrep_scale": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,

@@ -52,8 +52,9 @@ struct PathArgs {
   float* gw_partial;        // (gridDim.x, p, c) when they are shared
   const eqt_path_block* blocks;
   const eqt_path* paths;
+  const int32_t* rows;      // UV_BACKWARD: rows of g in the order of their use
   int64_t n;
-  int c, d1, d2, dout, p, num_blocks, num_paths;
+  int c, d1, d2, dout, p, num_blocks, num_paths, num_rows;
 };
 
 template <typename T> struct Chunk;
@@ -117,20 +118,49 @@ struct WeightStream {
   }
 };
 
-// Shared memory of both directions; host and kernels agree on the sizes through this one description.
+// The rows of the node-level gradient G (n, rows, c) of a sample in path order, a fixed number of rows ahead.
+constexpr int ROWS_AHEAD = 16;
+struct RowStream {
+  float* ring;              // this thread's column, ROWS_AHEAD rows
+  const float* g;           // the thread's channels of row 0 of its sample
+  const int32_t* order;     // rows in the order of their use
+  int row, c, count, at;
+  __device__ __forceinline__ void issue(int q) {
+    if (q < count) copy_v(ring + (q % ROWS_AHEAD) * row, g + (int64_t)order[q] * c);
+    copy_commit();
+  }
+  __device__ __forceinline__ void begin() {
+    at = 0;
+    for (int q = 0; q < ROWS_AHEAD; ++q) issue(q);
+  }
+  template <int N> __device__ __forceinline__ void next(float (&v)[N][V]) {
+    copy_wait<ROWS_AHEAD - N>();
+#pragma unroll
+    for (int m = 0; m < N; ++m) lds_v(ring + ((at + m) % ROWS_AHEAD) * row, v[m]);
+#pragma unroll
+    for (int m = 0; m < N; ++m) issue(at + m + ROWS_AHEAD);
+    at += N;
+  }
+};
+
+enum PathMode { UU_FORWARD, UU_BACKWARD, UV_EXPAND, UV_BACKWARD };
+
+// Shared memory of a kernel; host and kernels agree on the sizes through this one description.
 struct PathSmem {
-  size_t blocks, paths, ys, xcol, gcol, wring, gycol, gwcol, total;
-  __host__ __device__ PathSmem(bool backward, bool shared_gw, int elem, int threads, int slots, int d1, int dout, int d2, int p, int num_blocks,
-                               int num_paths) {
+  size_t blocks, paths, rows, ys, xcol, gcol, ring, gycol, gwcol, total;
+  __host__ __device__ PathSmem(PathMode mode, bool shared_gw, int elem, int threads, int slots, int d1, int dout, int d2, int p, int num_blocks,
+                               int num_paths, int num_rows) {
+    const bool backward = mode == UU_BACKWARD || mode == UV_BACKWARD;
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t r = at; at = (at + bytes + 15) & ~size_t(15); return r; };
     const size_t row = (size_t)elem * V * threads;
     blocks = take(sizeof(eqt_path_block) * num_blocks);
     paths = take(sizeof(eqt_path) * num_paths);
+    rows = take(mode == UV_BACKWARD ? sizeof(int32_t) * num_rows : 0);
     ys = take(sizeof(float) * slots * d2);
     xcol = take(row * d1);
-    gcol = take(backward ? row * dout : 0);
-    wring = take(row * AHEAD);
+    gcol = take(mode == UU_BACKWARD ? row * dout : 0);
+    ring = take(mode == UV_EXPAND ? 0 : row * (mode == UV_BACKWARD ? ROWS_AHEAD : AHEAD));
     gycol = take(backward ? sizeof(float) * threads * d2 : 0);
     gwcol = take(shared_gw ? sizeof(float) * V * threads * p : 0);
     total = at;
@@ -190,13 +220,13 @@ __global__ void __launch_bounds__(128, 4) so3_uu_forward_kernel(PathArgs a, int 
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, threads = blockDim.x, row = threads * V;
   const int tps = a.c / V, slots = threads / tps, slot = tid / tps, ch = (tid - slot * tps) * V;
-  const PathSmem L(false, false, sizeof(T), threads, slots, a.d1, a.dout, a.d2, a.p, a.num_blocks, a.num_paths);
+  const PathSmem L(UU_FORWARD, false, sizeof(T), threads, slots, a.d1, a.dout, a.d2, a.p, a.num_blocks, a.num_paths, 0);
   eqt_path_block* blocks = reinterpret_cast<eqt_path_block*>(smem + L.blocks);
   eqt_path* paths = reinterpret_cast<eqt_path*>(smem + L.paths);
   float* ys = reinterpret_cast<float*>(smem + L.ys);
   T* xc = reinterpret_cast<T*>(smem + L.xcol) + tid * V;
   WeightStream<T> ws;
-  ws.ring = reinterpret_cast<T*>(smem + L.wring) + tid * V;
+  ws.ring = reinterpret_cast<T*>(smem + L.ring) + tid * V;
   ws.row = row; ws.c = a.c;
   for (int i = tid; i < a.num_blocks; i += threads) blocks[i] = a.blocks[i];
   for (int i = tid; i < a.num_paths; i += threads) paths[i] = a.paths[i];
@@ -229,6 +259,23 @@ __global__ void __launch_bounds__(128, 4) so3_uu_forward_kernel(PathArgs a, int 
         case 3: forward_block<T, 3>(a, bd, ws, xc, row, yr, out); break;
       }
     }
+  }
+}
+
+// gy of the CTA's samples from the threads' columns: the threads of a sample hold theirs side by side; the start is
+// rotated to spread the banks
+template <typename T>
+__device__ __forceinline__ void sum_gy(const float* gy_all, T* gy, int64_t n0, int here, int d2, int threads, int tps) {
+  for (int i = threadIdx.x; i < here * d2; i += threads) {
+    const int sl = i / d2, k = i - sl * d2;
+    const float* col = gy_all + k * threads + sl * tps;
+    float v = 0.f;
+    int j = i % tps;
+    for (int u = 0; u < tps; ++u) {
+      v += col[j];
+      if (++j == tps) j = 0;
+    }
+    gy[n0 * d2 + i] = static_cast<T>(v);
   }
 }
 
@@ -312,7 +359,7 @@ __global__ void __launch_bounds__(128, 3) so3_uu_backward_kernel(PathArgs a, int
   const int tid = threadIdx.x, threads = blockDim.x, row = threads * V;
   const int tps = a.c / V, slots = threads / tps, slot = tid / tps, ch = (tid - slot * tps) * V;
   const bool shared_gw = a.gw_partial != nullptr;
-  const PathSmem L(true, shared_gw, sizeof(T), threads, slots, a.d1, a.dout, a.d2, a.p, a.num_blocks, a.num_paths);
+  const PathSmem L(UU_BACKWARD, shared_gw, sizeof(T), threads, slots, a.d1, a.dout, a.d2, a.p, a.num_blocks, a.num_paths, 0);
   eqt_path_block* blocks = reinterpret_cast<eqt_path_block*>(smem + L.blocks);
   eqt_path* paths = reinterpret_cast<eqt_path*>(smem + L.paths);
   float* ys = reinterpret_cast<float*>(smem + L.ys);
@@ -321,7 +368,7 @@ __global__ void __launch_bounds__(128, 3) so3_uu_backward_kernel(PathArgs a, int
   float* gy_all = reinterpret_cast<float*>(smem + L.gycol);
   float* gw_all = reinterpret_cast<float*>(smem + L.gwcol);
   WeightStream<T> ws;
-  ws.ring = reinterpret_cast<T*>(smem + L.wring) + tid * V;
+  ws.ring = reinterpret_cast<T*>(smem + L.ring) + tid * V;
   ws.paths = paths;
   ws.row = row; ws.c = a.c; ws.count = a.num_paths;
   for (int i = tid; i < a.num_blocks; i += threads) blocks[i] = a.blocks[i];
@@ -363,18 +410,7 @@ __global__ void __launch_bounds__(128, 3) so3_uu_backward_kernel(PathArgs a, int
     }
     if (a.gy) {
       __syncthreads();
-      // the threads of a sample hold its gy in consecutive columns; the start is rotated to spread the banks
-      for (int i = tid; i < here * a.d2; i += threads) {
-        const int sl = i / a.d2, k = i - sl * a.d2;
-        const float* col = gy_all + k * threads + sl * tps;
-        float v = 0.f;
-        int j = i % tps;
-        for (int u = 0; u < tps; ++u) {
-          v += col[j];
-          if (++j == tps) j = 0;
-        }
-        static_cast<T*>(a.gy)[n0 * a.d2 + i] = static_cast<T>(v);
-      }
+      sum_gy(gy_all, static_cast<T*>(a.gy), n0, here, a.d2, threads, tps);
     }
   }
   if (shared_gw) {
@@ -386,6 +422,172 @@ __global__ void __launch_bounds__(128, 3) so3_uu_backward_kernel(PathArgs a, int
       float v = 0.f;
       for (int sl = 0; sl < slots; ++sl) v += col[sl * a.c];
       part[i] = v;
+    }
+  }
+}
+
+// ---- full channel mixing ('uv'): the channel-wise half of the layer ---------------------------------------------------
+// S[n, row(p, M), c] = sum_{t: (p_t, M_t) = (p, M)} s_t x[n, M1_t, c] y[n, M2_t]: one row per (output component, path),
+// which the GEMM with the C_in x C_out matrices consumes.  Bound: the rows written (6.2 times the features at l_max 3).
+template <int LO>
+__device__ __forceinline__ void expand_block(const PathArgs& a, const eqt_path_block& b, const eqt_path* paths, const float* xc, int row,
+                                             const float* yr, float* out) {
+  for (int q = b.first; q < b.first + b.count; ++q) {
+    const eqt_path pd = paths[q];
+    const float wv[V] = {pd.scale, pd.scale, pd.scale, pd.scale};
+    float o[2 * LO + 1][V];
+#pragma unroll
+    for (int m = 0; m < 2 * LO + 1; ++m)
+#pragma unroll
+      for (int i = 0; i < V; ++i) o[m][i] = 0.f;
+    const float* xb = xc + pd.offset * row;
+    const float* yb = yr + pd.offset_y;
+    switch (pd.code) {
+#define EQT_CASE(L1, L2) case L1 * 4 + L2: forward_path<float, LO, L1, L2>(o, xb, row, yb, wv); break;
+      EQT_PATH_CASES(EQT_CASE)
+#undef EQT_CASE
+    }
+#pragma unroll
+    for (int m = 0; m < 2 * LO + 1; ++m) store_v<float>(out + (int64_t)(pd.row + m * pd.row_stride) * a.c, o[m]);
+  }
+}
+
+__global__ void __launch_bounds__(128, 4) so3_uv_expand_kernel(PathArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int tid = threadIdx.x, threads = blockDim.x, row = threads * V;
+  const int tps = a.c / V, slots = threads / tps, slot = tid / tps, ch = (tid - slot * tps) * V;
+  const PathSmem L(UV_EXPAND, false, sizeof(float), threads, slots, a.d1, a.dout, a.d2, a.p, a.num_blocks, a.num_paths, 0);
+  eqt_path_block* blocks = reinterpret_cast<eqt_path_block*>(smem + L.blocks);
+  eqt_path* paths = reinterpret_cast<eqt_path*>(smem + L.paths);
+  float* ys = reinterpret_cast<float*>(smem + L.ys);
+  float* xc = reinterpret_cast<float*>(smem + L.xcol) + tid * V;
+  for (int i = tid; i < a.num_blocks; i += threads) blocks[i] = a.blocks[i];
+  for (int i = tid; i < a.num_paths; i += threads) paths[i] = a.paths[i];
+  const float* x = static_cast<const float*>(a.x);
+  const float* y = static_cast<const float*>(a.y);
+  const int b0 = a.num_blocks * (int)blockIdx.y / (int)gridDim.y, b1 = a.num_blocks * ((int)blockIdx.y + 1) / (int)gridDim.y;
+  for (int64_t n0 = (int64_t)blockIdx.x * slots; n0 < a.n; n0 += (int64_t)gridDim.x * slots) {
+    const int here = (int)min((int64_t)slots, a.n - n0);
+    const int64_t n = n0 + slot;
+    __syncthreads();
+    if (slot < here) {
+      for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
+      copy_commit();
+    }
+    for (int i = tid; i < here * a.d2; i += threads) ys[i] = y[n0 * a.d2 + i];
+    copy_wait<0>();
+    __syncthreads();
+    if (slot >= here) continue;
+    float* out = static_cast<float*>(a.out) + n * a.num_rows * a.c + ch;
+    const float* yr = ys + slot * a.d2;
+    for (int b = b0; b < b1; ++b) {
+      const eqt_path_block bd = blocks[b];
+      switch (bd.l) {
+        case 0: expand_block<0>(a, bd, paths, xc, row, yr, out); break;
+        case 1: expand_block<1>(a, bd, paths, xc, row, yr, out); break;
+        case 2: expand_block<2>(a, bd, paths, xc, row, yr, out); break;
+        case 3: expand_block<3>(a, bd, paths, xc, row, yr, out); break;
+      }
+    }
+  }
+}
+
+// gx[n, M1, c] = sum_t s_t y[n, M2_t] G[n, row_t, c]  and  gy[n, M2] = sum_t s_t <x[n, M1_t], G[n, row_t]>  from one
+// pass over G: a row is used by one path, so it goes from memory through the ring into registers once, and neither a
+// second intermediate nor a second GEMM is needed for gx.
+template <int LO, int L1, int L2>
+__device__ __forceinline__ void uv_backward_path(float (&gx)[2 * L1 + 1][V], const float (&x)[2 * L1 + 1][V], RowStream& rs, const float* yr,
+                                                 float* gyc, int threads, float scale) {
+  if constexpr (is_path(LO, L1, L2)) {
+    float g[2 * LO + 1][V], y[2 * L2 + 1], gy[2 * L2 + 1];
+    rs.next<2 * LO + 1>(g);
+#pragma unroll
+    for (int m = 0; m < 2 * LO + 1; ++m)
+#pragma unroll
+      for (int i = 0; i < V; ++i) g[m][i] *= scale;
+#pragma unroll
+    for (int i = 0; i < 2 * L2 + 1; ++i) { y[i] = yr[i]; gy[i] = gyc[i * threads]; }
+    CgPath<LO, L1, L2>::template adjoint<V>(gx, g, y);
+    CgPath<LO, L1, L2>::template inner<V>(gy, g, x);
+#pragma unroll
+    for (int i = 0; i < 2 * L2 + 1; ++i) gyc[i * threads] = gy[i];
+  }
+}
+
+template <int L1>
+__device__ __forceinline__ void uv_backward_block(const PathArgs& a, const eqt_path_block& b, const eqt_path* paths, RowStream& rs,
+                                                  const float* xc, int row, int threads, const float* yr, float* gyc, float* gxout) {
+  float x[2 * L1 + 1][V], gx[2 * L1 + 1][V];
+#pragma unroll
+  for (int m = 0; m < 2 * L1 + 1; ++m) {
+    lds_v(xc + (b.offset + m) * row, x[m]);
+#pragma unroll
+    for (int i = 0; i < V; ++i) gx[m][i] = 0.f;
+  }
+  for (int q = b.first; q < b.first + b.count; ++q) {
+    const eqt_path pd = paths[q];
+    switch (pd.code) {
+#define EQT_CASE(LO, L2) \
+  case LO * 4 + L2: uv_backward_path<LO, L1, L2>(gx, x, rs, yr + pd.offset_y, gyc + pd.offset_y * threads, threads, pd.scale); break;
+      EQT_PATH_CASES(EQT_CASE)
+#undef EQT_CASE
+    }
+  }
+  if (gxout)
+#pragma unroll
+    for (int m = 0; m < 2 * L1 + 1; ++m) store_v<float>(gxout + (int64_t)(b.offset + m) * a.c, gx[m]);
+}
+
+__global__ void __launch_bounds__(128, 3) so3_uv_backward_kernel(PathArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int tid = threadIdx.x, threads = blockDim.x, row = threads * V;
+  const int tps = a.c / V, slots = threads / tps, slot = tid / tps, ch = (tid - slot * tps) * V;
+  const PathSmem L(UV_BACKWARD, false, sizeof(float), threads, slots, a.d1, a.dout, a.d2, a.p, a.num_blocks, a.num_paths, a.num_rows);
+  eqt_path_block* blocks = reinterpret_cast<eqt_path_block*>(smem + L.blocks);
+  eqt_path* paths = reinterpret_cast<eqt_path*>(smem + L.paths);
+  int32_t* rows = reinterpret_cast<int32_t*>(smem + L.rows);
+  float* ys = reinterpret_cast<float*>(smem + L.ys);
+  float* xc = reinterpret_cast<float*>(smem + L.xcol) + tid * V;
+  float* gy_all = reinterpret_cast<float*>(smem + L.gycol);
+  RowStream rs;
+  rs.ring = reinterpret_cast<float*>(smem + L.ring) + tid * V;
+  rs.order = rows;
+  rs.row = row; rs.c = a.c; rs.count = a.num_rows;
+  for (int i = tid; i < a.num_blocks; i += threads) blocks[i] = a.blocks[i];
+  for (int i = tid; i < a.num_paths; i += threads) paths[i] = a.paths[i];
+  for (int i = tid; i < a.num_rows; i += threads) rows[i] = a.rows[i];
+  const float* x = static_cast<const float*>(a.x);
+  const float* y = static_cast<const float*>(a.y);
+  for (int64_t n0 = (int64_t)blockIdx.x * slots; n0 < a.n; n0 += (int64_t)gridDim.x * slots) {
+    const int here = (int)min((int64_t)slots, a.n - n0);
+    const int64_t n = n0 + slot;
+    __syncthreads();                                   // tables loaded / harmonics and partial gy of the previous samples have been read
+    if (slot < here) {
+      for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
+      copy_commit();
+      rs.g = static_cast<const float*>(a.g) + n * a.num_rows * a.c + ch;
+      rs.begin();
+      for (int i = 0; i < a.d2; ++i) gy_all[i * threads + tid] = 0.f;
+    }
+    for (int i = tid; i < here * a.d2; i += threads) ys[i] = y[n0 * a.d2 + i];
+    __syncthreads();
+    if (slot < here) {
+      float* gx = a.gx ? static_cast<float*>(a.gx) + n * a.d1 * a.c + ch : nullptr;
+      const float* yr = ys + slot * a.d2;
+      copy_wait<ROWS_AHEAD>();                         // x
+      for (int b = 0; b < a.num_blocks; ++b) {
+        const eqt_path_block bd = blocks[b];
+        switch (bd.l) {
+          case 0: uv_backward_block<0>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
+          case 1: uv_backward_block<1>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
+          case 2: uv_backward_block<2>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
+          case 3: uv_backward_block<3>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
+        }
+      }
+    }
+    if (a.gy) {
+      __syncthreads();
+      sum_gy(gy_all, static_cast<float*>(a.gy), n0, here, a.d2, threads, tps);
     }
   }
 }
@@ -414,14 +616,15 @@ constexpr size_t PATH_SMEM_MAX = 220 * 1024;
 struct PathShape { int threads, slots, grid, split; size_t smem; };
 
 // 128 threads; fewer while that leaves SMs without a CTA (a sample's threads stay in one CTA)
-bool path_shape(bool backward, bool shared_gw, int64_t n, int c, int dtype, const eqt_path_table* t, PathShape* s) {
+bool path_shape(PathMode mode, bool shared_gw, int64_t n, int c, int dtype, const eqt_path_table* t, PathShape* s) {
   if (c < V || c % V || c / V > 128) return false;
+  const bool backward = mode == UU_BACKWARD || mode == UV_BACKWARD;
   int threads = 128;
   while (threads > 32 && threads / 2 >= c / V && ceil_div(n, threads / (c / V)) < sm_count()) threads /= 2;
   for (; threads >= c / V && threads >= 32; threads /= 2) {
     const int slots = threads / (c / V);
-    const PathSmem L(backward, shared_gw, dtype == EQT_F32 ? 4 : 2, threads, slots, t->d1, t->d_out, t->d2, t->num_weights,
-                     backward ? t->num_bwd_blocks : t->num_fwd_blocks, t->num_paths);
+    const PathSmem L(mode, shared_gw, dtype == EQT_F32 ? 4 : 2, threads, slots, t->d1, t->d_out, t->d2, t->num_weights,
+                     backward ? t->num_bwd_blocks : t->num_fwd_blocks, t->num_paths, t->num_rows);
     if (L.total > PATH_SMEM_MAX) continue;
     const int per_sm = std::max<int>(1, std::min<int>(512 / threads, (int)(PATH_SMEM_MAX / (L.total + 1024))));
     s->threads = threads; s->slots = slots; s->smem = L.total;
@@ -432,34 +635,43 @@ bool path_shape(bool backward, bool shared_gw, int64_t n, int c, int dtype, cons
   return false;
 }
 
-int path_run(bool backward, const eqt_path_table* t, bool per_sample_w, bool shared_gw, int64_t n, int c, int dtype, PathArgs a,
+int path_run(PathMode mode, const eqt_path_table* t, bool per_sample_w, bool shared_gw, int64_t n, int c, int dtype, PathArgs a,
              cudaStream_t st, int* grid) {
   a.n = n; a.c = c; a.d1 = t->d1; a.d2 = t->d2; a.dout = t->d_out; a.p = t->num_weights; a.num_paths = t->num_paths;
+  a.rows = t->bwd_rows; a.num_rows = t->num_rows;
+  const bool backward = mode == UU_BACKWARD || mode == UV_BACKWARD;
   a.num_blocks = backward ? t->num_bwd_blocks : t->num_fwd_blocks;
   a.blocks = backward ? t->bwd_blocks : t->fwd_blocks;
   a.paths = backward ? t->bwd_paths : t->fwd_paths;
   PathShape s;
-  if (!path_shape(backward, shared_gw, n, c, dtype, t, &s))
+  if (!path_shape(mode, shared_gw, n, c, dtype, t, &s))
     return fail(EQT_ERR_UNSUPPORTED, "paths and columns of %d channels do not fit shared memory", c);
   if (grid) *grid = s.grid;
   const uintptr_t mask = (uintptr_t)(V * (dtype == EQT_F32 ? 4 : 2)) - 1;
   if (((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.g) |
         reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.gx) | reinterpret_cast<uintptr_t>(a.gw)) & mask) != 0)
     return fail(EQT_ERR_UNSUPPORTED, "operands are not aligned to four elements");
-  auto kern = dtype == EQT_F32 ? (backward ? so3_uu_backward_kernel<float> : so3_uu_forward_kernel<float>)
-                               : (backward ? so3_uu_backward_kernel<__nv_bfloat16> : so3_uu_forward_kernel<__nv_bfloat16>);
-  if (s.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
-    if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  auto launch = [&](auto kern, auto... more) {
+    if (s.smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+      if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    }
+    kern<<<dim3((unsigned)s.grid, (unsigned)s.split), s.threads, s.smem, st>>>(a, more...);
+    return check_launch("so3 path kernel");
+  };
+  const int per_sample = per_sample_w;
+  switch (mode) {
+    case UU_FORWARD: return dtype == EQT_F32 ? launch(so3_uu_forward_kernel<float>, per_sample) : launch(so3_uu_forward_kernel<__nv_bfloat16>, per_sample);
+    case UU_BACKWARD: return dtype == EQT_F32 ? launch(so3_uu_backward_kernel<float>, per_sample) : launch(so3_uu_backward_kernel<__nv_bfloat16>, per_sample);
+    case UV_EXPAND: return launch(so3_uv_expand_kernel);
+    default: return launch(so3_uv_backward_kernel);
   }
-  kern<<<dim3((unsigned)s.grid, (unsigned)s.split), s.threads, s.smem, st>>>(a, per_sample_w);
-  return check_launch(backward ? "so3_uu_backward_kernel" : "so3_uu_forward_kernel");
 }
 
 int path_check(const eqt_path_table* t, int64_t n, int c, int dtype) {
-  if (!t || !t->fwd_blocks || !t->bwd_blocks || !t->fwd_paths || !t->bwd_paths) return fail(EQT_ERR_BAD_ARGUMENT, "incomplete table");
+  if (!t || !t->fwd_blocks || !t->bwd_blocks || !t->fwd_paths || !t->bwd_paths || !t->bwd_rows) return fail(EQT_ERR_BAD_ARGUMENT, "incomplete table");
   if (n < 0 || c <= 0 || t->d1 <= 0 || t->d2 <= 0 || t->d_out <= 0 || t->num_weights <= 0 || t->num_paths < 0 ||
-      t->num_fwd_blocks < 0 || t->num_bwd_blocks < 0)
+      t->num_fwd_blocks < 0 || t->num_bwd_blocks < 0 || t->num_rows < 0)
     return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
   if (dtype != EQT_F32 && dtype != EQT_BF16) return fail(EQT_ERR_UNSUPPORTED, "float32 or bfloat16 only");
   return EQT_OK;
@@ -472,7 +684,7 @@ extern "C" int64_t eqt_so3_uu_scratch_floats(const eqt_path_table* table, int64_
   using namespace eqt;
   if (!table || n < 0 || channels <= 0) return -1;
   PathShape s;
-  if (!path_shape(false, false, n, channels, dtype, table, &s) || !path_shape(true, !per_sample_weight, n, channels, dtype, table, &s)) return -1;
+  if (!path_shape(UU_FORWARD, false, n, channels, dtype, table, &s) || !path_shape(UU_BACKWARD, !per_sample_weight, n, channels, dtype, table, &s)) return -1;
   return per_sample_weight ? 0 : (int64_t)s.grid * table->num_weights * channels;
 }
 
@@ -484,7 +696,7 @@ extern "C" int eqt_so3_uu_forward(const eqt_path_table* table, const void* x, co
   if (!x || !y || !w || !out) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   PathArgs a{};
   a.x = x; a.y = y; a.w = w; a.out = out;
-  return path_run(false, table, per_sample_weight != 0, false, n, channels, dtype, a, static_cast<cudaStream_t>(stream), nullptr);
+  return path_run(UU_FORWARD, table, per_sample_weight != 0, false, n, channels, dtype, a, static_cast<cudaStream_t>(stream), nullptr);
 }
 
 extern "C" int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, const void* y, const void* w, const void* g, void* gx,
@@ -506,7 +718,7 @@ extern "C" int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, c
   a.gw_partial = shared_gw ? scratch : nullptr;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int blocks = 0;
-  if (int rc = path_run(true, table, per_sample_weight != 0, shared_gw, n, channels, dtype, a, st, &blocks)) return rc;
+  if (int rc = path_run(UU_BACKWARD, table, per_sample_weight != 0, shared_gw, n, channels, dtype, a, st, &blocks)) return rc;
   if (!shared_gw) return EQT_OK;
   const int count = table->num_weights * channels;
   const unsigned grid = (unsigned)ceil_div(count, 32);
@@ -515,4 +727,33 @@ extern "C" int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, c
   else
     so3_uu_reduce_kernel<__nv_bfloat16><<<grid, dim3(32, 8), 0, st>>>(scratch, static_cast<__nv_bfloat16*>(gw), blocks, count);
   return check_launch("so3_uu_reduce_kernel");
+}
+
+extern "C" int eqt_so3_uv_supported(const eqt_path_table* table, int32_t channels) {
+  using namespace eqt;
+  PathShape s;
+  return table && channels > 0 && path_shape(UV_EXPAND, false, 1 << 30, channels, EQT_F32, table, &s) &&
+         path_shape(UV_BACKWARD, false, 1 << 30, channels, EQT_F32, table, &s);
+}
+
+extern "C" int eqt_so3_uv_expand(const eqt_path_table* table, const float* x, const float* y, float* rows, int64_t n, int32_t channels,
+                                 void* stream) {
+  using namespace eqt;
+  if (int rc = path_check(table, n, channels, EQT_F32)) return rc;
+  if (n == 0) return EQT_OK;
+  if (!x || !y || !rows) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  PathArgs a{};
+  a.x = x; a.y = y; a.out = rows;
+  return path_run(UV_EXPAND, table, false, false, n, channels, EQT_F32, a, static_cast<cudaStream_t>(stream), nullptr);
+}
+
+extern "C" int eqt_so3_uv_backward(const eqt_path_table* table, const float* x, const float* y, const float* grad_rows, float* gx, float* gy,
+                                   int64_t n, int32_t channels, void* stream) {
+  using namespace eqt;
+  if (int rc = path_check(table, n, channels, EQT_F32)) return rc;
+  if (n == 0) return EQT_OK;
+  if (!x || !y || !grad_rows) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  PathArgs a{};
+  a.x = x; a.y = y; a.g = grad_rows; a.gx = gx; a.gy = gy;
+  return path_run(UV_BACKWARD, table, false, false, n, channels, EQT_F32, a, static_cast<cudaStream_t>(stream), nullptr);
 }

@@ -43,21 +43,55 @@ from ...structs import TensorProductInfo
 _CHECK_EVERY_CALL = os.environ.get("EQT_CHECK_STATUS", "0") not in ("", "0")
 
 
-class GraphTPPlan:
+class MixTables:
+    """Device tables of a layer's weight step and of its adjoints: ``out[n, M] = sum_{rows r of M} s[n, r] W[path(r)]``."""
+
+    def __init__(self, info: TensorProductInfo, device, out_dims=None):
+        self.mix_fwd, self.mix_bwd1, self.mix_bwd2 = (t.to(device) for t in (info.info_M_fwd, info.info_M_bwd1, info.info_M_bwd2))
+        # block structure of the weight step for the tensor-core GEMM (None: CUDA-core kernel)
+        self.tc_fwd = MixPlan(info.info_M_fwd, out_dims, device) if out_dims is not None else None
+
+    def forward(self, s: Tensor, weight: Tensor, mode: str) -> Tensor:
+        return _mix(s, weight, self.mix_fwd, mode, self.tc_fwd)
+
+    def grad_weight(self, s: Tensor, grad: Tensor, weight: Tensor, mode: str) -> Tensor:
+        tcw, b2 = self.tc_fwd, self.mix_bwd2
+        if (mode == "uv" and tcw is not None and tcw.regular and grad.dtype == torch.float32
+                and _tc_supported_w(weight.shape[-2], weight.shape[-1])):
+            return wgrad_tc(s, grad, tcw, weight.shape[0])
+        if mode == "uv":   # (P, Cout, Cin) summed over nodes, then transposed to the weight's layout
+            gw = _ops.indexed_outer_scale_gather(grad, s, b2.scale, b2.index1, b2.index2, b2.seg_out,
+                                                 out_accumulated=True, out_size=b2.out_size)
+            return gw.transpose(-1, -2).contiguous()
+        return _ops.indexed_mul_scale_gather(grad, s, b2.scale, b2.index1, b2.index2, b2.seg_out,
+                                             out_accumulated=True, out_size=b2.out_size)
+
+    def grad_inter(self, grad: Tensor, weight: Tensor, mode: str) -> Tensor:
+        """Gradient with respect to the intermediate: ``G[n, r] = grad[n, M(r)] W[path(r)]^T``."""
+        tc, b1 = self.tc_fwd, self.mix_bwd1
+        if (mode == "uv" and tc is not None and tc.regular
+                and _tc_supported_t(weight.shape[-2], weight.shape[-1])):
+            return mix_tc_transposed(grad, weight, tc)
+        if mode == "uv":
+            return _ops.indexed_vecmat_scale_gather(grad, weight.transpose(-1, -2).contiguous(), b1.scale, b1.index2, b1.index1,
+                                                    b1.seg_out, out_size=b1.out_size)
+        return _ops.indexed_mul_scale_gather(weight, grad, b1.scale, b1.index1, b1.index2, b1.seg_out,
+                                             out_size=b1.out_size)
+
+
+class GraphTPPlan(MixTables):
     """Device tables of one layer for the fused graph kernels (built once per layer and device)."""
 
     def __init__(self, tp_info_forward: TensorProductInfo, tp_info_backward1: TensorProductInfo,
                  d_in1: int, d_in2: int, d_out: int, device, out_dims=None, in1_dims=None):
         f, b1 = tp_info_forward, tp_info_backward1
+        super().__init__(f, device, out_dims)
         self.fwd_table = TpTable(f.info_Mij_fwd, True, d_in1, d_in2, device)
         # backward-1 tables: input1 is the channel-less operand, input2 the incoming gradient
         self.bwd1_table = TpTable(b1.info_Mij_fwd, False, d_out, d_in2, device)
-        self.mix_fwd, self.mix_bwd1, self.mix_bwd2 = (t.to(device) for t in (f.info_M_fwd, f.info_M_bwd1, f.info_M_bwd2))
         self.mix_src = b1.info_M_fwd.to(device)
         self.d_in1, self.d_in2, self.d_out = d_in1, d_in2, d_out
         self.device = torch.device(device)
-        # block structure of the two weight steps for the tensor-core GEMM (None: CUDA-core kernel)
-        self.tc_fwd = MixPlan(f.info_M_fwd, out_dims, device) if out_dims is not None else None
         self.tc_src = MixPlan(b1.info_M_fwd, in1_dims, device) if in1_dims is not None else None
 
 
@@ -82,7 +116,7 @@ class FusedGraphOps:
             s = cg_segment_sum(plan.fwd_table, node_x, y, graph.src_by_dst, graph.dst_order, graph.dst_ptr,
                                graph.num_dst)
         with _profile.timed("channel_mix[fwd]"):
-            out = _mix(s, weight, plan.mix_fwd, self.mode, plan.tc_fwd)
+            out = plan.forward(s, weight, self.mode)
         return out, (node_x, y, weight, s if weight.requires_grad else None)
 
     def _wt(self, weight: Tensor) -> Tensor:
@@ -90,34 +124,15 @@ class FusedGraphOps:
 
     def grad_weight(self, state, grad: Tensor) -> Tensor:
         _, _, weight, s = state
-        plan, mode, b2 = self.plan, self.mode, self.plan.mix_bwd2
         with _profile.timed("weight_grad"):
-            tcw = plan.tc_fwd
-            if (mode == "uv" and tcw is not None and tcw.regular and grad.dtype == torch.float32
-                    and _tc_supported_w(weight.shape[-2], weight.shape[-1])):
-                return wgrad_tc(s, grad, tcw, weight.shape[0])
-            if mode == "uv":   # (P, Cout, Cin) summed over nodes, then transposed to the weight's layout
-                gw = _ops.indexed_outer_scale_gather(grad, s, b2.scale, b2.index1, b2.index2, b2.seg_out,
-                                                     out_accumulated=True, out_size=b2.out_size)
-                return gw.transpose(-1, -2).contiguous()
-            return _ops.indexed_mul_scale_gather(grad, s, b2.scale, b2.index1, b2.index2, b2.seg_out,
-                                                 out_accumulated=True, out_size=b2.out_size)
+            return self.plan.grad_weight(s, grad, weight, self.mode)
 
     def grad_y(self, state, grad: Tensor) -> Tensor:
         node_x, y, weight, _ = state
-        graph, plan, mode, b1 = self.graph, self.plan, self.mode, self.plan.mix_bwd1
+        graph, plan = self.graph, self.plan
         # gradient w.r.t. the node-level intermediate: G[d, r] = g[d, M(r)] W[w(r)]^T
         with _profile.timed("channel_mix[grad_inter]"):
-            tc = plan.tc_fwd
-            if (mode == "uv" and tc is not None and tc.regular
-                    and _tc_supported_t(weight.shape[-2], weight.shape[-1])):
-                g_inter = mix_tc_transposed(grad, weight, tc)
-            elif mode == "uv":
-                g_inter = _ops.indexed_vecmat_scale_gather(grad, self._wt(weight), b1.scale, b1.index2, b1.index1,
-                                                           b1.seg_out, out_size=b1.out_size)
-            else:
-                g_inter = _ops.indexed_mul_scale_gather(weight, grad, b1.scale, b1.index1, b1.index2, b1.seg_out,
-                                                        out_size=b1.out_size)
+            g_inter = plan.grad_inter(grad, weight, self.mode)
         with _profile.timed("cg_inner[grad_y]"):
             return cg_inner(plan.fwd_table, node_x, g_inter, graph.src_by_dst, graph.dst_ptr, graph.dst_sorted,
                             graph.dst_order, y.shape[0])

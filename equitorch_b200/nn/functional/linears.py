@@ -18,7 +18,7 @@ import torch
 from torch import Tensor
 from torch.autograd import Function
 
-from ...ops import so3_uu_op as _uu
+from ...ops import so3_path_op as _path
 from ...ops.graph_ops import segment_sum  # noqa: F401  (re-exported for users of the functional API)
 from ...ops.indexed_product_scale_segment_op import indexed_vecmat_scale_segment
 from ...ops.indexed_product_segment_op import indexed_outer_segment
@@ -172,7 +172,7 @@ class SO3LinearUU(Function):
         input1, input2, weight = input1.contiguous(), input2.contiguous(), weight.contiguous()
         ctx.save_for_backward(input1, input2, weight)
         ctx.plan, ctx.infos = plan, infos
-        return _uu.so3_uu_forward(plan, input1, input2, weight)
+        return _path.so3_uu_forward(plan, input1, input2, weight)
 
     @staticmethod
     def backward(ctx, grad):
@@ -180,7 +180,7 @@ class SO3LinearUU(Function):
         need = ctx.needs_input_grad[:3]
         grad = grad.contiguous()
         if not torch.is_grad_enabled() and grad.dtype == input1.dtype and grad.data_ptr() % 16 == 0:
-            return (*_uu.so3_uu_backward(ctx.plan, input1, input2, weight, grad, need), None, None)
+            return (*_path.so3_uu_backward(ctx.plan, input1, input2, weight, grad, need), None, None)
         f = ctx.infos[0]
         r1, r2 = _rot(ctx.infos)
         g1 = tensor_product_1uu(input2, grad, weight, *r1) if need[0] else None
@@ -318,6 +318,45 @@ def tensor_product_vu1(input1, input2, weight, tp_info_forward, tp_info_backward
 
 
 so3_linear_uv = tensor_product_u1v
+
+
+class SO3LinearUV(Function):
+    """:func:`tensor_product_u1v` with weights shared by the batch: rows of the intermediate from straight-line
+    Clebsch-Gordan blocks, the GEMM, and both operand gradients from one pass over the gradient of the rows.  A backward
+    pass that is itself differentiated is composed of the differentiable products instead."""
+
+    @staticmethod
+    def forward(ctx, input1, input2, weight, plan, mix, infos):
+        input1, input2, weight = input1.contiguous(), input2.contiguous(), weight.contiguous()
+        rows = _path.so3_uv_expand(plan, input1, input2)
+        out = mix.forward(rows, weight, "uv")
+        ctx.save_for_backward(input1, input2, weight, rows if ctx.needs_input_grad[2] else None)
+        ctx.plan, ctx.mix, ctx.infos = plan, mix, infos
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        input1, input2, weight, rows = ctx.saved_tensors
+        need = ctx.needs_input_grad[:3]
+        grad = grad.contiguous()
+        g1 = g2 = gw = None
+        if not torch.is_grad_enabled() and grad.dtype == torch.float32 and grad.data_ptr() % 16 == 0:
+            if need[2]:
+                gw = ctx.mix.grad_weight(rows, grad, weight, "uv")
+            if need[0] or need[1]:
+                g1, g2 = _path.so3_uv_backward(ctx.plan, input1, input2, ctx.mix.grad_inter(grad, weight, "uv"), need[:2])
+            return g1, g2, gw, None, None, None
+        f = ctx.infos[0]
+        r1, r2 = _rot(ctx.infos)
+        wt = weight.transpose(-1, -2).contiguous()
+        if need[0]:
+            g1 = tensor_product_1vu(input2, grad, wt, *r1)
+        if need[1]:
+            g2 = tensor_product_vu1(grad, input1, wt, *r2)
+        if need[2]:
+            inter = sparse_vecsca(input1, input2, *_mij(f, 0))
+            gw = sparse_outer(grad, inter, *_m(f, 2), out_accumulated=True).transpose(-1, -2).contiguous()
+        return g1, g2, gw, None, None, None
 
 
 # ------------------------------------------------------------------------------------------

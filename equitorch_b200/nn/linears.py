@@ -12,11 +12,12 @@ import torch
 from torch import Tensor
 
 from ..irreps import check_irreps
-from ..ops.so3_uu_op import PathPlan
+from ..ops.so3_path_op import PathPlan
 from ..tables import (generate_fully_connected_tp_paths, irreps_info, irreps_linear_infos, so2_linear_infos, so3_path_norms,
                       tp_infos)
 from ._base import _WeightedTableModule
-from .functional.linears import SO3LinearUU, irrep_wise_linear, irreps_linear, so3_linear_uu, so3_linear_uv
+from .functional.graph_tp import MixTables
+from .functional.linears import SO3LinearUU, SO3LinearUV, irrep_wise_linear, irreps_linear, so3_linear_uu, so3_linear_uv
 from .functional.sparse_product import sparse_mul, sparse_vecmat
 from .init import initialize_linear, initialize_so3_so2_linear
 
@@ -91,11 +92,14 @@ class SO3Linear(_WeightedTableModule):
         assert self.channels_in is None or input1.shape[-1] == self.channels_in, \
             f"Input1 channel dim mismatch: expected {self.channels_in}, got {input1.shape[-1]}"
         weight = self._resolve_weight(weight)
-        if self.feature_mode == "uu" and input1.is_cuda:
-            plan = self._path_plan(input1.device)
-            if plan is not None and plan.supported(input1, input2, weight):
-                return SO3LinearUU.apply(input1, input2, weight, plan,
-                                         (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2))
+        if input1.is_cuda:
+            plan, infos = self._path_plan(input1.device), (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2)
+            if plan is not None and self.feature_mode == "uu" and plan.supported(input1, input2, weight):
+                return SO3LinearUU.apply(input1, input2, weight, plan, infos)
+            if plan is not None and self.feature_mode == "uv" and plan.uv_supported(input1, input2, weight):
+                if plan.mix is None:
+                    plan.mix = MixTables(self.tp_info_forward, input1.device, [ir.dim for ir in self.irreps_out])
+                return SO3LinearUV.apply(input1, input2, weight, plan, plan.mix, infos)
         fn = so3_linear_uu if self.feature_mode == "uu" else so3_linear_uv
         return fn(input1, input2, weight, self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2)
 

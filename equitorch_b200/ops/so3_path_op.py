@@ -1,4 +1,5 @@
-"""Channel-wise ``SO3Linear`` in one kernel per direction (operator layer over ``eqt_so3_uu_*``)."""
+"""``SO3Linear`` on straight-line Clebsch-Gordan blocks: 'uu' in one kernel per direction, the channel-wise half of
+'uv' (operator layer over ``eqt_so3_uu_*`` / ``eqt_so3_uv_*``)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -11,7 +12,8 @@ from torch import Tensor
 from .. import _lib
 from ..csrc.gen_path_specs import MAX_L as PATH_MAX_L
 
-_PATH = np.dtype([("code", "<i4"), ("offset", "<i4"), ("offset_y", "<i4"), ("weight", "<i4"), ("scale", "<f4")])
+_PATH = np.dtype([("code", "<i4"), ("offset", "<i4"), ("offset_y", "<i4"), ("weight", "<i4"), ("scale", "<f4"),
+                  ("row", "<i4"), ("row_stride", "<i4")])
 _BLOCK = np.dtype([("l", "<i4"), ("offset", "<i4"), ("first", "<i4"), ("count", "<i4")])
 
 
@@ -20,19 +22,27 @@ class PathPlan:
     second operand irrep - and ``scales`` the factors on their Clebsch-Gordan blocks."""
 
     def __init__(self, paths: Sequence[Tuple[int, int, int]], scales: Sequence[float], irreps_out, irreps1, irreps2, device):
-        self.device, self._fits = torch.device(device), {}
+        self.device, self._fits, self.mix = torch.device(device), {}, None      # mix: tables of the weight step ('uv')
         ls = [[ir.l for ir in irs] for irs in (irreps_out, irreps1, irreps2)]
         self.usable = len(paths) > 0 and all(0 <= l <= PATH_MAX_L for degrees in ls for l in degrees)
         if not self.usable:
             return
         start = [np.cumsum([0] + [2 * l + 1 for l in degrees]).tolist() for degrees in ls]
+        # rows of the intermediate: per output irrep, component by component, its paths ordered by (i, j, weight)
+        row, fan, num_rows = {}, {}, 0
+        for k, l in enumerate(ls[0]):
+            mine = sorted((w for w in range(len(paths)) if paths[w][0] == k), key=lambda w: (paths[w][1], paths[w][2], w))
+            row.update((w, num_rows + n) for n, w in enumerate(mine))
+            fan[k] = len(mine)
+            num_rows += len(mine) * (2 * l + 1)
         parts = []
         for key, other in ((0, 1), (1, 0)):
             order = sorted(range(len(paths)), key=lambda w: paths[w][key])
             parts.append(np.array([(4 * ls[other][paths[w][other]] + ls[2][paths[w][2]], start[other][paths[w][other]],
-                                    start[2][paths[w][2]], w, scales[w]) for w in order], dtype=_PATH))
+                                    start[2][paths[w][2]], w, scales[w], row[w], fan[paths[w][0]]) for w in order], dtype=_PATH))
             first = np.searchsorted([paths[w][key] for w in order], np.arange(len(ls[key]) + 1)).tolist()
             parts.append(np.array([(l, start[key][n], first[n], first[n + 1] - first[n]) for n, l in enumerate(ls[key])], dtype=_BLOCK))
+        parts.append(np.array([row[w] + m * fan[paths[w][0]] for w in order for m in range(2 * ls[0][paths[w][0]] + 1)], dtype=np.int32))
         # one upload: the parts back to back, each on a 16-byte boundary
         blob, at, size = [], [], 0
         for part in parts:
@@ -43,8 +53,9 @@ class PathPlan:
         self.blob = torch.frombuffer(bytearray(b"".join(blob)), dtype=torch.uint8).to(device)
         base = self.blob.data_ptr()
         self.sizes = (start[1][-1], start[2][-1], start[0][-1], len(paths))
-        self.struct = _lib.PathTableStruct(base + at[1], base + at[3], base + at[0], base + at[2], *self.sizes, len(paths),
-                                           len(ls[0]), len(ls[1]))
+        self.num_rows = num_rows
+        self.struct = _lib.PathTableStruct(base + at[1], base + at[3], base + at[0], base + at[2], base + at[4], *self.sizes,
+                                           len(paths), len(ls[0]), len(ls[1]), num_rows)
         self.ref = C.byref(self.struct)
 
     def supported(self, x: Tensor, y: Tensor, w: Tensor) -> bool:
@@ -59,6 +70,40 @@ class PathPlan:
             self._fits[key] = all(_lib.lib().eqt_so3_uu_scratch_floats(self.ref, n, x.shape[2], int(w.ndim == 3),
                                                                        _lib.DTYPE_CODE[x.dtype]) >= 0 for n in (1, 1 << 30))
         return self._fits[key] and (x.data_ptr() | w.data_ptr()) % 16 == 0
+
+
+    def uv_supported(self, x: Tensor, y: Tensor, w: Tensor) -> bool:
+        """Whether the channel-wise kernels of the 'uv' layer take these operands (float32, weights shared by the batch)."""
+        if not (self.usable and x.is_cuda and x.dtype == torch.float32 and x.dtype == y.dtype == w.dtype
+                and x.ndim == 3 and y.ndim == 2 and x.shape[0] == y.shape[0] and x.shape[0] > 0 and w.ndim == 3
+                and x.shape[2] == w.shape[1] and x.shape[1] == self.sizes[0] and y.shape[1] == self.sizes[1]
+                and w.shape[0] == self.sizes[3] and y.device == x.device == w.device == self.device):
+            return False
+        key = ("uv", x.shape[2])
+        if key not in self._fits:
+            self._fits[key] = bool(_lib.lib().eqt_so3_uv_supported(self.ref, x.shape[2]))
+        return self._fits[key] and (x.data_ptr() | w.data_ptr()) % 16 == 0
+
+
+def so3_uv_expand(plan: PathPlan, x: Tensor, y: Tensor) -> Tensor:
+    """``rows[n, r, c]``: the entries of (output component, path) row r contracted with x and y; contiguous float32."""
+    n, _, c = x.shape
+    rows = torch.empty(n, plan.num_rows, c, dtype=torch.float32, device=x.device)
+    with _lib.on_device(x.device):
+        _lib.check(_lib.lib().eqt_so3_uv_expand(plan.ref, x.data_ptr(), y.data_ptr(), rows.data_ptr(), n, c, _lib.stream_ptr(x.device)),
+                   "eqt_so3_uv_expand")
+    return rows
+
+
+def so3_uv_backward(plan: PathPlan, x: Tensor, y: Tensor, grad_rows: Tensor,
+                    need: Tuple[bool, bool]) -> Tuple[Optional[Tensor], Optional[Tensor]]:
+    """Gradients of :func:`so3_uv_expand` with respect to x and y, from one pass over ``grad_rows``."""
+    n, _, c = x.shape
+    gx, gy = (torch.empty_like(t) if wanted else None for t, wanted in zip((x, y), need))
+    with _lib.on_device(x.device):
+        _lib.check(_lib.lib().eqt_so3_uv_backward(plan.ref, x.data_ptr(), y.data_ptr(), grad_rows.data_ptr(), _lib.ptr(gx), _lib.ptr(gy),
+                                                  n, c, _lib.stream_ptr(x.device)), "eqt_so3_uv_backward")
+    return gx, gy
 
 
 def so3_uu_forward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor) -> Tensor:

@@ -335,6 +335,7 @@ typedef struct eqt_path {
   int32_t offset_y;    /* first component of its y irrep                                    */
   int32_t weight;
   float scale;         /* factor on the Clebsch-Gordan values                               */
+  int32_t row, row_stride; /* row of the intermediate for component M of the output irrep: row + M row_stride */
 } eqt_path;
 typedef struct eqt_path_block {
   int32_t l, offset;   /* degree and first component of the block's irrep                   */
@@ -345,7 +346,8 @@ typedef struct eqt_path_table {
   const eqt_path_block* bwd_blocks;
   const eqt_path* fwd_paths;
   const eqt_path* bwd_paths;
-  int32_t d1, d2, d_out, num_weights, num_paths, num_fwd_blocks, num_bwd_blocks;
+  const int32_t* bwd_rows;   /* (num_rows) rows of the intermediate in backward path order   */
+  int32_t d1, d2, d_out, num_weights, num_paths, num_fwd_blocks, num_bwd_blocks, num_rows;
 } eqt_path_table;
 int64_t eqt_so3_uu_scratch_floats(const eqt_path_table* table, int64_t n, int32_t channels, int32_t per_sample_weight,
                                   int32_t dtype);
@@ -354,6 +356,21 @@ int eqt_so3_uu_forward(const eqt_path_table* table, const void* x, const void* y
 int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, const void* y, const void* w, const void* g, void* gx,
                         void* gy, void* gw, float* scratch, int64_t scratch_floats, int64_t n, int32_t channels,
                         int32_t per_sample_weight, int32_t dtype, void* stream);
+
+/*
+ * The channel-wise half of the layer with full channel mixing ('uv' SO3Linear), float32, same tables:
+ *   expand:   rows[n, r, c] = sum_t s_t x[n, M1_t, c] y[n, M2_t] over the entries of row r = (output component, path)
+ *   backward: gx and gy from the gradient of the rows, in one pass over it
+ * rows / grad_rows (n, num_rows, c); gx (n, d1, c) and gy (n, d2) may be NULL.  eqt_so3_uv_supported: 1 if this many
+ * channels fit.
+ * replaces: the vec-scalar step of TensorProductU1V and the three-step TensorProductVU1 adjoint
+ *   (equitorch/nn/functional/linears.py:254-336, 415-492).
+ */
+int eqt_so3_uv_supported(const eqt_path_table* table, int32_t channels);
+int eqt_so3_uv_expand(const eqt_path_table* table, const float* x, const float* y, float* rows, int64_t n,
+                      int32_t channels, void* stream);
+int eqt_so3_uv_backward(const eqt_path_table* table, const float* x, const float* y, const float* grad_rows, float* gx,
+                        float* gy, int64_t n, int32_t channels, void* stream);
 
 /*
  * Gather, lay out and split shared weights w (num_paths, cin, cout) for the tensor-core entry points:

@@ -1,4 +1,4 @@
-"""``SO3Linear`` 'uu' through the one-pass kernels against the dense float64 oracle: channel counts that give 1 to 64
+"""``SO3Linear`` through the kernels on straight-line Clebsch-Gordan blocks ('uu': one pass per direction) against the dense float64 oracle: channel counts that give 1 to 64
 threads per sample (powers of two and not), batches from one sample (output irreps spread over the grid, smaller
 blocks) to several waves, degrees 0 to 3 with even and odd degree sums, shared and per-sample weights, float32 and bfloat16; and a differentiated
 backward pass against the composed products."""
@@ -9,7 +9,7 @@ import torch
 
 from equitorch_b200 import _lib
 from equitorch_b200 import nn as enn
-from equitorch_b200.nn.functional.linears import tensor_product_u1u
+from equitorch_b200.nn.functional.linears import tensor_product_u1u, tensor_product_u1v
 from oracle import tensor_products as otp
 
 pytestmark = pytest.mark.gpu
@@ -49,17 +49,43 @@ def test_one_pass_kernels(ir, ir_y, n, c, per_sample, dtype):
     assert torch.equal(gy, got[2])
 
 
-def test_differentiated_backward_pass():
+@pytest.mark.parametrize("ir,ir_y,n,c,c_out", [("0e+1o", "0e+1o", 1, 4, 8), ("0e+1o+2e", "0e+1o+2e", 7, 12, 20),
+                                               ("0e+1o+2e+3o", "0e+1o+2e+3o", 513, 64, 32), ("4x0e+2x1o+2e", "0e+1o+2e", 1501, 32, 64),
+                                               ("0o+1e+2e+3e", "0e+1e+2o+3e", 300, 16, 16), ("0e+1o+2e+3o", "0e+1o+2e+3o", 2003, 128, 48)])
+def test_channel_mixing_layer(ir, ir_y, n, c, c_out):
+    """'uv' through the row kernels: every degree triple, channel counts with and without a tensor-core GEMM."""
+    g = torch.Generator().manual_seed(n + c)
+    layer = enn.SO3Linear(ir, ir_y, ir, c, c_out, internal_weights=False, feature_mode="uv").to(DEV)
+    dim, dim_y, p = layer.irreps_in1_dim, layer.irreps_in2_dim, layer.num_paths
+    x, y, cot = torch.randn(n, dim, c, generator=g), torch.randn(n, dim_y, generator=g), torch.randn(n, dim, c_out, generator=g)
+    w = torch.randn(p, c, c_out, generator=g) / c ** 0.5
+    xo, yo, wo = (t.double().requires_grad_(True) for t in (x, y, w))
+    want = otp.so3_linear_dense(xo, yo, wo, ir, ir_y, ir, feature_mode="uv")
+    want = [want, *torch.autograd.grad(want, [xo, yo, wo], cot.double())]
+    xg, yg, wg = (t.to(DEV).requires_grad_(True) for t in (x, y, w))
+    assert layer._path_plan(xg.device).uv_supported(xg, yg, wg)
+    got = layer(xg, yg, wg)
+    got = [got, *torch.autograd.grad(got, [xg, yg, wg], cot.to(DEV))]
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and _rel(a, b) < BOUND[torch.float32]
+    (gy,) = torch.autograd.grad(layer(xg.detach(), yg, wg.detach()), [yg], cot.to(DEV))
+    assert torch.equal(gy, got[2])
+
+
+@pytest.mark.parametrize("mode", ["uu", "uv"])
+def test_differentiated_backward_pass(mode):
     g = torch.Generator().manual_seed(0)
     ir, n, c = "0e+1o+2e", 33, 8
-    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode="uu").to(DEV)
+    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode=mode).to(DEV)
+    weight = torch.randn(*layer.weight_shape, generator=g)
     leaves = [t.to(DEV).requires_grad_(True) for t in (torch.randn(n, 9, c, generator=g), torch.randn(n, 9, generator=g),
-                                                       torch.randn(11, c, generator=g), torch.randn(n, 9, c, generator=g))]
+                                                       weight, torch.randn(n, 9, c, generator=g))]
+    product = tensor_product_u1u if mode == "uu" else tensor_product_u1v
     infos = (layer.tp_info_forward, layer.tp_info_backward1, layer.tp_info_backward2)
 
     def second(fn):
         x, y, w, cot = leaves
         first = torch.autograd.grad(fn(x, y, w), [x, y, w], cot, create_graph=True)
         return torch.autograd.grad(sum((t * t).sum() for t in first), leaves)
-    for a, b in zip(second(layer), second(lambda x, y, w: tensor_product_u1u(x, y, w, *infos))):
+    for a, b in zip(second(layer), second(lambda x, y, w: product(x, y, w, *infos))):
         assert _rel(a, b.cpu()) < 1e-5
