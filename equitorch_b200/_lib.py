@@ -139,6 +139,13 @@ SIGNATURES = {
                                   C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
     "eqt_irrep_dot": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,
                                 C.c_int32, C.c_int32, C.c_void_p]),
+    "eqt_irrep_scale_backward": (C.c_int, [C.c_void_p] * 6 + [C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
+    "eqt_batch_rms_scratch": (C.c_int64, [C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "eqt_batch_rms_forward": (C.c_int, [C.c_void_p] * 5 + [C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,
+                                                           C.c_int32, C.c_int32, C.c_double, C.c_int32, C.c_void_p]),
+    "eqt_batch_rms_backward": (C.c_int, [C.c_void_p] * 7 + [C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,
+                                                            C.c_int32, C.c_int32, C.c_double, C.c_int32, C.c_void_p]),
+    "eqt_row_sum": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p]),
     "eqt_layer_rms_num_partials": (C.c_int, [C.c_int64]),
     "eqt_layer_rms_forward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32,
                                         C.c_int32, C.c_int32, C.c_int32, C.c_double, C.c_int32, C.c_void_p]),

@@ -7,6 +7,7 @@ Each gradient is again one of the two operators, so derivatives of any order are
 """
 from __future__ import annotations
 
+import torch
 from torch import Tensor
 from torch.autograd import Function
 
@@ -25,6 +26,8 @@ class IrrepScale(Function):
     def backward(ctx, grad: Tensor):
         x, s = ctx.saved_tensors
         gx = gs = None
+        if ctx.mode == _ops.PER_SAMPLE_CHANNEL and all(ctx.needs_input_grad[:2]) and not torch.is_grad_enabled():
+            return (*_ops.irrep_scale_backward(x, s, grad, ctx.info.irrep_seg), None, None)    # first derivatives only
         if ctx.needs_input_grad[0]:
             gx = IrrepScale.apply(grad, s, ctx.info, ctx.mode)
         if ctx.needs_input_grad[1]:

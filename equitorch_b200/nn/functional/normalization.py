@@ -12,8 +12,37 @@ from torch.autograd.function import once_differentiable
 from ...ops import irrep_ops as _iops
 from ...ops.irrep_ops import PER_SAMPLE, SHARED
 from ...structs import IrrepsInfo
-from ._irrep import irrep_scale
+from ._irrep import irrep_dot, irrep_scale
 from .norm import batch_mean_squared_norm, channel_mean_squared_norm
+
+
+class _BatchRMSNormFused(Function):
+    """Training-mode BatchRMSNorm: column sums, fold and one streaming pass per direction.  Returns (out, stat)."""
+
+    @staticmethod
+    def forward(ctx, x: Tensor, weight: Optional[Tensor], info: IrrepsInfo, scaled: bool, eps: float):
+        out, stat = _iops.batch_rms_forward(x, weight, info.irrep_seg, info.irrep_index, scaled, eps)
+        ctx.save_for_backward(x, weight, stat)
+        ctx.info, ctx.scaled, ctx.eps = info, scaled, eps
+        ctx.mark_non_differentiable(stat)
+        return out, stat
+
+    @staticmethod
+    def backward(ctx, grad: Tensor, _):
+        x, weight, stat = ctx.saved_tensors
+        need_x, need_w = ctx.needs_input_grad[0], weight is not None and ctx.needs_input_grad[1]
+        if not torch.is_grad_enabled():
+            return (*_iops.batch_rms_backward(x, grad, weight, stat, ctx.info.irrep_seg, ctx.info.irrep_index, ctx.scaled, ctx.eps,
+                                              need_x, need_w), None, None, None)
+        # higher derivatives: the same gradients from differentiable per-irrep operators
+        r = torch.rsqrt(batch_mean_squared_norm(x, ctx.info, ctx.scaled) + ctx.eps)
+        q = irrep_dot(grad, x, ctx.info).sum(dim=0)
+        wr = r if weight is None else weight * r
+        coef = q * wr * r * r / x.shape[0]
+        if ctx.scaled:
+            coef = coef * ctx.info.rdims.unsqueeze(-1)
+        gx = irrep_scale(grad, wr, ctx.info, SHARED) - irrep_scale(x, coef.to(x.dtype), ctx.info, SHARED) if need_x else None
+        return gx, (q * r if need_w else None), None, None, None
 
 
 def batch_rms_norm(input: Tensor, running_squared_norm: Tensor, irreps_info: IrrepsInfo, weight: Optional[Tensor] = None,
@@ -21,6 +50,10 @@ def batch_rms_norm(input: Tensor, running_squared_norm: Tensor, irreps_info: Irr
     """``out[n, i, c] = x[n, i, c] * weight[k, c] / sqrt(stat[k, c] + eps)``, ``k = irrep(i)``; ``stat`` is the
     batch mean of the (scaled) squared norms when training (``running_squared_norm`` is updated in place),
     else ``running_squared_norm``."""
+    if training and _iops.batch_rms_supported(input, weight):
+        out, stat = _BatchRMSNormFused.apply(input, weight, irreps_info, scaled, eps)
+        running_squared_norm.data.lerp_(stat.to(running_squared_norm.dtype), momentum)
+        return out
     if training:
         stat = batch_mean_squared_norm(input, irreps_info, scaled)
         running_squared_norm.data.lerp_(stat.detach().to(running_squared_norm.dtype), momentum)

@@ -53,6 +53,80 @@ def irrep_dot(a: Tensor, b: Tensor, irrep_seg: Tensor) -> Tensor:
     return out
 
 
+def irrep_scale_backward(x: Tensor, s: Tensor, grad: Tensor, irrep_seg: Tensor):
+    """Gradients of ``irrep_scale(x, s, .., PER_SAMPLE_CHANNEL)`` with respect to ``x`` and ``s`` in one pass over ``grad``."""
+    _check(grad)
+    dev = _lib.require_cuda(x, s, grad, irrep_seg)
+    if x.shape != grad.shape or x.dtype != grad.dtype:
+        raise ValueError("features and gradient must have the same shape and dtype")
+    x, s, grad = x.contiguous(), s.to(x.dtype).contiguous(), grad.contiguous()
+    n, d, c = x.shape
+    k = irrep_seg.numel() - 1
+    if tuple(s.shape) != (n, k, c):
+        raise ValueError(f"scale operand must be {(n, k, c)}, got {tuple(s.shape)}")
+    gx, gs = torch.empty_like(x), torch.empty_like(s)
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().eqt_irrep_scale_backward(x.data_ptr(), s.data_ptr(), grad.data_ptr(), gx.data_ptr(), gs.data_ptr(),
+                                                       irrep_seg.data_ptr(), n, d, k, c, _lib.DTYPE_CODE[x.dtype],
+                                                       _lib.stream_ptr(dev)), "eqt_irrep_scale_backward")
+    return gx, gs
+
+
+def batch_rms_supported(x: Tensor, weight) -> bool:
+    """Whether the fused BatchRMSNorm (training mode) takes these operands."""
+    return (x.is_cuda and x.ndim == 3 and x.dtype in (torch.float32, torch.float64) and x.shape[0] > 0 and x.shape[2] > 0
+            and x.shape[1] <= 1024 and (weight is None or weight.dtype == x.dtype))
+
+
+def _batch_rms_scratch(x: Tensor, k: int) -> Tensor:
+    n, d, c = x.shape
+    return torch.empty(_lib.lib().eqt_batch_rms_scratch(n, d, k, c, _lib.DTYPE_CODE[x.dtype]), dtype=x.dtype, device=x.device)
+
+
+def _batch_weight(weight, k: int, c: int):
+    if weight is not None and tuple(weight.shape) != (k, c):
+        raise ValueError(f"weight must be {(k, c)}, got {tuple(weight.shape)}")
+    return None if weight is None else weight.contiguous()
+
+
+def batch_rms_forward(x: Tensor, weight, irrep_seg: Tensor, irrep_index: Tensor, scaled: bool, eps: float):
+    """Returns (out, stat (K, C)): ``stat`` is the batch mean of the (scaled) squared norms."""
+    _check(x)
+    dev = _lib.require_cuda(x, weight, irrep_seg, irrep_index)
+    n, d, c = x.shape
+    k = irrep_seg.numel() - 1
+    x, w = x.contiguous(), _batch_weight(weight, k, c)
+    out = torch.empty_like(x)
+    stat = torch.empty(k, c, dtype=x.dtype, device=dev)
+    with _lib.on_device(dev):
+        scratch = _batch_rms_scratch(x, k)
+        _lib.check(_lib.lib().eqt_batch_rms_forward(x.data_ptr(), _lib.ptr(w), out.data_ptr(), stat.data_ptr(), scratch.data_ptr(),
+                                                    scratch.numel(), irrep_seg.data_ptr(), irrep_index.data_ptr(), n, d, k, c,
+                                                    int(scaled), float(eps), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)),
+                   "eqt_batch_rms_forward")
+    return out, stat
+
+
+def batch_rms_backward(x: Tensor, grad_out: Tensor, weight, stat: Tensor, irrep_seg: Tensor, irrep_index: Tensor, scaled: bool,
+                       eps: float, need_x: bool, need_weight: bool):
+    """Returns (grad_x or None, grad_weight or None)."""
+    dev = _lib.require_cuda(x, grad_out, weight, stat, irrep_seg, irrep_index)
+    if x.shape != grad_out.shape or x.dtype != grad_out.dtype:
+        raise ValueError("features and gradient must have the same shape and dtype")
+    n, d, c = x.shape
+    k = irrep_seg.numel() - 1
+    x, grad_out, w = x.contiguous(), grad_out.contiguous(), _batch_weight(weight, k, c)
+    gx = torch.empty_like(x) if need_x else None
+    gw = torch.empty(k, c, dtype=x.dtype, device=dev) if need_weight else None
+    with _lib.on_device(dev):
+        scratch = _batch_rms_scratch(x, k)
+        _lib.check(_lib.lib().eqt_batch_rms_backward(x.data_ptr(), grad_out.data_ptr(), _lib.ptr(w), stat.data_ptr(), _lib.ptr(gx),
+                                                     _lib.ptr(gw), scratch.data_ptr(), scratch.numel(), irrep_seg.data_ptr(),
+                                                     irrep_index.data_ptr(), n, d, k, c, int(scaled), float(eps),
+                                                     _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)), "eqt_batch_rms_backward")
+    return gx, gw
+
+
 def layer_rms_supported(x: Tensor, num_irreps: int) -> bool:
     """Whether the fused LayerRMSNorm kernels take this input."""
     if not (x.is_cuda and x.ndim == 3 and x.dtype in (torch.float32, torch.float64)):
@@ -87,7 +161,7 @@ def layer_rms_backward(x: Tensor, grad_out: Tensor, weight, rsigma: Tensor, irre
     n, d, c = x.shape
     k = irrep_seg.numel() - 1
     gx = torch.empty_like(x)
-    partial = None
+    partial = gw = None
     if need_weight_grad:
         partial = torch.empty(_lib.lib().eqt_layer_rms_num_partials(n), k, c, dtype=x.dtype, device=dev)
     with _lib.on_device(dev):
@@ -95,4 +169,10 @@ def layer_rms_backward(x: Tensor, grad_out: Tensor, weight, rsigma: Tensor, irre
                                                      gx.data_ptr(), _lib.ptr(partial), irrep_seg.data_ptr(), n, d, k, c,
                                                      int(scaled), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)),
                    "eqt_layer_rms_backward")
-    return gx, (None if partial is None else partial.sum(dim=0))
+        if need_weight_grad and n > 0:
+            gw = torch.empty(k, c, dtype=x.dtype, device=dev)
+            _lib.check(_lib.lib().eqt_row_sum(partial.data_ptr(), gw.data_ptr(), partial.shape[0], k * c, _lib.DTYPE_CODE[x.dtype],
+                                              _lib.stream_ptr(dev)), "eqt_row_sum")
+        elif need_weight_grad:
+            gw = torch.zeros(k, c, dtype=x.dtype, device=dev)
+    return gx, gw

@@ -407,16 +407,42 @@ int eqt_irrep_dot(const void* a, const void* b, void* out, const int64_t* irrep_
                   int32_t k, int32_t c, int32_t dtype, void* stream);
 
 /*
+ * Both gradients of eqt_irrep_scale with s_mode 0 in one pass over the gradient g of its output:
+ *   gx[n, i, c] = g[n, i, c] * s[n, irrep(i), c],   gs[n, k, c] = sum_{i in irrep k} g[n, i, c] * x[n, i, c]
+ * replaces: the backward pass of gating, equitorch/nn/functional/activations.py:31-36.
+ */
+int eqt_irrep_scale_backward(const void* x, const void* s, const void* g, void* gx, void* gs, const int64_t* irrep_seg,
+                             int64_t n, int32_t d, int32_t k, int32_t c, int32_t dtype, void* stream);
+
+/*
+ * BatchRMSNorm with the statistics of the batch (float32 / float64, n >= 1):
+ *   stat[k, c] = mean_n sum_{i in k} x[n, i, c]^2 (/ dim_k if scaled)
+ *   out[n, i, c] = x[n, i, c] * weight[k(i), c] * (stat[k(i), c] + eps)^-1/2          (weight may be NULL)
+ * and its backward from x, stat and the gradient of out (the statistics depend on x); grad_x and grad_weight may be NULL.
+ * scratch: eqt_batch_rms_scratch(...) elements of the tensors' type, 16-byte aligned; contents need not survive the call.
+ * replaces: batch_rms_norm in training mode, equitorch/nn/functional/normalization.py:8-63.
+ */
+int64_t eqt_batch_rms_scratch(int64_t n, int32_t d, int32_t k, int32_t c, int32_t dtype);
+int eqt_batch_rms_forward(const void* x, const void* weight, void* out, void* stat, void* scratch, int64_t scratch_size,
+                          const int64_t* irrep_seg, const int64_t* irrep_index, int64_t n, int32_t d, int32_t k, int32_t c,
+                          int32_t scaled, double eps, int32_t dtype, void* stream);
+int eqt_batch_rms_backward(const void* x, const void* grad_out, const void* weight, const void* stat, void* grad_x,
+                           void* grad_weight, void* scratch, int64_t scratch_size, const int64_t* irrep_seg,
+                           const int64_t* irrep_index, int64_t n, int32_t d, int32_t k, int32_t c, int32_t scaled, double eps,
+                           int32_t dtype, void* stream);
+
+/*
  * Fused LayerRMSNorm (float32 / float64): per sample n and irrep k
  *   rsigma[n, k] = (mean_c sum_{i in k} x[n, i, c]^2 (/ dim_k if scaled) + eps)^-1/2
  *   out[n, i, c] = x[n, i, c] * rsigma[n, k(i)] * weight[k(i), c]            (weight may be NULL)
- * in one pass (one warp per sample), and its backward: grad_x, plus per-warp partial sums of grad_weight,
+ * in one pass (one warp per sample), and its backward: grad_x, plus per-block partial sums of grad_weight,
  * grad_weight_partial (eqt_layer_rms_num_partials(n), k, c), which the caller sums over the first dimension
  * (NULL = not wanted).  Needs k <= 16, C / 4 (float32) or C / 2 (float64) dividing 32, 16-byte aligned tensors;
  * EQT_ERR_UNSUPPORTED otherwise.
  * replaces: layer_rms_norm, equitorch/nn/functional/normalization.py:112-160 (channel_mean_squared_norm,
  * sparse_vecsca, sparse_mul and their backward passes).
  */
+int eqt_row_sum(const void* in, void* out, int64_t rows, int64_t cols, int32_t dtype, void* stream); /* sum over the rows of (rows, cols) */
 int eqt_layer_rms_num_partials(int64_t n);
 int eqt_layer_rms_forward(const void* x, const void* weight, void* out, void* rsigma, const int64_t* irrep_seg,
                           int64_t n, int32_t d, int32_t k, int32_t c, int32_t scaled, double eps, int32_t dtype,
