@@ -112,6 +112,11 @@ SIGNATURES = {
                                      C.c_int32, C.c_void_p]),
     "eqt_dense_rotation_grad_matrix": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p,
                                                  C.c_int32, C.c_void_p]),
+    "eqt_block_rotation_supported": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
+    "eqt_block_rotation": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
+                                     C.c_void_p]),
+    "eqt_block_rotation_grad_matrix": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_int32,
+                                                 C.c_void_p]),
     "eqt_vecmat_tc": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                 C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
                                 C.c_void_p]),

@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "wigner_blocks.cuh"
 
 namespace eqt {
 namespace {
@@ -443,6 +444,11 @@ extern "C" int eqt_wigner_d_forward(const eqt_wigner_table* table, const void* a
   a.coef = table->coef; a.comp = table->comp; a.alpha = alpha; a.beta = beta; a.gamma = gamma; a.d = d; a.n = n;
   a.dim = table->dim; a.max_l = table->max_l; a.coef_count = table->coef_count;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == EQT_F32) {
+    const int rc = wigner_quads_forward(table, static_cast<const float*>(alpha), static_cast<const float*>(beta),
+                                        static_cast<const float*>(gamma), static_cast<float*>(d), n, st);
+    if (rc != NOT_TAKEN) return rc;
+  }
   return dtype == EQT_F32 ? wig_launch<float>(false, table, a, st) : wig_launch<double>(false, table, a, st);
 }
 
@@ -459,6 +465,13 @@ extern "C" int eqt_wigner_d_backward(const eqt_wigner_table* table, const void* 
   a.d = const_cast<void*>(grad_d); a.ga = grad_alpha; a.gb = grad_beta; a.gc = grad_gamma; a.n = n;
   a.dim = table->dim; a.max_l = table->max_l; a.coef_count = table->coef_count;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == EQT_F32) {
+    const int rc = wigner_quads_backward(table, static_cast<const float*>(alpha), static_cast<const float*>(beta),
+                                         static_cast<const float*>(gamma), static_cast<const float*>(grad_d),
+                                         static_cast<float*>(grad_alpha), static_cast<float*>(grad_beta),
+                                         static_cast<float*>(grad_gamma), n, st);
+    if (rc != NOT_TAKEN) return rc;
+  }
   return dtype == EQT_F32 ? wig_launch<float>(true, table, a, st) : wig_launch<double>(true, table, a, st);
 }
 

@@ -35,7 +35,7 @@ def sparse_wigner_rotation(input: Tensor, sincos_alpha: Optional[Tensor], sincos
 
 class _DenseRotation(torch.autograd.Function):
     """``matrix (N, D, D) @ x (N, D, C)`` (``transposed``: ``matrix^T @ x``) on the shared-memory kernels.
-    ``row_range``: the matrices are block diagonal (see ``ops.wigner_op.block_row_range``)."""
+    ``row_range``: the matrices are block diagonal (``ops.wigner_op.block_row_range`` or ``block_diagonal``)."""
 
     @staticmethod
     def forward(ctx, x: Tensor, matrix: Tensor, transposed: bool, row_range):
@@ -75,7 +75,7 @@ class _RotationGradMatrix(torch.autograd.Function):
         return ga, gb, None
 
 
-def dense_wigner_rotation(input: Tensor, wigner_d: Tensor, row_range: Optional[Tensor] = None) -> Tensor:
+def dense_wigner_rotation(input: Tensor, wigner_d: Tensor, row_range=None) -> Tensor:
     """``wigner_d (N, dim, dim) @ input (N, dim, C)``.  A ``wigner_d`` that is the transposed view of a contiguous
     tensor (``d.transpose(-1, -2)``, the inverse rotation) is applied without materialising the transpose.
     ``row_range`` declares the matrices block diagonal over the irreps: only the blocks are read and multiplied, and

@@ -49,8 +49,8 @@ class DenseWignerRotation(nn.Module):
     def forward(self, input: Tensor, wigner_d: Tensor) -> Tensor:
         row_range = None
         if self.block_diagonal and input.is_cuda and wigner_d.shape[-1] == self.irreps.dim:
-            from ..ops.wigner_op import block_row_range
-            row_range = block_row_range(self.irreps, input.device)
+            from ..ops.wigner_op import block_diagonal
+            row_range = block_diagonal(self.irreps, input.device)
         return dense_wigner_rotation(input, wigner_d, row_range)
 
     def extra_repr(self) -> str:

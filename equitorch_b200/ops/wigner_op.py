@@ -113,26 +113,63 @@ def block_row_range(irreps: Irreps, device) -> Tensor:
     return _row_ranges[key]
 
 
-def dense_rotation(matrix: Tensor, x: Tensor, transposed: bool = False, row_range: Tensor = None) -> Tensor:
+class BlockDiagonal:
+    """Diagonal block structure of a matrix: the row ranges on the device and the block sizes on the host."""
+
+    def __init__(self, irreps: Irreps, device):
+        self.row_range = block_row_range(irreps, device)
+        self.sizes = (C.c_int32 * len(irreps))(*[ir.dim for ir in irreps])
+
+    def takes(self, *features: Tensor) -> bool:
+        """Whether the float32 block kernels take these (N, dim, C) features."""
+        return (all(x.dtype == torch.float32 and x.data_ptr() % 16 == 0 for x in features)
+                and bool(_lib.lib().eqt_block_rotation_supported(self.sizes, len(self.sizes), features[0].shape[2])))
+
+
+_blocks: Dict[Tuple, BlockDiagonal] = {}
+
+
+def block_diagonal(irreps: Irreps, device) -> BlockDiagonal:
+    key = (tuple(ir.dim for ir in irreps), torch.device(device))
+    if key not in _blocks:
+        _blocks[key] = BlockDiagonal(irreps, device)
+    return _blocks[key]
+
+
+def dense_rotation(matrix: Tensor, x: Tensor, transposed: bool = False, row_range=None) -> Tensor:
     """``out[n] = matrix[n] @ x[n]`` (or ``matrix[n].T @ x[n]``); matrix (N, D, D), x (N, D, C), contiguous.
-    ``row_range`` (see :func:`block_row_range`): the matrices are block diagonal, entries outside the blocks are
-    neither read nor multiplied."""
+    ``row_range`` (see :func:`block_row_range`, :func:`block_diagonal`): the matrices are block diagonal, entries outside
+    the blocks are neither read nor multiplied."""
     dev = _lib.require_cuda(matrix, x)
     n, d, c = x.shape
     out = torch.empty_like(x)
     with _lib.on_device(dev):
+        if isinstance(row_range, BlockDiagonal):
+            if matrix.dtype == x.dtype and row_range.takes(x, out):
+                _lib.check(_lib.lib().eqt_block_rotation(matrix.data_ptr(), x.data_ptr(), out.data_ptr(), n, row_range.sizes,
+                                                         len(row_range.sizes), c, int(transposed), _lib.stream_ptr(dev)),
+                           "eqt_block_rotation")
+                return out
+            row_range = row_range.row_range
         _lib.check(_lib.lib().eqt_dense_rotation(matrix.data_ptr(), x.data_ptr(), out.data_ptr(), n, d, c, int(transposed),
                                                  _lib.ptr(row_range), _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(dev)),
                    "eqt_dense_rotation")
     return out
 
 
-def dense_rotation_grad_matrix(grad_out: Tensor, x: Tensor, row_range: Tensor = None) -> Tensor:
+def dense_rotation_grad_matrix(grad_out: Tensor, x: Tensor, row_range=None) -> Tensor:
     """``grad_matrix[n] = grad_out[n] @ x[n].T`` (with ``row_range``: zero outside the diagonal blocks)."""
     dev = _lib.require_cuda(grad_out, x)
     n, d, c = x.shape
     gm = torch.empty(n, d, d, dtype=x.dtype, device=dev)
     with _lib.on_device(dev):
+        if isinstance(row_range, BlockDiagonal):
+            if grad_out.dtype == x.dtype and row_range.takes(x, grad_out):
+                _lib.check(_lib.lib().eqt_block_rotation_grad_matrix(grad_out.data_ptr(), x.data_ptr(), gm.data_ptr(), n,
+                                                                     row_range.sizes, len(row_range.sizes), c,
+                                                                     _lib.stream_ptr(dev)), "eqt_block_rotation_grad_matrix")
+                return gm
+            row_range = row_range.row_range
         _lib.check(_lib.lib().eqt_dense_rotation_grad_matrix(grad_out.data_ptr(), x.data_ptr(), gm.data_ptr(), n, d, c,
                                                              _lib.ptr(row_range), _lib.DTYPE_CODE[x.dtype],
                                                              _lib.stream_ptr(dev)),

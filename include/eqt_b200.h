@@ -489,6 +489,17 @@ int eqt_dense_rotation_grad_matrix(const void* grad_out, const void* x, void* gr
                                    int32_t channels, const int32_t* row_range, int32_t dtype, void* stream);
 
 /*
+ * The same two operations for float32 matrices that are block diagonal with the given block sizes (host array, in order; their
+ * sum is the matrix size): only the blocks are read and multiplied, grad_matrix is zero outside them.  channels a multiple of
+ * 4, x / out / grad_out 16-byte aligned.  eqt_block_rotation_supported: 1 if blocks and channels fit (at most 128 components).
+ */
+int eqt_block_rotation_supported(const int32_t* block_sizes, int32_t num_blocks, int32_t channels);
+int eqt_block_rotation(const float* matrix, const float* x, float* out, int64_t n, const int32_t* block_sizes, int32_t num_blocks,
+                       int32_t channels, int32_t transposed, void* stream);
+int eqt_block_rotation_grad_matrix(const float* grad_out, const float* x, float* grad_matrix, int64_t n,
+                                   const int32_t* block_sizes, int32_t num_blocks, int32_t channels, void* stream);
+
+/*
  * Radius graph and edge features in one pass over a cell list (float32).
  * The caller bins the n points into cubic cells of side cell_size >= r - `dims` cells per axis, x fastest:
  * cell = ((graph * dims[2] + z) * dims[1] + y) * dims[0] + x, one slab of cells per graph of the batch - and
