@@ -350,33 +350,40 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
 // ------------------------------------------------------------------------------------------
 // The reference's indexed products with shared weights on the same machinery
 // ------------------------------------------------------------------------------------------
-extern "C" int eqt_vecmat_tc(const float* x, const float* w, const int64_t* index2, const float* scale, float* w_big,
-                             float* w_small, float* out, int64_t n, int32_t rows1, int32_t cin, int32_t cout,
-                             int32_t num_out, int64_t entries, const int32_t* kb_begin, const int32_t* a_col,
-                             int32_t* status, void* stream) {
+extern "C" int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64_t* index2, const float* scale, float* w_big,
+                                     float* w_small, float* out, int64_t n, int32_t rows1, int32_t cin, int32_t cout,
+                                     int32_t num_out, int64_t slots, int32_t group, int32_t num_groups, const int32_t* group_rows,
+                                     const int32_t* slot_entry, const int32_t* kb_begin, const int32_t* a_col, int32_t* status,
+                                     void* stream) {
   using namespace eqt;
-  if (n < 0 || rows1 <= 0 || cin <= 0 || cout <= 0 || num_out < 0 || entries < 0) return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
-  if (n == 0 || num_out == 0) return EQT_OK;
+  if (n < 0 || rows1 <= 0 || cin <= 0 || cout <= 0 || num_out < 0 || slots < 0 || group <= 0 || num_groups < 0)
+    return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
+  if (n == 0 || num_out == 0 || num_groups == 0) return EQT_OK;
   if (!x || !w || !w_big || !w_small || !out || !kb_begin || !a_col || !status) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
-  if (cin % KB != 0 || cout % 16 != 0 || cout > 128)
-    return fail(EQT_ERR_UNSUPPORTED, "tensor-core vecmat needs C_in %% 32 == 0, C_out %% 16 == 0, C_out <= 128");
+  if (group > 1 && (!group_rows || !slot_entry)) return fail(EQT_ERR_BAD_ARGUMENT, "groups of rows need their tables");
+  if (!group_rows && num_groups != num_out) return fail(EQT_ERR_BAD_ARGUMENT, "one group per output row without a row table");
+  if (cin % KB != 0 || cout % 16 != 0 || cout > 128 || (group > 1 && (cout % 32 != 0 || group * cout > 128)))
+    return fail(EQT_ERR_UNSUPPORTED, "tensor-core vecmat needs C_in %% 32 == 0, C_out %% 16 == 0, C_out <= 128 (all rows of a group)");
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w_big) |
        reinterpret_cast<uintptr_t>(w_small)) & 15u)
     return fail(EQT_ERR_UNSUPPORTED, "tensor-core vecmat needs 16-byte aligned operands");
-  if (n > 0x7fffffffll || (int64_t)rows1 * cin > 0x7fffffffll || entries * cin > 0x7fffffffll)
+  if (n > 0x7fffffffll || (int64_t)rows1 * cin > 0x7fffffffll || slots * cin > 0x7fffffffll)
     return fail(EQT_ERR_UNSUPPORTED, "operands too large for one TMA coordinate");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t ktot = entries * cin;
-  if (entries > 0) {
-    pack_vecmat_weights_kernel<<<flat_grid(ktot * cout, 256), 256, 0, st>>>(w, index2, scale, w_big, w_small, entries, cin, cout);
+  const int64_t ktot = slots * cin;
+  const int n_cols = group * cout;
+  if (slots > 0) {
+    pack_vecmat_weights_kernel<<<flat_grid(ktot * n_cols, 256), 256, 0, st>>>(w, index2, scale, slot_entry, w_big, w_small, slots, group,
+                                                                              cin, cout);
     if (int rc = check_launch("pack_vecmat_weights_kernel")) return rc;
   }
   VecmatLaunch L{};
-  L.out = out; L.kb_begin = kb_begin; L.a_col = a_col; L.n = n; L.num_out = num_out; L.n_cols = cout; L.status = status;
-  L.total_items = (int64_t)num_out * ceil_div(n, TILE_M);
-  const uint32_t stage_bytes = TILE_M * KB * 4 + 2u * (uint32_t)cout * KB * 4;
-  L.acc_sets = cout <= 64 ? 2 : 1;               // a pair of accumulators each: at least four A slots stay free
-  const int acc_cols = 2 * L.acc_sets * cout;
+  L.out = out; L.kb_begin = kb_begin; L.rows = group_rows; L.a_col = a_col; L.n = n; L.num_out = num_out; L.status = status;
+  L.num_groups = num_groups; L.group = group; L.cout = cout; L.n_cols = n_cols;
+  L.total_items = (int64_t)num_groups * ceil_div(n, TILE_M);
+  const uint32_t stage_bytes = TILE_M * KB * 4 + 2u * (uint32_t)n_cols * KB * 4;
+  L.acc_sets = n_cols <= 64 ? 2 : 1;             // a pair of accumulators each: at least four A slots stay free
+  const int acc_cols = 2 * L.acc_sets * n_cols;
   L.stages = (int)std::min<size_t>(std::min<size_t>(8, (220 * 1024 - 1024 - EPI_PATCH_BYTES) / stage_bytes), (512 - acc_cols) / 64);
   if (L.stages < 2) return fail(EQT_ERR_UNSUPPORTED, "tile too wide for the shared-memory ring");
   L.tmem_cols = 32;
@@ -389,9 +396,9 @@ extern "C" int eqt_vecmat_tc(const float* x, const float* w, const int64_t* inde
   }
   {
     // an empty table still needs valid maps: describe at least one k-block
-    cuuint64_t dims[2] = {(cuuint64_t)std::max<int64_t>(ktot, KB), (cuuint64_t)cout};
+    cuuint64_t dims[2] = {(cuuint64_t)std::max<int64_t>(ktot, KB), (cuuint64_t)n_cols};
     cuuint64_t strides[1] = {(cuuint64_t)std::max<int64_t>(ktot, KB) * 4};
-    cuuint32_t box[2] = {KB, (cuuint32_t)cout};
+    cuuint32_t box[2] = {KB, (cuuint32_t)n_cols};
     if (int rc = make_map(&L.map_bb, w_big, 2, dims, strides, box)) return rc;
     if (int rc = make_map(&L.map_bs, w_small, 2, dims, strides, box)) return rc;
   }
@@ -402,50 +409,59 @@ extern "C" int eqt_vecmat_tc(const float* x, const float* w, const int64_t* inde
   return check_launch("vecmat_tc_kernel");
 }
 
-extern "C" int64_t eqt_outer_tc_scratch_floats(int64_t n, int32_t c2, int32_t m_tiles) {
-  using namespace eqt;
-  if (n < 0 || c2 <= 0 || c2 % 32 || m_tiles <= 0) return -1;
-  const int splits = std::max(1, sm_count() / m_tiles);
-  return (int64_t)splits * m_tiles * 128 * c2;
+extern "C" int eqt_vecmat_tc(const float* x, const float* w, const int64_t* index2, const float* scale, float* w_big,
+                             float* w_small, float* out, int64_t n, int32_t rows1, int32_t cin, int32_t cout,
+                             int32_t num_out, int64_t entries, const int32_t* kb_begin, const int32_t* a_col,
+                             int32_t* status, void* stream) {
+  return eqt_vecmat_tc_grouped(x, w, index2, scale, w_big, w_small, out, n, rows1, cin, cout, num_out, entries, 1, num_out, nullptr,
+                               nullptr, kb_begin, a_col, status, stream);
 }
 
-extern "C" int eqt_outer_tc(const float* in1, const float* in2, float* out, float* scratch, int64_t scratch_floats, int64_t n,
-                            int32_t rows1, int32_t c1, int32_t rows2, int32_t c2, const int32_t* a_cols, const int32_t* b_cols,
-                            int32_t m_tiles, const int32_t* red_ptr, const int32_t* red_slot, const float* red_scale,
-                            int32_t num_w, int32_t* status, void* stream) {
+extern "C" int64_t eqt_outer_tc_scratch_floats(int64_t n, int32_t columns, int32_t m_tiles) {
   using namespace eqt;
-  if (n < 0 || rows1 <= 0 || rows2 <= 0 || c1 <= 0 || c2 <= 0 || m_tiles < 0 || num_w < 0) return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
+  if (n < 0 || columns <= 0 || columns % 32 || m_tiles <= 0) return -1;
+  const int splits = std::max(1, sm_count() / m_tiles);
+  return (int64_t)splits * m_tiles * 128 * columns;
+}
+
+extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* out, float* scratch, int64_t scratch_floats, int64_t n,
+                                    int32_t rows1, int32_t c1, int32_t rows2, int32_t c2, int32_t group, const int32_t* a_cols,
+                                    const int32_t* b_cols, int32_t m_tiles, const int32_t* red_ptr, const int32_t* red_slot,
+                                    const float* red_scale, int32_t num_w, int32_t* status, void* stream) {
+  using namespace eqt;
+  if (n < 0 || rows1 <= 0 || rows2 <= 0 || c1 <= 0 || c2 <= 0 || group <= 0 || m_tiles < 0 || num_w < 0) return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
   if (num_w == 0) return EQT_OK;
   if (!in1 || !in2 || !out || !scratch || !a_cols || !b_cols || !red_ptr || !red_slot || !red_scale || !status)
     return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
-  if (c1 % 32 != 0 || c2 % 32 != 0 || c2 > 128)
-    return fail(EQT_ERR_UNSUPPORTED, "tensor-core outer product needs C1 %% 32 == 0, C2 %% 32 == 0, C2 <= 128");
+  if (c1 % 32 != 0 || c2 % 32 != 0 || c2 > 128 || group > 128 / c2)
+    return fail(EQT_ERR_UNSUPPORTED, "tensor-core outer product needs C1 %% 32 == 0, C2 %% 32 == 0, C2 <= 128 (all rows of a group)");
   if ((reinterpret_cast<uintptr_t>(in1) | reinterpret_cast<uintptr_t>(in2) | reinterpret_cast<uintptr_t>(out) |
        reinterpret_cast<uintptr_t>(scratch)) & 15u)
     return fail(EQT_ERR_UNSUPPORTED, "tensor-core outer product needs 16-byte aligned operands");
-  if (n > 0x7fffffffll || (int64_t)rows1 * c1 > 0x7fffffffll || (int64_t)rows2 * c2 > 0x7fffffffll)
+  if (n > 0x7fffffffll || (int64_t)rows1 * c1 > 0x7fffffffll || (int64_t)rows2 * c2 > 0x7fffffffll || m_tiles >= (1 << 22))
     return fail(EQT_ERR_UNSUPPORTED, "operands too large for one TMA coordinate");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int columns = group * c2;
   int splits = 1;
   if (n > 0 && m_tiles > 0) {
-    const int b_boxes = c2 / 32;
+    const int b_boxes = columns / 32;
     const size_t budget = 220 * 1024 - 1024;
     const size_t bytes_per_row = 2 * (size_t)(4 + b_boxes) * 128;
     const int npt = std::max(8, (int)(budget / 3 / bytes_per_row) / 8 * 8);          // reduction rows per tile
     WgradBatch B{};
-    B.count = 1; B.n = n; B.n_cols = c2; B.status = status;
+    B.count = 1; B.n = n; B.n_cols = columns; B.status = status;
     WgradBlock& a = B.blk[0];
     a.dim = 1; a.npt = npt; a.rows_pad = npt;
     const size_t stage_bytes = bytes_per_row * (size_t)npt;
     a.stages = (int)std::min<size_t>(8, budget / stage_bytes);
     a.issuers = npt / 8 >= 2 ? 2 : 1;
     B.tmem_cols = 32;
-    while (B.tmem_cols < 2 * a.issuers * c2) B.tmem_cols <<= 1;
+    while (B.tmem_cols < 2 * a.issuers * columns) B.tmem_cols <<= 1;
     a.chunk_tiles = std::max(1, 512 / npt);
-    a.a_cols = a_cols; a.b_cols = b_cols;
+    a.a_cols = a_cols; a.b_cols = b_cols; a.b_row_boxes = c2 / 32;
     const int64_t tiles = ceil_div(n, npt);
     splits = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count() / m_tiles));
-    const int64_t need = (int64_t)splits * m_tiles * 128 * c2;
+    const int64_t need = (int64_t)splits * m_tiles * 128 * columns;
     if (need > scratch_floats) return fail(EQT_ERR_BAD_ARGUMENT, "scratch too small: %lld floats needed", (long long)need);
     a.partial = scratch;
     a.m_tiles = m_tiles; a.splits = splits; a.cta_begin = 0;
@@ -471,8 +487,16 @@ extern "C" int eqt_outer_tc(const float* in1, const float* in2, float* out, floa
     return EQT_OK;
   }
   outer_reduce_kernel<<<flat_grid((int64_t)num_w * c1 * c2 / 4, 256), 256, 0, st>>>(scratch, out, red_ptr, red_slot, red_scale, splits,
-                                                                                   (int64_t)m_tiles * 128, num_w, c1, c2);
+                                                                                   (int64_t)m_tiles * 128, num_w, c1, c2, columns);
   return check_launch("outer_reduce_kernel");
+}
+
+extern "C" int eqt_outer_tc(const float* in1, const float* in2, float* out, float* scratch, int64_t scratch_floats, int64_t n,
+                            int32_t rows1, int32_t c1, int32_t rows2, int32_t c2, const int32_t* a_cols, const int32_t* b_cols,
+                            int32_t m_tiles, const int32_t* red_ptr, const int32_t* red_slot, const float* red_scale,
+                            int32_t num_w, int32_t* status, void* stream) {
+  return eqt_outer_tc_grouped(in1, in2, out, scratch, scratch_floats, n, rows1, c1, rows2, c2, 1, a_cols, b_cols, m_tiles, red_ptr,
+                              red_slot, red_scale, num_w, status, stream);
 }
 
 // ------------------------------------------------------------------------------------------

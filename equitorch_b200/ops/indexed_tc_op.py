@@ -2,7 +2,7 @@
 
 ``indexed_vecmat_scale_gather`` with a 3-D matrix operand and ``indexed_outer_scale_gather`` with
 ``out_accumulated=True`` are GEMMs over the batch; for float32 operands with channel counts that are multiples of 32
-they run on tcgen05 (``eqt_vecmat_tc`` / ``eqt_outer_tc``) instead of the table-driven CUDA-core kernels.  What the
+they run on tcgen05 (``eqt_vecmat_tc_grouped`` / ``eqt_outer_tc_grouped``) instead of the table-driven CUDA-core kernels.  What the
 kernels need besides the operands depends on the index tables only (k-block columns, packing of entries into
 128-row slices, reduction lists) and is built once per table and device and cached.
 """
@@ -53,16 +53,47 @@ def _buffer(dev, floats: int) -> Tensor:
     return buf
 
 
+def _same_reads(reads):
+    """Classes of rows that read the same rows, ``{(what they read, sorted): [rows]}``, in order of first appearance;
+    ``reads[r]`` lists what row r reads, repeats included."""
+    classes: "OrderedDict[tuple, list]" = OrderedDict()
+    for row, r in enumerate(reads):
+        classes.setdefault(tuple(sorted(r)), []).append(row)
+    return classes
+
+
 class VecmatPlan:
-    def __init__(self, index1, seg, entries: int, num_out: int, cin: int, dev):
+    """Output rows that read the same input rows share work items of up to ``group`` rows (see ``eqt_vecmat_tc_grouped``)."""
+
+    def __init__(self, index1, seg, entries: int, num_out: int, cin: int, cout: int, dev):
         chunks = cin // 32
         i1 = _host(index1, np.arange(entries, dtype=np.int64))
         sg = _host(seg, np.arange(num_out + 1, dtype=np.int64))
-        a_col = (i1[:, None] * cin + np.arange(chunks)[None, :] * 32).reshape(-1)
-        self.kb_begin = torch.from_numpy((sg * chunks).astype(np.int32)).to(dev)
-        self.a_col = torch.from_numpy(a_col.astype(np.int32)).to(dev)
-        if self.a_col.numel() == 0:
-            self.a_col = torch.zeros(1, dtype=torch.int32, device=dev)
+        classes = _same_reads([i1[sg[r]:sg[r + 1]].tolist() for r in range(num_out)])
+
+        # A k-block costs 16 KB of x and 256 bytes of weights per column.  With the one-row groups at 413 entries of 32 x 32
+        # (l = 0..6) a pass moved 9.9 MB per 128 samples and issued 4956 small MMAs; four rows a group make it 5.5 MB and 1368.
+        def cost(g):
+            return sum(-(-len(rows) // g) * len(reads) for reads, rows in classes.items()) * (64 + g * cout)
+        sizes = [1] + [g for g in (2, 3, 4) if cout % 32 == 0 and g * cout <= 128]
+        self.group = min(sizes, key=cost)
+        group_rows, slot_entry, a_col, kb_begin = [], [], [], [0]
+        for reads, rows in classes.items():
+            for k in range(0, len(rows), self.group):
+                part = rows[k:k + self.group]
+                group_rows.append(part + [-1] * (self.group - len(part)))
+                # the j-th of the sorted reads of every row of the class is the same input row
+                order = [sg[r] + np.argsort(i1[sg[r]:sg[r + 1]], kind="stable") for r in part]
+                for j, row1 in enumerate(reads):
+                    slot_entry.append([int(o[j]) for o in order] + [-1] * (self.group - len(part)))
+                    a_col += [row1 * cin + ch * 32 for ch in range(chunks)]
+                kb_begin.append(len(a_col))
+        self.slots, self.num_groups = len(slot_entry), len(group_rows)
+
+        def dev_i32(v):
+            return torch.tensor(v if len(v) else [0], dtype=torch.int32, device=dev)
+        self.kb_begin, self.a_col = dev_i32(kb_begin), dev_i32(a_col)
+        self.group_rows, self.slot_entry = dev_i32(group_rows), dev_i32(slot_entry)
 
 
 def vecmat_supported(x: Tensor, w: Tensor, gather_index, index_out, out_accumulated, out_size, num_out) -> bool:
@@ -79,20 +110,22 @@ def vecmat_tc(x: Tensor, w: Tensor, scale, index1, index2, seg, num_out: int) ->
     cout = w.shape[2]
     entries = (index1.shape[0] if index1 is not None else index2.shape[0] if index2 is not None
                else int(seg[-1]) if seg is not None else rows1)
-    plan = _cached("vecmat", dev, (index1, seg), (entries, num_out, cin),
-                   lambda: VecmatPlan(index1, seg, entries, num_out, cin, dev))
-    packed = torch.empty(2, max(entries, 1) * cin * cout, dtype=torch.float32, device=dev)
+    plan = _cached("vecmat", dev, (index1, seg), (entries, num_out, cin, cout),
+                   lambda: VecmatPlan(index1, seg, entries, num_out, cin, cout, dev))
+    packed = torch.empty(2, max(plan.slots, 1) * cin * plan.group * cout, dtype=torch.float32, device=dev)
     out = torch.empty(n, num_out, cout, dtype=torch.float32, device=dev)
     with _lib.on_device(dev):
-        _lib.check(_lib.lib().eqt_vecmat_tc(x.data_ptr(), w.data_ptr(), _lib.ptr(index2), _lib.ptr(scale), packed[0].data_ptr(),
-                                            packed[1].data_ptr(), out.data_ptr(), n, rows1, cin, cout, num_out, entries,
-                                            plan.kb_begin.data_ptr(), plan.a_col.data_ptr(), status_flag(dev).data_ptr(),
-                                            _lib.stream_ptr(dev)), "eqt_vecmat_tc")
+        _lib.check(_lib.lib().eqt_vecmat_tc_grouped(x.data_ptr(), w.data_ptr(), _lib.ptr(index2), _lib.ptr(scale),
+                                                    packed[0].data_ptr(), packed[1].data_ptr(), out.data_ptr(), n, rows1, cin, cout,
+                                                    num_out, plan.slots, plan.group, plan.num_groups, plan.group_rows.data_ptr(),
+                                                    plan.slot_entry.data_ptr(), plan.kb_begin.data_ptr(), plan.a_col.data_ptr(),
+                                                    status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_vecmat_tc_grouped")
     return out
 
 
 class OuterPlan:
-    """Packing of the entries of an accumulated outer product into 128-row slices (see ``eqt_outer_tc``)."""
+    """Packing of the entries of an accumulated outer product into 128-row slices (see ``eqt_outer_tc_grouped``): second
+    operand rows that meet the same rows of the first share slices, ``group`` of them at a time."""
 
     def __init__(self, scale, index1, index2, seg, entries: int, num_w: int, c1: int, c2: int, dev):
         chunks = c1 // 32
@@ -101,22 +134,29 @@ class OuterPlan:
         sg = _host(seg, np.arange(num_w + 1, dtype=np.int64))
         sc = _host(scale, np.ones(entries, dtype=np.float32)).astype(np.float32)
         w_of = np.repeat(np.arange(num_w), np.diff(sg))
+        rows2 = np.unique(i2)
+        meets = {int(r): np.nonzero(i2 == r)[0] for r in rows2}
+        classes = _same_reads([sorted(set(i1[meets[int(r)]].tolist())) for r in rows2])
+
+        # a slice reads four 128-byte columns of the first operand and c2 / 32 per row of the second, for every sample
+        def cost(g):
+            return sum(-(-len(reads) * chunks // 4) * -(-len(rows) // g) for reads, rows in classes.items()) * (4 + g * c2 // 32)
+        self.group = min([g for g in (1, 2, 3, 4) if g * c2 <= 128], key=cost)
         a_cols, b_cols, units = [], [], []            # units: (weight, chunk, slot, scale)
-        for row2 in np.unique(i2):
-            ts = np.nonzero(i2 == row2)[0]
-            slots = [(t, ch) for t in ts for ch in range(chunks)]
-            for s0 in range(0, len(slots), 4):
-                group = slots[s0:s0 + 4]
-                tile = len(b_cols)
-                b_cols.append(int(row2) * c2)
-                for q in range(4):
-                    if q < len(group):
-                        t, ch = group[q]
-                        a_cols.append(int(i1[t]) * c1 + ch * 32)
-                        units.append((int(w_of[t]), ch, tile * 4 + q, float(sc[t])))
-                    else:
-                        a_cols.append(0)
-        self.m_tiles = len(b_cols)
+        for reads, rows in classes.items():
+            slots = [(r1, ch) for r1 in reads for ch in range(chunks)]
+            for k in range(0, len(rows), self.group):
+                part = [int(rows2[r]) for r in rows[k:k + self.group]]
+                for s0 in range(0, len(slots), 4):
+                    tile = len(a_cols) // 4
+                    b_cols += [r2 * c2 for r2 in part] + [part[0] * c2] * (self.group - len(part))
+                    for q, (r1, ch) in enumerate(slots[s0:s0 + 4]):
+                        a_cols.append(int(r1) * c1 + ch * 32)
+                        for which, r2 in enumerate(part):
+                            units += [(int(w_of[t]), ch, (which << 24) + tile * 4 + q, float(sc[t]))
+                                      for t in meets[r2] if i1[t] == r1]
+                    a_cols += [0] * (-len(a_cols) % 4)
+        self.m_tiles = len(a_cols) // 4
         units.sort(key=lambda u: (u[0], u[1], u[2]))
         keys = np.array([u[0] * chunks + u[1] for u in units], dtype=np.int64)
         red_ptr = np.searchsorted(keys, np.arange(num_w * chunks + 1)).astype(np.int32)
@@ -147,10 +187,11 @@ def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Te
                    lambda: OuterPlan(scale, index1, index2, seg, entries, num_w, c1, c2, dev))
     out = torch.empty(num_w, c1, c2, dtype=torch.float32, device=dev)
     with _lib.on_device(dev):
-        need = int(_lib.lib().eqt_outer_tc_scratch_floats(n, c2, max(plan.m_tiles, 1)))
+        need = int(_lib.lib().eqt_outer_tc_scratch_floats(n, plan.group * c2, max(plan.m_tiles, 1)))
         scratch = _buffer(dev, max(need, 1))
-        _lib.check(_lib.lib().eqt_outer_tc(a.data_ptr(), b.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(), n,
-                                           rows1, c1, rows2, c2, plan.a_cols.data_ptr(), plan.b_cols.data_ptr(), plan.m_tiles,
-                                           plan.red_ptr.data_ptr(), plan.red_slot.data_ptr(), plan.red_scale.data_ptr(), num_w,
-                                           status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_outer_tc")
+        _lib.check(_lib.lib().eqt_outer_tc_grouped(a.data_ptr(), b.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(),
+                                                   n, rows1, c1, rows2, c2, plan.group, plan.a_cols.data_ptr(),
+                                                   plan.b_cols.data_ptr(), plan.m_tiles, plan.red_ptr.data_ptr(),
+                                                   plan.red_slot.data_ptr(), plan.red_scale.data_ptr(), num_w,
+                                                   status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_outer_tc_grouped")
     return out
