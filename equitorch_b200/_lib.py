@@ -130,6 +130,12 @@ SIGNATURES = {
     "eqt_outer_tc_scratch_floats": (C.c_int64, [C.c_int64, C.c_int32, C.c_int32]),
     "eqt_radius_count": (C.c_int, [C.POINTER(RadiusGridStruct), C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_int32, C.c_int32,
                                    C.c_void_p, C.c_void_p, C.c_void_p]),
+    "eqt_radius_bin": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_float, C.c_void_p, C.c_int32, C.c_void_p,
+                                 C.c_void_p, C.c_void_p, C.c_void_p]),
+    "eqt_radius_place": (C.c_int, [C.c_void_p] * 5 + [C.c_int64, C.c_void_p]),
+    "eqt_radius_search": (C.c_int, [C.c_void_p] * 4 + [C.c_int64, C.c_void_p, C.c_float, C.c_int32, C.c_int32] + [C.c_void_p] * 4),
+    "eqt_radius_list_edges": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p,
+                                        C.POINTER(EdgeFeaturesStruct), C.c_void_p]),
     "eqt_radius_edges": (C.c_int, [C.POINTER(RadiusGridStruct), C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_int32, C.c_int32,
                                    C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(EdgeFeaturesStruct), C.c_void_p, C.c_void_p]),
     "eqt_so3_uu_scratch_floats": (C.c_int64, [C.POINTER(PathTableStruct), C.c_int64, C.c_int32, C.c_int32, C.c_int32]),

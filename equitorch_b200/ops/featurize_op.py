@@ -1,4 +1,4 @@
-"""Radius graph and fused edge features (operator layer over ``eqt_radius_count`` / ``eqt_radius_edges``)."""
+"""Radius graph and fused edge features (operator layer over the ``eqt_radius_*`` entry points)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -11,18 +11,25 @@ from torch import Tensor
 from .. import _lib
 
 CUTOFF_KINDS = {"polynomial": 0, "cosine": 1, "mollifier": 2}
-_status = {}
 
-
-def _flag(dev) -> Tensor:
-    if dev not in _status:
-        _status[dev] = torch.zeros(1, dtype=torch.int32, device=dev)
-    return _status[dev]
+#: neighbour lists of at most this many entries (256 MB) are kept between the search and the pass that writes the edges;
+#: above it that pass searches again
+MAX_LIST_ENTRIES = 1 << 26
+_LIST_ROW = 512          # most candidates of one target
 
 
 class CellList(NamedTuple):
-    struct: "_lib.RadiusGridStruct"
-    keep: tuple          # tensors the struct points at
+    cell_start: Tensor       # (cells + 1,) int32 first place of every cell
+    sorted: Tensor           # (N, 4) float32: x, y, z and index (its bits) of the points by cell
+    point_cell: Tensor       # (N,) int32, -1 for a graph index out of range
+    dims: "C.Array"
+    cell_size: float
+
+    def struct(self):
+        """The struct of the searching entry points and what it points at."""
+        index = self.sorted[:, 3].contiguous().view(torch.int32)
+        return _lib.RadiusGridStruct(self.cell_start.data_ptr(), index.data_ptr(), self.point_cell.data_ptr(), self.cell_size,
+                                     self.dims), index
 
 
 def build_cell_list(pos: Tensor, r: float, batch: Optional[Tensor] = None) -> CellList:
@@ -30,25 +37,28 @@ def build_cell_list(pos: Tensor, r: float, batch: Optional[Tensor] = None) -> Ce
     n = pos.shape[0]
     dev = pos.device
     cell_size = float(r) * (1.0 + 1e-5)
-    lo = pos.min(dim=0).values
-    extent = (pos.max(dim=0).values - lo).tolist()                      # one host synchronisation
-    dims = [max(1, int(math.floor(e / cell_size)) + 1) for e in extent]
+    lo, hi = torch.stack(torch.aminmax(pos, dim=0)).tolist()            # one host synchronisation
+    dims = [max(1, int(math.floor((b - a) / cell_size)) + 1) for a, b in zip(lo, hi)]
     per_graph = dims[0] * dims[1] * dims[2]
-    graphs = 1 if batch is None else int(batch.max()) + 1
+    graphs = 1 if batch is None else max(0, int(batch.max()) + 1)
     if graphs * per_graph >= 2 ** 31:
         raise ValueError("cell grid too large; the positions are too spread out for this cutoff")
-    c = ((pos - lo) / cell_size).floor().long()
-    for k in range(3):
-        c[:, k].clamp_(0, dims[k] - 1)
-    cell = (c[:, 2] * dims[1] + c[:, 1]) * dims[0] + c[:, 0]
-    if batch is not None:
-        cell = cell + batch.long() * per_graph
-    order = torch.argsort(cell, stable=True)
-    cell_start = torch.searchsorted(cell[order], torch.arange(graphs * per_graph + 1, device=dev)).int()
-    point_cell, sorted_index = cell.int().contiguous(), order.int().contiguous()
-    struct = _lib.RadiusGridStruct(cell_start.data_ptr(), sorted_index.data_ptr(), point_cell.data_ptr(), cell_size,
-                                   (C.c_int32 * 3)(*dims))
-    return CellList(struct, (cell_start, sorted_index, point_cell))
+    cells = graphs * per_graph
+    batch = None if batch is None else batch.long().contiguous()
+    counts = torch.zeros(2 * cells + 1, dtype=torch.int32, device=dev)  # [starts, counts]
+    cell_start, cell_count = counts[:cells + 1], counts[cells + 1:]
+    point_cell, rank = torch.empty(2, n, dtype=torch.int32, device=dev)
+    placed = torch.empty(n, 4, dtype=torch.float32, device=dev)
+    c_dims = (C.c_int32 * 3)(*dims)
+    lib = _lib.lib()
+    with _lib.on_device(dev):
+        _lib.check(lib.eqt_radius_bin(pos.data_ptr(), _lib.ptr(batch), n, (C.c_float * 3)(*lo), cell_size, c_dims, graphs,
+                                      point_cell.data_ptr(), rank.data_ptr(), cell_count.data_ptr(), _lib.stream_ptr(dev)),
+                   "eqt_radius_bin")
+        torch.cumsum(cell_count, 0, dtype=torch.int32, out=cell_start[1:])
+        _lib.check(lib.eqt_radius_place(pos.data_ptr(), point_cell.data_ptr(), rank.data_ptr(), cell_start.data_ptr(),
+                                        placed.data_ptr(), n, _lib.stream_ptr(dev)), "eqt_radius_place")
+    return CellList(cell_start, placed, point_cell, c_dims, cell_size)
 
 
 class EdgeFeatures(NamedTuple):
@@ -82,17 +92,24 @@ def radius_graph_features(pos: Tensor, r: float, batch: Optional[Tensor] = None,
         raise ValueError("the fused kernel takes l_max <= 4; use SphericalHarmonics on edge_vec for higher degrees")
     cells = build_cell_list(pos, r, batch)
     degree = torch.empty(n, dtype=torch.int32, device=dev)
-    flag = _flag(dev)
+    tail = torch.zeros(n + 2, dtype=torch.long, device=dev)              # CSR pointer, then the status of the search
+    ptr, flag = tail[:n + 1], tail[n + 1:].view(torch.int32)
+    row = min(int(max_num_neighbors), _LIST_ROW)
+    lists = torch.empty(n, row, dtype=torch.int32, device=dev) if 0 < row and n * row <= MAX_LIST_ENTRIES else None
     lib = _lib.lib()
     with _lib.on_device(dev):
-        _lib.check(lib.eqt_radius_count(C.byref(cells.struct), pos.data_ptr(), _lib.ptr(batch), n, float(r), int(loop),
-                                        int(max_num_neighbors), degree.data_ptr(), flag.data_ptr(), _lib.stream_ptr(dev)),
-                   "eqt_radius_count")
-    ptr = torch.zeros(n + 1, dtype=torch.long, device=dev)
+        if lists is not None:
+            _lib.check(lib.eqt_radius_search(pos.data_ptr(), cells.sorted.data_ptr(), cells.cell_start.data_ptr(),
+                                             cells.point_cell.data_ptr(), n, cells.dims, float(r), int(loop), row,
+                                             degree.data_ptr(), lists.data_ptr(), flag.data_ptr(), _lib.stream_ptr(dev)),
+                       "eqt_radius_search")
+        else:
+            grid, index = cells.struct()
+            _lib.check(lib.eqt_radius_count(C.byref(grid), pos.data_ptr(), None, n, float(r), int(loop), int(max_num_neighbors),
+                                            degree.data_ptr(), flag.data_ptr(), _lib.stream_ptr(dev)), "eqt_radius_count")
     torch.cumsum(degree, 0, out=ptr[1:])
-    e = int(ptr[-1])                                                     # host synchronisation: the output size
-    if int(flag.item()) != 0:
-        flag.zero_()
+    e, failed = tail[n:].tolist()                                        # host synchronisation: the output size
+    if failed:
         raise _lib.EqtError("a node has more than 512 candidate neighbours; lower the cutoff")
     src = torch.empty(e, dtype=torch.long, device=dev)
     dst = torch.empty(e, dtype=torch.long, device=dev)
@@ -112,7 +129,11 @@ def radius_graph_features(pos: Tensor, r: float, batch: Optional[Tensor] = None,
                                     CUTOFF_KINDS[cutoff] if cutoff is not None else 0, float(bessel_r_max or 1.0),
                                     float(cutoff_r_min), float(cutoff_r_max or 1.0), float(cutoff_p), float(cutoff_eps))
     with _lib.on_device(dev):
-        _lib.check(lib.eqt_radius_edges(C.byref(cells.struct), pos.data_ptr(), _lib.ptr(batch), n, float(r), int(loop),
-                                        int(max_num_neighbors), ptr.data_ptr(), src.data_ptr(), dst.data_ptr(), C.byref(feats),
-                                        flag.data_ptr(), _lib.stream_ptr(dev)), "eqt_radius_edges")
+        if lists is not None:
+            _lib.check(lib.eqt_radius_list_edges(pos.data_ptr(), n, ptr.data_ptr(), lists.data_ptr(), row, src.data_ptr(),
+                                                 dst.data_ptr(), C.byref(feats), _lib.stream_ptr(dev)), "eqt_radius_list_edges")
+        else:
+            _lib.check(lib.eqt_radius_edges(C.byref(grid), pos.data_ptr(), None, n, float(r), int(loop), int(max_num_neighbors),
+                                            ptr.data_ptr(), src.data_ptr(), dst.data_ptr(), C.byref(feats), flag.data_ptr(),
+                                            _lib.stream_ptr(dev)), "eqt_radius_edges")
     return EdgeFeatures(src, dst, ptr, vec, length, sh, bes, cut)

@@ -562,6 +562,24 @@ int eqt_radius_count(const eqt_radius_grid* grid, const float* pos, const int64_
 int eqt_radius_edges(const eqt_radius_grid* grid, const float* pos, const int64_t* batch, int64_t n, float r, int32_t loop,
                      int32_t max_neighbors, const int64_t* ptr, int64_t* src, int64_t* dst, const eqt_edge_features* features,
                      int32_t* status, void* stream);
+/*
+ * The same with the cells filled by a counting sort and the neighbour lists kept between the two passes.
+ * eqt_radius_bin: point_cell (n) from cell = floor((pos - lo) / cell_size) per axis, clamped to `dims`, plus the slab of
+ * batch[i] (batch may be NULL; -1 where it is not in [0, graphs)); rank[i] numbers the points of a cell, cell_count (zeroed by
+ * the caller, dims[0] * dims[1] * dims[2] * graphs) counts them.  lo and dims are host arrays of three.
+ * eqt_radius_place: with cell_start = exclusive scan of cell_count, sorted (n, 4) = x, y, z, index (as bits) by cell.
+ * eqt_radius_search: degree as eqt_radius_count with max_neighbors = row <= 512, and list (n, row): the neighbours, ascending.
+ * eqt_radius_list_edges: what eqt_radius_edges writes, from the lists.
+ */
+int eqt_radius_bin(const float* pos, const int64_t* batch, int64_t n, const float* lo, float cell_size, const int32_t* dims,
+                   int32_t graphs, int32_t* point_cell, int32_t* rank, int32_t* cell_count, void* stream);
+int eqt_radius_place(const float* pos, const int32_t* point_cell, const int32_t* rank, const int32_t* cell_start, float* sorted,
+                     int64_t n, void* stream);
+int eqt_radius_search(const float* pos, const float* sorted, const int32_t* cell_start, const int32_t* point_cell, int64_t n,
+                      const int32_t* dims, float r, int32_t loop, int32_t row, int32_t* degree, int32_t* list, int32_t* status,
+                      void* stream);
+int eqt_radius_list_edges(const float* pos, int64_t n, const int64_t* ptr, const int32_t* list, int32_t row, int64_t* src,
+                          int64_t* dst, const eqt_edge_features* features, void* stream);
 
 #ifdef __cplusplus
 }
