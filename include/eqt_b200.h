@@ -275,12 +275,13 @@ int eqt_vecmat_tc(const float* x, const float* w, const int64_t* index2, const f
  * group > 1: cout % 32 == 0, group * cout <= 128).  A slot is (group, x row): kb_begin (num_groups + 1) and a_col count the
  * k-blocks of slots, group_rows (num_groups, group) names the output rows (-1: none; every row once), slot_entry (slots, group)
  * the entry t of a slot's x row in each output row (-1: none).  w_big / w_small hold slots * cin * group * cout floats.
+ * longest: k-blocks of the longest group where the caller knows them (1 adds a correction product), else 0.
  */
 int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64_t* index2, const float* scale, float* w_big,
                           float* w_small, float* out, int64_t n, int32_t rows1, int32_t cin, int32_t cout, int32_t num_out,
                           int64_t slots, int32_t group, int32_t num_groups, const int32_t* group_rows,
-                          const int32_t* slot_entry, const int32_t* kb_begin, const int32_t* a_col, int32_t* status,
-                          void* stream);
+                          const int32_t* slot_entry, const int32_t* kb_begin, const int32_t* a_col, int32_t longest,
+                          int32_t* status, void* stream);
 
 /*
  * The reference's indexed outer product accumulated over the batch (the gradient of shared weights), on tensor
@@ -304,12 +305,13 @@ int eqt_outer_tc(const float* in1, const float* in2, float* out, float* scratch,
 int64_t eqt_outer_tc_scratch_floats(int64_t n, int32_t columns, int32_t m_tiles);   /* columns = c2, or group * c2 below */
 /*
  * The same with `group` in2 rows per slice (group * c2 <= 128): b_cols is (m_tiles, group) (any valid column where a slice has
- * fewer rows), and red_slot names slot + 2^24 * (which of the group's rows).
+ * fewer rows), and red_slot names slot + 2^24 * (which of the group's rows).  transposed != 0 writes out (num_w, c2, c1): for
+ * callers that hand the operands over the other way round.
  */
 int eqt_outer_tc_grouped(const float* in1, const float* in2, float* out, float* scratch, int64_t scratch_floats, int64_t n,
                          int32_t rows1, int32_t c1, int32_t rows2, int32_t c2, int32_t group, const int32_t* a_cols,
                          const int32_t* b_cols, int32_t m_tiles, const int32_t* red_ptr, const int32_t* red_slot,
-                         const float* red_scale, int32_t num_w, int32_t* status, void* stream);
+                         const float* red_scale, int32_t num_w, int32_t transposed, int32_t* status, void* stream);
 
 /*
  * eqt_wgrad_tc for callers that cannot hand over a scratch buffer because they cannot allocate device

@@ -56,7 +56,7 @@ def test_vecmat_plan_covers_every_entry_once(kind, cin, cout):
     assert sorted(seen) == list(range(len(i1)))
 
 
-@pytest.mark.parametrize("c1,c2", [(32, 32), (64, 32), (96, 64), (32, 128)])
+@pytest.mark.parametrize("c1,c2", [(32, 32), (64, 32), (96, 64), (32, 128), (64, 128), (256, 64)])
 @pytest.mark.parametrize("kind", ["shared", "own"])
 def test_outer_plan_covers_every_entry_once(kind, c1, c2):
     # the second operand's rows are the table's output rows, so that classes of them meet the same first-operand rows
@@ -64,21 +64,22 @@ def test_outer_plan_covers_every_entry_once(kind, c1, c2):
     i2 = torch.repeat_interleave(torch.arange(num_out), seg.diff())
     w_seg = torch.arange(len(i1) + 1)
     plan = tc.OuterPlan(None, i1, i2, w_seg, len(i1), len(i1), c1, c2, "cpu")
-    chunks, group = c1 // 32, plan.group
+    first, second, cf, cs = (i2, i1, c2, c1) if plan.swapped else (i1, i2, c1, c2)
+    chunks, group = cf // 32, plan.group
     a, b = plan.a_cols.numpy().reshape(-1, 4), plan.b_cols.numpy().reshape(-1, group)
-    assert len(a) == len(b) == plan.m_tiles and group * c2 <= 128
+    assert len(a) == len(b) == plan.m_tiles and group * cs <= 128
     ptr, slot = plan.red_ptr.numpy(), plan.red_slot.numpy()
     for w in range(len(i1)):
         for ch in range(chunks):
             units = slot[ptr[w * chunks + ch]:ptr[w * chunks + ch + 1]]
             assert len(units) == 1
             which, at = units[0] >> 24, units[0] & 0xffffff
-            assert a[at // 4, at % 4] == int(i1[w]) * c1 + 32 * ch and b[at // 4, which] == int(i2[w]) * c2
+            assert a[at // 4, at % 4] == int(first[w]) * cf + 32 * ch and b[at // 4, which] == int(second[w]) * cs
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [512, 700])
-@pytest.mark.parametrize("cin,cout", [(32, 32), (64, 64), (160, 32), (32, 96), (32, 16)])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (64, 64), (160, 32), (32, 96), (64, 128), (128, 32), (32, 16)])
 @pytest.mark.parametrize("kind", ["shared", "own"])
 def test_kernels_on_grouped_tables(kind, cin, cout, n):
     from equitorch_b200.ops import batched_sparse_dense_op as gops
