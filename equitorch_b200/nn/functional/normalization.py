@@ -50,7 +50,7 @@ def batch_rms_norm(input: Tensor, running_squared_norm: Tensor, irreps_info: Irr
     """``out[n, i, c] = x[n, i, c] * weight[k, c] / sqrt(stat[k, c] + eps)``, ``k = irrep(i)``; ``stat`` is the
     batch mean of the (scaled) squared norms when training (``running_squared_norm`` is updated in place),
     else ``running_squared_norm``."""
-    if training and _iops.batch_rms_supported(input, weight):
+    if training and _iops.batch_rms_supported(input, weight, irreps_info.num_irreps):
         out, stat = _BatchRMSNormFused.apply(input, weight, irreps_info, scaled, eps)
         running_squared_norm.data.lerp_(stat.to(running_squared_norm.dtype), momentum)
         return out

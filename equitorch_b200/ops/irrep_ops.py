@@ -72,10 +72,11 @@ def irrep_scale_backward(x: Tensor, s: Tensor, grad: Tensor, irrep_seg: Tensor):
     return gx, gs
 
 
-def batch_rms_supported(x: Tensor, weight) -> bool:
-    """Whether the fused BatchRMSNorm (training mode) takes these operands."""
+def batch_rms_supported(x: Tensor, weight, num_irreps: int) -> bool:
+    """Whether the fused BatchRMSNorm (training mode) takes these operands; a weight that broadcasts to (K, C) does not."""
     return (x.is_cuda and x.ndim == 3 and x.dtype in (torch.float32, torch.float64) and x.shape[0] > 0 and x.shape[2] > 0
-            and x.shape[1] <= 1024 and (weight is None or weight.dtype == x.dtype))
+            and x.shape[1] <= 1024
+            and (weight is None or (weight.dtype == x.dtype and tuple(weight.shape) == (num_irreps, x.shape[2]))))
 
 
 def _batch_rms_scratch(x: Tensor, k: int) -> Tensor:

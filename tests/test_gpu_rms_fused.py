@@ -98,3 +98,15 @@ def test_transposed_gradient_and_features():
         results.append([out, *torch.autograd.grad(out, [a, sg, bn.weight], b)])
     for p, q in zip(*results):
         assert torch.equal(p, q)
+
+
+def test_weights_that_broadcast_are_taken_as_before():
+    from equitorch_b200.nn import functional as F
+    ir, c, n = Irreps("0e+1o+2e"), 8, 11
+    x, _, w, _ = (t.to(DEV) for t in _inputs(ir, n, c, torch.float32))
+    info = _info(ir, torch.float32)
+    for weight in (w[:, :1], w[:1], w[0]):
+        a, b = torch.ones(len(ir), c, device=DEV), torch.ones(len(ir), c, device=DEV)
+        got = F.batch_rms_norm(x, a, info, weight, True, True, 0.1, 1e-5)
+        want = F.batch_rms_norm(x, b, info, weight.expand(len(ir), c), True, True, 0.1, 1e-5)
+        assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max()) and torch.allclose(a, b, rtol=1e-5)
