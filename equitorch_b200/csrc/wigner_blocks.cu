@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(BR_THREADS) block_rotation_kernel(const float*
                                                                     int samples, const __grid_constant__ RowTiles given) {
   extern __shared__ __align__(16) float sm[];
   __shared__ RowTiles tiles;                                         // indexed by lane
-  if (threadIdx.x < sizeof(RowTiles) / 4) reinterpret_cast<uint32_t*>(&tiles)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&given)[threadIdx.x];
+  static_assert(sizeof(RowTiles) % 4 == 0 && sizeof(RowTiles) / 4 > BR_THREADS, "copied by words, more of them than threads");
+  for (int i = threadIdx.x; i < (int)(sizeof(RowTiles) / 4); i += blockDim.x) reinterpret_cast<uint32_t*>(&tiles)[i] = reinterpret_cast<const uint32_t*>(&given)[i];
   __syncthreads();
   const int mat_room = tiles.floats, list_room = (tiles.first[tiles.count] + 3) & ~3;
   uint32_t* list = reinterpret_cast<uint32_t*>(sm);                  // (offset in the matrix << 16) | offset in shared memory

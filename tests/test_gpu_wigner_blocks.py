@@ -66,6 +66,17 @@ def test_rotation_and_its_gradients(name, n, c):
         assert float((got[2] * (1 - mask.to(DEV))).abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("name,c", [("109x0e", 4), ("96x0e", 32), ("60x0e+12x1o+2e", 4), ("9x5o", 8), ("64x0e", 128)])
+def test_as_many_blocks_as_are_accepted(name, c):
+    """Every word of the list of row tiles is in use: the block sizes of the largest matrices that the block kernels take."""
+    ir, n, gen = Irreps(name), 5, torch.Generator().manual_seed(c)
+    assert block_diagonal(ir, DEV).takes(torch.empty(n, ir.dim, c, device=DEV))
+    m = torch.stack([torch.block_diag(*[torch.randn(i.dim, i.dim, generator=gen) for i in ir]) for _ in range(n)]).to(DEV)
+    x = torch.randn(n, ir.dim, c, generator=gen).to(DEV)
+    for t in (m, m.transpose(-1, -2)):
+        assert _err(enn.DenseWignerRotation(ir)(x, t), t.double() @ x.double()) < TOL
+
+
 def test_what_lies_outside_the_blocks_is_not_read():
     ir = Irreps("0e+1o+2e")
     gen = torch.Generator().manual_seed(2)
