@@ -50,8 +50,11 @@ class MixTables:
         self.mix_fwd, self.mix_bwd1, self.mix_bwd2 = (t.to(device) for t in (info.info_M_fwd, info.info_M_bwd1, info.info_M_bwd2))
         # block structure of the weight step for the tensor-core GEMM (None: CUDA-core kernel)
         self.tc_fwd = MixPlan(info.info_M_fwd, out_dims, device) if out_dims is not None else None
+        w, seg = info.info_M_fwd.index2, info.info_M_fwd.seg_out
+        self.rows = w.numel() if w is not None else info.info_M_fwd.out_size if seg is None else int(seg[-1])
 
     def forward(self, s: Tensor, weight: Tensor, mode: str) -> Tensor:
+        assert s.shape[1] == self.rows, f"{s.shape[1]} rows for a table of {self.rows}"
         return _mix(s, weight, self.mix_fwd, mode, self.tc_fwd)
 
     def grad_weight(self, s: Tensor, grad: Tensor, weight: Tensor, mode: str) -> Tensor:

@@ -22,16 +22,19 @@ class PathPlan:
     second operand irrep - and ``scales`` the factors on their Clebsch-Gordan blocks."""
 
     def __init__(self, paths: Sequence[Tuple[int, int, int]], scales: Sequence[float], irreps_out, irreps1, irreps2, device):
-        self.device, self._fits, self.mix = torch.device(device), {}, None      # mix: tables of the weight step ('uv')
+        self.device, self._fits, self.mix = torch.device(device), {}, None      # mix: tables of the weight step ('uv'), False: other rows
         ls = [[ir.l for ir in irs] for irs in (irreps_out, irreps1, irreps2)]
-        self.usable = len(paths) > 0 and all(0 <= l <= PATH_MAX_L for degrees in ls for l in degrees)
+        # a path of degrees that do not couple has no block (its entries in the layer's tables are none either)
+        self.usable = (len(paths) > 0 and all(0 <= l <= PATH_MAX_L for degrees in ls for l in degrees)
+                       and all(abs(ls[1][i] - ls[2][j]) <= ls[0][k] <= ls[1][i] + ls[2][j] for k, i, j in paths))
         if not self.usable:
             return
         start = [np.cumsum([0] + [2 * l + 1 for l in degrees]).tolist() for degrees in ls]
         # rows of the intermediate: per output irrep, component by component, its paths ordered by (i, j, weight)
-        row, fan, num_rows = {}, {}, 0
+        row, fan, num_rows, self.row_weights = {}, {}, 0, []
         for k, l in enumerate(ls[0]):
             mine = sorted((w for w in range(len(paths)) if paths[w][0] == k), key=lambda w: (paths[w][1], paths[w][2], w))
+            self.row_weights += [mine] * (2 * l + 1)              # of every output component
             row.update((w, num_rows + n) for n, w in enumerate(mine))
             fan[k] = len(mine)
             num_rows += len(mine) * (2 * l + 1)
@@ -58,6 +61,17 @@ class PathPlan:
                                            len(paths), len(ls[0]), len(ls[1]), num_rows)
         self.ref = C.byref(self.struct)
 
+    def rows_match(self, info) -> bool:
+        """Whether the rows of the intermediate that ``info`` (the forward table of the weight step) consumes are the rows
+        of this plan.  They are not where a path is listed twice: the table then has a row per run of a weight among the
+        entries of a component, several for one (component, weight)."""
+        if not self.usable or info.index1 is not None or info.scale is not None or info.gather_index is not None \
+                or info.index_out is not None or info.out_size != len(self.row_weights):
+            return False
+        seg = list(range(info.out_size + 1)) if info.seg_out is None else info.seg_out.tolist()
+        weights = list(range(seg[-1])) if info.index2 is None else info.index2.tolist()
+        return len(weights) == self.num_rows and [weights[a:b] for a, b in zip(seg, seg[1:])] == self.row_weights
+
     def supported(self, x: Tensor, y: Tensor, w: Tensor) -> bool:
         if not (self.usable and x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and x.dtype == y.dtype == w.dtype
                 and x.ndim == 3 and y.ndim == 2 and x.shape[0] == y.shape[0] and x.shape[0] > 0 and w.ndim in (2, 3)
@@ -70,7 +84,6 @@ class PathPlan:
             self._fits[key] = all(_lib.lib().eqt_so3_uu_scratch_floats(self.ref, n, x.shape[2], int(w.ndim == 3),
                                                                        _lib.DTYPE_CODE[x.dtype]) >= 0 for n in (1, 1 << 30))
         return self._fits[key] and (x.data_ptr() | w.data_ptr()) % 16 == 0
-
 
     def uv_supported(self, x: Tensor, y: Tensor, w: Tensor) -> bool:
         """Whether the channel-wise kernels of the 'uv' layer take these operands (float32, weights shared by the batch)."""

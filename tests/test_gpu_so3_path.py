@@ -10,9 +10,9 @@ import torch
 from equitorch_b200 import _lib
 from equitorch_b200 import nn as enn
 from equitorch_b200.nn.functional.linears import tensor_product_u1u, tensor_product_u1v
+from equitorch_b200.ops.so3_path_op import PathPlan
 from oracle import tensor_products as otp
 
-pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 # float32: an element is a sum of up to 40 terms of random sign, a weight gradient of 40 n; bfloat16: one rounding of the result
 BOUND = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -7}
@@ -22,6 +22,7 @@ def _rel(a, b):
     return float((a.detach().double().cpu() - b.detach().double()).abs().max() / b.detach().double().abs().max())
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("per_sample", [False, True])
 @pytest.mark.parametrize("ir,ir_y,n,c", [("0e+1o", "0e+1o", 1, 4), ("0e+1o+2e", "0e+1o+2e", 7, 12), ("0e+1o+2e+3o", "0e+1o+2e+3o", 129, 64),
@@ -49,6 +50,7 @@ def test_one_pass_kernels(ir, ir_y, n, c, per_sample, dtype):
     assert torch.equal(gy, got[2])
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("ir,ir_y,n,c,c_out", [("0e+1o", "0e+1o", 1, 4, 8), ("0e+1o+2e", "0e+1o+2e", 7, 12, 20),
                                                ("0e+1o+2e+3o", "0e+1o+2e+3o", 513, 64, 32), ("4x0e+2x1o+2e", "0e+1o+2e", 1501, 32, 64),
                                                ("0o+1e+2e+3e", "0e+1e+2o+3e", 300, 16, 16), ("0e+1o+2e+3o", "0e+1o+2e+3o", 2003, 128, 48)])
@@ -72,6 +74,7 @@ def test_channel_mixing_layer(ir, ir_y, n, c, c_out):
     assert torch.equal(gy, got[2])
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["uu", "uv"])
 def test_differentiated_backward_pass(mode):
     g = torch.Generator().manual_seed(0)
@@ -89,3 +92,42 @@ def test_differentiated_backward_pass(mode):
         return torch.autograd.grad(sum((t * t).sum() for t in first), leaves)
     for a, b in zip(second(layer), second(lambda x, y, w: product(x, y, w, *infos))):
         assert _rel(a, b.cpu()) < 1e-5
+
+
+# (irreps, paths, whether the one-pass kernels take them, whether their rows are the rows of the layer's weight step)
+PATH_LISTS = [("0e+1e", None, True, True), ("0e+1o+2e+3o", None, True, True), ("0e", None, True, True),
+              ("0e+1e", [(1, 0, 1), (1, 1, 0), (0, 0, 0)], True, True), ("2x0e", [(1, 1, 1), (0, 0, 0)], True, True),
+              ("0e+1e+2e", [(2, 1, 1), (0, 2, 2), (2, 2, 0), (1, 1, 1), (2, 0, 2)], True, True),
+              ("0e+1e", [(1, 1, 0), (0, 0, 0), (1, 1, 0)], True, True),                    # twice, one entry a component
+              ("0e+1e", [(1, 1, 1), (1, 1, 1)], True, False), ("0e+1e", [(0, 0, 0), (1, 1, 1), (1, 0, 1), (1, 1, 1)], True, False),
+              ("0e+1e", [(0, 0, 0), (1, 0, 0), (0, 1, 1)], False, False)]                  # 0 x 0 -> 1 does not couple
+
+
+@pytest.mark.parametrize("ir,path,usable,match", PATH_LISTS)
+def test_rows_of_the_plan_and_of_the_weight_step(ir, path, usable, match):
+    layer = enn.SO3Linear(ir, ir, ir, 8, 8, feature_mode="uv", path=path)
+    plan, table = PathPlan(*layer._paths, layer.irreps_out, layer.irreps_in1, layer.irreps_in2, "cpu"), layer.tp_info_forward.info_M_fwd
+    assert plan.usable == usable and plan.rows_match(table) == match
+    if match:                     # the rows in number and, row by row, in what they are multiplied with
+        rows = [w for weights in plan.row_weights for w in weights]
+        assert len(rows) == plan.num_rows and rows == (list(range(len(rows))) if table.index2 is None else table.index2.tolist())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["uu", "uv"])
+@pytest.mark.parametrize("n,c", [(5, 8), (600, 32)])
+@pytest.mark.parametrize("ir,path,usable,match", PATH_LISTS[:-1])        # the composition refuses the last
+def test_path_lists(ir, path, usable, match, n, c, mode):
+    g = torch.Generator().manual_seed(n)
+    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode=mode, path=path).to(DEV)
+    dim = layer.irreps_in1_dim
+    leaves = [torch.randn(n, dim, c, generator=g), torch.randn(n, dim, generator=g), torch.randn(*layer.weight_shape, generator=g)]
+    cot = torch.randn(n, dim, c, generator=g)
+    lo = [t.double().requires_grad_(True) for t in leaves]
+    want = otp.so3_linear_dense(*lo, ir, ir, ir, feature_mode=mode, path=path)
+    want = [want, *torch.autograd.grad(want, lo, cot.double())]
+    lg = [t.to(DEV).requires_grad_(True) for t in leaves]
+    got = layer(*lg)
+    got = [got, *torch.autograd.grad(got, lg, cot.to(DEV))]
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and _rel(a, b) < BOUND[torch.float32]
