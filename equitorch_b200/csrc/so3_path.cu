@@ -98,11 +98,11 @@ constexpr int AHEAD = 8;
 template <typename T>
 struct WeightStream {
   T* ring;                  // this thread's column, AHEAD rows
-  const T* w;               // the thread's channels of weight 0
+  const T* w;               // the thread's channels of weight 0; NULL: the weights are not wanted, what next() gives is not used
   const eqt_path* paths;
   int row, c, count, at;
   __device__ __forceinline__ void issue(int q) {
-    if (q < count) copy_v(ring + (q % AHEAD) * row, w + (int64_t)paths[q].weight * c);
+    if (q < count && w) copy_v(ring + (q % AHEAD) * row, w + (int64_t)paths[q].weight * c);
     copy_commit();
   }
   // everything committed before begin() - the sample's columns - is complete once the first weights are
@@ -353,6 +353,8 @@ __device__ __forceinline__ void backward_block(const PathArgs& a, const eqt_path
     for (int m = 0; m < 2 * L1 + 1; ++m) store_v<T>(gxout + (int64_t)(b.offset + m) * a.c, gx[m]);
 }
 
+// An operand that none of the wanted gradients takes may be NULL: its columns are then left as they are and reach only
+// gradients that are not stored.
 template <typename T>
 __global__ void __launch_bounds__(128, 3) so3_uu_backward_kernel(PathArgs a, int per_sample) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -384,13 +386,15 @@ __global__ void __launch_bounds__(128, 3) so3_uu_backward_kernel(PathArgs a, int
     const int64_t n = n0 + slot;
     __syncthreads();                                   // tables loaded / harmonics and partial gy of the previous samples have been read
     if (slot < here) {
-      for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
+      if (x)
+        for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
       for (int i = 0; i < a.dout; ++i) copy_v(gc + i * row, g + (n * a.dout + i) * a.c + ch);
-      ws.w = static_cast<const T*>(a.w) + (per_sample ? n * a.p * a.c : 0) + ch;
+      ws.w = a.w ? static_cast<const T*>(a.w) + (per_sample ? n * a.p * a.c : 0) + ch : nullptr;
       ws.begin();
       for (int i = 0; i < a.d2; ++i) gy_all[i * threads + tid] = 0.f;
     }
-    for (int i = tid; i < here * a.d2; i += threads) ys[i] = static_cast<float>(y[n0 * a.d2 + i]);
+    if (y)
+      for (int i = tid; i < here * a.d2; i += threads) ys[i] = static_cast<float>(y[n0 * a.d2 + i]);
     __syncthreads();
     if (slot < here) {
       T* gx = a.gx ? static_cast<T*>(a.gx) + n * a.d1 * a.c + ch : nullptr;
@@ -563,13 +567,15 @@ __global__ void __launch_bounds__(128, 3) so3_uv_backward_kernel(PathArgs a) {
     const int64_t n = n0 + slot;
     __syncthreads();                                   // tables loaded / harmonics and partial gy of the previous samples have been read
     if (slot < here) {
-      for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
+      if (x)
+        for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
       copy_commit();
       rs.g = static_cast<const float*>(a.g) + n * a.num_rows * a.c + ch;
       rs.begin();
       for (int i = 0; i < a.d2; ++i) gy_all[i * threads + tid] = 0.f;
     }
-    for (int i = tid; i < here * a.d2; i += threads) ys[i] = y[n0 * a.d2 + i];
+    if (y)
+      for (int i = tid; i < here * a.d2; i += threads) ys[i] = y[n0 * a.d2 + i];
     __syncthreads();
     if (slot < here) {
       float* gx = a.gx ? static_cast<float*>(a.gx) + n * a.d1 * a.c + ch : nullptr;
@@ -705,7 +711,7 @@ extern "C" int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, c
   using namespace eqt;
   if (int rc = path_check(table, n, channels, dtype)) return rc;
   if (n == 0) return EQT_OK;
-  if (!x || !y || !w || !g) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  if (!g || (gx && (!y || !w)) || (gy && (!x || !w)) || (gw && (!x || !y))) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   const bool shared_gw = gw && !per_sample_weight;
   if (shared_gw) {
     const int64_t need = eqt_so3_uu_scratch_floats(table, n, channels, 0, dtype);
@@ -752,7 +758,7 @@ extern "C" int eqt_so3_uv_backward(const eqt_path_table* table, const float* x, 
   using namespace eqt;
   if (int rc = path_check(table, n, channels, EQT_F32)) return rc;
   if (n == 0) return EQT_OK;
-  if (!x || !y || !grad_rows) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  if (!grad_rows || (gx && !y) || (gy && !x)) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   PathArgs a{};
   a.x = x; a.y = y; a.g = grad_rows; a.gx = gx; a.gy = gy;
   return path_run(UV_BACKWARD, table, false, false, n, channels, EQT_F32, a, static_cast<cudaStream_t>(stream), nullptr);

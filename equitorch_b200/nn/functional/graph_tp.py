@@ -57,11 +57,11 @@ class MixTables:
         assert s.shape[1] == self.rows, f"{s.shape[1]} rows for a table of {self.rows}"
         return _mix(s, weight, self.mix_fwd, mode, self.tc_fwd)
 
-    def grad_weight(self, s: Tensor, grad: Tensor, weight: Tensor, mode: str) -> Tensor:
+    def grad_weight(self, s: Tensor, grad: Tensor, num_paths: int, mode: str) -> Tensor:
         tcw, b2 = self.tc_fwd, self.mix_bwd2
         if (mode == "uv" and tcw is not None and tcw.regular and grad.dtype == torch.float32
-                and _tc_supported_w(weight.shape[-2], weight.shape[-1])):
-            return wgrad_tc(s, grad, tcw, weight.shape[0])
+                and _tc_supported_w(s.shape[-1], grad.shape[-1])):
+            return wgrad_tc(s, grad, tcw, num_paths)
         if mode == "uv":   # (P, Cout, Cin) summed over nodes, then transposed to the weight's layout
             gw = _ops.indexed_outer_scale_gather(grad, s, b2.scale, b2.index1, b2.index2, b2.seg_out,
                                                  out_accumulated=True, out_size=b2.out_size)
@@ -128,7 +128,7 @@ class FusedGraphOps:
     def grad_weight(self, state, grad: Tensor) -> Tensor:
         _, _, weight, s = state
         with _profile.timed("weight_grad"):
-            return self.plan.grad_weight(s, grad, weight, self.mode)
+            return self.plan.grad_weight(s, grad, weight.shape[0], self.mode)
 
     def grad_y(self, state, grad: Tensor) -> Tensor:
         node_x, y, weight, _ = state

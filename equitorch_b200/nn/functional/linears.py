@@ -163,24 +163,30 @@ def tensor_product_uu1(input1, input2, weight, tp_info_forward, tp_info_backward
 so3_linear_uu = tensor_product_u1u
 
 
+def _dense(*tensors):
+    return [None if t is None else t.contiguous() for t in tensors]
+
+
 class SO3LinearUU(Function):
     """:func:`tensor_product_u1u` in one kernel per direction (``plan``: the layer's tables on the device).  A backward
-    pass that is itself differentiated is composed of the differentiable products instead."""
+    pass that is itself differentiated is composed of the differentiable products instead, on the operands as they were
+    given: a contiguous copy made in here has no history."""
 
     @staticmethod
     def forward(ctx, input1, input2, weight, plan, infos):
-        input1, input2, weight = input1.contiguous(), input2.contiguous(), weight.contiguous()
-        ctx.save_for_backward(input1, input2, weight)
-        ctx.plan, ctx.infos = plan, infos
-        return _path.so3_uu_forward(plan, input1, input2, weight)
+        n1, n2, nw = ctx.needs_input_grad[:3]
+        ctx.save_for_backward(input1 if n2 or nw else None, input2 if n1 or nw else None, weight if n1 or n2 else None)
+        ctx.plan, ctx.infos, ctx.weight_ndim = plan, infos, weight.ndim
+        return _path.so3_uu_forward(plan, *_dense(input1, input2, weight))
 
     @staticmethod
     def backward(ctx, grad):
         input1, input2, weight = ctx.saved_tensors
         need = ctx.needs_input_grad[:3]
-        grad = grad.contiguous()
-        if not torch.is_grad_enabled() and grad.dtype == input1.dtype and grad.data_ptr() % 16 == 0:
-            return (*_path.so3_uu_backward(ctx.plan, input1, input2, weight, grad, need), None, None)
+        if not torch.is_grad_enabled():
+            operands = _dense(input1, input2, weight, grad)
+            if _path.aligned(*operands):
+                return (*_path.so3_uu_backward(ctx.plan, *operands, need, ctx.weight_ndim == 3), None, None)
         f = ctx.infos[0]
         r1, r2 = _rot(ctx.infos)
         g1 = tensor_product_1uu(input2, grad, weight, *r1) if need[0] else None
@@ -188,7 +194,7 @@ class SO3LinearUU(Function):
         gw = None
         if need[2]:
             inter = sparse_vecsca(input1, input2, *_mij(f, 0))
-            gw = sparse_mul(grad, inter, *_m(f, 2), out_accumulated=weight.ndim == 2)
+            gw = sparse_mul(grad, inter, *_m(f, 2), out_accumulated=ctx.weight_ndim == 2)
         return g1, g2, gw, None, None
 
 
@@ -322,41 +328,31 @@ so3_linear_uv = tensor_product_u1v
 
 class SO3LinearUV(Function):
     """:func:`tensor_product_u1v` with weights shared by the batch: rows of the intermediate from straight-line
-    Clebsch-Gordan blocks, the GEMM, and both operand gradients from one pass over the gradient of the rows.  A backward
-    pass that is itself differentiated is composed of the differentiable products instead."""
+    Clebsch-Gordan blocks, the GEMM, and both operand gradients from one pass over the gradient of the rows.  The rows are
+    the intermediate of the two-step product, row by row, and an output like it: a backward pass that is itself
+    differentiated is that product's."""
 
     @staticmethod
     def forward(ctx, input1, input2, weight, plan, mix, infos):
-        input1, input2, weight = input1.contiguous(), input2.contiguous(), weight.contiguous()
-        rows = _path.so3_uv_expand(plan, input1, input2)
-        out = mix.forward(rows, weight, "uv")
-        ctx.save_for_backward(input1, input2, weight, rows if ctx.needs_input_grad[2] else None)
-        ctx.plan, ctx.mix, ctx.infos = plan, mix, infos
-        return out
+        x, y, w = _dense(input1, input2, weight)
+        rows = _path.so3_uv_expand(plan, x, y)
+        save_for_tp_backward(ctx, input1, input2, weight, rows, infos)
+        ctx.plan, ctx.mix = plan, mix
+        return mix.forward(rows, w, "uv"), rows
 
     @staticmethod
-    def backward(ctx, grad):
-        input1, input2, weight, rows = ctx.saved_tensors
+    def backward(ctx, grad, grad_rows):
         need = ctx.needs_input_grad[:3]
-        grad = grad.contiguous()
-        g1 = g2 = gw = None
-        if not torch.is_grad_enabled() and grad.dtype == torch.float32 and grad.data_ptr() % 16 == 0:
-            if need[2]:
-                gw = ctx.mix.grad_weight(rows, grad, weight, "uv")
-            if need[0] or need[1]:
-                g1, g2 = _path.so3_uv_backward(ctx.plan, input1, input2, ctx.mix.grad_inter(grad, weight, "uv"), need[:2])
-            return g1, g2, gw, None, None, None
-        f = ctx.infos[0]
-        r1, r2 = _rot(ctx.infos)
-        wt = weight.transpose(-1, -2).contiguous()
-        if need[0]:
-            g1 = tensor_product_1vu(input2, grad, wt, *r1)
-        if need[1]:
-            g2 = tensor_product_vu1(grad, input1, wt, *r2)
-        if need[2]:
-            inter = sparse_vecsca(input1, input2, *_mij(f, 0))
-            gw = sparse_outer(grad, inter, *_m(f, 2), out_accumulated=True).transpose(-1, -2).contiguous()
-        return g1, g2, gw, None, None, None
+        if grad is not None and grad_rows is None and not torch.is_grad_enabled():
+            input1, input2, weight, rows = ctx.saved_tensors
+            x, y, w, grad = _dense(input1, input2, weight, grad)
+            if _path.aligned(x, rows, grad):
+                g1 = g2 = None
+                gw = ctx.mix.grad_weight(rows, grad, ctx.plan.sizes[3], "uv") if need[2] else None
+                if need[0] or need[1]:
+                    g1, g2 = _path.so3_uv_backward(ctx.plan, x, y, ctx.mix.grad_inter(grad, w, "uv"), need[:2])
+                return g1, g2, gw, None, None, None
+        return TensorProductU1VDummy.backward(ctx, grad, grad_rows)
 
 
 # ------------------------------------------------------------------------------------------

@@ -101,7 +101,7 @@ class SO3Linear(_WeightedTableModule):
                     plan.mix = plan.rows_match(self.tp_info_forward.info_M_fwd) and \
                         MixTables(self.tp_info_forward, input1.device, [ir.dim for ir in self.irreps_out])
                 if plan.mix:
-                    return SO3LinearUV.apply(input1, input2, weight, plan, plan.mix, infos)
+                    return SO3LinearUV.apply(input1, input2, weight, plan, plan.mix, infos)[0]
         fn = so3_linear_uu if self.feature_mode == "uu" else so3_linear_uv
         return fn(input1, input2, weight, self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2)
 

@@ -108,14 +108,21 @@ def so3_uv_expand(plan: PathPlan, x: Tensor, y: Tensor) -> Tensor:
     return rows
 
 
-def so3_uv_backward(plan: PathPlan, x: Tensor, y: Tensor, grad_rows: Tensor,
+def aligned(*tensors: Optional[Tensor]) -> bool:
+    return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def so3_uv_backward(plan: PathPlan, x: Optional[Tensor], y: Optional[Tensor], grad_rows: Tensor,
                     need: Tuple[bool, bool]) -> Tuple[Optional[Tensor], Optional[Tensor]]:
-    """Gradients of :func:`so3_uv_expand` with respect to x and y, from one pass over ``grad_rows``."""
-    n, _, c = x.shape
-    gx, gy = (torch.empty_like(t) if wanted else None for t, wanted in zip((x, y), need))
-    with _lib.on_device(x.device):
-        _lib.check(_lib.lib().eqt_so3_uv_backward(plan.ref, x.data_ptr(), y.data_ptr(), grad_rows.data_ptr(), _lib.ptr(gx), _lib.ptr(gy),
-                                                  n, c, _lib.stream_ptr(x.device)), "eqt_so3_uv_backward")
+    """Gradients of :func:`so3_uv_expand` with respect to x and y, from one pass over ``grad_rows``; the gradient of x takes
+    y and that of y takes x."""
+    n, _, c = grad_rows.shape
+    gx = grad_rows.new_empty(n, plan.sizes[0], c) if need[0] else None
+    gy = grad_rows.new_empty(n, plan.sizes[1]) if need[1] else None
+    dev = grad_rows.device
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().eqt_so3_uv_backward(plan.ref, _lib.ptr(x), _lib.ptr(y), grad_rows.data_ptr(), _lib.ptr(gx), _lib.ptr(gy),
+                                                  n, c, _lib.stream_ptr(dev)), "eqt_so3_uv_backward")
     return gx, gy
 
 
@@ -130,17 +137,19 @@ def so3_uu_forward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor) -> Tensor:
     return out
 
 
-def so3_uu_backward(plan: PathPlan, x: Tensor, y: Tensor, w: Tensor, g: Tensor,
-                    need: Tuple[bool, bool, bool]) -> Tuple[Optional[Tensor], Optional[Tensor], Optional[Tensor]]:
-    """Gradients with respect to x, y and w (``None`` where not needed), all from one launch."""
-    n, _, c = x.shape
-    gx, gy, gw = (torch.empty_like(t) if wanted else None for t, wanted in zip((x, y, w), need))
-    lib, scratch, floats = _lib.lib(), None, 0
-    with _lib.on_device(x.device):
-        if need[2] and w.ndim == 2:
-            floats = int(lib.eqt_so3_uu_scratch_floats(plan.ref, n, c, 0, _lib.DTYPE_CODE[x.dtype]))
-            scratch = torch.empty(floats, dtype=torch.float32, device=x.device)
-        _lib.check(lib.eqt_so3_uu_backward(plan.ref, x.data_ptr(), y.data_ptr(), w.data_ptr(), g.data_ptr(), _lib.ptr(gx),
-                                           _lib.ptr(gy), _lib.ptr(gw), _lib.ptr(scratch), floats, n, c, int(w.ndim == 3),
-                                           _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(x.device)), "eqt_so3_uu_backward")
+def so3_uu_backward(plan: PathPlan, x: Optional[Tensor], y: Optional[Tensor], w: Optional[Tensor], g: Tensor, need: Tuple[bool, bool, bool],
+                    per_sample: bool) -> Tuple[Optional[Tensor], Optional[Tensor], Optional[Tensor]]:
+    """Gradients with respect to x, y and w (``None`` where not needed), all from one launch; each takes the other two."""
+    n, _, c = g.shape
+    d1, d2, _, p = plan.sizes
+    shapes = ((n, d1, c), (n, d2), (n, p, c) if per_sample else (p, c))
+    gx, gy, gw = (g.new_empty(shape) if wanted else None for shape, wanted in zip(shapes, need))
+    lib, scratch, floats, dev = _lib.lib(), None, 0, g.device
+    with _lib.on_device(dev):
+        if need[2] and not per_sample:
+            floats = int(lib.eqt_so3_uu_scratch_floats(plan.ref, n, c, 0, _lib.DTYPE_CODE[g.dtype]))
+            scratch = torch.empty(floats, dtype=torch.float32, device=dev)
+        _lib.check(lib.eqt_so3_uu_backward(plan.ref, _lib.ptr(x), _lib.ptr(y), _lib.ptr(w), g.data_ptr(), _lib.ptr(gx), _lib.ptr(gy),
+                                           _lib.ptr(gw), _lib.ptr(scratch), floats, n, c, int(per_sample), _lib.DTYPE_CODE[g.dtype],
+                                           _lib.stream_ptr(dev)), "eqt_so3_uu_backward")
     return gx, gy, gw

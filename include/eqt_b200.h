@@ -344,7 +344,8 @@ int64_t eqt_wgrad_tc_static_capacity(void);
  * float32 or bfloat16 storage, float32 arithmetic.  The table lists the paths (output irrep, x irrep, y irrep, weight)
  * with the factor of their Clebsch-Gordan block, once in blocks of one output irrep each (every output irrep has a
  * block, of zero paths if nothing reaches it) and once in blocks of one x irrep each; device memory.  Every weight
- * belongs to exactly one path.  Gradients that are NULL are not written.  Shared weights need
+ * belongs to exactly one path.  Gradients that are NULL are not written, and an operand that no written gradient takes
+ * (each takes the other two) may be NULL.  Shared weights need
  * eqt_so3_uu_scratch_floats() floats of scratch (the sums of the thread blocks, added in a fixed order); -1 means that
  * this many channels are not supported (a multiple of 4 up to 512 whose columns fit shared memory).  Operands with a
  * channel axis must be aligned to four elements.
@@ -382,7 +383,7 @@ int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, const void* 
  * The channel-wise half of the layer with full channel mixing ('uv' SO3Linear), float32, same tables:
  *   expand:   rows[n, r, c] = sum_t s_t x[n, M1_t, c] y[n, M2_t] over the entries of row r = (output component, path)
  *   backward: gx and gy from the gradient of the rows, in one pass over it
- * rows / grad_rows (n, num_rows, c); gx (n, d1, c) and gy (n, d2) may be NULL.  eqt_so3_uv_supported: 1 if this many
+ * rows / grad_rows (n, num_rows, c); gx (n, d1, c) and gy (n, d2) may be NULL, x without gy and y without gx too.  eqt_so3_uv_supported: 1 if this many
  * channels fit.
  * replaces: the vec-scalar step of TensorProductU1V and the three-step TensorProductVU1 adjoint
  *   (equitorch/nn/functional/linears.py:254-336, 415-492).

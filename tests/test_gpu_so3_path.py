@@ -131,3 +131,52 @@ def test_path_lists(ir, path, usable, match, n, c, mode):
     got = [got, *torch.autograd.grad(got, lg, cot.to(DEV))]
     for a, b in zip(got, want):
         assert a.shape == b.shape and _rel(a, b) < BOUND[torch.float32]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["uu", "uv"])
+@pytest.mark.parametrize("n,c,per_sample", [(33, 8, False), (600, 32, False), (33, 8, True)])
+def test_second_derivatives_with_operands_that_are_views(mode, n, c, per_sample):
+    """A transposed x, a slice as y and a strided weight: gradients of the energy and of a loss on them (training on forces)
+    against the composed products."""
+    g = torch.Generator().manual_seed(n)
+    ir = "0e+1o+2e"
+    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode=mode).to(DEV)
+    shape = ((n,) if per_sample else ()) + tuple(layer.weight_shape)
+    leaves = [t.to(DEV).requires_grad_(True) for t in (torch.randn(n, c, 9, generator=g), torch.randn(n, 13, generator=g),
+                                                       torch.randn(*shape, generator=g), torch.randn(n, 9, c, generator=g))]
+    product = tensor_product_u1u if mode == "uu" else tensor_product_u1v
+    infos = (layer.tp_info_forward, layer.tp_info_backward1, layer.tp_info_backward2)
+
+    def both(fn):
+        x0, y0, w0, cot = leaves
+        x, y, w = x0.transpose(1, 2), y0[:, 4:], torch.cat([w0, w0], dim=-1)[..., :c]
+        assert not (x.is_contiguous() or y.is_contiguous() or w.is_contiguous())
+        first = torch.autograd.grad(fn(x, y, w), [x0, y0, w0], cot, create_graph=True)
+        return [t.detach() for t in first] + list(torch.autograd.grad(sum((t * t).sum() for t in first), leaves))
+    for a, b in zip(both(layer), both(lambda x, y, w: product(x, y, w, *infos))):
+        assert _rel(a, b.cpu()) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,dtype,per_sample", [("uu", torch.float32, False), ("uu", torch.bfloat16, True), ("uv", torch.float32, False)])
+def test_gradients_of_some_operands(mode, dtype, per_sample):
+    """Every subset of operands that want a gradient: the same values, and no operand is kept that none of them takes."""
+    g = torch.Generator().manual_seed(5)
+    ir, n, c = "0e+1o+2e", 301, 32
+    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode=mode).to(DEV)
+    shape = ((n,) if per_sample else ()) + tuple(layer.weight_shape)
+    values = [torch.randn(*s, generator=g).to(dtype).to(DEV) for s in ((n, 9, c), (n, 9), shape)]
+    cot = torch.randn(n, 9, c, generator=g).to(dtype).to(DEV)
+
+    def run(wanted, after=lambda out, operands: None):
+        operands = [v.clone().requires_grad_(k in wanted) for k, v in enumerate(values)]
+        out = layer(*operands)
+        after(out, operands)
+        return dict(zip(wanted, torch.autograd.grad(out, [operands[k] for k in wanted], cot)))
+    full = run((0, 1, 2))
+    for wanted in ((0,), (1,), (2,), (0, 1), (0, 2), (1, 2)):
+        part = run(wanted)
+        assert all(torch.equal(part[k], full[k]) for k in wanted)
+    if mode == "uv":                   # the rows are kept for the weight gradient, so that x may change in place
+        assert torch.equal(run((2,), lambda out, operands: operands[0].mul_(2))[2], full[2])
