@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 from collections import OrderedDict
-from typing import Dict, Optional
+from typing import Optional
 
 import numpy as np
 import torch
@@ -22,7 +22,6 @@ from .mix_tc_op import status_flag
 MIN_BATCH = 512          # below this the table-driven kernels are as fast and have no set-up cost
 MAX_PLANS = 256
 _plans: "OrderedDict[tuple, tuple]" = OrderedDict()
-_scratch: Dict[torch.device, Tensor] = {}
 
 
 def _cached(kind, dev, tensors, extra, build):
@@ -43,14 +42,6 @@ def _cached(kind, dev, tensors, extra, build):
 
 def _host(t: Optional[Tensor], default: np.ndarray) -> np.ndarray:
     return default if t is None else t.detach().cpu().numpy()
-
-
-def _buffer(dev, floats: int) -> Tensor:
-    buf = _scratch.get(dev)
-    if buf is None or buf.numel() < floats:
-        buf = torch.empty(max(floats, 1), dtype=torch.float32, device=dev)
-        _scratch[dev] = buf
-    return buf
 
 
 def _same_reads(reads):
@@ -203,7 +194,7 @@ def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Te
         a, b, rows1, c1, rows2, c2 = b, a, rows2, c2, rows1, c1
     with _lib.on_device(dev):
         need = int(_lib.lib().eqt_outer_tc_scratch_floats(n, plan.group * c2, max(plan.m_tiles, 1)))
-        scratch = _buffer(dev, max(need, 1))
+        scratch = torch.empty(max(need, 1), dtype=torch.float32, device=dev)     # of this call: calls on other streams may overlap it
         _lib.check(_lib.lib().eqt_outer_tc_grouped(a.data_ptr(), b.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(),
                                                    n, rows1, c1, rows2, c2, plan.group, plan.a_cols.data_ptr(),
                                                    plan.b_cols.data_ptr(), plan.m_tiles, plan.red_ptr.data_ptr(),

@@ -95,21 +95,6 @@ def mix_tc_transposed(g: Tensor, weight: Tensor, plan: MixPlan) -> Tensor:
     return out
 
 
-_scratch = {}
-
-
-def wgrad_scratch(device, cout: int, need: int = 0) -> Tensor:
-    """Per-device scratch for the split reduction of :func:`wgrad_tc` (at least 128 * cout floats per SM)."""
-    device = torch.device(device)
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
-    need = max(need, 128 * cout * sms)
-    buf = _scratch.get(device)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(need, dtype=torch.float32, device=device)
-        _scratch[device] = buf
-    return buf
-
-
 def wgrad_tc(s: Tensor, g: Tensor, plan: MixPlan, num_paths: int) -> Tensor:
     """``gw[p] = sum_n sum_{rows r of path p} s[n, r, :]^T g[n, M(r), :]`` -> (num_paths, cin, cout), deterministic."""
     dev = _lib.require_cuda(s, g)
@@ -123,7 +108,7 @@ def wgrad_tc(s: Tensor, g: Tensor, plan: MixPlan, num_paths: int) -> Tensor:
         need = int(_lib.lib().eqt_wgrad_tc_scratch_floats(n, cin, cout, blocks, len(blocks)))
         if need < 0:
             raise _lib.EqtError("eqt_wgrad_tc refuses these blocks")
-        scratch = wgrad_scratch(dev, cout, need)
+        scratch = torch.empty(need, dtype=torch.float32, device=dev)       # of this call: calls on other streams may overlap it
         _lib.check(_lib.lib().eqt_wgrad_tc(s.data_ptr(), g.data_ptr(), packed.data_ptr(), scratch.data_ptr(),
                                            scratch.numel(), n, rows, plan.comps, cin, cout, blocks, len(blocks),
                                            status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_wgrad_tc")

@@ -134,3 +134,35 @@ def test_tensor_product_uvw_sliced_over_samples(monkeypatch):
     ro = torch.autograd.grad(ref, [ao, bo, wo], cot[:m].double())
     for u, v in zip((gx1[:m], gx2[:m], gw), ro):
         assert _rel(u, v) < 1e-5
+
+
+@pytest.mark.parametrize("which", ["indexed", "blocks"])
+def test_weight_gradients_on_two_streams(which):
+    """Two streams at once, each with its own inputs: every result is the one of the call alone (the partial sums of the
+    split reduction belong to the call)."""
+    from equitorch_b200.irreps import Irreps
+    from equitorch_b200.ops.mix_tc_op import MixPlan, wgrad_tc
+    from equitorch_b200.tables import tp_infos
+    g = torch.Generator(device=DEV).manual_seed(0)
+    n, c = 20000, 64
+    ir = Irreps("0e+1o+2e")
+    table, _, _, paths = tp_infos(ir, ir, ir)
+    plan = MixPlan(table.info_M_fwd.to(DEV), [i.dim for i in ir], DEV)
+    index, seg = torch.arange(9, device=DEV), torch.arange(10, device=DEV)
+    inputs = [[torch.randn(n, rows, c, generator=g, device=DEV) for rows in ((9, 9) if which == "indexed" else (plan.rows, 9))] for _ in range(2)]
+
+    def call(a, b):
+        if which == "blocks":
+            return wgrad_tc(a, b, plan, paths)
+        return gops.indexed_outer_scale_gather(a, b, None, index, index, seg, out_accumulated=True)
+    want = [call(*pair) for pair in inputs]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(40):
+        for k, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[k].append(call(*inputs[k]))
+    torch.cuda.synchronize()
+    for k in range(2):
+        assert all(torch.equal(t, want[k]) for t in got[k])
