@@ -1,7 +1,8 @@
 """Edge <-> node data movement around a layer: gather node rows by edge source, sum edge rows
 into their destination node.  The reference leaves both to ``torch_geometric.utils.scatter``
 and fancy indexing with ``edge_index`` (``equitorch/transforms/__init__.py:99-101``); here they
-are two kernels that work on CSR-sorted edges and use no atomics."""
+are two kernels.  The sum works on CSR-sorted edges and uses no atomics; the adjoint of the gather adds its rows with
+atomics in float32, or with ``index_add_`` in a fixed order where ``torch.use_deterministic_algorithms`` asks for one."""
 from __future__ import annotations
 
 from typing import Optional
@@ -55,7 +56,7 @@ class _ScatterAddRows(torch.autograd.Function):
     @staticmethod
     def forward(ctx, grad, index, rows):
         ctx.save_for_backward(index)
-        if grad.dtype not in (torch.float32, torch.bfloat16):
+        if grad.dtype not in (torch.float32, torch.bfloat16) or torch.are_deterministic_algorithms_enabled():
             out = torch.zeros(rows, *grad.shape[1:], dtype=grad.dtype, device=grad.device)
             return out.index_add_(0, index, grad)
         dev = _lib.require_cuda(grad, index)
