@@ -47,7 +47,23 @@ class _GatherRows(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         (index,) = ctx.saved_tensors
-        return _ScatterAddRows.apply(grad, index, ctx.rows), None
+        adjoint = _ScatterAddRows.apply if torch.is_grad_enabled() else _scatter_add_rows_raw
+        return adjoint(grad, index, ctx.rows), None
+
+
+def _scatter_add_rows_raw(grad: Tensor, index: Tensor, rows: int) -> Tensor:
+    if grad.dtype not in (torch.float32, torch.bfloat16) or torch.are_deterministic_algorithms_enabled():
+        out = torch.zeros(rows, *grad.shape[1:], dtype=grad.dtype, device=grad.device)
+        return out.index_add_(0, index, grad)
+    dev = _lib.require_cuda(grad, index)
+    grad = grad.contiguous()
+    out = torch.zeros(rows, *grad.shape[1:], dtype=torch.float32, device=dev)       # sums in float32 for bfloat16 too
+    width = grad[0].numel() if grad.shape[0] else 0
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().eqt_scatter_add_rows(_lib.DTYPE_CODE[grad.dtype], grad.data_ptr(), index.contiguous().data_ptr(),
+                                                   out.data_ptr(), grad.shape[0], width, rows, _lib.stream_ptr(dev)),
+                   "eqt_scatter_add_rows")
+    return out if grad.dtype == torch.float32 else out.to(grad.dtype)
 
 
 class _ScatterAddRows(torch.autograd.Function):
@@ -56,18 +72,7 @@ class _ScatterAddRows(torch.autograd.Function):
     @staticmethod
     def forward(ctx, grad, index, rows):
         ctx.save_for_backward(index)
-        if grad.dtype not in (torch.float32, torch.bfloat16) or torch.are_deterministic_algorithms_enabled():
-            out = torch.zeros(rows, *grad.shape[1:], dtype=grad.dtype, device=grad.device)
-            return out.index_add_(0, index, grad)
-        dev = _lib.require_cuda(grad, index)
-        grad = grad.contiguous()
-        out = torch.zeros(rows, *grad.shape[1:], dtype=torch.float32, device=dev)       # sums in float32 for bfloat16 too
-        width = grad[0].numel() if grad.shape[0] else 0
-        with _lib.on_device(dev):
-            _lib.check(_lib.lib().eqt_scatter_add_rows(_lib.DTYPE_CODE[grad.dtype], grad.data_ptr(), index.contiguous().data_ptr(),
-                                                       out.data_ptr(), grad.shape[0], width, rows, _lib.stream_ptr(dev)),
-                       "eqt_scatter_add_rows")
-        return out.to(grad.dtype)
+        return _scatter_add_rows_raw(grad, index, rows)
 
     @staticmethod
     def backward(ctx, g):
@@ -85,7 +90,8 @@ class _SegmentSum(torch.autograd.Function):
     def backward(ctx, grad):
         ptr, perm = ctx.saved_tensors
         if perm is None:
-            return _ExpandSegments.apply(grad, ptr, ctx.rows), None, None
+            adjoint = _ExpandSegments.apply if torch.is_grad_enabled() else _expand_segments_raw
+            return adjoint(grad, ptr, ctx.rows), None, None
         # node of every summed position without a host round trip (the step stays capturable in a CUDA graph):
         # position e lies in segment d when ptr[d] <= e < ptr[d+1]; positions outside [ptr[0], ptr[-1]) get zero
         count = perm.shape[0]
@@ -99,21 +105,25 @@ class _SegmentSum(torch.autograd.Function):
         return out.index_add_(0, perm, g), None, None
 
 
+def _expand_segments_raw(grad: Tensor, ptr: Tensor, rows: int) -> Tensor:
+    dev = _lib.require_cuda(grad, ptr)
+    grad = grad.contiguous()
+    out = torch.empty(rows, *grad.shape[1:], dtype=grad.dtype, device=dev)
+    width = out[0].numel() if rows else 0
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().eqt_expand_segments(_lib.DTYPE_CODE[grad.dtype], grad.data_ptr(), ptr.contiguous().data_ptr(),
+                                                  out.data_ptr(), ptr.shape[0] - 1, rows, width, _lib.stream_ptr(dev)),
+                   "eqt_expand_segments")
+    return out
+
+
 class _ExpandSegments(torch.autograd.Function):
     """Row d of the input to every row of segment d, zero to rows of no segment: the adjoint of the segment sum."""
 
     @staticmethod
     def forward(ctx, grad, ptr, rows):
         ctx.save_for_backward(ptr)
-        dev = _lib.require_cuda(grad, ptr)
-        grad = grad.contiguous()
-        out = torch.empty(rows, *grad.shape[1:], dtype=grad.dtype, device=dev)
-        width = out[0].numel() if rows else 0
-        with _lib.on_device(dev):
-            _lib.check(_lib.lib().eqt_expand_segments(_lib.DTYPE_CODE[grad.dtype], grad.data_ptr(), ptr.contiguous().data_ptr(),
-                                                      out.data_ptr(), ptr.shape[0] - 1, rows, width, _lib.stream_ptr(dev)),
-                       "eqt_expand_segments")
-        return out
+        return _expand_segments_raw(grad, ptr, rows)
 
     @staticmethod
     def backward(ctx, g):

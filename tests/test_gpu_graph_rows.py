@@ -25,3 +25,23 @@ def test_the_adjoint_of_the_gather_is_deterministic_on_request(dtype):
     want = torch.zeros(7, 33, device=DEV, dtype=torch.float64).index_add_(0, index, cot.double())
     # sums of 5700 terms: in order in float32 1e-5 of the largest, in bfloat16 storage one rounding per addition
     assert float((runs[0].double() - want).abs().max() / want.abs().max()) < {torch.float32: 1e-5, torch.float64: 1e-12}.get(dtype, 1.0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_derivatives_of_the_adjoints(dtype):
+    """A gradient that is itself differentiated, for the gather and the segment sum."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x = torch.randn(11, 5, generator=g, device=DEV, dtype=dtype).requires_grad_(True)
+    index = torch.randint(0, 11, (40,), generator=g, device=DEV)
+    ptr = torch.tensor([2, 2, 9, 30, 36], device=DEV)
+
+    def second(fn):
+        out = fn(x)
+        (first,) = torch.autograd.grad((out ** 3).sum(), x, create_graph=True)
+        return [out, first, *torch.autograd.grad((first ** 2).sum(), x)]
+
+    def plain(t):
+        rows = t[index]
+        return torch.stack([rows[a:b].sum(0) for a, b in zip(ptr[:-1].tolist(), ptr[1:].tolist())])
+    for a, b in zip(second(lambda t: segment_sum(gather_rows(t, index), ptr)), second(plain)):
+        assert float((a - b).abs().max() / b.abs().max()) < (1e-5 if dtype == torch.float32 else 1e-12)
