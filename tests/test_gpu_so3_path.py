@@ -163,7 +163,7 @@ def test_second_derivatives_with_operands_that_are_views(mode, n, c, per_sample)
 def test_gradients_of_some_operands(mode, dtype, per_sample):
     """Every subset of operands that want a gradient: the same values, and no operand is kept that none of them takes."""
     g = torch.Generator().manual_seed(5)
-    ir, n, c = "0e+1o+2e", 301, 32
+    ir, n, c = "0e+1o+2e", 601, 32
     layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode=mode).to(DEV)
     shape = ((n,) if per_sample else ()) + tuple(layer.weight_shape)
     values = [torch.randn(*s, generator=g).to(dtype).to(DEV) for s in ((n, 9, c), (n, 9), shape)]
