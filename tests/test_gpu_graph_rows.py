@@ -45,3 +45,21 @@ def test_derivatives_of_the_adjoints(dtype):
         return torch.stack([rows[a:b].sum(0) for a, b in zip(ptr[:-1].tolist(), ptr[1:].tolist())])
     for a, b in zip(second(lambda t: segment_sum(gather_rows(t, index), ptr)), second(plain)):
         assert float((a - b).abs().max() / b.abs().max()) < (1e-5 if dtype == torch.float32 else 1e-12)
+
+
+@pytest.mark.parametrize("width,dtype", [(64, torch.float32), (3, torch.float32), (1, torch.float32), (45, torch.bfloat16),
+                                         (480, torch.bfloat16), (6, torch.float64), (1028, torch.float32)])
+@pytest.mark.parametrize("bounds", [[0, 0], [0, 1], [5, 12], [0, 15, 16, 17, 64, 64, 64, 200], [3, 3, 3, 40, 41], [0, 200], [0, 16, 32, 48, 200],
+                                    [0] * 40 + list(range(0, 100, 3)) + [100] * 70 + [190]])
+def test_adjoint_of_the_segment_sum(bounds, width, dtype):
+    """Few long and many short segments; segments that end at, before and after the runs of 16 rows, empty ones, and rows before
+    the first and after the last."""
+    g = torch.Generator(device=DEV).manual_seed(width)
+    rows, ptr = 200, torch.tensor(bounds, device=DEV)
+    x = torch.randn(rows, width, generator=g, device=DEV).to(dtype).requires_grad_(True)
+    cot = torch.randn(len(bounds) - 1, width, generator=g, device=DEV).to(dtype)
+    (got,) = torch.autograd.grad(segment_sum(x, ptr), x, cot)
+    want = torch.zeros_like(got)
+    for d, (a, b) in enumerate(zip(bounds, bounds[1:])):
+        want[a:b] = cot[d]
+    assert torch.equal(got, want)
