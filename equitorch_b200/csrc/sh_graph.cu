@@ -547,12 +547,16 @@ extern "C" int eqt_scatter_add_rows(int32_t dtype, const void* in, const int64_t
                                     int64_t out_rows, void* stream) {
   using namespace eqt;
   if (num_rows < 0 || width < 0 || out_rows < 0) return fail(EQT_ERR_BAD_ARGUMENT, "negative size");
-  if (num_rows == 0 || width == 0) return EQT_OK;
-  if (!in || !index || !out) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  if (out_rows == 0 || width == 0) return EQT_OK;
+  if (!out || (num_rows > 0 && (!in || !index))) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  if (dtype != EQT_F32 && dtype != EQT_BF16) return fail(EQT_ERR_UNSUPPORTED, "row scatter sums float32 or bfloat16 rows");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float) * (size_t)(out_rows * width), s);
+  if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+  if (num_rows == 0) return EQT_OK;
   switch (dtype) {
     case EQT_F32: return run_scatter_add((const float*)in, index, out, num_rows, width, out_rows, s);
     case EQT_BF16: return run_scatter_add((const __nv_bfloat16*)in, index, out, num_rows, width, out_rows, s);
-    default: return fail(EQT_ERR_UNSUPPORTED, "row scatter sums float32 or bfloat16 rows");
+    default: return EQT_ERR_UNSUPPORTED;
   }
 }

@@ -5,6 +5,7 @@ are two kernels.  The sum works on CSR-sorted edges and uses no atomics; the adj
 atomics in float32, or with ``index_add_`` in a fixed order where ``torch.use_deterministic_algorithms`` asks for one."""
 from __future__ import annotations
 
+import math
 from typing import Optional
 
 import torch
@@ -57,8 +58,8 @@ def _scatter_add_rows_raw(grad: Tensor, index: Tensor, rows: int) -> Tensor:
         return out.index_add_(0, index, grad)
     dev = _lib.require_cuda(grad, index)
     grad = grad.contiguous()
-    out = torch.zeros(rows, *grad.shape[1:], dtype=torch.float32, device=dev)       # sums in float32 for bfloat16 too
-    width = grad[0].numel() if grad.shape[0] else 0
+    out = torch.empty(rows, *grad.shape[1:], dtype=torch.float32, device=dev)       # sums in float32 for bfloat16 too
+    width = math.prod(grad.shape[1:])
     with _lib.on_device(dev):
         _lib.check(_lib.lib().eqt_scatter_add_rows(_lib.DTYPE_CODE[grad.dtype], grad.data_ptr(), index.contiguous().data_ptr(),
                                                    out.data_ptr(), grad.shape[0], width, rows, _lib.stream_ptr(dev)),

@@ -130,9 +130,9 @@ int eqt_gather_rows(int32_t dtype, const void* in, const int64_t* index, void* o
 /*
  * Their adjoints:
  *   eqt_expand_segments:  out[e, :] = in[d, :] for e in [ptr[d], ptr[d+1]), zero for rows of no segment (ptr ascending)
- *   eqt_scatter_add_rows: out[index[e], :] += in[e, :] in float32 (EQT_F32 / EQT_BF16 rows), out zero-filled by the
- *                         caller; the order of the additions is not fixed; rows with index outside [0, out_rows) are
- *                         skipped.
+ *   eqt_scatter_add_rows: out[index[e], :] += in[e, :] in float32 (EQT_F32 / EQT_BF16 rows), out (out_rows, width)
+ *                         zeroed first; the order of the additions is not fixed; rows with index outside [0, out_rows)
+ *                         are skipped.
  */
 int eqt_expand_segments(int32_t dtype, const void* in, const int64_t* ptr, void* out, int64_t num_segments,
                         int64_t num_rows, int64_t width, void* stream);

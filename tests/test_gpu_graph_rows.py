@@ -3,7 +3,7 @@ and segments end."""
 import pytest
 import torch
 
-from equitorch_b200.ops.graph_ops import gather_rows, segment_sum
+from equitorch_b200.ops.graph_ops import _scatter_add_rows_raw, gather_rows, segment_sum
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -63,3 +63,46 @@ def test_adjoint_of_the_segment_sum(bounds, width, dtype):
     for d, (a, b) in enumerate(zip(bounds, bounds[1:])):
         want[a:b] = cot[d]
     assert torch.equal(got, want)
+
+
+def _rows(g, rows, width, dtype, offset):
+    """Rows whose first element lies ``offset`` elements behind a 16-byte boundary."""
+    return torch.randn(rows * width + offset, generator=g, device=DEV).to(dtype)[offset:].view(rows, width)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4])
+@pytest.mark.parametrize("width,dtype", [(64, torch.float32), (3, torch.float32), (1, torch.float32), (6, torch.float32), (1028, torch.float32),
+                                         (45, torch.bfloat16), (480, torch.bfloat16), (12, torch.bfloat16), (1, torch.bfloat16),
+                                         (6, torch.float64), (5, torch.float64)])
+def test_gather_sum_and_the_adjoint_of_the_gather(width, dtype, offset):
+    """Units of 16 bytes, of four elements and of one; rows off the 16-byte grid; segments that are empty, shorter and longer than
+    the four rows in flight; a permutation of the rows."""
+    g = torch.Generator(device=DEV).manual_seed(width + offset)
+    x = _rows(g, 57, width, dtype, offset)
+    index = torch.randint(0, 57, (301,), generator=g, device=DEV)
+    leaf = x.detach().requires_grad_(True)
+    picked = gather_rows(leaf, index)
+    assert torch.equal(picked, x[index])
+    # sums of up to 12 (adjoint), 240 (segments) terms of both signs: float32 1e-6 of the largest, bfloat16 the rounding of the result
+    tol = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -8, torch.float64: 1e-13}[dtype]
+    cot = _rows(g, 301, width, dtype, offset)
+    (got,) = torch.autograd.grad(picked, leaf, cot)
+    want = torch.zeros(57, width, device=DEV, dtype=torch.float64).index_add_(0, index, cot.double())
+    assert got.dtype == dtype and float((got.double() - want).abs().max()) <= tol * float(want.abs().max())
+    bounds = [0, 0, 1, 4, 9, 249, 249, 290]
+    ptr, perm = torch.tensor(bounds, device=DEV), torch.randperm(301, generator=g, device=DEV)
+    for order in (None, perm):
+        got = segment_sum(cot, ptr) if order is None else segment_sum(cot, ptr, order)
+        rows = cot.double() if order is None else cot.double()[order]
+        want = torch.stack([rows[a:b].sum(0) for a, b in zip(bounds, bounds[1:])])
+        assert got.dtype == dtype and float((got.double() - want).abs().max()) <= tol * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_added_outside_the_result_are_skipped(dtype):
+    g = torch.Generator(device=DEV).manual_seed(2)
+    rows, index = torch.randn(6, 8, generator=g, device=DEV).to(dtype), torch.tensor([0, -1, 2, 3, 1 << 40, 0], device=DEV)
+    want = torch.zeros(3, 8, device=DEV).index_add_(0, index[[0, 2, 5]], rows[[0, 2, 5]].float())
+    assert torch.equal(_scatter_add_rows_raw(rows, index, 3), want.to(dtype))
+    assert torch.equal(_scatter_add_rows_raw(rows[:0], index[:0], 3), torch.zeros(3, 8, device=DEV, dtype=dtype))
+    assert _scatter_add_rows_raw(rows[:0], index[:0], 0).shape == (0, 8)
