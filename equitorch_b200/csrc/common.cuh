@@ -24,6 +24,13 @@ inline int check_launch(const char* what) {
   return EQT_OK;
 }
 
+// Limit of the dynamic shared memory of a kernel on the current device: the most that any launch of it asks for, not what the
+// next one needs.  The limit belongs to the kernel, and between setting and launching, another host thread may set it too.
+template <typename K> inline int allow_shared(K kernel, size_t most) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  return e == cudaSuccess ? EQT_OK : fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+}
+
 // ---- storage <-> arithmetic types --------------------------------------------------------
 template <typename T> struct Acc { using type = float; };
 template <> struct Acc<double> { using type = double; };

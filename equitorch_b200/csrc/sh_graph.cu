@@ -121,8 +121,7 @@ template <typename Kern>
 int configure_smem(Kern kern, size_t bytes) {
   if (bytes > 48 * 1024) {
     if (bytes > 227 * 1024) return fail(EQT_ERR_UNSUPPORTED, "l_max needs %zu bytes of shared memory", bytes);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    return allow_shared(kern, 227 * 1024);
   }
   return EQT_OK;
 }

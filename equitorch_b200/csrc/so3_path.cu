@@ -658,10 +658,8 @@ int path_run(PathMode mode, const eqt_path_table* t, bool per_sample_w, bool sha
         reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.gx) | reinterpret_cast<uintptr_t>(a.gw)) & mask) != 0)
     return fail(EQT_ERR_UNSUPPORTED, "operands are not aligned to four elements");
   auto launch = [&](auto kern, auto... more) {
-    if (s.smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
-      if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
+    if (s.smem > 48 * 1024)
+      if (int rc = allow_shared(kern, PATH_SMEM_MAX)) return rc;
     kern<<<dim3((unsigned)s.grid, (unsigned)s.split), s.threads, s.smem, st>>>(a, more...);
     return check_launch("so3 path kernel");
   };

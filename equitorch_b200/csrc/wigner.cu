@@ -399,6 +399,8 @@ int wig_check(const eqt_wigner_table* t, int32_t dtype) {
   return EQT_OK;
 }
 
+constexpr size_t WIG_SMEM_MOST = 200 * 1024;
+
 template <typename T>
 int wig_launch(bool backward, const eqt_wigner_table* t, WigArgs a, cudaStream_t st) {
   const int L1 = t->max_l + 1;
@@ -407,9 +409,8 @@ int wig_launch(bool backward, const eqt_wigner_table* t, WigArgs a, cudaStream_t
     const size_t bytes = sizeof(T) * ((size_t)t->coef_count + WIG_EPB * 3 * L1 * 2 + (size_t)t->dim * t->dim) +
                          sizeof(int32_t) * 2 * a.block_elems;
     if (t->max_l > 7 || t->coef_count >= (1 << 19)) return fail(EQT_ERR_UNSUPPORTED, "element codes hold degrees up to 7");
-    if (bytes > 200 * 1024) return fail(EQT_ERR_UNSUPPORTED, "Wigner coefficient table too large for shared memory");
-    cudaError_t e = cudaFuncSetAttribute(wigner_d_forward_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    if (bytes > WIG_SMEM_MOST) return fail(EQT_ERR_UNSUPPORTED, "Wigner coefficient table too large for shared memory");
+    if (int rc = allow_shared(wigner_d_forward_kernel<T>, WIG_SMEM_MOST)) return rc;
     // one resident wave (the per-CTA tables make a second, partial wave expensive)
     int per_sm = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wigner_d_forward_kernel<T>, 256, bytes) != cudaSuccess || per_sm < 1)
@@ -419,9 +420,8 @@ int wig_launch(bool backward, const eqt_wigner_table* t, WigArgs a, cudaStream_t
     return check_launch("wigner_d_forward_kernel");
   }
   const size_t bytes = sizeof(T) * ((size_t)t->coef_count + 8 * 3 * L1 * 2);
-  if (bytes > 200 * 1024) return fail(EQT_ERR_UNSUPPORTED, "Wigner coefficient table too large for shared memory");
-  cudaError_t e = cudaFuncSetAttribute(wigner_d_backward_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  if (bytes > WIG_SMEM_MOST) return fail(EQT_ERR_UNSUPPORTED, "Wigner coefficient table too large for shared memory");
+  if (int rc = allow_shared(wigner_d_backward_kernel<T>, WIG_SMEM_MOST)) return rc;
   int per_sm = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wigner_d_backward_kernel<T>, 256, bytes) != cudaSuccess || per_sm < 1)
     per_sm = 1;
@@ -485,11 +485,11 @@ extern "C" int eqt_dense_rotation(const void* matrix, const void* x, void* out, 
   const size_t es = dtype == EQT_F32 ? 4 : 8;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t bytes = es * ((size_t)dim * ((dim + 3) & ~3) + (size_t)dim * ((channels + 3) & ~3));
-  if (bytes > 200 * 1024) return fail(EQT_ERR_UNSUPPORTED, "matrix and features of one sample do not fit shared memory");
+  if (bytes > WIG_SMEM_MOST) return fail(EQT_ERR_UNSUPPORTED, "matrix and features of one sample do not fit shared memory");
   // one resident wave: samples are strided over the CTAs, and a second, partial wave would run at a fraction of the occupancy
   auto wave = [&](auto kernel, int threads) {
     int per_sm = 1;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    allow_shared(kernel, WIG_SMEM_MOST);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes) != cudaSuccess || per_sm < 1) per_sm = 1;
     return (unsigned)std::min<int64_t>(n, (int64_t)sm_count() * per_sm);
   };
@@ -514,11 +514,11 @@ extern "C" int eqt_dense_rotation_grad_matrix(const void* grad_out, const void* 
   if (!grad_out || !x || !grad_matrix) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   const size_t es = dtype == EQT_F32 ? 4 : 8;
   const size_t bytes = es * (2 * (size_t)channels * ((dim + 3) & ~3) + (size_t)dim * dim);
-  if (bytes > 200 * 1024) return fail(EQT_ERR_UNSUPPORTED, "features of one sample do not fit shared memory");
+  if (bytes > WIG_SMEM_MOST) return fail(EQT_ERR_UNSUPPORTED, "features of one sample do not fit shared memory");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto wave = [&](auto kernel, int threads) {
     int per_sm = 1;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    allow_shared(kernel, WIG_SMEM_MOST);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes) != cudaSuccess || per_sm < 1) per_sm = 1;
     return (unsigned)std::min<int64_t>(n, (int64_t)sm_count() * per_sm);
   };

@@ -399,10 +399,11 @@ __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const f
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+constexpr size_t SMEM_MOST = 200 * 1024;
+
 template <typename K>
 int resident_grid(K kernel, int threads, size_t bytes, int64_t want, unsigned* grid) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  if (int rc = allow_shared(kernel, SMEM_MOST)) return rc;
   int per_sm = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes) != cudaSuccess || per_sm < 1) per_sm = 1;
   *grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count() * per_sm));
@@ -417,8 +418,6 @@ int quad_bound(const eqt_wigner_table* t) {
   const int l1 = t->max_l + 1;
   return (int)std::min<int64_t>((int64_t)t->dim * l1 * l1 / (2 * t->max_l + 1), INT32_MAX);
 }
-
-constexpr size_t SMEM_MOST = 200 * 1024;
 
 bool rotation_tiles(const int32_t* sizes, int blocks, RowTiles& t, int* dim) {
   t = RowTiles{};
