@@ -115,14 +115,19 @@ __global__ void __launch_bounds__(256) ew_kernel(P p) {
 // at a time, so that its place, the row's segment and the first entry are found once and four 128-bit loads per operand are in
 // flight.  With one flattened index over samples, rows and channels every element paid three divisions and the chain of table
 // loads in front of its operands (7k nodes, 35 rows x 128 channels: 44 us a pass, 40 us so; the tables in shared memory
-// instead: 42).
+// instead: 42).  Where all rows of a sample have fewer items than the block threads, `sets` = threads / items of them take every
+// sets-th sample of the block's range (1M samples of one row of 4 channels: 130 us with the other threads idle, 6.5 us so, 9.5 us
+// with the flattened index; 100k samples of 9 rows x 16 channels: 38.6, 28.9 and 34.7 us).
 constexpr int EW_THREADS = 128;
-template <int OP>
-__global__ void __launch_bounds__(EW_THREADS) ew_kernel_f4(P p, int64_t chunk) {
+template <int OP, bool SETS>
+__global__ void __launch_bounds__(EW_THREADS) ew_kernel_f4(P p, int64_t chunk, int several) {
+  const int sets = SETS ? several : 1;
   const float* x = static_cast<const float*>(p.in1);
   const float* y = static_cast<const float*>(p.in2);
-  const int64_t C = p.c1, c4 = C / 4, item = blockIdx.x * (int64_t)EW_THREADS + threadIdx.x;
-  if (item >= p.num_out * c4) return;
+  const int64_t C = p.c1, c4 = C / 4, items = p.num_out * c4;
+  const int64_t set = SETS ? threadIdx.x / items : 0;
+  const int64_t item = SETS ? threadIdx.x - set * items : blockIdx.x * (int64_t)EW_THREADS + threadIdx.x;
+  if (item >= items || set >= sets) return;
   const int64_t o = item / c4, c = (item - o * c4) * 4;
   const int64_t n0 = blockIdx.y * chunk, n1 = min(n0 + chunk, p.n);
   int64_t t0, t1;
@@ -131,7 +136,7 @@ __global__ void __launch_bounds__(EW_THREADS) ew_kernel_f4(P p, int64_t chunk) {
   const float first_scale = t0 < t1 ? scale_of<float>(p, first.tt) : 0.f;
   float* out = static_cast<float*>(p.out) + out_row(p, o) * C + c;
   const int64_t out_stride = p.out_size * C;
-  for (int64_t n = n0; n < n1; n += 4) {
+  for (int64_t n = n0 + set; n < n1; n += 4 * sets) {                 // its samples: n, n + sets, n + 2 sets, n + 3 sets
     float4 acc[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -143,21 +148,21 @@ __global__ void __launch_bounds__(EW_THREADS) ew_kernel_f4(P p, int64_t chunk) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         s[u] = scale;
-        if (n + u >= n1) continue;
-        v[u] = __ldg(reinterpret_cast<const float4*>(x + (n + u) * p.bs1 + e.r1 * C + c));
-        if (OP == EQT_OP_MUL) w[u] = __ldg(reinterpret_cast<const float4*>(y + (n + u) * p.bs2 + e.r2 * C + c));
-        if (OP == EQT_OP_VECSCA) s[u] *= __ldg(y + (n + u) * p.bs2 + e.r2);
+        if (n + u * sets >= n1) continue;
+        v[u] = __ldg(reinterpret_cast<const float4*>(x + (n + u * sets) * p.bs1 + e.r1 * C + c));
+        if (OP == EQT_OP_MUL) w[u] = __ldg(reinterpret_cast<const float4*>(y + (n + u * sets) * p.bs2 + e.r2 * C + c));
+        if (OP == EQT_OP_VECSCA) s[u] *= __ldg(y + (n + u * sets) * p.bs2 + e.r2);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        if (n + u >= n1) continue;
+        if (n + u * sets >= n1) continue;
         if (OP == EQT_OP_MUL) { v[u].x *= w[u].x; v[u].y *= w[u].y; v[u].z *= w[u].z; v[u].w *= w[u].w; }
         acc[u].x += v[u].x * s[u]; acc[u].y += v[u].y * s[u]; acc[u].z += v[u].z * s[u]; acc[u].w += v[u].w * s[u];
       }
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (n + u < n1) *reinterpret_cast<float4*>(out + (n + u) * out_stride) = acc[u];
+      if (n + u * sets < n1) *reinterpret_cast<float4*>(out + (n + u * sets) * out_stride) = acc[u];
   }
 }
 
@@ -699,15 +704,17 @@ int launch(const eqt_product_args& a, P p, cudaStream_t s) {
     }
     if (std::is_same<T, float>::value && p.c1 % 4 == 0 && aligned16(p.in1) && aligned16(p.out) &&
         (op != EQT_OP_MUL || aligned16(p.in2))) {
-      const int64_t blocks_x = ceil_div(p.num_out * (p.c1 / 4), EW_THREADS);
-      int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)sm_count() * 32, blocks_x), ceil_div(p.n, 4)));
+      const int64_t items = p.num_out * (p.c1 / 4), blocks_x = ceil_div(items, EW_THREADS);
+      const int sets = (int)std::max<int64_t>(1, EW_THREADS / items), step = 4 * sets;        // samples a block takes at a time
+      int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)sm_count() * 32, blocks_x), ceil_div(p.n, step)));
       chunks = std::min<int64_t>(chunks, 65535);
-      const int64_t chunk = ceil_div(ceil_div(p.n, chunks), 4) * 4;
+      const int64_t chunk = ceil_div(ceil_div(p.n, chunks), step) * step;
       if (blocks_x > INT32_MAX) return fail(EQT_ERR_UNSUPPORTED, "too many output rows");
       const dim3 grid((unsigned)blocks_x, (unsigned)ceil_div(p.n, chunk));
-      if (op == EQT_OP_MUL) ew_kernel_f4<EQT_OP_MUL><<<grid, EW_THREADS, 0, s>>>(p, chunk);
-      if (op == EQT_OP_VECSCA) ew_kernel_f4<EQT_OP_VECSCA><<<grid, EW_THREADS, 0, s>>>(p, chunk);
-      if (op == EQT_OP_SCALE) ew_kernel_f4<EQT_OP_SCALE><<<grid, EW_THREADS, 0, s>>>(p, chunk);
+      auto run = [&](auto* whole, auto* side) { (sets > 1 ? side : whole)<<<grid, EW_THREADS, 0, s>>>(p, chunk, sets); };
+      if (op == EQT_OP_MUL) run(ew_kernel_f4<EQT_OP_MUL, false>, ew_kernel_f4<EQT_OP_MUL, true>);
+      if (op == EQT_OP_VECSCA) run(ew_kernel_f4<EQT_OP_VECSCA, false>, ew_kernel_f4<EQT_OP_VECSCA, true>);
+      if (op == EQT_OP_SCALE) run(ew_kernel_f4<EQT_OP_SCALE, false>, ew_kernel_f4<EQT_OP_SCALE, true>);
       return check_launch("ew_kernel_f4");
     }
     if (std::is_same<T, __nv_bfloat16>::value && p.c1 % 8 == 0 && aligned16(p.in1) && aligned16(p.out) &&

@@ -48,3 +48,16 @@ def test_operands_off_the_16_byte_grid():
         a = gops.indexed_mul_scale_gather(off, y, sc, i1, i2, seg, **kw)
         b = gops.indexed_mul_scale_gather(off.clone(), y, sc, i1, i2, seg, **kw)
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("n,c,num_out", [(1, 4, 1), (511, 4, 1), (513, 4, 1), (70001, 4, 1), (1025, 20, 3), (300, 8, 63), (300, 8, 64), (300, 8, 65), (77, 24, 21)])
+def test_rows_that_do_not_fill_a_block(n, c, num_out):
+    """One item a sample up to as many as a block has threads and one more; samples that end within a block's step."""
+    g = torch.Generator().manual_seed(n + c)
+    sc, i1, i2, seg = _table(g, num_out, 2 * num_out + 1, 7)
+    x, y, scalar = torch.randn(n, 7, c, generator=g), torch.randn(n, 7, c, generator=g), torch.randn(n, 7, generator=g)
+    dev = lambda t: t.to(DEV)
+    for name, second in (("indexed_mul_scale_gather", y), ("indexed_vecsca_scale_gather", scalar)):
+        want = getattr(oops, name)(x.double(), second.double(), sc.double(), i1, i2, seg)
+        got = getattr(gops, name)(*map(dev, (x, second, sc, i1, i2, seg)))
+        assert got.shape == want.shape and float((got.cpu().double() - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max()))
