@@ -744,9 +744,10 @@ int launch(const eqt_product_args& a, P p, cudaStream_t s) {
       outer_acc_kernel<T><<<grid, 256, 0, s>>>(p, chunk);
       return check_launch("outer_acc_kernel");
     }
-    // lanes own four columns each: 4, 8, ... 128 columns and operands whose rows allow 4-wide accesses
+    // lanes own four columns each: 4, 8, ... 128 columns and operands whose rows allow 4-wide accesses; below 32 products a
+    // row most lanes would idle (20k samples x 9 rows: 4 x 4 62 us, 34 us a thread per element; 4 x 8 62 and 64; 8 x 8 62 and 122)
     const int64_t q = p.c2 / 4;
-    if (p.c2 % 4 == 0 && q <= 32 && (q & (q - 1)) == 0 && p.c1 <= 0x7fffff && p.num_out <= 0x7fffffff &&
+    if (p.c2 % 4 == 0 && p.c1 * p.c2 >= 32 && q <= 32 && (q & (q - 1)) == 0 && p.c1 <= 0x7fffff && p.num_out <= 0x7fffffff &&
         ((reinterpret_cast<uintptr_t>(p.in2) | reinterpret_cast<uintptr_t>(p.out)) & (4 * sizeof(T) - 1)) == 0) {
       outer_rows_kernel<T><<<flat_grid(p.n * p.num_out, 8, 8), 256, 0, s>>>(p);
       return check_launch("outer_rows_kernel");
