@@ -44,21 +44,29 @@ _CHECK_EVERY_CALL = os.environ.get("EQT_CHECK_STATUS", "0") not in ("", "0")
 
 
 class MixTables:
-    """Device tables of a layer's weight step and of its adjoints: ``out[n, M] = sum_{rows r of M} s[n, r] W[path(r)]``."""
+    """Device tables of a layer's weight step and of its adjoints: ``out[n, M] = sum_{rows r of M} s[n, r] W[path(r)]``.
 
-    def __init__(self, info: TensorProductInfo, device, out_dims=None):
+    ``min_batch``, ``most_columns``: the tensor-core kernels take batches and output widths from / up to these.  Their
+    products of TF32 pairs, summed by an adder that truncates, are further from 64 bits than float32 multiply-adds (448 terms,
+    64 channels: 1.5e-6 of the norm against 3.6e-7), so a layer whose other route is float32 there stays on it."""
+
+    def __init__(self, info: TensorProductInfo, device, out_dims=None, min_batch: int = 0, most_columns: int = 256):
         self.mix_fwd, self.mix_bwd1, self.mix_bwd2 = (t.to(device) for t in (info.info_M_fwd, info.info_M_bwd1, info.info_M_bwd2))
         # block structure of the weight step for the tensor-core GEMM (None: CUDA-core kernel)
         self.tc_fwd = MixPlan(info.info_M_fwd, out_dims, device) if out_dims is not None else None
+        self.min_batch, self.most_columns = min_batch, most_columns
         w, seg = info.info_M_fwd.index2, info.info_M_fwd.seg_out
         self.rows = w.numel() if w is not None else info.info_M_fwd.out_size if seg is None else int(seg[-1])
 
     def forward(self, s: Tensor, weight: Tensor, mode: str) -> Tensor:
         assert s.shape[1] == self.rows, f"{s.shape[1]} rows for a table of {self.rows}"
-        return _mix(s, weight, self.mix_fwd, mode, self.tc_fwd)
+        return _mix(s, weight, self.mix_fwd, mode, self._tensor_cores(s, weight.shape[-1]))
+
+    def _tensor_cores(self, batch: Tensor, columns: int) -> Optional[MixPlan]:
+        return self.tc_fwd if batch.shape[0] >= self.min_batch and columns <= self.most_columns else None
 
     def grad_weight(self, s: Tensor, grad: Tensor, num_paths: int, mode: str) -> Tensor:
-        tcw, b2 = self.tc_fwd, self.mix_bwd2
+        tcw, b2 = self._tensor_cores(grad, 0), self.mix_bwd2
         if (mode == "uv" and tcw is not None and tcw.regular and grad.dtype == torch.float32
                 and _tc_supported_w(s.shape[-1], grad.shape[-1])):
             return wgrad_tc(s, grad, tcw, num_paths)
@@ -71,7 +79,7 @@ class MixTables:
 
     def grad_inter(self, grad: Tensor, weight: Tensor, mode: str) -> Tensor:
         """Gradient with respect to the intermediate: ``G[n, r] = grad[n, M(r)] W[path(r)]^T``."""
-        tc, b1 = self.tc_fwd, self.mix_bwd1
+        tc, b1 = self._tensor_cores(grad, weight.shape[-2]), self.mix_bwd1
         if (mode == "uv" and tc is not None and tc.regular
                 and _tc_supported_t(weight.shape[-2], weight.shape[-1])):
             return mix_tc_transposed(grad, weight, tc)

@@ -12,6 +12,7 @@ import torch
 from torch import Tensor
 
 from ..irreps import check_irreps
+from ..ops.indexed_tc_op import MAX_COLUMNS, MIN_BATCH
 from ..ops.so3_path_op import PathPlan
 from ..tables import (generate_fully_connected_tp_paths, irreps_info, irreps_linear_infos, so2_linear_infos, so3_path_norms,
                       tp_infos)
@@ -99,7 +100,7 @@ class SO3Linear(_WeightedTableModule):
             if plan is not None and self.feature_mode == "uv" and plan.uv_supported(input1, input2, weight):
                 if plan.mix is None:
                     plan.mix = plan.rows_match(self.tp_info_forward.info_M_fwd) and \
-                        MixTables(self.tp_info_forward, input1.device, [ir.dim for ir in self.irreps_out])
+                        MixTables(self.tp_info_forward, input1.device, [ir.dim for ir in self.irreps_out], MIN_BATCH, MAX_COLUMNS)
                 if plan.mix:
                     return SO3LinearUV.apply(input1, input2, weight, plan, plan.mix, infos)[0]
         fn = so3_linear_uu if self.feature_mode == "uu" else so3_linear_uv

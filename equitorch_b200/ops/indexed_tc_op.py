@@ -20,6 +20,7 @@ from .. import _lib
 from .mix_tc_op import status_flag
 
 MIN_BATCH = 512          # below this the table-driven kernels are as fast and have no set-up cost
+MAX_COLUMNS = 128        # widest output row of a GEMM: its accumulators have to fit tensor memory beside the split operand
 MAX_PLANS = 256
 _plans: "OrderedDict[tuple, tuple]" = OrderedDict()
 
@@ -91,7 +92,7 @@ class VecmatPlan:
 def vecmat_supported(x: Tensor, w: Tensor, gather_index, index_out, out_accumulated, out_size, num_out) -> bool:
     return (x.is_cuda and x.dtype == torch.float32 and w.dtype == torch.float32 and x.ndim == 3 and w.ndim == 3
             and gather_index is None and index_out is None and not out_accumulated and out_size == num_out
-            and x.shape[0] >= MIN_BATCH and x.shape[2] % 32 == 0 and w.shape[2] % 16 == 0 and w.shape[2] <= 128
+            and x.shape[0] >= MIN_BATCH and x.shape[2] % 32 == 0 and w.shape[2] % 16 == 0 and w.shape[2] <= MAX_COLUMNS
             and x.data_ptr() % 16 == 0)
 
 
@@ -177,7 +178,7 @@ def outer_supported(a: Tensor, b: Tensor, gather_index, index_out, out_accumulat
     return (a.is_cuda and a.dtype == torch.float32 and b.dtype == torch.float32 and a.ndim == 3 and b.ndim == 3
             and out_accumulated and gather_index is None and index_out is None and out_size == num_out
             and a.shape[0] == b.shape[0] and a.shape[0] >= MIN_BATCH and a.shape[2] % 32 == 0 and b.shape[2] % 32 == 0
-            and b.shape[2] <= 128 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)
+            and b.shape[2] <= MAX_COLUMNS and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)
 
 
 def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Tensor:
