@@ -122,8 +122,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // points at that row's first served column (column offset included), bit i of `vmask` says whether the row exists.
 constexpr int EPI_PITCH = 36;
 constexpr int EPI_PATCH_BYTES = 4 * 32 * EPI_PITCH * 4;      // four epilogue warps
+// `add`: onto what this thread stored there before
 __device__ __forceinline__ void store_block_rows(float* patch, const float (&v)[32], int lane, float* const (&orow)[8],
-                                                 unsigned vmask, int c0, int n_cols) {
+                                                 unsigned vmask, int c0, int n_cols, bool add = false) {
   __syncwarp();                                 // the previous block has been read out of the patch
 #pragma unroll
   for (int c = 0; c < 32; c += 4)
@@ -131,8 +132,14 @@ __device__ __forceinline__ void store_block_rows(float* patch, const float (&v)[
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const float4 t = *reinterpret_cast<const float4*>(patch + (i * 4 + (lane >> 3)) * EPI_PITCH + (lane & 7) * 4);
-    if (((vmask >> i) & 1) && c0 + (lane & 7) * 4 < n_cols) *reinterpret_cast<float4*>(orow[i] + c0) = t;
+    float4 t = *reinterpret_cast<const float4*>(patch + (i * 4 + (lane >> 3)) * EPI_PITCH + (lane & 7) * 4);
+    if (!((vmask >> i) & 1) || c0 + (lane & 7) * 4 >= n_cols) continue;
+    float4* to = reinterpret_cast<float4*>(orow[i] + c0);
+    if (add) {
+      const float4 o = *to;
+      t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
+    }
+    *to = t;
   }
 }
 

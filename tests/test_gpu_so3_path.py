@@ -208,3 +208,13 @@ def test_channel_mixing_in_float32_where_it_was(ir, n, c, c_out, bounds):
     are 1.5 to 5 times those."""
     for e, bound in zip(_norm_errors("uv", ir, n, c, c_out), bounds):
         assert bound is None or e < bound
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ir,n,c,c_out,bound", [("0e+1o+2e+3o", 700, 128, 128, 4e-6), ("0e+1o+2e+3o", 700, 128, 64, 4e-6),
+                                                ("8x0e+4x1o+4x2e", 600, 32, 32, 4e-6), ("8x0e+4x1o+4x2e", 520, 64, 96, 4e-6)])
+def test_long_sums_are_added_up_in_pieces(ir, n, c, c_out, bound):
+    """Sums of 16 to 112 k-blocks of 32 terms: no further from 64 bits than pieces of 16 in one accumulator.  Bound: 192
+    truncated additions of 1.7e-8 of the norm each and the split's 6.5e-8, 3.3e-6, and a fifth for the draw (the composed
+    products are at 3.2e-6 with 28 k-blocks; in one piece 5.6e-6, growing with the length)."""
+    assert _norm_errors("uv", ir, n, c, c_out)[0] < bound
