@@ -218,3 +218,12 @@ def test_long_sums_are_added_up_in_pieces(ir, n, c, c_out, bound):
     truncated additions of 1.7e-8 of the norm each and the split's 6.5e-8, 3.3e-6, and a fifth for the draw (the composed
     products are at 3.2e-6 with 28 k-blocks; in one piece 5.6e-6, growing with the length)."""
     assert _norm_errors("uv", ir, n, c, c_out)[0] < bound
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ir,n,c,per_sample,composed", [("0e+1o+2e+3o", 1001, 64, False, (7.5e-8, 7.6e-8, 9.9e-8, 1.5e-7)),
+                                                        ("0e+1o+2e", 4001, 32, True, (6.4e-8, 6.4e-8, 8.8e-8, 6.1e-8))])
+def test_channelwise_sums_are_no_further_from_64_bits(ir, n, c, per_sample, composed):
+    """Against the errors of the composed products on such operands; a tenth for other draws of them."""
+    for e, bound in zip(_norm_errors("uu", ir, n, c, c, per_sample), composed):
+        assert e < 1.1 * bound
