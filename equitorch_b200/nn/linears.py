@@ -23,6 +23,11 @@ from .functional.sparse_product import sparse_mul, sparse_vecmat
 from .init import initialize_linear, initialize_so3_so2_linear
 
 
+def _version(info) -> Optional[int]:
+    scale = info.info_Mij_fwd.scale
+    return None if scale is None or scale.is_inference() else scale._version
+
+
 class SO3Linear(_WeightedTableModule):
     r"""Tensor product of channelled features with a channel-less second operand
     (typically spherical harmonics of an edge direction).
@@ -57,31 +62,45 @@ class SO3Linear(_WeightedTableModule):
             channel_norm=self.channel_norm, channel_scale=fan_in ** (-0.5) if fan_in else 1.0)
         paths = path or generate_fully_connected_tp_paths(self.irreps_out, self.irreps_in1, self.irreps_in2)
         self._paths = (list(paths), so3_path_norms(paths, path_norm, self.channel_norm, fan_in ** (-0.5) if fan_in else 1.0))
-        self._own_info, self._path_plans = self.tp_info_forward, {}
+        self._own_tables()
         shape = (self.num_paths, channels_in, channels_out) if feature_mode == "uv" else (self.num_paths, channels_out)
         self._setup_weight(shape, internal_weights,
                            lambda w: initialize_so3_so2_linear(w, feature_mode, channel_normed=self.channel_norm))
 
+    def _tables(self):
+        return self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2
+
+    def _own_tables(self, own: bool = True) -> None:
+        """``own``: the layer's tables are those of its paths, in the state that they are in now."""
+        self._path_plans, self._own = {}, ((self._tables(), _version(self.tp_info_forward)) if own else None)
+
+    def _is_own(self) -> bool:
+        return (self._own is not None and all(a is b for a, b in zip(self._tables(), self._own[0]))
+                and _version(self.tp_info_forward) == self._own[1])
+
     def _path_plan(self, device) -> Optional[PathPlan]:
         """The tables of the one-pass kernels on ``device``, built at the first call there; ``None`` when the layer's
-        own tables have been exchanged."""
-        if self.tp_info_forward is not self._own_info:
+        own tables have been exchanged or written to, and while a stream is being captured that would have to wait for
+        their copy to the device."""
+        if not self._is_own():
             return None
         plan = self._path_plans.get(device)
-        if plan is None:
+        if plan is None and not torch.cuda.is_current_stream_capturing():
             plan = self._path_plans[device] = PathPlan(*self._paths, self.irreps_out, self.irreps_in1, self.irreps_in2, device)
         return plan
 
     def _apply(self, fn, *args, **kwargs):
-        own = self.tp_info_forward is self._own_info
+        own = self._is_own()
         module = super()._apply(fn, *args, **kwargs)
-        module._path_plans = {}
-        if own:
-            module._own_info = module.tp_info_forward
+        module._own_tables(own)
         return module
 
     def __getstate__(self):
-        return {k: ({} if k in ("_path_plans", "_plans") else v) for k, v in self.__dict__.items()}   # device tables are rebuilt
+        return {**{k: v for k, v in self.__dict__.items() if k not in ("_path_plans", "_plans")}, "_own": self._is_own()}
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._own_tables(bool(state.get("_own", False)))          # a layer stored without its paths runs the composed products
 
     def forward(self, input1: Tensor, input2: Tensor, weight: Optional[Tensor] = None) -> Tensor:
         assert input1.shape[-2] == self.irreps_in1_dim, \
@@ -98,7 +117,7 @@ class SO3Linear(_WeightedTableModule):
             if plan is not None and self.feature_mode == "uu" and plan.supported(input1, input2, weight):
                 return SO3LinearUU.apply(input1, input2, weight, plan, infos)
             if plan is not None and self.feature_mode == "uv" and plan.uv_supported(input1, input2, weight):
-                if plan.mix is None:
+                if plan.mix is None and not torch.cuda.is_current_stream_capturing():
                     plan.mix = plan.rows_match(self.tp_info_forward.info_M_fwd) and \
                         MixTables(self.tp_info_forward, input1.device, [ir.dim for ir in self.irreps_out], MIN_BATCH, MAX_COLUMNS)
                 if plan.mix:

@@ -9,6 +9,7 @@ kernels need besides the operands depends on the index tables only (k-block colu
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from collections import OrderedDict
 from typing import Optional
 
@@ -23,21 +24,31 @@ MIN_BATCH = 512          # below this the table-driven kernels are as fast and h
 MAX_COLUMNS = 128        # widest output row of a GEMM: its accumulators have to fit tensor memory beside the split operand
 MAX_PLANS = 256
 _plans: "OrderedDict[tuple, tuple]" = OrderedDict()
+_plans_lock = threading.Lock()
 
 
 def _cached(kind, dev, tensors, extra, build):
     """Plan for these index tensors.  A plan is keyed by the identity and version of the tensors it was built from
     and keeps them alive, so that neither a recycled address nor an in-place update can alias another table; the
-    tables of a module are persistent buffers, so layers hit the cache on every call after the first."""
+    tables of a module are persistent buffers, so layers hit the cache on every call after the first.
+
+    ``None`` where no plan can be had and the table-driven kernels have to run: building one copies the tables to the host,
+    which a stream that is being captured does not allow, and tensors of inference mode have no version."""
+    if any(t is not None and t.is_inference() for t in tensors):
+        return None
     key = (kind, dev, tuple(None if t is None else (id(t), t._version) for t in tensors)) + tuple(extra)
-    hit = _plans.get(key)
-    if hit is not None:
-        _plans.move_to_end(key)
-        return hit[0]
+    with _plans_lock:
+        hit = _plans.get(key)
+        if hit is not None:
+            _plans.move_to_end(key)
+            return hit[0]
+    if torch.cuda.is_current_stream_capturing():
+        return None
     plan = build()
-    _plans[key] = (plan, tensors)
-    if len(_plans) > MAX_PLANS:
-        _plans.popitem(last=False)
+    with _plans_lock:
+        _plans[key] = (plan, tensors)
+        if len(_plans) > MAX_PLANS:
+            _plans.popitem(last=False)
     return plan
 
 
@@ -59,8 +70,8 @@ class VecmatPlan:
 
     def __init__(self, index1, seg, entries: int, num_out: int, cin: int, cout: int, dev):
         chunks = cin // 32
-        i1 = _host(index1, np.arange(entries, dtype=np.int64))
         sg = _host(seg, np.arange(num_out + 1, dtype=np.int64))
+        i1 = _host(index1, np.arange(entries if entries >= 0 else sg[-1], dtype=np.int64))
         classes = _same_reads([i1[sg[r]:sg[r + 1]].tolist() for r in range(num_out)])
 
         # A k-block costs 16 KB of x and 256 bytes of weights per column.  With the one-row groups at 413 entries of 32 x 32
@@ -96,15 +107,21 @@ def vecmat_supported(x: Tensor, w: Tensor, gather_index, index_out, out_accumula
             and x.data_ptr() % 16 == 0)
 
 
-def vecmat_tc(x: Tensor, w: Tensor, scale, index1, index2, seg, num_out: int) -> Tensor:
-    """``out[i, M, :] = sum_{t in seg[M]} scale[t] x[i, index1[t], :] @ w[index2[t]]`` on tensor cores."""
+def _entries(index1, index2, seg, rows1: int) -> int:
+    return (index1.shape[0] if index1 is not None else index2.shape[0] if index2 is not None
+            else rows1 if seg is None else -1)          # -1: as many as the last segment ends at, read with the plan
+
+
+def vecmat_tc(x: Tensor, w: Tensor, scale, index1, index2, seg, num_out: int) -> Optional[Tensor]:
+    """``out[i, M, :] = sum_{t in seg[M]} scale[t] x[i, index1[t], :] @ w[index2[t]]`` on tensor cores; ``None`` without a plan."""
     dev = x.device
     n, rows1, cin = x.shape
     cout = w.shape[2]
-    entries = (index1.shape[0] if index1 is not None else index2.shape[0] if index2 is not None
-               else int(seg[-1]) if seg is not None else rows1)
+    entries = _entries(index1, index2, seg, rows1)
     plan = _cached("vecmat", dev, (index1, seg), (entries, num_out, cin, cout),
                    lambda: VecmatPlan(index1, seg, entries, num_out, cin, cout, dev))
+    if plan is None:
+        return None
     packed = torch.empty(2, max(plan.slots, 1) * cin * plan.group * cout, dtype=torch.float32, device=dev)
     out = torch.empty(n, num_out, cout, dtype=torch.float32, device=dev)
     with _lib.on_device(dev):
@@ -122,9 +139,10 @@ class OuterPlan:
     change places and the result is written transposed."""
 
     def __init__(self, scale, index1, index2, seg, entries: int, num_w: int, c1: int, c2: int, dev):
+        sg = _host(seg, np.arange(num_w + 1, dtype=np.int64))
+        entries = entries if entries >= 0 else int(sg[-1])
         i1 = _host(index1, np.arange(entries, dtype=np.int64))
         i2 = _host(index2, np.arange(entries, dtype=np.int64))
-        sg = _host(seg, np.arange(num_w + 1, dtype=np.int64))
         sc = _host(scale, np.ones(entries, dtype=np.float32)).astype(np.float32)
         w_of = np.repeat(np.arange(num_w), np.diff(sg))
 
@@ -181,15 +199,17 @@ def outer_supported(a: Tensor, b: Tensor, gather_index, index_out, out_accumulat
             and b.shape[2] <= MAX_COLUMNS and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)
 
 
-def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Tensor:
-    """``out[w] = sum_i sum_{t in seg[w]} scale[t] a[i, index1[t], :, None] b[i, index2[t], None, :]`` on tensor cores."""
+def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Optional[Tensor]:
+    """``out[w] = sum_i sum_{t in seg[w]} scale[t] a[i, index1[t], :, None] b[i, index2[t], None, :]`` on tensor cores; ``None``
+    without a plan."""
     dev = a.device
     n, rows1, c1 = a.shape
     rows2, c2 = b.shape[1], b.shape[2]
-    entries = (index1.shape[0] if index1 is not None else index2.shape[0] if index2 is not None
-               else int(seg[-1]) if seg is not None else rows1)
+    entries = _entries(index1, index2, seg, rows1)
     plan = _cached("outer", dev, (scale, index1, index2, seg), (entries, num_w, c1, c2),
                    lambda: OuterPlan(scale, index1, index2, seg, entries, num_w, c1, c2, dev))
+    if plan is None:
+        return None
     out = torch.empty(num_w, c1, c2, dtype=torch.float32, device=dev)
     if plan.swapped:
         a, b, rows1, c1, rows2, c2 = b, a, rows2, c2, rows1, c1

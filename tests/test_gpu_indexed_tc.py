@@ -166,3 +166,23 @@ def test_weight_gradients_on_two_streams(which):
     torch.cuda.synchronize()
     for k in range(2):
         assert all(torch.equal(t, want[k]) for t in got[k])
+
+
+def test_calls_that_can_have_no_plan_take_the_table_driven_kernels():
+    """A first call while a stream is captured, and tables that belong to inference mode."""
+    ir, n, c = "0e+1o+2e", 600, 32
+    g = torch.Generator().manual_seed(3)
+    x, w = torch.randn(n, 9, c, generator=g).to(DEV), torch.randn(3, c, c, generator=g).to(DEV)
+    new = lambda: enn.IrrepsLinear(ir, ir, c, c, internal_weights=False).to(DEV)
+    want = new()(x, w)
+    layer, graph = new(), torch.cuda.CUDAGraph()
+    with torch.no_grad():
+        new()(x[:100], w)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            got = layer(x, w)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert _rel(got, want) < 1e-5
+    with torch.inference_mode():
+        assert _rel(new()(x, w).clone(), want) < 1e-5

@@ -3,6 +3,7 @@ threads per sample (powers of two and not), batches from one sample (output irre
 blocks) to several waves, degrees 0 to 3 with even and odd degree sums, shared and per-sample weights, float32 and bfloat16; and a differentiated
 backward pass against the composed products."""
 import copy
+import pickle
 
 import pytest
 import torch
@@ -227,3 +228,57 @@ def test_channelwise_sums_are_no_further_from_64_bits(ir, n, c, per_sample, comp
     """Against the errors of the composed products on such operands; a tenth for other draws of them."""
     for e, bound in zip(_norm_errors("uu", ir, n, c, c, per_sample), composed):
         assert e < 1.1 * bound
+
+
+def _composed(layer, x, y, w):
+    product = tensor_product_u1u if layer.feature_mode == "uu" else tensor_product_u1v
+    return product(x, y, w, *layer._tables())
+
+
+def _small_layer(mode, n=100, c=32, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    ir = "0e+1o+2e"
+    layer = enn.SO3Linear(ir, ir, ir, c, c, internal_weights=False, feature_mode=mode).to(DEV)
+    return layer, [t.to(DEV) for t in (torch.randn(n, 9, c, generator=g), torch.randn(n, 9, generator=g),
+                                       torch.randn(*layer.weight_shape, generator=g))]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["uu", "uv"])
+def test_first_call_while_a_stream_is_captured(mode):
+    """A layer whose tables are not on the device yet takes the composed products, as before there were one-pass kernels."""
+    warm, operands = _small_layer(mode, seed=1)
+    want = _composed(warm, *operands).clone()
+    layer, _ = _small_layer(mode)
+    graph = torch.cuda.CUDAGraph()
+    with torch.no_grad():
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            got = layer(*operands)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    assert layer._path_plans == {} and _rel(layer(*operands), want.cpu()) < 1e-5 and layer._path_plans != {}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["uu", "uv"])
+def test_tables_that_are_exchanged_written_to_or_stored(mode):
+    layer, operands = _small_layer(mode)
+    want = layer(*operands).cpu()
+    for other in (copy.deepcopy(layer), pickle.loads(pickle.dumps(layer)), copy.deepcopy(layer).cpu().to(DEV)):
+        assert other._is_own() and torch.equal(other(*operands).cpu(), want)
+    stored = layer.__getstate__()                      # as a layer is stored that knows nothing of the one-pass kernels
+    for name in ("_paths", "_own"):
+        del stored[name]
+    old = enn.SO3Linear.__new__(enn.SO3Linear)
+    old.__setstate__(stored)
+    assert _rel(old(*operands), want) < 1e-5 and old._path_plans == {}
+    old = old.to("cpu").to(DEV)
+    assert _rel(old(*operands), want) < 1e-5
+    layer.tp_info_forward.info_Mij_fwd.scale.mul_(2)   # written to in place
+    assert not layer._is_own() and _rel(layer(*operands), 2 * want) < 1e-5
+    layer, _ = _small_layer(mode)
+    scale = layer.tp_info_forward.info_Mij_fwd.scale
+    layer.tp_info_forward = layer.tp_info_forward._replace(info_Mij_fwd=layer.tp_info_forward.info_Mij_fwd._replace(scale=3 * scale))
+    assert _rel(layer(*operands), 3 * want) < 1e-5
