@@ -29,7 +29,7 @@ from torch.autograd import Function
 
 from ... import _profile
 from ...graph import EdgeGraph
-from ...ops import batched_sparse_dense_op as _ops
+from ...ops import batched_sparse_dense_op as _ops, indexed_tc_op
 from ...ops.fused_tp_op import TpTable, cg_inner, cg_segment_sum, check_status
 from ...ops.mix_tc_op import (MixPlan, mix_tc, mix_tc_transposed, wgrad_tc, supported as _tc_supported,
                               supported_transposed as _tc_supported_t, supported_wgrad as _tc_supported_w)
@@ -48,7 +48,9 @@ class MixTables:
 
     ``min_batch``, ``most_columns``: the tensor-core kernels take batches and output widths from / up to these.  Their
     products of TF32 pairs, summed by an adder that truncates, are further from 64 bits than float32 multiply-adds (448 terms,
-    64 channels: 1.5e-6 of the norm against 3.6e-7), so a layer whose other route is float32 there stays on it."""
+    64 channels: 1.5e-6 of the norm against 3.6e-7), so a layer whose other route is float32 there keeps to sums that are no
+    further: the indexed products with one row an item (2.0e-7; 300 samples, l_max 3, 64 channels 35 us, float32 88 us; 2000
+    samples, 128 -> 256 channels 231 and 735 us) where the shapes allow it, the table-driven kernels elsewhere."""
 
     def __init__(self, info: TensorProductInfo, device, out_dims=None, min_batch: int = 0, most_columns: int = 256):
         self.mix_fwd, self.mix_bwd1, self.mix_bwd2 = (t.to(device) for t in (info.info_M_fwd, info.info_M_bwd1, info.info_M_bwd2))
@@ -60,7 +62,14 @@ class MixTables:
 
     def forward(self, s: Tensor, weight: Tensor, mode: str) -> Tensor:
         assert s.shape[1] == self.rows, f"{s.shape[1]} rows for a table of {self.rows}"
-        return _mix(s, weight, self.mix_fwd, mode, self._tensor_cores(s, weight.shape[-1]))
+        tc, info, (cin, cout) = self._tensor_cores(s, weight.shape[-1]), self.mix_fwd, weight.shape[-2:]
+        if (mode == "uv" and tc is None and self.most_columns <= indexed_tc_op.MAX_COLUMNS and s.dtype == torch.float32
+                and cin % 32 == 0 and cout % 16 == 0):
+            parts = [indexed_tc_op.vecmat_tc(s, w.contiguous(), info.scale, info.index1, info.index2, info.seg_out, info.out_size)
+                     for w in weight.split(self.most_columns, dim=-1)]
+            if parts[0] is not None:
+                return parts[0] if len(parts) == 1 else torch.cat(parts, dim=-1)
+        return _mix(s, weight, info, mode, tc)
 
     def _tensor_cores(self, batch: Tensor, columns: int) -> Optional[MixPlan]:
         return self.tc_fwd if batch.shape[0] >= self.min_batch and columns <= self.most_columns else None
