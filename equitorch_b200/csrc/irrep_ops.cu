@@ -591,16 +591,19 @@ __global__ void __launch_bounds__(256) layer_rms_bwd_kernel(const T* __restrict_
     // the block's warps in order
     for (int i = threadIdx.x; i < k * c; i += blockDim.x) fold[i] = T(0);
     __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < LRN_MAX_IRREPS; ++kk) {          // all warps at once: only the additions below take turns
+      if (kk >= k) break;
+#pragma unroll
+      for (int q = 0; q < V; ++q)
+        for (int o = 16; o >= cv; o >>= 1) gwa[kk][q] += __shfl_xor_sync(0xffffffffu, gwa[kk][q], o);
+    }
     for (int turn = 0; turn < 8; ++turn) {
 #pragma unroll
       for (int kk = 0; kk < LRN_MAX_IRREPS; ++kk) {
-        if (kk >= k || (threadIdx.x >> 5) != turn) break;
+        if (kk >= k || (threadIdx.x >> 5) != turn || lane >= cv) break;
 #pragma unroll
-        for (int q = 0; q < V; ++q) {
-          T v = gwa[kk][q];
-          for (int o = 16; o >= cv; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane < cv) fold[kk * c + lane * V + q] += v;
-        }
+        for (int q = 0; q < V; ++q) fold[kk * c + lane * V + q] += gwa[kk][q];
       }
       __syncthreads();
     }
@@ -611,7 +614,9 @@ __global__ void __launch_bounds__(256) layer_rms_bwd_kernel(const T* __restrict_
 // Float32 rows of at most 32 * NV vectors: the warp holds its sample in registers, so all of a sample's loads are in flight
 // at once and nothing is read twice; an element's irrep and channels depend on its position alone and are found before
 // the loop.  The kernels above walk the irreps one after the other (a load, a butterfly and a second read per irrep) and
-// stay for longer rows and float64.  100k x 16 x 64: forward 222 -> 170 us, backward 380 + 58 -> 235 + 4 us.
+// stay for longer rows, rows of fewer than four vectors and float64.  100k x 16 x 64: forward 222 -> 170 us, backward 380 + 58
+// -> 235 + 4 us.  (16 vectors a lane leave one block of eight warps per SM: 50k x 9 x 128 forward 178 us, 96 us above; 500k rows
+// of one vector 136 and 114 us.)
 //
 // sum[u] over the warp of the values that belong to irrep k0 + u: four butterflies side by side, so that their latencies
 // overlap.
@@ -630,7 +635,7 @@ __device__ __forceinline__ void irrep_sums(const float (&v)[NV], const int (&kj)
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256, NV <= 5 ? 3 : NV <= 8 ? 2 : 1) layer_rms_fwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(256, NV <= 5 ? 3 : 2) layer_rms_fwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                  float* __restrict__ out, float* __restrict__ rsigma,
                                                                  const int64_t* __restrict__ irrep_seg, int64_t n, int d, int k, int c,
                                                                  int scaled, float eps) {
@@ -780,11 +785,10 @@ __global__ void __launch_bounds__(lrn_bwd_threads(NV), NV <= 3 || NV > 5 ? 3 : 2
   }
 }
 
-// The smallest instance that holds a row of `vecs` vectors, 0 where none does (two operands and the weight gradient of 16
-// vectors do not fit the registers: forward only).
-int layer_rms_row_vectors(int vecs, int most) {
-  for (int nv : {2, 3, 5, 8, 16})
-    if (nv <= most && vecs <= 32 * nv) return nv;
+// The smallest instance that holds a row of `vecs` vectors, 0 where the kernels that walk the irreps are the better ones.
+int layer_rms_row_vectors(int vecs, int fewest) {
+  for (int nv : {2, 3, 5, 8})
+    if (vecs >= fewest && vecs <= 32 * nv) return nv;
   return 0;
 }
 
@@ -844,11 +848,11 @@ extern "C" int eqt_layer_rms_forward(const void* x, const void* weight, void* ou
     return fail(EQT_ERR_UNSUPPORTED, "fused LayerRMSNorm needs <= %d irreps, C / %d dividing 32 and 16-byte aligned tensors",
                 LRN_MAX_IRREPS, v);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = layer_rms_grid(n);
-  const int nv = dtype == EQT_F32 ? layer_rms_row_vectors(d * (c / 4), 16) : 0;
+  const int nv = dtype == EQT_F32 ? layer_rms_row_vectors(d * (c / 4), 4) : 0;
+  const int grid = nv ? layer_rms_grid(n) : (int)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)sm_count() * 8));
   if (nv) {
     auto* kernel = nv == 2 ? layer_rms_fwd_rows_kernel<2> : nv == 3 ? layer_rms_fwd_rows_kernel<3> : nv == 5 ? layer_rms_fwd_rows_kernel<5>
-                 : nv == 8 ? layer_rms_fwd_rows_kernel<8> : layer_rms_fwd_rows_kernel<16>;
+                 : layer_rms_fwd_rows_kernel<8>;
     kernel<<<grid, 256, 0, st>>>(static_cast<const float*>(x), static_cast<const float*>(weight), static_cast<float*>(out),
                                  static_cast<float*>(rsigma), irrep_seg, n, d, k, c, scaled, (float)eps);
   } else if (dtype == EQT_F32)
@@ -876,7 +880,7 @@ extern "C" int eqt_layer_rms_backward(const void* x, const void* grad_out, const
                 LRN_MAX_IRREPS, v);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = layer_rms_grid(n);
-  const int nv = dtype == EQT_F32 ? layer_rms_row_vectors(d * (c / 4), 8) : 0;
+  const int nv = dtype == EQT_F32 ? layer_rms_row_vectors(d * (c / 4), 1) : 0;
   if (nv) {
     auto* kernel = nv == 2 ? layer_rms_bwd_rows_kernel<2> : nv == 3 ? layer_rms_bwd_rows_kernel<3> : nv == 5 ? layer_rms_bwd_rows_kernel<5>
                                                        : layer_rms_bwd_rows_kernel<8>;
