@@ -87,10 +87,10 @@ struct GemmJob {
 };
 
 int launch_jobs(const GemmJob* jobs, int count, int64_t n, int* status, cudaStream_t st) {
-  {   // per device / context, so set on every call (a cheap host-side call)
-    cudaError_t e = cudaFuncSetAttribute(mix_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  }
+  auto* kernel = mix_tc_kernel<false>;
+  for (int q = 0; q < count; ++q)
+    if (jobs[q].K / KB > MIX_CHUNK_KB) kernel = mix_tc_kernel<true>;
+  if (int rc = allow_shared(kernel, 220 * 1024)) return rc;      // per device / context, so set on every call (a cheap host-side call)
   for (int first = 0; first < count; first += MAX_JOBS) {
     const int m = std::min(MAX_JOBS, count - first);
     MixLaunch L{};
@@ -144,7 +144,7 @@ int launch_jobs(const GemmJob* jobs, int count, int64_t n, int* status, cudaStre
     }
     L.total_tiles = total;
     const unsigned grid = (unsigned)std::min<int64_t>(total, sm_count());
-    mix_tc_kernel<<<grid, TC_THREADS + 32, (size_t)L.stages * stage_bytes + 1024 + epi_bytes, st>>>(L);
+    kernel<<<grid, TC_THREADS + 32, (size_t)L.stages * stage_bytes + 1024 + epi_bytes, st>>>(L);
     if (int rc = check_launch("mix_tc_kernel")) return rc;
   }
   return EQT_OK;
