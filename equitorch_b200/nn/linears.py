@@ -23,11 +23,6 @@ from .functional.sparse_product import sparse_mul, sparse_vecmat
 from .init import initialize_linear, initialize_so3_so2_linear
 
 
-def _version(info) -> Optional[int]:
-    scale = info.info_Mij_fwd.scale
-    return None if scale is None or scale.is_inference() else scale._version
-
-
 class SO3Linear(_WeightedTableModule):
     r"""Tensor product of channelled features with a channel-less second operand
     (typically spherical harmonics of an edge direction).
@@ -72,11 +67,16 @@ class SO3Linear(_WeightedTableModule):
 
     def _own_tables(self, own: bool = True) -> None:
         """``own``: the layer's tables are those of its paths, in the state that they are in now."""
-        self._path_plans, self._own = {}, ((self._tables(), _version(self.tp_info_forward)) if own else None)
+        scale = self.tp_info_forward.info_Mij_fwd.scale
+        version = None if scale is None or scale.is_inference() else scale._version        # inference mode: none to compare
+        self._path_plans, self._own = {}, ((*self._tables(), scale, version) if own else None)
 
     def _is_own(self) -> bool:
-        return (self._own is not None and all(a is b for a, b in zip(self._tables(), self._own[0]))
-                and _version(self.tp_info_forward) == self._own[1])
+        if self._own is None:
+            return False
+        forward, backward1, backward2, scale, version = self._own
+        return (self.tp_info_forward is forward and self.tp_info_backward1 is backward1 and self.tp_info_backward2 is backward2
+                and (version is None or scale._version == version))
 
     def _path_plan(self, device) -> Optional[PathPlan]:
         """The tables of the one-pass kernels on ``device``, built at the first call there; ``None`` when the layer's
