@@ -78,6 +78,16 @@ class PathTableStruct(C.Structure):
                 ("num_fwd_blocks", C.c_int32), ("num_bwd_blocks", C.c_int32), ("num_rows", C.c_int32)]
 
 
+class UvwGroupStruct(C.Structure):
+    _fields_ = [("l", C.c_int32), ("offset", C.c_int32), ("count", C.c_int32)]
+
+
+class UvwRoleStruct(C.Structure):
+    _fields_ = [("paths", C.c_void_p), ("groups", C.c_void_p), ("num_paths", C.c_int32), ("num_groups", C.c_int32), ("ds", C.c_int32),
+                ("df", C.c_int32), ("d_out", C.c_int32), ("ci", C.c_int32), ("ck", C.c_int32), ("cj", C.c_int32), ("stride_i", C.c_int32),
+                ("stride_k", C.c_int32), ("stride_j", C.c_int32), ("stride_p", C.c_int32)]
+
+
 # name -> (restype, argtypes); every symbol declared in include/eqt_b200.h appears here
 SIGNATURES = {
     "eqt_sparse_product": (C.c_int, [C.POINTER(ProductArgs), C.c_void_p]),
@@ -138,6 +148,11 @@ SIGNATURES = {
                                         C.POINTER(EdgeFeaturesStruct), C.c_void_p]),
     "eqt_radius_edges": (C.c_int, [C.POINTER(RadiusGridStruct), C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_int32, C.c_int32,
                                    C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(EdgeFeaturesStruct), C.c_void_p, C.c_void_p]),
+    "eqt_uvw_scratch_floats": (C.c_int64, [C.POINTER(UvwRoleStruct), C.c_int32, C.c_int64]),
+    "eqt_uvw_contract": (C.c_int, [C.POINTER(UvwRoleStruct), C.c_int32] + [C.POINTER(C.c_void_p)] * 3
+                         + [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
+    "eqt_uvw_wgrad_scratch_floats": (C.c_int64, [C.POINTER(UvwRoleStruct), C.c_void_p, C.c_int64]),
+    "eqt_uvw_wgrad": (C.c_int, [C.POINTER(UvwRoleStruct)] + [C.c_void_p] * 6 + [C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
     "eqt_so3_uu_scratch_floats": (C.c_int64, [C.POINTER(PathTableStruct), C.c_int64, C.c_int32, C.c_int32, C.c_int32]),
     "eqt_so3_uu_forward": (C.c_int, [C.POINTER(PathTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                      C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),

@@ -4,7 +4,10 @@ A layer's table is a list of paths (k, i, j) between irreps; what a path does de
 degrees up to ``MAX_L`` the block's multiply-adds are emitted with the CG values as immediates, on register blocks of V
 channels: products of several y components with the same (M, m1) are summed before they meet the channels.
 
-    python -m equitorch_b200.csrc.gen_path_specs        # rewrites generated/path_specs.inc
+``generated/triple_specs.inc`` holds the blocks of a product of two channelled operands in the forms that its kernels take:
+one component of the contracted operand at a time, and all of them from a pair of channels.
+
+    python -m equitorch_b200.csrc.gen_path_specs        # rewrites generated/path_specs.inc and triple_specs.inc
 """
 from __future__ import annotations
 
@@ -12,11 +15,13 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(HERE, "generated", "path_specs.inc")
+TRIPLE_OUT = os.path.join(HERE, "generated", "triple_specs.inc")
 MAX_L = 3
+TRIPLE_MAX_L = 2
 
 
-def triples():
-    return [(lo, l1, l2) for lo in range(MAX_L + 1) for l1 in range(MAX_L + 1) for l2 in range(MAX_L + 1)
+def triples(max_l: int = MAX_L):
+    return [(lo, l1, l2) for lo in range(max_l + 1) for l1 in range(max_l + 1) for l2 in range(max_l + 1)
             if abs(l1 - l2) <= lo <= l1 + l2]
 
 
@@ -58,12 +63,42 @@ def _emit(lo: int, l1: int, l2: int) -> str:
     return "\n".join(out)
 
 
-def generate(path: str = OUT) -> str:
-    body = ["// AUTO-GENERATED by equitorch_b200/csrc/gen_path_specs.py - do not edit.", "#pragma once",
-            "template <int LO, int L1, int L2> struct CgPath;", ""]
-    body += [_emit(*t) for t in triples()]
-    body.append(f"constexpr int PATH_MAX_L = {MAX_L};")
-    text = "\n".join(body) + "\n"
+def _emit_triple(lo: int, ls: int, lf: int) -> str:
+    from ..constants import so3_clebsch_gordan
+    cg = so3_clebsch_gordan(lo, ls, lf)
+    no, ns, nf = 2 * lo + 1, 2 * ls + 1, 2 * lf + 1
+    out = [f"template <> struct CgTriple<{lo}, {ls}, {lf}> {{",
+           "  // o[a] += (sum_b cg[a, b, C] s[b]) z for component C of the contracted operand",
+           f"  template <int C, int V> __device__ __forceinline__ static void column(float (&o)[{no}][V], const float (&s)[{ns}], const float (&z)[V]) {{"]
+    for c in range(nf):
+        out.append(f"    if constexpr (C == {c}) {{")
+        for a in range(no):
+            ts = [(b, float(cg[a, b, c])) for b in range(ns) if cg[a, b, c]]
+            if ts:
+                expr = f"{_lit(ts[0][1])} * s[{ts[0][0]}]"
+                for b, v in ts[1:]:
+                    expr = f"fmaf({_lit(v)}, s[{b}], {expr})"
+                out.append(f"      axpy<V>(o[{a}], {expr}, z);")
+        out.append("    }")
+    out += ["  }",
+            "  // q[c] = sum_(a, b) cg[a, b, c] s[b] g[a], V samples side by side",
+            f"  template <int V> __device__ __forceinline__ static void pair(float (&q)[{nf}][V], const float (&s)[{ns}][V], const float (&g)[{no}][V]) {{",
+            "    float d[V];"]
+    seen = set()
+    for a in range(no):
+        for b in range(ns):
+            cs = [(c, float(cg[a, b, c])) for c in range(nf) if cg[a, b, c]]
+            if not cs:
+                continue
+            out.append(f"    times<V>(d, s[{b}], g[{a}]);")
+            for c, v in cs:
+                out.append(f"    axpy<V>(q[{c}], {_lit(v)}, d);" if c in seen else f"    scaled<V>(q[{c}], {_lit(v)}, d);")
+                seen.add(c)
+    out += ["  }", "};"]
+    return "\n".join(out)
+
+
+def _write(path: str, text: str) -> str:
     os.makedirs(os.path.dirname(path), exist_ok=True)
     if not os.path.exists(path) or open(path).read() != text:
         with open(path, "w") as fh:
@@ -71,5 +106,21 @@ def generate(path: str = OUT) -> str:
     return path
 
 
+def generate_triples(path: str = TRIPLE_OUT) -> str:
+    body = ["// AUTO-GENERATED by equitorch_b200/csrc/gen_path_specs.py - do not edit.", "#pragma once",
+            "template <int LO, int LS, int LF> struct CgTriple;", ""]
+    body += [_emit_triple(*t) for t in triples(TRIPLE_MAX_L)]
+    body.append(f"constexpr int TRIPLE_MAX_L = {TRIPLE_MAX_L};")
+    return _write(path, "\n".join(body) + "\n")
+
+
+def generate(path: str = OUT) -> str:
+    body = ["// AUTO-GENERATED by equitorch_b200/csrc/gen_path_specs.py - do not edit.", "#pragma once",
+            "template <int LO, int L1, int L2> struct CgPath;", ""]
+    body += [_emit(*t) for t in triples()]
+    body.append(f"constexpr int PATH_MAX_L = {MAX_L};")
+    return _write(path, "\n".join(body) + "\n")
+
+
 if __name__ == "__main__":
-    print(generate())
+    print(generate(), generate_triples())

@@ -12,10 +12,11 @@ import torch
 from torch import Tensor
 from torch.autograd import Function
 
+from ...ops import uvw_op as _uvw
 from ...structs import IrrepsInfo, SparseProductInfo, TensorProductInfo
 from ._irrep import irrep_dot
 from ._tp_common import add, expand_like_inter, save_for_tp_backward
-from .linears import _m, _mij, _rot
+from .linears import _dense, _m, _mij, _rot
 from .sparse_product import sparse_mat_t_vec, sparse_mul, sparse_outer, sparse_vecmat
 
 
@@ -92,6 +93,42 @@ class TensorProductUVWDummy(Function):
             gw = sparse_outer(grad, inter.flatten(-2), *_m(f, 2), out_accumulated=ctx.weight_ndim == 4)
             gw = gw.transpose(-1, -2).contiguous().unflatten(-2, inter.shape[-2:])
         return g1, g2, gw, None, None, None
+
+
+class TensorProductUVW(Function):
+    """:func:`tensor_product_uvw` without an intermediate in memory (``plan``: the layer's tables on the device): the output and
+    both operand gradients are the same product with the roles of the operands exchanged.  A backward pass that is itself
+    differentiated is composed of the differentiable products, on the operands as they were given."""
+
+    @staticmethod
+    def forward(ctx, input1, input2, weight, plan, infos):
+        n1, n2, nw = ctx.needs_input_grad[:3]
+        ctx.save_for_backward(input1 if n2 or nw else None, input2 if n1 or nw else None, weight if n1 or n2 else None)
+        ctx.plan, ctx.infos = plan, infos
+        x1, x2, w = _dense(input1, input2, weight)
+        return _uvw.uvw_contract(plan, (None, x1, x2), w, (_uvw.FORWARD,))[0]
+
+    @staticmethod
+    def backward(ctx, grad):
+        input1, input2, weight = ctx.saved_tensors
+        need = ctx.needs_input_grad[:3]
+        if not torch.is_grad_enabled():
+            x1, x2, w, g = _dense(input1, input2, weight, grad)
+            if all(t is None or t.data_ptr() % 16 == 0 for t in (x1, x2, w, g)):
+                roles = tuple(r for r, n in zip((_uvw.GRAD_1, _uvw.GRAD_2), need) if n)
+                grads = iter(_uvw.uvw_contract(ctx.plan, (g, x1, x2), w, roles) if roles else ())
+                gw = _uvw.uvw_wgrad(ctx.plan, x1, x2, g) if need[2] else None
+                return next(grads) if need[0] else None, next(grads) if need[1] else None, gw, None, None
+        r1, r2 = _rot(ctx.infos)
+        g1 = tensor_product_uvw(input2, grad, weight.permute(0, 2, 3, 1).contiguous(), *r1) if need[0] else None
+        g2 = tensor_product_uvw(grad, input1, weight.permute(0, 3, 1, 2).contiguous(), *r2) if need[1] else None
+        gw = None
+        if need[2]:
+            f = ctx.infos[0]
+            inter = sparse_outer(input1, input2, *_mij(f, 0))
+            gw = sparse_outer(grad, inter.flatten(-2), *_m(f, 2), out_accumulated=True)
+            gw = gw.transpose(-1, -2).contiguous().unflatten(-2, inter.shape[-2:])
+        return g1, g2, gw, None, None
 
 
 #: largest per-call intermediate (N, num_Mij, C1, C2) of the 'uvw' product in bytes; larger batches are processed in

@@ -14,16 +14,15 @@ from torch import Tensor
 from ..irreps import check_irreps
 from ..ops.indexed_tc_op import MAX_COLUMNS, MIN_BATCH
 from ..ops.so3_path_op import PathPlan
-from ..tables import (generate_fully_connected_tp_paths, irreps_info, irreps_linear_infos, so2_linear_infos, so3_path_norms,
-                      tp_infos)
-from ._base import _WeightedTableModule
+from ..tables import irreps_info, irreps_linear_infos, so2_linear_infos, tp_infos
+from ._base import _PathModule, _WeightedTableModule
 from .functional.graph_tp import MixTables
 from .functional.linears import SO3LinearUU, SO3LinearUV, irrep_wise_linear, irreps_linear, so3_linear_uu, so3_linear_uv
 from .functional.sparse_product import sparse_mul, sparse_vecmat
 from .init import initialize_linear, initialize_so3_so2_linear
 
 
-class SO3Linear(_WeightedTableModule):
+class SO3Linear(_PathModule):
     r"""Tensor product of channelled features with a channel-less second operand
     (typically spherical harmonics of an edge direction).
 
@@ -34,7 +33,7 @@ class SO3Linear(_WeightedTableModule):
     path by the square root of the number of paths into its output irrep; ``channel_norm``
     (``'uv'`` only) divides by ``sqrt(channels_in)``.
     """
-    _table_attrs = ("tp_info_forward", "tp_info_backward1", "tp_info_backward2")
+    _plan_type = PathPlan
 
     def __init__(self, irreps_in1, irreps_in2, irreps_out, channels_in=None, channels_out=None,
                  internal_weights=True, feature_mode="uu", path_norm=True, channel_norm=False, path=None):
@@ -55,52 +54,10 @@ class SO3Linear(_WeightedTableModule):
         (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2, self.num_paths) = tp_infos(
             self.irreps_out, self.irreps_in1, self.irreps_in2, path=path, path_norm=path_norm,
             channel_norm=self.channel_norm, channel_scale=fan_in ** (-0.5) if fan_in else 1.0)
-        paths = path or generate_fully_connected_tp_paths(self.irreps_out, self.irreps_in1, self.irreps_in2)
-        self._paths = (list(paths), so3_path_norms(paths, path_norm, self.channel_norm, fan_in ** (-0.5) if fan_in else 1.0))
-        self._own_tables()
+        self._set_paths(path, fan_in)
         shape = (self.num_paths, channels_in, channels_out) if feature_mode == "uv" else (self.num_paths, channels_out)
         self._setup_weight(shape, internal_weights,
                            lambda w: initialize_so3_so2_linear(w, feature_mode, channel_normed=self.channel_norm))
-
-    def _tables(self):
-        return self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2
-
-    def _own_tables(self, own: bool = True) -> None:
-        """``own``: the layer's tables are those of its paths, in the state that they are in now."""
-        scale = self.tp_info_forward.info_Mij_fwd.scale
-        version = None if scale is None or scale.is_inference() else scale._version        # inference mode: none to compare
-        self._path_plans, self._own = {}, ((*self._tables(), scale, version) if own else None)
-
-    def _is_own(self) -> bool:
-        if self._own is None:
-            return False
-        forward, backward1, backward2, scale, version = self._own
-        return (self.tp_info_forward is forward and self.tp_info_backward1 is backward1 and self.tp_info_backward2 is backward2
-                and (version is None or scale._version == version))
-
-    def _path_plan(self, device) -> Optional[PathPlan]:
-        """The tables of the one-pass kernels on ``device``, built at the first call there; ``None`` when the layer's
-        own tables have been exchanged or written to, and while a stream is being captured that would have to wait for
-        their copy to the device."""
-        if not self._is_own():
-            return None
-        plan = self._path_plans.get(device)
-        if plan is None and not torch.cuda.is_current_stream_capturing():
-            plan = self._path_plans[device] = PathPlan(*self._paths, self.irreps_out, self.irreps_in1, self.irreps_in2, device)
-        return plan
-
-    def _apply(self, fn, *args, **kwargs):
-        own = self._is_own()
-        module = super()._apply(fn, *args, **kwargs)
-        module._own_tables(own)
-        return module
-
-    def __getstate__(self):
-        return {**{k: v for k, v in self.__dict__.items() if k not in ("_path_plans", "_plans")}, "_own": self._is_own()}
-
-    def __setstate__(self, state):
-        super().__setstate__(state)
-        self._own_tables(bool(state.get("_own", False)))          # a layer stored without its paths runs the composed products
 
     def forward(self, input1: Tensor, input2: Tensor, weight: Optional[Tensor] = None) -> Tensor:
         assert input1.shape[-2] == self.irreps_in1_dim, \

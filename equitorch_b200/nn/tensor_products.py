@@ -6,19 +6,20 @@ from typing import Optional
 from torch import Tensor, nn
 
 from ..irreps import check_irreps
+from ..ops.uvw_op import UvwPlan
 from ..tables import irreps_info, tp_infos
-from ._base import _WeightedTableModule
-from .functional.tensor_products import tensor_dot_uu, tensor_dot_uv, tensor_product_uuu, tensor_product_uvw
+from ._base import _PathModule
+from .functional.tensor_products import TensorProductUVW, tensor_dot_uu, tensor_dot_uv, tensor_product_uuu, tensor_product_uvw
 from .init import initialize_tensor_product
 
 
-class TensorProduct(_WeightedTableModule):
+class TensorProduct(_PathModule):
     """Weighted Clebsch-Gordan tensor product of two channelled feature tensors.
 
     ``'uvw'``: ``(N, D1, C1) x (N, D2, C2)`` with weight ``(num_paths, C1, C2, Cout)`` -> ``(N, Dout, Cout)``.
     ``'uuu'``: equal channel counts, weight ``(num_paths, C)``, channels are not mixed.
     """
-    _table_attrs = ("tp_info_forward", "tp_info_backward1", "tp_info_backward2")
+    _plan_type = UvwPlan
 
     def __init__(self, irreps_in1, irreps_in2, irreps_out, channels_in1=None, channels_in2=None,
                  channels_out=None, internal_weights=True, feature_mode="uuu", path_norm=True,
@@ -38,6 +39,7 @@ class TensorProduct(_WeightedTableModule):
         (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2, self.num_paths) = tp_infos(
             self.irreps_out, self.irreps_in1, self.irreps_in2, path=path, path_norm=path_norm,
             channel_norm=self.channel_norm, channel_scale=fan_in ** (-0.5))
+        self._set_paths(path, fan_in)
         shape = ((self.num_paths, channels_in1, channels_in2, channels_out) if feature_mode == "uvw"
                  else (self.num_paths, channels_out))
         self._setup_weight(shape, internal_weights,
@@ -54,6 +56,11 @@ class TensorProduct(_WeightedTableModule):
         else:
             assert input1.shape[-1] == input2.shape[-1], "Input channel dims must match in 'uuu' mode"
         weight = self._resolve_weight(weight)
+        if self.feature_mode == "uvw" and input1.is_cuda:
+            plan = self._path_plan(input1.device)
+            if plan is not None and plan.supported(input1, input2, weight):
+                return TensorProductUVW.apply(input1, input2, weight, plan,
+                                              (self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2))
         fn = tensor_product_uuu if self.feature_mode == "uuu" else tensor_product_uvw
         return fn(input1, input2, weight, self.tp_info_forward, self.tp_info_backward1, self.tp_info_backward2)
 

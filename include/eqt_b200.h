@@ -380,6 +380,41 @@ int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, const void* 
                         int32_t per_sample_weight, int32_t dtype, void* stream);
 
 /*
+ * Product of two channelled operands with full channel mixing ('uvw' TensorProduct), float32, weights shared by the batch,
+ * degrees up to 2, 16 or 32 channels per operand, without an intermediate in memory.  A role says which operand is which:
+ *   out[n, a, j] = sum_p scale_p sum_(b, c) cg[a, b, c] sum_(i, k) s[n, b, i] f[n, c, k] W[p, i, k, j]
+ * with cg the Clebsch-Gordan block of the path's three degrees in the order (out, s, f).  The output of the layer and the
+ * gradients of its two operands are three roles of the same product (for the exchanged ones `scale` also holds the ratio of the
+ * blocks' normalisations); eqt_uvw_contract evaluates up to two of them at a time (with the same cj).  Paths are listed by
+ * irrep of f (`groups`, host memory, in the order of the list) and by output component inside; device memory.
+ * eqt_uvw_wgrad: gw[p, i, k, j] = scale_p sum_n sum_(a, b, c) cg[a, b, c] s[n, b, i] f[n, c, k] g[n, a, j], every weight written;
+ * `degrees` (host, 3 per path: out, s, f) in the order of the list.
+ * Scratch: *_scratch_floats(); -1 = these sizes are not supported.  All operands 16-byte aligned.  Sums of the thread blocks
+ * are added in a fixed order.
+ * replaces: TensorProductUVWDummy and its adjoints (equitorch/nn/functional/tensor_products.py:92-172).
+ */
+typedef struct eqt_uvw_path {
+  int32_t l_o, l_s, l_f, offset_o, offset_s, offset_f, weight;
+  float scale;
+} eqt_uvw_path;
+typedef struct eqt_uvw_group {
+  int32_t l, offset, count;    /* irrep of f: degree, first component, paths                       */
+} eqt_uvw_group;
+typedef struct eqt_uvw_role {
+  const eqt_uvw_path* paths;   /* device                                                           */
+  const eqt_uvw_group* groups; /* host                                                             */
+  int32_t num_paths, num_groups, ds, df, d_out;
+  int32_t ci, ck, cj;          /* channels of s, f and out                                         */
+  int32_t stride_i, stride_k, stride_j, stride_p; /* of the weights (and of gw), in floats         */
+} eqt_uvw_role;
+int64_t eqt_uvw_scratch_floats(const eqt_uvw_role* roles, int32_t jobs, int64_t n);
+int eqt_uvw_contract(const eqt_uvw_role* roles, int32_t jobs, const float* const* s, const float* const* f, float* const* out,
+                     const float* w, float* scratch, int64_t scratch_floats, int64_t n, int32_t* status, void* stream);
+int64_t eqt_uvw_wgrad_scratch_floats(const eqt_uvw_role* role, const int32_t* degrees, int64_t n);
+int eqt_uvw_wgrad(const eqt_uvw_role* role, const int32_t* degrees, const float* s, const float* f, const float* g, float* gw,
+                  float* scratch, int64_t scratch_floats, int64_t n, int32_t* status, void* stream);
+
+/*
  * The channel-wise half of the layer with full channel mixing ('uv' SO3Linear), float32, same tables:
  *   expand:   rows[n, r, c] = sum_t s_t x[n, M1_t, c] y[n, M2_t] over the entries of row r = (output component, path)
  *   backward: gx and gy from the gradient of the rows, in one pass over it

@@ -1,0 +1,68 @@
+"""'uvw' ``TensorProduct`` without an intermediate (tensor-core contraction of one operand with the weights, the other operand and the
+Clebsch-Gordan blocks in the epilogue) against the dense float64 oracle: sample tiles and chunks of 32 with remainders, one sample,
+batches of several waves, 16 and 32 channels on every side, degrees of either parity, repeated irreps, output components that
+no path reaches; and the exchange of roles against the blocks themselves."""
+import numpy as np
+import pytest
+import torch
+
+from equitorch_b200 import nn as enn
+from equitorch_b200.constants import so3_clebsch_gordan
+from equitorch_b200.nn.functional.tensor_products import TensorProductUVW, tensor_product_uvw
+from equitorch_b200.ops.uvw_op import FORWARD, GRAD_1, GRAD_2, exchanged_scale
+from oracle import tensor_products as otp
+
+DEV = "cuda:0"
+
+
+def _rel(a, b):
+    return float((a.detach().double().cpu() - b.detach().double()).norm() / b.detach().double().norm())
+
+
+@pytest.mark.parametrize("degrees", [(0, 0, 0), (1, 1, 0), (0, 2, 2), (2, 1, 1), (1, 1, 1), (2, 2, 1), (2, 2, 2)])
+def test_exchanged_roles_are_multiples(degrees):
+    ours = so3_clebsch_gordan(*degrees)
+    for role in (FORWARD, GRAD_1, GRAD_2):
+        block = so3_clebsch_gordan(*(degrees[a] for a in role))
+        assert np.abs(ours.transpose(role) - exchanged_scale(degrees, role) * block).max() < 1e-14
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ir1,ir2,ir_out,n,c1,c2,c_out", [
+    ("0e+1o", "0e+1o", "0e+1o", 1, 16, 16, 16), ("0e+1o+2e", "0e+1o+2e", "0e+1o+2e", 31, 32, 32, 32),
+    ("0e+1o+2e", "0e+1o+2e", "0e+1o+2e", 129, 16, 32, 32), ("0e+1o+2e", "0e+1o+2e", "0e+1o+2e", 2003, 32, 16, 16),
+    ("2x0e+1o+1e", "0e+1o+2e+2o", "1e+2x2o+0o+1o", 257, 32, 32, 16), ("0e+1o+2e", "0e+1o+2e", "0e+1o+2e", 20011, 16, 16, 32),
+    ("0e", "1o", "1o+2e", 100, 16, 16, 16)])
+def test_against_the_oracle(ir1, ir2, ir_out, n, c1, c2, c_out):
+    g = torch.Generator().manual_seed(n)
+    layer = enn.TensorProduct(ir1, ir2, ir_out, c1, c2, c_out, internal_weights=False, feature_mode="uvw").to(DEV)
+    x1, x2 = torch.randn(n, layer.irreps_in1_dim, c1, generator=g), torch.randn(n, layer.irreps_in2_dim, c2, generator=g)
+    w, cot = torch.randn(*layer.weight_shape, generator=g), torch.randn(n, layer.irreps_out_dim, c_out, generator=g)
+    leaves = [t.to(DEV).requires_grad_(True) for t in (x1, x2, w)]
+    out = layer(*leaves)
+    assert type(out.grad_fn).__name__ == TensorProductUVW.__name__ + "Backward"
+    got = [out, *torch.autograd.grad(out, leaves, cot.to(DEV))]
+    where = DEV if n > 1000 else "cpu"                                    # the oracle's float64 sums of large batches
+    ref = [t.to(where).double().requires_grad_(True) for t in (x1, x2, w)]
+    want = [otp.tensor_product_dense(*ref, layer.irreps_in1, layer.irreps_in2, layer.irreps_out, feature_mode="uvw")]
+    want += torch.autograd.grad(want[0], ref, cot.to(where).double())
+    # split of both factors 2^-22 each, rounding of the sums and, per step of eight terms, one truncation by the tensor core
+    for a, b in zip(got, want):
+        assert _rel(a, b.cpu()) < 1e-6
+    (only,) = torch.autograd.grad(layer(leaves[0].detach(), leaves[1], w.to(DEV)), [leaves[1]], cot.to(DEV))
+    assert _rel(only, want[2].cpu()) < 1e-6
+
+
+@pytest.mark.gpu
+def test_second_derivatives_are_those_of_the_composed_product():
+    g = torch.Generator(device=DEV).manual_seed(3)
+    ir, c, n = "0e+1o+2e", 16, 70
+    layer = enn.TensorProduct(ir, ir, ir, c, c, c, internal_weights=False, feature_mode="uvw").to(DEV)
+    leaves = [torch.randn(*s, generator=g, device=DEV).requires_grad_(True) for s in ((n, 9, c), (n, 9, c), layer.weight_shape)]
+    cot = torch.randn(n, 9, c, generator=g, device=DEV)
+    results = []
+    for fn in (layer, lambda *a: tensor_product_uvw(*a, layer.tp_info_forward, layer.tp_info_backward1, layer.tp_info_backward2)):
+        first = torch.autograd.grad(fn(*leaves), leaves, cot, create_graph=True)
+        results.append([*first, *torch.autograd.grad(sum(t.square().sum() for t in first), leaves)])
+    for a, b in zip(*results):
+        assert _rel(a, b.cpu()) < 1e-5
