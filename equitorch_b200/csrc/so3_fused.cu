@@ -503,7 +503,6 @@ constexpr int THREADS = 16 * 32;
 constexpr int GE = 8;                  // edges per group (one tf32 MMA k-step)
 constexpr int NS = 4;                  // ring slots
 constexpr int ROWF = 1024;             // floats per gathered row (16 components x 64 channels)
-constexpr int NODES_PER_CHUNK = 16;
 constexpr uint32_t TMEM_COLS = 512;    // 2 x 128 accumulators + 2 x 128 A slots
 constexpr uint32_t COL_A = 256;
 
@@ -529,27 +528,27 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
       : "memory");
 }
 
-// The node walk every role performs: nodes come in chunks of NODES_PER_CHUNK dealt round-robin to the CTAs.  The
+// The node walk every role performs: nodes come in chunks of nodes_per_cta dealt round-robin to the CTAs.  The
 // segment pointers are read two nodes ahead of their use, so the walk does not wait for a load per node.
 struct Walk {
   const int64_t* ptr;
-  int n_out;            // 32-bit state: the launcher checks that nodes and edges fit
+  int n_out, per;       // 32-bit state: the launcher checks that nodes and edges fit
   int chunk;            // current chunk
   int d_in;             // next node inside the chunk
   int p0, p1, p2;       // ptr[d], ptr[d + 1], ptr[d + 2] of the next node d
   __device__ int at(int i) const { return (int)__ldg(ptr + min(i, n_out)); }
   __device__ void prime() {
-    const int d = chunk * NODES_PER_CHUNK;
+    const int d = chunk * per;
     p0 = at(d); p1 = at(d + 1); p2 = at(d + 2);
   }
-  __device__ Walk(const FusedArgs& a) : ptr(a.ptr), n_out((int)a.n_out), chunk(blockIdx.x), d_in(0) { prime(); }
+  __device__ Walk(const FusedArgs& a) : ptr(a.ptr), n_out((int)a.n_out), per(a.nodes_per_cta), chunk(blockIdx.x), d_in(0) { prime(); }
   // next node of this CTA: returns false at the end; d = node, e0 = its first edge, deg = its edge count
   __device__ bool next(int& d, int& e0, int& deg) {
-    d = chunk * NODES_PER_CHUNK + d_in;
-    if (d_in >= NODES_PER_CHUNK || d >= n_out) {
+    d = chunk * per + d_in;
+    if (d_in >= per || d >= n_out) {
       chunk += gridDim.x;
       d_in = 0;
-      d = chunk * NODES_PER_CHUNK;
+      d = chunk * per;
       if (d >= n_out) return false;
       prime();
     }
@@ -776,15 +775,18 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
   }
 }
 
+// Nodes that a CTA of the persistent kernel takes at a time: at most 16, and sixteen rounds of the CTAs where there are that many
+// nodes, so that the last round weighs little (10k nodes in chunks of 16 were 4.2 rounds of 148 CTAs, i.e. five: 230 us for 200k edges,
+// 202 us in chunks of four; below 2400 nodes chunks of 16 leave SMs without any).
 template <class S>
-int launch_segsum_tc(const FusedArgs& a, cudaStream_t s) {
+int launch_segsum_tc(FusedArgs a, cudaStream_t s) {
   if constexpr (S::HAS_TC) {
+    a.nodes_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(16, a.n_out / ((int64_t)sm_count() * 16)));
     constexpr size_t bytes = segtc::OFF_SC + sizeof(float) * ((S::T + 3) & ~3) + 1024;
     auto kern = tp_segsum_tc_kernel<S>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    const int64_t chunks = ceil_div(a.n_out, segtc::NODES_PER_CHUNK);
-    kern<<<(unsigned)std::min<int64_t>(chunks, sm_count()), segtc::THREADS, bytes, s>>>(a);
+    kern<<<(unsigned)std::min<int64_t>(ceil_div(a.n_out, a.nodes_per_cta), sm_count()), segtc::THREADS, bytes, s>>>(a);
     return check_launch("tp_segsum_tc_kernel");
   } else {
     return -1;
