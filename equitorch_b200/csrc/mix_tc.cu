@@ -404,6 +404,25 @@ extern "C" int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64
     if (int rc = make_map(&L.map_bb, w_big, 2, dims, strides, box)) return rc;
     if (int rc = make_map(&L.map_bs, w_small, 2, dims, strides, box)) return rc;
   }
+  // Resident weights: one-row groups of short sums over rows of x that are read about once (an output row's items run one after
+  // the other, so a row that several output rows read would come from memory each time), 128 columns with two A slots.
+  const int b_bytes = longest * n_cols * KB * 8;
+  if (group == 1 && longest >= 1 && longest <= VM_SHORT_CHUNK_KB && slots <= rows1 + rows1 / 2 && b_bytes <= 96 * 1024 &&
+      (n_cols <= 64 || (n_cols == 128 && longest <= 2))) {
+    ResidentLaunch R{};
+    R.map_a = L.map_a; R.map_bb = L.map_bb; R.map_bs = L.map_bs;
+    R.out = out; R.kb_begin = kb_begin; R.rows = group_rows; R.a_col = a_col; R.status = status;
+    R.n = n; R.tiles = ceil_div(n, TILE_M); R.total_items = L.total_items;
+    R.num_out = num_out; R.n_cols = n_cols; R.units = n_cols > 64 ? 2 : 1; R.unit_cols = n_cols / R.units;
+    R.slots = std::min(4, (512 - 6 * R.unit_cols) / 64);
+    R.b_bytes = b_bytes;
+    R.raw_stages = (int)std::min<size_t>(8, (220 * 1024 - 1024 - EPI_PATCH_BYTES - b_bytes) / (TILE_M * KB * 4));
+    auto* resident = longest == 1 ? vecmat_resident_kernel<true> : vecmat_resident_kernel<false>;
+    if (int rc = allow_shared(resident, 220 * 1024)) return rc;
+    resident<<<(unsigned)std::min<int64_t>(R.total_items, sm_count()), TC_THREADS,
+               (size_t)b_bytes + (size_t)R.raw_stages * TILE_M * KB * 4 + 1024 + EPI_PATCH_BYTES, st>>>(R);
+    return check_launch("vecmat_resident_kernel");
+  }
   auto* kernel = group == 1 && longest == 1 ? vecmat_tc_kernel<true> : vecmat_tc_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));

@@ -1,0 +1,41 @@
+"""``IrrepsLinear`` on the tensor-core product that keeps an output row's weights in shared memory, against float64: widths of one and
+of two accumulator units, sums of one to four k-blocks (the most it takes) and of five (not taken), batches that end inside a
+sample tile, ranges that begin and end inside an output row, a row that no path reaches, and rows that several outputs read."""
+import pytest
+import torch
+
+from equitorch_b200 import nn as enn
+from equitorch_b200.ops.fused_tp_op import check_status
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("ir_in,ir_out,n,cin,cout", [
+    ("0e+1o+2e+3o", "0e+1o+2e+3o", 513, 64, 128), ("0e+1o", "0e+1o", 20011, 32, 128), ("0e+1o+2e", "0e+1o+2e", 1000, 64, 48),
+    ("0e+1o", "0e+1o", 5003, 128, 64), ("0e+1o+2e", "0e+1o+2e", 700, 96, 16), ("0e+1o", "0e+1o", 640, 160, 32),
+    ("0e+1o", "0e+1e+1o", 2049, 64, 64), ("0e+1o", "2x0e+2x1o", 1500, 32, 64), ("2x0e+1o", "0e+1o", 1281, 64, 128), ("0e", "0e", 512, 128, 128)])
+def test_against_float64(ir_in, ir_out, n, cin, cout):
+    g = torch.Generator(device=DEV).manual_seed(n)
+    layer = enn.IrrepsLinear(ir_in, ir_out, cin, cout, internal_weights=False).to(DEV)
+    x = torch.randn(n, layer.irreps_in.dim, cin, generator=g, device=DEV).requires_grad_(True)
+    w = (torch.randn(*layer.weight_shape, generator=g, device=DEV) * cin ** -0.5).requires_grad_(True)
+    cot = torch.randn(n, layer.irreps_out.dim, cout, generator=g, device=DEV)
+    out = layer(x, w)
+    got = [out, *torch.autograd.grad(out, [x, w], cot)]
+    check_status(torch.device(DEV))
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    f = layer.forward_info
+    want = xd.new_zeros(n, layer.irreps_out.dim, cout)
+    seg = f.M_seg_MM0.tolist()
+    rows = []
+    for r in range(len(seg) - 1):
+        rows.append(sum(f.scale_MM0[t].double() * xd[:, f.M0_MM0[t]] @ wd[f.ii0_MM0[t]] for t in range(seg[r], seg[r + 1])))
+    want = want.index_add(1, f.M_out, torch.stack(rows, dim=1))
+    # three products of TF32 pairs, at most eight truncating steps per accumulator: a few units of 2^-24
+    for a, b in zip(got, [want, *torch.autograd.grad(want, [xd, wd], cot.double())]):
+        assert _rel(a.detach(), b.detach()) < 2e-6
