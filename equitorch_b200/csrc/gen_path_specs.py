@@ -68,8 +68,8 @@ def _emit_triple(lo: int, ls: int, lf: int) -> str:
     cg = so3_clebsch_gordan(lo, ls, lf)
     no, ns, nf = 2 * lo + 1, 2 * ls + 1, 2 * lf + 1
     out = [f"template <> struct CgTriple<{lo}, {ls}, {lf}> {{",
-           "  // o[a] += (sum_b cg[a, b, C] s[b]) z for component C of the contracted operand",
-           f"  template <int C, int V> __device__ __forceinline__ static void column(float (&o)[{no}][V], const float (&s)[{ns}], const float (&z)[V]) {{"]
+           "  // o[a] += (sum_b cg[a, b, C] s[b]) z for component C of the contracted operand, 2 V columns",
+           f"  template <int C, int V> __device__ __forceinline__ static void column(Two (&o)[{no}][V], const float (&s)[{ns}], const Two (&z)[V]) {{"]
     for c in range(nf):
         out.append(f"    if constexpr (C == {c}) {{")
         for a in range(no):
@@ -81,9 +81,9 @@ def _emit_triple(lo: int, ls: int, lf: int) -> str:
                 out.append(f"      axpy<V>(o[{a}], {expr}, z);")
         out.append("    }")
     out += ["  }",
-            "  // q[c] = sum_(a, b) cg[a, b, c] s[b] g[a], V samples side by side",
-            f"  template <int V> __device__ __forceinline__ static void pair(float (&q)[{nf}][V], const float (&s)[{ns}][V], const float (&g)[{no}][V]) {{",
-            "    float d[V];"]
+            "  // q[c] = sum_(a, b) cg[a, b, c] s[b] g[a], 2 V samples side by side",
+            f"  template <int V> __device__ __forceinline__ static void pair(Two (&q)[{nf}][V], const Two (&s)[{ns}][V], const Two (&g)[{no}][V]) {{",
+            "    Two d[V];"]
     seen = set()
     for a in range(no):
         for b in range(ns):

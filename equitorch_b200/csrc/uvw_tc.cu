@@ -34,17 +34,37 @@ namespace eqt {
 namespace {
 using namespace tc;
 
-template <int N> __device__ __forceinline__ void axpy(float (&o)[N], float s, const float (&x)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = fmaf(s, x[i], o[i]);
+// Two float32 values in one 64-bit register pair: packed multiply-adds (fma.rn.f32x2) take half the issue slots.
+struct Two { unsigned long long v; };
+__device__ __forceinline__ Two two(float x, float y) {
+  Two r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
 }
-template <int N> __device__ __forceinline__ void times(float (&o)[N], const float (&a)[N], const float (&b)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = a[i] * b[i];
+__device__ __forceinline__ void apart(const Two& t, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(t.v)); }
+__device__ __forceinline__ Two fma2(const Two& a, const Two& b, const Two& c) {
+  Two r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
 }
-template <int N> __device__ __forceinline__ void scaled(float (&o)[N], float s, const float (&x)[N]) {
+__device__ __forceinline__ Two mul2(const Two& a, const Two& b) {
+  Two r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+template <int N> __device__ __forceinline__ void axpy(Two (&o)[N], float s, const Two (&x)[N]) {
+  const Two k = two(s, s);
 #pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = s * x[i];
+  for (int i = 0; i < N; ++i) o[i] = fma2(k, x[i], o[i]);
+}
+template <int N> __device__ __forceinline__ void times(Two (&o)[N], const Two (&a)[N], const Two (&b)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) o[i] = mul2(a[i], b[i]);
+}
+template <int N> __device__ __forceinline__ void scaled(Two (&o)[N], float s, const Two (&x)[N]) {
+  const Two k = two(s, s);
+#pragma unroll
+  for (int i = 0; i < N; ++i) o[i] = mul2(k, x[i]);
 }
 
 #include "generated/triple_specs.inc"
@@ -70,7 +90,7 @@ __device__ __forceinline__ void split4(const float4 v, float4& hi, float4& lo) {
 }
 
 struct ContractJob {
-  const float* s;                  // (n, ds, ci)
+  const float* s;                  // (ds, ci, padded n): transposed, so that the samples of a warp are one run
   const float* f;                  // (n, df, ck)
   float* out;                      // (slices, n, d_out, J): partial sums, or the output itself with one slice
   float* sum;                      // (n, d_out, J)
@@ -83,7 +103,7 @@ struct Segment { short job, group, q0, q1; int slice; };       // channel groups
 struct ContractLaunch {
   ContractJob job[2];
   Segment seg[MAX_SEGMENTS];
-  int64_t n;
+  int64_t n, pad;                  // samples, and that rounded up to whole tiles
   int segments, tiles;
   int* status;
 };
@@ -124,32 +144,46 @@ struct ContractBars {
   uint64_t b_full[B_STAGES], b_empty[B_STAGES], full[SLOTS], empty[SLOTS];
 };
 
-// The contraction of one thread: sample `n` (clamped to the batch), columns [half * JH, (half + 1) * JH) of every channel.
+// The contraction of one thread: one sample, columns [half * J / 2, (half + 1) * J / 2) of every channel, two side by side.
 template <int J> struct Contraction {
   static constexpr int JH = J / 2, IQ = COLS / J;
   const ContractJob& job;
   ContractBars& bars;
   volatile int* ab;
   uint32_t taddr;            // TMEM lane of the thread's sample, first column of its half
-  int64_t n;
+  const float* s;            // the sample in the transposed operand
+  int64_t pad;
   int q0, q1, lane;
   Ring slot;
   bool ok = true;
 
+  // The accumulator of channel i + 1 and its coefficients are on their way while those of channel i are used.
   template <int LO, int LS, int LF, int C>
-  __device__ __forceinline__ void column(float (&acc)[2 * LO + 1][JH], const float (&s)[IQ][2 * LS + 1]) {
+  __device__ __forceinline__ void column(Two (&acc)[2 * LO + 1][JH / 2], const float* sp) {
     if (!ok || !bar_wait(&bars.full[slot.s], slot.ph, ab)) { ok = false; return; }
     tc_fence_after();
     const uint32_t at = taddr + (uint32_t)(slot.s * COLS);
+    const int64_t step = job.ci * pad;
+    uint32_t z[JH];
+    float next[2 * LS + 1];
+    tmem_request<JH>(at, z);
+#pragma unroll
+    for (int b = 0; b < 2 * LS + 1; ++b) next[b] = __ldg(sp + b * step);
 #pragma unroll
     for (int i = 0; i < IQ; ++i) {
-      uint32_t z[JH];
-      tmem_request<JH>(at + i * J, z);
       tmem_arrived<JH>(z);
-      float v[JH];
+      Two v[JH / 2];
+      float now[2 * LS + 1];
 #pragma unroll
-      for (int j = 0; j < JH; ++j) v[j] = __uint_as_float(z[j]);
-      CgTriple<LO, LS, LF>::template column<C, JH>(acc, s[i], v);
+      for (int j = 0; j < JH / 2; ++j) v[j] = two(__uint_as_float(z[2 * j]), __uint_as_float(z[2 * j + 1]));
+#pragma unroll
+      for (int b = 0; b < 2 * LS + 1; ++b) now[b] = next[b];
+      if (i + 1 < IQ) {
+        tmem_request<JH>(at + (i + 1) * J, z);
+#pragma unroll
+        for (int b = 0; b < 2 * LS + 1; ++b) next[b] = __ldg(sp + b * step + (i + 1) * pad);
+      }
+      CgTriple<LO, LS, LF>::template column<C, JH / 2>(acc, now, v);
     }
     tc_fence_before();
     __syncwarp();
@@ -157,26 +191,18 @@ template <int J> struct Contraction {
     slot.next(SLOTS);
   }
 
-  template <int LO, int LS, int LF> __device__ __forceinline__ void path(float (&acc)[2 * LO + 1][JH], int offset_s) {
+  template <int LO, int LS, int LF> __device__ __forceinline__ void path(Two (&acc)[2 * LO + 1][JH / 2], int offset_s) {
     if constexpr (couples(LO, LS, LF)) {
-      const float* sp = job.s + (n * job.ds + offset_s) * job.ci + q0 * IQ;
-      for (int q = q0; q < q1; ++q, sp += IQ) {
-        float s[IQ][2 * LS + 1];
-#pragma unroll
-        for (int b = 0; b < 2 * LS + 1; ++b)
-#pragma unroll
-          for (int i = 0; i < IQ; i += 4) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(sp + b * job.ci + i));
-            s[i][b] = v.x; s[i + 1][b] = v.y; s[i + 2][b] = v.z; s[i + 3][b] = v.w;
-          }
-        column<LO, LS, LF, 0>(acc, s);
+      const float* sp = s + ((int64_t)offset_s * job.ci + q0 * IQ) * pad;
+      for (int q = q0; q < q1; ++q, sp += IQ * pad) {
+        column<LO, LS, LF, 0>(acc, sp);
         if constexpr (LF > 0) {
-          column<LO, LS, LF, 1>(acc, s);
-          column<LO, LS, LF, 2>(acc, s);
+          column<LO, LS, LF, 1>(acc, sp);
+          column<LO, LS, LF, 2>(acc, sp);
         }
         if constexpr (LF > 1) {
-          column<LO, LS, LF, 3>(acc, s);
-          column<LO, LS, LF, 4>(acc, s);
+          column<LO, LS, LF, 3>(acc, sp);
+          column<LO, LS, LF, 4>(acc, sp);
         }
       }
     }
@@ -184,11 +210,11 @@ template <int J> struct Contraction {
 
   // all paths of an irrep of f into one output irrep; returns the path behind them
   template <int LO, int LF> __device__ __forceinline__ int block(int q, int end, float* out, bool store) {
-    float acc[2 * LO + 1][JH];
+    Two acc[2 * LO + 1][JH / 2];
 #pragma unroll
     for (int a = 0; a < 2 * LO + 1; ++a)
 #pragma unroll
-      for (int j = 0; j < JH; ++j) acc[a][j] = 0.f;
+      for (int j = 0; j < JH / 2; ++j) acc[a][j] = two(0.f, 0.f);
     const int offset_o = __ldg(&job.paths[q].offset_o);
     for (; q < end && ok && __ldg(&job.paths[q].offset_o) == offset_o; ++q) {
       const int offset_s = __ldg(&job.paths[q].offset_s);
@@ -203,7 +229,7 @@ template <int J> struct Contraction {
       for (int a = 0; a < 2 * LO + 1; ++a)
 #pragma unroll
         for (int j = 0; j < JH; j += 4)
-          *reinterpret_cast<float4*>(out + (offset_o + a) * J + j) = make_float4(acc[a][j], acc[a][j + 1], acc[a][j + 2], acc[a][j + 3]);
+          *reinterpret_cast<ulonglong2*>(out + (offset_o + a) * J + j) = make_ulonglong2(acc[a][j / 2].v, acc[a][j / 2 + 1].v);
     return q;
   }
 
@@ -343,9 +369,9 @@ __global__ void __launch_bounds__(CONTRACT_THREADS, 1) uvw_contract_kernel(const
     // ---------------- contraction ----------------
     const int quarter = warp & 3, half = warp >> 2;
     const int64_t n = tile * 128 + quarter * 32 + lane;
-    Contraction<J> w{job, bars, ab, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * (J / 2)), min(n, p.n - 1),
+    Contraction<J> w{job, bars, ab, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * (J / 2)), job.s + n, p.pad,
                      seg.q0, seg.q1, lane};
-    float* out = job.out + (((int64_t)seg.slice * p.n + w.n) * job.d_out) * J + half * (J / 2);
+    float* out = job.out + (((int64_t)seg.slice * p.n + min(n, p.n - 1)) * job.d_out) * J + half * (J / 2);
     switch (lf) {
       case 0: w.template run<0>(first, first + count, out, n < p.n); break;
       case 1: w.template run<1>(first, first + count, out, n < p.n); break;
@@ -369,17 +395,36 @@ __global__ void __launch_bounds__(CONTRACT_THREADS, 1) uvw_contract_kernel(const
   }
 }
 
-// Weights of every (path, channel group) as the image that a stage of the contraction holds: row (i, j) of the group, K = k,
-// scaled, split and swizzled.  A thread writes four k of one row.
+// What a contraction reads, one slice of the grid per job and kind.  Weights of every (path, channel group) as the image that a
+// stage holds: row (i, j) of the group, K = k, scaled, split and swizzled; a thread writes four k of one row.  And s with the
+// samples last, through shared memory in blocks of 32 x 32 (rows past the batch are zero).
 struct PackJob {
   const eqt_uvw_path* paths;
   unsigned char* packed;
   int64_t si, sk, sj, sp;          // strides of the weights: i, k, j, path
   int ci, ck, cj, num_paths;
+  const float* s;                  // (n, columns)
+  float* st;                       // (columns, pad)
+  int columns;
 };
-struct PackLaunch { PackJob job[2]; const float* w; };
+struct PackLaunch { PackJob job[2]; const float* w; int64_t n, pad; };
 __global__ void __launch_bounds__(256) uvw_pack_kernel(const __grid_constant__ PackLaunch p) {
-  const PackJob& job = p.job[blockIdx.y];
+  const PackJob& job = p.job[blockIdx.y / 2];
+  if (blockIdx.y & 1) {
+    __shared__ float block[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int64_t across = ceil_div(job.columns, 32), blocks = across * (p.pad / 32);
+    for (int64_t t = blockIdx.x; t < blocks; t += gridDim.x) {
+      const int64_t n0 = t / across * 32;
+      const int c0 = (int)(t % across) * 32;
+      __syncthreads();
+      for (int r = y; r < 32; r += 8) block[r][x] = n0 + r < p.n && c0 + x < job.columns ? __ldg(job.s + (n0 + r) * job.columns + c0 + x) : 0.f;
+      __syncthreads();
+      for (int r = y; r < 32; r += 8)
+        if (c0 + r < job.columns) job.st[(int64_t)(c0 + r) * p.pad + n0 + x] = block[x][r];
+    }
+    return;
+  }
   const int quads = job.ck / 4, iq = COLS / job.cj, groups = job.ci / iq;
   const int64_t total = (int64_t)job.num_paths * groups * quads * COLS;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -484,7 +529,8 @@ extern "C" int64_t eqt_uvw_scratch_floats(const eqt_uvw_role* roles, int32_t job
   int slices[2];
   if (ceil_div(n, 128) * MAX_SEGMENTS > 0x7fffffffll || cut(roles, jobs, ceil_div(n, 128), nullptr, slices) < 0) return -1;
   int64_t need = 0;
-  for (int j = 0; j < jobs; ++j) need += packed_floats(roles[j]) + (slices[j] > 1 ? slices[j] * n * roles[j].d_out * roles[j].cj : 0);
+  for (int j = 0; j < jobs; ++j)
+    need += packed_floats(roles[j]) + ceil_div(n, 128) * 128 * roles[j].ds * roles[j].ci + (slices[j] > 1 ? slices[j] * n * roles[j].d_out * roles[j].cj : 0);
   return need;
 }
 
@@ -508,7 +554,7 @@ extern "C" int eqt_uvw_contract(const eqt_uvw_role* roles, int32_t jobs, const f
   PackLaunch P{};
   SumLaunch S{};
   int slices[2];
-  L.n = n; L.tiles = (int)ceil_div(n, 128); L.status = status;
+  L.n = P.n = n; L.tiles = (int)ceil_div(n, 128); L.pad = P.pad = (int64_t)L.tiles * 128; L.status = status;
   L.segments = cut(roles, jobs, L.tiles, &L, slices);
   P.w = w;
   size_t smem = 0;
@@ -516,13 +562,15 @@ extern "C" int eqt_uvw_contract(const eqt_uvw_role* roles, int32_t jobs, const f
   for (int j = 0; j < jobs; ++j) {
     const eqt_uvw_role& r = roles[j];
     ContractJob& c = L.job[j];
-    c.s = s[j]; c.f = f[j]; c.sum = out[j]; c.paths = r.paths;
+    c.f = f[j]; c.sum = out[j]; c.paths = r.paths;
     c.ds = r.ds; c.df = r.df; c.d_out = r.d_out; c.ci = r.ci; c.ck = r.ck; c.slices = slices[j];
     c.packed = reinterpret_cast<unsigned char*>(scratch + at);
     P.job[j] = PackJob{r.paths, reinterpret_cast<unsigned char*>(scratch + at), r.stride_i, r.stride_k, r.stride_j, r.stride_p,
-                       r.ci, r.ck, r.cj, r.num_paths};
+                       r.ci, r.ck, r.cj, r.num_paths, s[j], nullptr, r.ds * r.ci};
     at += packed_floats(r);
-    widest = std::max(widest, (int64_t)r.num_paths * r.ci * r.cj * (r.ck / 4));
+    c.s = P.job[j].st = scratch + at;
+    at += L.pad * r.ds * r.ci;
+    widest = std::max({widest, (int64_t)r.num_paths * r.ci * r.cj * (r.ck / 4), L.pad * r.ds * r.ci / 4});
     int q = 0;
     for (int g = 0; g < r.num_groups; ++g) {
       c.first[g] = q; c.count[g] = r.groups[g].count; c.offset[g] = r.groups[g].offset; c.degree[g] = r.groups[g].l;
@@ -545,7 +593,7 @@ extern "C" int eqt_uvw_contract(const eqt_uvw_role* roles, int32_t jobs, const f
     }
     S.from[j] = c.out;
   }
-  uvw_pack_kernel<<<dim3(flat_grid(widest, 256), jobs), 256, 0, st>>>(P);
+  uvw_pack_kernel<<<dim3(flat_grid(widest, 256), 2 * jobs), 256, 0, st>>>(P);
   if (int rc = check_launch("uvw_pack_kernel")) return rc;
   if (int rc = roles[0].cj == 32 ? launch_contract<32>(L, smem + 1024, st) : launch_contract<16>(L, smem + 1024, st)) return rc;
   if (rows) {
@@ -645,23 +693,23 @@ template <int J> struct RowMaker {
         for (int u = set; u < 4; u += 2) {
           if (!bar_wait(&bars.a_free[u], a_phase ^ 1, ab)) return false;
           tc_fence_after();
-          float q[2][NF][4];
+          Two q[2][NF][2];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            float s[NS][4], g[NO][4];
+            Two s[NS][2], g[NO][2];
             const float4* sp = reinterpret_cast<const float4*>(stage + s_off);
             const float4* gp = reinterpret_cast<const float4*>(stage + g_off);
 #pragma unroll
             for (int b = 0; b < NS; ++b) {
               const float4 v = sp[(b * IQ + i) * 8 + chunk_of(b * IQ + i, u * 2 + h)];
-              s[b][0] = v.x; s[b][1] = v.y; s[b][2] = v.z; s[b][3] = v.w;
+              s[b][0] = two(v.x, v.y); s[b][1] = two(v.z, v.w);
             }
 #pragma unroll
             for (int a = 0; a < NO; ++a) {
               const float4 v = gp[(a * J + j) * 8 + chunk_of(a * J + j, u * 2 + h)];
-              g[a][0] = v.x; g[a][1] = v.y; g[a][2] = v.z; g[a][3] = v.w;
+              g[a][0] = two(v.x, v.y); g[a][1] = two(v.z, v.w);
             }
-            CgTriple<LO, LS, LF>::template pair<4>(q[h], s, g);
+            CgTriple<LO, LS, LF>::template pair<2>(q[h], s, g);
           }
 #pragma unroll
           for (int c = 0; c < NF; ++c) {
@@ -669,10 +717,12 @@ template <int J> struct RowMaker {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float hi = rn_tf32(q[h][c][e]);
-                v[h * 4 + e] = hi;
-                v[8 + h * 4 + e] = rn_tf32(q[h][c][e] - hi);
+              for (int e = 0; e < 4; e += 2) {       // the MMA drops what of the small part is past TF32
+                float x, y;
+                apart(q[h][c][e / 2], x, y);
+                v[h * 4 + e] = rn_tf32(x);
+                v[h * 4 + e + 1] = rn_tf32(y);
+                apart(fma2(two(v[h * 4 + e], v[h * 4 + e + 1]), two(-1.f, -1.f), q[h][c][e / 2]), v[8 + h * 4 + e], v[8 + h * 4 + e + 1]);
               }
             tmem_put16(tmem + (uint32_t)(u * 80 + c * 16), v);
           }
