@@ -2,7 +2,8 @@
 
 A layer's table is a list of paths (k, i, j) between irreps; what a path does depends on its three degrees only.  For
 degrees up to ``MAX_L`` the block's multiply-adds are emitted with the CG values as immediates, on register blocks of V
-channels: products of several y components with the same (M, m1) are summed before they meet the channels.
+channels: products of several y components with the same (M, m1) are summed before they meet the channels.  P: two channels at a
+time in packed instructions.
 
 ``generated/triple_specs.inc`` holds the blocks of a product of two channelled operands in the forms that its kernels take:
 one component of the contracted operand at a time, and all of them from a pair of channels.
@@ -44,20 +45,20 @@ def _emit(lo: int, l1: int, l2: int) -> str:
     no, n1, n2 = 2 * lo + 1, 2 * l1 + 1, 2 * l2 + 1
     out = [f"template <> struct CgPath<{lo}, {l1}, {l2}> {{",
            f"  // o[M] += sum_m1 (sum_m2 cg y[m2]) x[m1]",
-           f"  template <int V> __device__ __forceinline__ static void forward(float (&o)[{no}][V], const float (&x)[{n1}][V], const float (&y)[{n2}]) {{"]
+           f"  template <int V, bool P = false> __device__ __forceinline__ static void forward(float (&o)[{no}][V], const float (&x)[{n1}][V], const float (&y)[{n2}]) {{"]
     for (M, m1), ts in pairs.items():
-        out.append(f"    axpy<V>(o[{M}], {coef(ts)}, x[{m1}]);")
+        out.append(f"    axpy<V, P>(o[{M}], {coef(ts)}, x[{m1}]);")
     out += ["  }",
             f"  // r[m1] += sum_M (sum_m2 cg y[m2]) g[M]",
-            f"  template <int V> __device__ __forceinline__ static void adjoint(float (&r)[{n1}][V], const float (&g)[{no}][V], const float (&y)[{n2}]) {{"]
+            f"  template <int V, bool P = false> __device__ __forceinline__ static void adjoint(float (&r)[{n1}][V], const float (&g)[{no}][V], const float (&y)[{n2}]) {{"]
     for (M, m1), ts in pairs.items():
-        out.append(f"    axpy<V>(r[{m1}], {coef(ts)}, g[{M}]);")
+        out.append(f"    axpy<V, P>(r[{m1}], {coef(ts)}, g[{M}]);")
     out += ["  }",
             f"  // gy[m2] += sum_(M, m1) cg <g[M], x[m1]> over the V channels",
-            f"  template <int V> __device__ __forceinline__ static void inner(float (&gy)[{n2}], const float (&g)[{no}][V], const float (&x)[{n1}][V]) {{",
+            f"  template <int V, bool P = false> __device__ __forceinline__ static void inner(float (&gy)[{n2}], const float (&g)[{no}][V], const float (&x)[{n1}][V]) {{",
             "    float d;"]
     for (M, m1), ts in pairs.items():
-        out.append(f"    d = dot<V>(g[{M}], x[{m1}]);")
+        out.append(f"    d = dot<V, P>(g[{M}], x[{m1}]);")
         out += [f"    gy[{m2}] = fmaf({_lit(v)}, d, gy[{m2}]);" for m2, v in ts]
     out += ["  }", "};"]
     return "\n".join(out)

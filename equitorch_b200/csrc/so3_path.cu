@@ -27,15 +27,44 @@ namespace {
 
 constexpr int V = 4;                              // channels per thread
 
-template <int N> __device__ __forceinline__ void axpy(float (&o)[N], float s, const float (&x)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = fmaf(s, x[i], o[i]);
+// P: two values at a time in packed instructions (fma.rn.f32x2).  Fewer instructions, but the scalar operand needs a pair of its own:
+// 'uv' backward 279 -> 214 us (20,011 samples, l_max 3, 64 channels), 'uu' forward 55 -> 52 us (20,480 samples, bfloat16, weights per
+// sample); 'uu' backward, which is at its register limit without, 107 -> 114 us, so that one does without.
+__device__ __forceinline__ unsigned long long two(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
 }
-template <int N> __device__ __forceinline__ float dot(const float (&a)[N], const float (&b)[N]) {
-  float d = a[0] * b[0];
+__device__ __forceinline__ void apart(unsigned long long t, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(t)); }
+template <int N, bool P> __device__ __forceinline__ void axpy(float (&o)[N], float s, const float (&x)[N]) {
+  if constexpr (P) {
+    const unsigned long long k = two(s, s);
 #pragma unroll
-  for (int i = 1; i < N; ++i) d = fmaf(a[i], b[i], d);
-  return d;
+    for (int i = 0; i < N; i += 2) {
+      unsigned long long r;
+      asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(k), "l"(two(x[i], x[i + 1])), "l"(two(o[i], o[i + 1])));
+      apart(r, o[i], o[i + 1]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) o[i] = fmaf(s, x[i], o[i]);
+  }
+}
+template <int N, bool P> __device__ __forceinline__ float dot(const float (&a)[N], const float (&b)[N]) {
+  if constexpr (P) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(two(a[0], a[1])), "l"(two(b[0], b[1])));
+#pragma unroll
+    for (int i = 2; i < N; i += 2) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r) : "l"(two(a[i], a[i + 1])), "l"(two(b[i], b[i + 1])));
+    float x, y;
+    apart(r, x, y);
+    return x + y;
+  } else {
+    float d = a[0] * b[0];
+#pragma unroll
+    for (int i = 1; i < N; ++i) d = fmaf(a[i], b[i], d);
+    return d;
+  }
 }
 
 #include "generated/path_specs.inc"
@@ -158,7 +187,7 @@ struct PathSmem {
     paths = take(sizeof(eqt_path) * num_paths);
     rows = take(mode == UV_BACKWARD ? sizeof(int32_t) * num_rows : 0);
     ys = take(sizeof(float) * slots * d2);
-    xcol = take(row * d1);
+    xcol = take(mode == UV_BACKWARD ? 0 : row * d1);
     gcol = take(mode == UU_BACKWARD ? row * dout : 0);
     ring = take(mode == UV_EXPAND ? 0 : row * (mode == UV_BACKWARD ? ROWS_AHEAD : AHEAD));
     gycol = take(backward ? sizeof(float) * threads * d2 : 0);
@@ -188,7 +217,7 @@ __device__ __forceinline__ void forward_path(float (&o)[2 * LO + 1][V], const T*
     for (int m = 0; m < 2 * LO + 1; ++m)
 #pragma unroll
       for (int i = 0; i < V; ++i) t[m][i] = 0.f;
-    CgPath<LO, L1, L2>::template forward<V>(t, x, y);
+    CgPath<LO, L1, L2>::template forward<V, true>(t, x, y);
 #pragma unroll
     for (int m = 0; m < 2 * LO + 1; ++m)
 #pragma unroll
@@ -509,7 +538,11 @@ __global__ void __launch_bounds__(128, 4) so3_uv_expand_kernel(PathArgs a) {
 
 // gx[n, M1, c] = sum_t s_t y[n, M2_t] G[n, row_t, c]  and  gy[n, M2] = sum_t s_t <x[n, M1_t], G[n, row_t]>  from one
 // pass over G: a row is used by one path, so it goes from memory through the ring into registers once, and neither a
-// second intermediate nor a second GEMM is needed for gx.
+// second intermediate nor a second GEMM is needed for gx.  The straight-line blocks of a layer are more code than the
+// instruction caches hold (4 k instructions a sample at l_max 3), and walking through them takes a CTA some 65 k cycles whatever its
+// size, most of it waiting for instructions: what counts is the samples in flight.  x is therefore loaded a block at a time instead
+// of kept in columns of shared memory, which leaves room for three CTAs: 294 -> 279 us (20,011
+// samples, l_max 3, 64 channels); twelve warps in one CTA that keep together: 295 us.  Packed multiply-adds make the walk shorter: 214 us.
 template <int LO, int L1, int L2>
 __device__ __forceinline__ void uv_backward_path(float (&gx)[2 * L1 + 1][V], const float (&x)[2 * L1 + 1][V], RowStream& rs, const float* yr,
                                                  float* gyc, int threads, float scale) {
@@ -518,27 +551,28 @@ __device__ __forceinline__ void uv_backward_path(float (&gx)[2 * L1 + 1][V], con
     rs.next<2 * LO + 1>(g);
 #pragma unroll
     for (int i = 0; i < 2 * L2 + 1; ++i) { y[i] = yr[i]; gy[i] = 0.f; }
-    CgPath<LO, L1, L2>::template inner<V>(gy, g, x);
+    CgPath<LO, L1, L2>::template inner<V, true>(gy, g, x);
 #pragma unroll
     for (int i = 0; i < 2 * L2 + 1; ++i) gyc[i * threads] = fmaf(gy[i], scale, gyc[i * threads]);
 #pragma unroll
     for (int m = 0; m < 2 * LO + 1; ++m)
 #pragma unroll
       for (int i = 0; i < V; ++i) g[m][i] *= scale;
-    CgPath<LO, L1, L2>::template adjoint<V>(gx, g, y);
+    CgPath<LO, L1, L2>::template adjoint<V, true>(gx, g, y);
   }
 }
 
 template <int L1>
 __device__ __forceinline__ void uv_backward_block(const PathArgs& a, const eqt_path_block& b, const eqt_path* paths, RowStream& rs,
-                                                  const float* xc, int row, int threads, const float* yr, float* gyc, float* gxout) {
+                                                  const float* x_from, int threads, const float* yr, float* gyc, float* gxout) {
   float x[2 * L1 + 1][V], gx[2 * L1 + 1][V];
 #pragma unroll
-  for (int m = 0; m < 2 * L1 + 1; ++m) {
-    lds_v(xc + (b.offset + m) * row, x[m]);
+  for (int m = 0; m < 2 * L1 + 1; ++m)
 #pragma unroll
-    for (int i = 0; i < V; ++i) gx[m][i] = 0.f;
-  }
+    for (int i = 0; i < V; ++i) x[m][i] = gx[m][i] = 0.f;
+  if (x_from)
+#pragma unroll
+    for (int m = 0; m < 2 * L1 + 1; ++m) load_v(x_from + (int64_t)(b.offset + m) * a.c, x[m]);
   for (int q = b.first; q < b.first + b.count; ++q) {
     const eqt_path pd = paths[q];
     switch (pd.code) {
@@ -562,7 +596,6 @@ __global__ void __launch_bounds__(128, 3) so3_uv_backward_kernel(PathArgs a) {
   eqt_path* paths = reinterpret_cast<eqt_path*>(smem + L.paths);
   int32_t* rows = reinterpret_cast<int32_t*>(smem + L.rows);
   float* ys = reinterpret_cast<float*>(smem + L.ys);
-  float* xc = reinterpret_cast<float*>(smem + L.xcol) + tid * V;
   float* gy_all = reinterpret_cast<float*>(smem + L.gycol);
   RowStream rs;
   rs.ring = reinterpret_cast<float*>(smem + L.ring) + tid * V;
@@ -578,9 +611,6 @@ __global__ void __launch_bounds__(128, 3) so3_uv_backward_kernel(PathArgs a) {
     const int64_t n = n0 + slot;
     __syncthreads();                                   // tables loaded / harmonics and partial gy of the previous samples have been read
     if (slot < here) {
-      if (x)
-        for (int i = 0; i < a.d1; ++i) copy_v(xc + i * row, x + (n * a.d1 + i) * a.c + ch);
-      copy_commit();
       rs.g = static_cast<const float*>(a.g) + n * a.num_rows * a.c + ch;
       rs.begin();
       for (int i = 0; i < a.d2; ++i) gy_all[i * threads + tid] = 0.f;
@@ -590,15 +620,15 @@ __global__ void __launch_bounds__(128, 3) so3_uv_backward_kernel(PathArgs a) {
     __syncthreads();
     if (slot < here) {
       float* gx = a.gx ? static_cast<float*>(a.gx) + n * a.d1 * a.c + ch : nullptr;
+      const float* xn = x ? x + n * a.d1 * a.c + ch : nullptr;
       const float* yr = ys + slot * a.d2;
-      copy_wait<ROWS_AHEAD>();                         // x
       for (int b = 0; b < a.num_blocks; ++b) {
         const eqt_path_block bd = blocks[b];
         switch (bd.l) {
-          case 0: uv_backward_block<0>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
-          case 1: uv_backward_block<1>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
-          case 2: uv_backward_block<2>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
-          case 3: uv_backward_block<3>(a, bd, paths, rs, xc, row, threads, yr, gy_all + tid, gx); break;
+          case 0: uv_backward_block<0>(a, bd, paths, rs, xn, threads, yr, gy_all + tid, gx); break;
+          case 1: uv_backward_block<1>(a, bd, paths, rs, xn, threads, yr, gy_all + tid, gx); break;
+          case 2: uv_backward_block<2>(a, bd, paths, rs, xn, threads, yr, gy_all + tid, gx); break;
+          case 3: uv_backward_block<3>(a, bd, paths, rs, xn, threads, yr, gy_all + tid, gx); break;
         }
       }
     }
