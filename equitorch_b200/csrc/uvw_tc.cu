@@ -611,12 +611,15 @@ extern "C" int eqt_uvw_contract(const eqt_uvw_role* roles, int32_t jobs, const f
 // A GEMM whose reduction runs over samples and components of f, with M = 128 pairs (i, j) of one path, N = channels of f.  A
 // thread is one pair: it computes its row of Q from the two operands in shared memory, eight samples at a time, splits it and
 // stores it to tensor memory, where the MMA reads it; f arrives as [big | small] tiles of 32 samples, so that one MMA of 2 K
-// columns makes big * big and big * small, and one of K columns small * big.  The accumulator is folded into float32 registers
-// every 12 to 20 k-steps (the adder of the tensor core truncates).  The work - (path, channel group) x chunks of 32 samples -
+// columns makes big * big and big * small, and one of K columns small * big.  An MMA waits for the one
+// before it into the same accumulator, so even and odd k-steps and the two kinds of MMA have accumulators of their own, folded into
+// float32 registers every 12 to 20 k-steps each (the adder of the tensor core truncates); and every instruction of the issuing
+// thread counts, so the MMAs of a stage are straight-line code by the degree of f (one accumulator and a loop: 211 us at 2000 samples,
+// l_max 2, 32 channels; four: 201 us; without the loop 167 us; a third stage changes nothing).  The work - (path, channel group) x chunks of 32 samples -
 // is one line that is cut into equal costs, one range per SM; a range that ends inside a (path, channel group) leaves a partial sum,
 // and a second launch adds the partial sums of each in order.
 //   warps 0-7   rows of Q (two sets of four, alternating groups of eight samples)
-//   warps 8-11  accumulator -> registers -> partial sums; warp 8 also TMEM allocation and MMA issue, one fold ahead
+//   warps 8-11  accumulators -> registers -> partial sums; warp 8 also TMEM allocation and MMA issue
 //   warps 12-15 operands -> shared memory
 // Bound: the multiply-adds of Q and its split.
 namespace eqt {
@@ -647,7 +650,7 @@ struct WLaunch {
   WPiece piece[MAX_PIECES];
 };
 
-struct WBars { uint64_t full[W_STAGES], empty[W_STAGES], a_ready[4], a_free[4], d_full[2], d_free[2]; };
+struct WBars { uint64_t full[W_STAGES], empty[W_STAGES], a_ready[4], a_free[4], d_full, d_free; };
 
 __device__ __forceinline__ void tmem_put16(uint32_t taddr, const float (&v)[16]) {
   asm volatile(
@@ -659,7 +662,8 @@ __device__ __forceinline__ void tmem_put16(uint32_t taddr, const float (&v)[16])
       : "memory");
 }
 
-__host__ __device__ constexpr int fold_every(int lf) { return lf == 2 ? 1 : lf == 1 ? 2 : 4; }      // stages between folds
+__host__ __device__ constexpr int fold_every(int lf) { return lf == 2 ? 2 : lf == 1 ? 4 : 8; }      // stages between folds
+constexpr int A_COL0 = 192;                // TMEM: [even | odd k-steps: big, corrections][small * big, even | odd], then the A slots
 
 struct WSmem {
   int s, g, b, stage;                      // byte offsets inside a stage; the tiles of f first (1024-byte aligned)
@@ -753,7 +757,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) uvw_wgrad_kernel(const __grid_co
     abort_flag = 0;
     for (int i = 0; i < W_STAGES; ++i) { bar_init(&bars.full[i], W_LOADERS); bar_init(&bars.empty[i], 9); }      // makers + the MMAs' commit
     for (int i = 0; i < 4; ++i) { bar_init(&bars.a_ready[i], 4); bar_init(&bars.a_free[i], 1); }
-    for (int i = 0; i < 2; ++i) { bar_init(&bars.d_full[i], 1); bar_init(&bars.d_free[i], 4); }
+    bar_init(&bars.d_full, 1);
+    bar_init(&bars.d_free, 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 8) {
@@ -763,7 +768,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) uvw_wgrad_kernel(const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_slot;         // [two accumulators of 2 K columns][four slots of 80 columns from column 128]
+  const uint32_t tmem = tmem_slot;
   volatile int* ab = &abort_flag;
   const int p0 = p.cta[blockIdx.x], p1 = p.cta[blockIdx.x + 1];
 
@@ -771,7 +776,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) uvw_wgrad_kernel(const __grid_co
     // ---------------- rows of Q ----------------
     const int quarter = warp & 3, row = quarter * 32 + lane;
     RowMaker<J> w{bars, ab, base, L.stage, L.s, L.g, row / J, row % J,
-                  tmem + ((uint32_t)(quarter * 32) << 16) + 128, warp >> 2, lane};
+                  tmem + ((uint32_t)(quarter * 32) << 16) + A_COL0, warp >> 2, lane};
     for (int x = p0; x < p1; ++x) {
       const WPiece pc = p.piece[x];
       const eqt_uvw_path* path = p.paths + pc.unit / p.groups;
@@ -788,84 +793,79 @@ __global__ void __launch_bounds__(W_THREADS, 1) uvw_wgrad_kernel(const __grid_co
     }
   } else if (warp < 12) {
     // ---------------- MMA issue and accumulators -> partial sums ----------------
-    // A fold covers up to fold_every() stages of one piece.  Warp 8 issues the MMAs of a fold before it reads the accumulator of
-    // the one before, so that they run meanwhile.
+    // A fold covers up to fold_every() stages of one piece.
     const int quarter = warp & 3;
     const uint32_t wide = umma_idesc_tf32(2 * k), narrow = umma_idesc_tf32(k);
-    Ring st, d, e;                           // stages; accumulator being filled; accumulator being read
-    uint32_t a_phase = 0;
-    auto issue = [&](int stages, int nf) {     // one thread
-      if (!bar_wait(&bars.d_free[d.s], d.ph ^ 1, ab)) return false;
+    Ring st;
+    uint32_t a_phase = 0, d_phase = 0;
+    // MMAs of a stage, issued by one thread; nf is odd, so that a stage begins with an even k-step again
+    auto stage = [&](auto count, bool first) __attribute__((always_inline)) {
+      constexpr int NF = decltype(count)::value;
+      const uint32_t tiles = umma_lo(s32(base + st.s * L.stage));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (!bar_wait(&bars.a_ready[u], a_phase, ab)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < NF; ++c) {
+          const int step = u * NF + c, odd = step & 1;
+          const uint32_t a = tmem + A_COL0 + u * 80 + c * 16, b = tiles + c * 2 * k * 128 / 16 + u * 2;
+          const uint32_t more = step > 1 ? 1 : !first;
+          umma_tf32_ta_lo(tmem + odd * (2 * k), a, b, wide, more);                 // big * [big | small]
+          umma_tf32_ta_lo(tmem + 4 * k + odd * k, a + 8, b, narrow, more);         // small * big
+        }
+        umma_commit(&bars.a_free[u]);
+      }
+      umma_commit(&bars.empty[st.s]);
+      return true;
+    };
+    auto issue = [&](int stages, int nf) {
+      if (!bar_wait(&bars.d_free, d_phase ^ 1, ab)) return false;
       tc_fence_after();
-      const uint32_t acc = tmem + (uint32_t)(d.s * 64);
       for (int t = 0; t < stages; ++t, st.next(W_STAGES), a_phase ^= 1) {
         if (!bar_wait(&bars.full[st.s], st.ph, ab)) return false;
-        const uint32_t tiles = umma_lo(s32(base + st.s * L.stage));
-        for (int u = 0; u < 4; ++u) {
-          if (!bar_wait(&bars.a_ready[u], a_phase, ab)) return false;
-          tc_fence_after();
-          for (int c = 0; c < nf; ++c) {
-            const uint32_t a = tmem + 128 + (uint32_t)(u * 80 + c * 16);
-            const uint32_t b = tiles + (uint32_t)(c * 2 * k * 128 / 16 + u * 2);
-            umma_tf32_ta_lo(acc, a, b, wide, t != 0 || u != 0 || c != 0);        // big * [big | small]
-            umma_tf32_ta_lo(acc + k, a + 8, b, narrow, 1);                       // small * big, onto the corrections
-          }
-          umma_commit(&bars.a_free[u]);
-        }
-        umma_commit(&bars.empty[st.s]);
+        const bool done = nf == 5   ? stage(std::integral_constant<int, 5>(), t == 0)
+                          : nf == 3 ? stage(std::integral_constant<int, 3>(), t == 0)
+                                    : stage(std::integral_constant<int, 1>(), t == 0);
+        if (!done) return false;
       }
-      umma_commit(&bars.d_full[d.s]);
+      umma_commit(&bars.d_full);
       return true;
     };
-    float sum[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) sum[i] = 0.f;
-    int open = -1;                             // piece of the fold that was issued last and is not read yet, its last fold or not
-    bool closes = false, ok = true;
-    auto fold = [&]() {
-      if (!bar_wait(&bars.d_full[e.s], e.ph, ab)) return false;
-      tc_fence_after();
-      const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(e.s * 64);
-      float big[32];
-      tmem_ld32(at, big);                    // K = 16: [big | corrections] are the 32 columns
-      if (k > 16) {
-        float small[32];
-        tmem_ld32(at + 32, small);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) sum[i] += big[i] + small[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) sum[i] += big[i] + big[i + 16];
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) bar_arrive(&bars.d_free[e.s]);
-      e.next(2);
-      if (closes) {
-        float* out = p.partial + ((int64_t)open * 128 + quarter * 32 + lane) * k;
-#pragma unroll
-        for (int i = 0; i < k; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) sum[i] = 0.f;
-      }
-      return true;
-    };
+    bool ok = true;
     for (int x = p0; x < p1 && ok; ++x) {
       const WPiece pc = p.piece[x];
       const int lf = __ldg(&p.paths[pc.unit / p.groups].l_f), every = fold_every(lf);
-      for (int t = pc.chunk0; t < pc.chunk1 && ok; t += every) {
+      float sum[k];
+#pragma unroll
+      for (int i = 0; i < k; ++i) sum[i] = 0.f;
+      for (int t = pc.chunk0; t < pc.chunk1; t += every) {
         if (warp == 8) {
           int issued = lane == 0 ? (int)issue(min(every, pc.chunk1 - t), 2 * lf + 1) : 1;
           issued = __shfl_sync(0xffffffffu, issued, 0);
           if (!issued) { ok = false; break; }
-          d.next(2);
         }
-        if (open >= 0) ok = fold();
-        open = x;
-        closes = t + every >= pc.chunk1;
+        if (!bar_wait(&bars.d_full, d_phase, ab)) { ok = false; break; }
+        d_phase ^= 1;
+        tc_fence_after();
+        // every fold has at least four k-steps, so that all accumulators are written
+        const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+        for (int o = 0; o < 6 * k; o += 32) {
+          float v[32];
+          tmem_ld32(at + o, v);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sum[(o + i) % k] += v[i];
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(&bars.d_free);
       }
+      if (!ok) break;
+      float* out = p.partial + ((int64_t)x * 128 + quarter * 32 + lane) * k;
+#pragma unroll
+      for (int i = 0; i < k; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
     }
-    if (ok && open >= 0) fold();
   } else {
     // ---------------- operands -> shared memory ----------------
     // A lane has one float4 of every component for FP (GP) samples of f (g): neighbouring lanes a run of channels of few samples.
