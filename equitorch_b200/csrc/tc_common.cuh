@@ -103,6 +103,17 @@ __device__ __forceinline__ void umma_tf32_ta_lo(uint32_t d_tmem, uint32_t a_tmem
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], b, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI) : "memory");
 }
+// operands MN-major with 32-byte atoms (umma_desc_mn32): the low words carry the leading byte offset
+constexpr uint32_t UMMA_DESC_MN32_HI = (512 >> 4) | (1u << 14) | (1u << 29);
+__device__ __forceinline__ uint32_t umma_lo_mn32(uint32_t smem_byte_addr, uint32_t lbo_bytes) {
+  return ((smem_byte_addr & 0x3FFFF) >> 4) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
+}
+__device__ __forceinline__ void umma_tf32_mn32_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_MN32_HI) : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
 }
