@@ -765,13 +765,9 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
-  if (sh.abort_flag) {
-    if (tid == 0) atomicExch(a.status, 1);
-    // copies that may still be in flight get a bounded chance to land before shared memory is released
-    if (tid == 0)
-      for (int i = 0; i < NS; ++i)
-        for (int ph = 0; ph < 2; ++ph)
-          for (int k = 0; k < 1024 && !bar_try(&sh.full[i], ph); ++k) __nanosleep(256);
+  if (sh.abort_flag && tid == 0) {
+    atomicExch(a.status, 1);
+    let_copies_land(sh.full, NS);
   }
 }
 

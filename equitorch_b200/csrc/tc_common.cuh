@@ -46,6 +46,14 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, volatile 
   return false;
 }
 
+// After an expired wait: copies that may still be in flight to the buffers behind `bars` get a bounded chance to land before the
+// CTA's shared memory is released (one of the two parities is the phase before, which is complete).
+__device__ __forceinline__ void let_copies_land(uint64_t* bars, int count) {
+  for (int i = 0; i < count; ++i)
+    for (int ph = 0; ph < 2; ++ph)
+      for (int t = 0; t < 1024 && !bar_try(&bars[i], ph); ++t) __nanosleep(256);
+}
+
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"

@@ -388,10 +388,7 @@ __global__ void __launch_bounds__(CONTRACT_THREADS, 1) uvw_contract_kernel(const
   }
   if (abort_flag && tid == 0) {
     atomicExch(p.status, 2);
-    // copies that may still be in flight get a bounded chance to land before shared memory is released
-    for (int i = 0; i < B_STAGES; ++i)
-      for (int ph = 0; ph < 2; ++ph)
-        for (int t = 0; t < 1024 && !bar_try(&bars.b_full[i], ph); ++t) __nanosleep(256);
+    let_copies_land(bars.b_full, B_STAGES);
   }
 }
 
