@@ -415,7 +415,7 @@ extern "C" int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64
     R.n = n; R.tiles = ceil_div(n, TILE_M); R.total_items = L.total_items;
     R.num_out = num_out; R.n_cols = n_cols; R.units = n_cols > 64 ? 2 : 1; R.unit_cols = n_cols / R.units;
     R.slots = std::min(4, (512 - 6 * R.unit_cols) / 64);
-    R.b_bytes = b_bytes;
+    R.b_bytes = b_bytes; R.longest = longest;
     R.raw_stages = (int)std::min<size_t>(8, (220 * 1024 - 1024 - EPI_PATCH_BYTES - b_bytes) / (TILE_M * KB * 4));
     auto* resident = longest == 1 ? vecmat_resident_kernel<true> : vecmat_resident_kernel<false>;
     if (int rc = allow_shared(resident, 220 * 1024)) return rc;

@@ -28,12 +28,16 @@ def status_flag(device: torch.device) -> Tensor:
 
 
 def check_status(device=None) -> None:
-    """Synchronise and raise if any fused kernel reported a timed-out wait since the last check."""
+    """Synchronise and raise if any fused kernel reported a timed-out wait, or tables that contradict its arguments, since the
+    last check."""
     for dev, flag in _status.items():
         if device is None or dev == torch.device(device):
-            if int(flag.item()) != 0:
+            code = int(flag.item())
+            if code != 0:
                 flag.zero_()
-                raise _lib.EqtError(f"a fused tensor-product kernel on {dev} gave up waiting for an asynchronous copy")
+                raise _lib.EqtError(f"a fused tensor-product kernel on {dev} " + (
+                    "met a group of k-blocks longer than its caller had announced" if code == 4
+                    else "gave up waiting for an asynchronous copy"))
 
 
 class TpTable:

@@ -275,7 +275,9 @@ int eqt_vecmat_tc(const float* x, const float* w, const int64_t* index2, const f
  * group > 1: cout % 32 == 0, group * cout <= 128).  A slot is (group, x row): kb_begin (num_groups + 1) and a_col count the
  * k-blocks of slots, group_rows (num_groups, group) names the output rows (-1: none; every row once), slot_entry (slots, group)
  * the entry t of a slot's x row in each output row (-1: none).  w_big / w_small hold slots * cin * group * cout floats.
- * longest: k-blocks of the longest group where the caller knows them (1 adds a correction product), else 0.
+ * longest: k-blocks of the longest group where the caller knows them, else 0.  1 adds a correction product, and buffers of a kernel
+ * for short groups are sized by it: a value other than 0 has to bound every group; where it does not, `status` is set to 4 and the
+ * results are incomplete.
  */
 int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64_t* index2, const float* scale, float* w_big,
                           float* w_small, float* out, int64_t n, int32_t rows1, int32_t cin, int32_t cout, int32_t num_out,

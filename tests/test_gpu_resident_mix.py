@@ -4,8 +4,10 @@ sample tile, ranges that begin and end inside an output row, a row that no path 
 import pytest
 import torch
 
+from equitorch_b200 import _lib
 from equitorch_b200 import nn as enn
-from equitorch_b200.ops.fused_tp_op import check_status
+from equitorch_b200.ops import indexed_tc_op as tc
+from equitorch_b200.ops.fused_tp_op import check_status, status_flag
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -39,3 +41,28 @@ def test_against_float64(ir_in, ir_out, n, cin, cout):
     # three products of TF32 pairs, at most eight truncating steps per accumulator: a few units of 2^-24
     for a, b in zip(got, [want, *torch.autograd.grad(want, [xd, wd], cot.double())]):
         assert _rel(a.detach(), b.detach()) < 2e-6
+
+
+def test_groups_longer_than_announced_are_reported():
+    """The buffers are sized by the caller's ``longest``: a group past it must end in an error, not past the buffers."""
+    n, cin, cout, dim = 20000, 128, 64, 4
+    x, w = torch.randn(n, dim, cin, device=DEV), torch.randn(dim, cin, cout, device=DEV)
+    index = torch.arange(dim, device=DEV)
+    plan = tc.VecmatPlan(index, None, dim, dim, cin, cout, torch.device(DEV))
+    assert plan.group == 1 and plan.longest == 4
+    want = tc.vecmat_tc(x, w, None, index, index, None, dim)
+    plan.longest = 1
+    packed, out = torch.empty(2, dim * cin * cout, device=DEV), torch.empty(n, dim, cout, device=DEV)
+
+    def call():
+        _lib.check(_lib.lib().eqt_vecmat_tc_grouped(
+            x.data_ptr(), w.data_ptr(), index.data_ptr(), None, packed[0].data_ptr(), packed[1].data_ptr(), out.data_ptr(), n, dim, cin,
+            cout, dim, plan.slots, plan.group, plan.num_groups, plan.group_rows.data_ptr(), plan.slot_entry.data_ptr(),
+            plan.kb_begin.data_ptr(), plan.a_col.data_ptr(), plan.longest, status_flag(x.device).data_ptr(), _lib.stream_ptr(x.device)), "call")
+    call()
+    with pytest.raises(_lib.EqtError, match="longer than"):
+        check_status(x.device)
+    plan.longest = 4
+    call()
+    check_status(x.device)
+    assert torch.equal(out, want)
