@@ -405,10 +405,16 @@ extern "C" int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64
     if (int rc = make_map(&L.map_bs, w_small, 2, dims, strides, box)) return rc;
   }
   // Resident weights: one-row groups of short sums over rows of x that are read about once (an output row's items run one after
-  // the other, so a row that several output rows read would come from memory each time), 128 columns with two A slots.
+  // the other, so a row that several output rows read would come from memory each time), 128 columns with two A slots.  Only
+  // where the ring kernel has one accumulator set (more than 42 columns: with two its epilogue overlaps as well, and it is 7-10 %
+  // faster: 50k nodes of 4 rows, 64 -> 32 channels, 23.9 against 26.0 us) and where CTAs have more than one item to overlap: with at
+  // most one, loading the weights first costs 2-8 % (48 and 64 columns; 160 items: 3-5 % gained, 640: 10-20 %, 6256: 17-32 %).  Two units of two
+  // k-blocks hold both A slots to the end, so they take three items a CTA to gain (376 items: 16.0 -> 16.3 us, 640: 24.0 -> 22.2, 6256:
+  // 180 -> 154).
   const int b_bytes = longest * n_cols * KB * 8;
   if (group == 1 && longest >= 1 && longest <= VM_SHORT_CHUNK_KB && slots <= rows1 + rows1 / 2 && b_bytes <= 96 * 1024 &&
-      (n_cols <= 64 || (n_cols == 128 && longest <= 2))) {
+      L.acc_sets == 1 && (n_cols <= 64 || (n_cols == 128 && longest <= 2)) &&
+      L.total_items > (int64_t)sm_count() * (n_cols == 128 && longest == 2 ? 3 : 1)) {
     ResidentLaunch R{};
     R.map_a = L.map_a; R.map_bb = L.map_bb; R.map_bs = L.map_bs;
     R.out = out; R.kb_begin = kb_begin; R.rows = group_rows; R.a_col = a_col; R.status = status;

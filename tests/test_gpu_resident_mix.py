@@ -1,8 +1,10 @@
 """``IrrepsLinear`` on the tensor-core product that keeps an output row's weights in shared memory, against float64: widths of one and
-of two accumulator units, sums of one to four k-blocks (the most it takes) and of five (not taken), batches that end inside a
-sample tile, ranges that begin and end inside an output row, a row that no path reaches, and rows that several outputs read."""
+of two accumulator units, sums of one to four k-blocks (the most it takes), batches that end inside a sample tile, ranges that begin and
+end inside an output row, a row that no path reaches, and rows that several outputs read; and the calls that the kernel with a
+ring of weights keeps (narrow outputs, fewer items than SMs, longer sums)."""
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 from equitorch_b200 import _lib
 from equitorch_b200 import nn as enn
@@ -17,19 +19,24 @@ def _rel(a, b):
     return float((a.double() - b).norm() / b.norm())
 
 
-@pytest.mark.parametrize("ir_in,ir_out,n,cin,cout", [
-    ("0e+1o+2e+3o", "0e+1o+2e+3o", 513, 64, 128), ("0e+1o", "0e+1o", 20011, 32, 128), ("0e+1o+2e", "0e+1o+2e", 1000, 64, 48),
-    ("0e+1o", "0e+1o", 5003, 128, 64), ("0e+1o+2e", "0e+1o+2e", 700, 96, 16), ("0e+1o", "0e+1o", 640, 160, 32),
-    ("0e+1o", "0e+1e+1o", 2049, 64, 64), ("0e+1o", "2x0e+2x1o", 1500, 32, 64), ("2x0e+1o", "0e+1o", 1281, 64, 128), ("0e", "0e", 512, 128, 128)])
-def test_against_float64(ir_in, ir_out, n, cin, cout):
+@pytest.mark.parametrize("ir_in,ir_out,n,cin,cout,passes", [
+    ("0e+1o+2e+3o", "0e+1o+2e+3o", 4003, 64, 128, 2), ("0e+1o", "0e+1o", 20011, 32, 128, 1), ("0e+1o+2e", "0e+1o+2e", 2100, 64, 48, 1),
+    ("0e+1o", "0e+1o", 5003, 128, 64, 1), ("0e+1o+2e", "0e+1o+2e", 2500, 96, 16, 0), ("0e+1o", "0e+1o", 6400, 160, 32, 0),
+    ("0e+1o", "0e+1e+1o", 5003, 64, 64, 1), ("0e+1o", "2x0e+2x1o", 5003, 64, 64, 1), ("2x0e+1o", "0e+1o", 5003, 64, 128, 1),
+    ("0e", "0e", 19000, 96, 64, 1), ("0e+1o+2e+3o", "0e+1o+2e+3o", 4003, 64, 64, 2),
+    ("0e+1o+2e+3o", "0e+1o+2e+3o", 513, 64, 128, 0), ("0e+1o", "0e+1o", 700, 32, 64, 0), ("0e", "0e", 512, 128, 128, 0)])
+def test_against_float64(ir_in, ir_out, n, cin, cout, passes):
+    """``passes``: how many of the two products (output, gradient of x) take the resident kernel."""
     g = torch.Generator(device=DEV).manual_seed(n)
     layer = enn.IrrepsLinear(ir_in, ir_out, cin, cout, internal_weights=False).to(DEV)
     x = torch.randn(n, layer.irreps_in.dim, cin, generator=g, device=DEV).requires_grad_(True)
     w = (torch.randn(*layer.weight_shape, generator=g, device=DEV) * cin ** -0.5).requires_grad_(True)
     cot = torch.randn(n, layer.irreps_out.dim, cout, generator=g, device=DEV)
-    out = layer(x, w)
-    got = [out, *torch.autograd.grad(out, [x, w], cot)]
-    check_status(torch.device(DEV))
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        out = layer(x, w)
+        got = [out, *torch.autograd.grad(out, [x, w], cot)]
+        check_status(torch.device(DEV))
+    assert sum(e.count for e in prof.key_averages() if "vecmat_resident_kernel" in e.key) == passes
     xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
     f = layer.forward_info
     want = xd.new_zeros(n, layer.irreps_out.dim, cout)
