@@ -79,3 +79,18 @@ def test_wgrad_tc_matches_float64_and_is_reproducible(irreps, n, cin, cout):
     want = torch.zeros(paths, cin, cout, dtype=torch.float64, device=DEV).index_add_(0, info.index2, per_row)
     err = float((got.double() - want).abs().max() / want.abs().max())
     assert err < 8e-6, f"relative error {err:.2e}"
+
+
+@pytest.mark.parametrize("cout", [96, 128])
+def test_sums_run_in_the_order_of_the_channels(cout):
+    """One issuer (more than 64 columns): terms of one accumulator are added in the order of the channels, eight at a time.  2^30 + 1 is
+    not a float32, so what cancels 2^30 in the last eight leaves 0, and 1 where the 1 comes after it."""
+    ir = Irreps("2x0e+1o")
+    fwd, _, _, paths = tp_infos(ir, ir, ir)
+    plan = MixPlan(fwd.info_M_fwd.to(DEV), [i.dim for i in ir], DEV)
+    s, w = torch.zeros(200, plan.rows, 32, device=DEV), torch.ones(paths, 32, cout, device=DEV)
+    for place, value in ((0, 2. ** 30), (16, 1.), (24, -2. ** 30)):
+        s[:, 0, place] = value
+    got = mix_tc(s, w, plan)
+    check_status()
+    assert torch.count_nonzero(got) == 0
