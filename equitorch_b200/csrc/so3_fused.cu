@@ -528,8 +528,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
       : "memory");
 }
 
-// The node walk every role performs: nodes come in chunks of nodes_per_cta dealt round-robin to the CTAs.  The
-// segment pointers are read two nodes ahead of their use, so the walk does not wait for a load per node.
+constexpr int NODES_PER_CHUNK = 16;    // nodes that a CTA takes at a time, fewer on small graphs (launch_segsum_tc)
+
+// The node walk every role performs: nodes come in chunks of PER nodes (0: nodes_per_cta) dealt round-robin to the CTAs.  Inside a
+// chunk the segment pointers are read two nodes ahead of their use, so the walk does not wait for a load per node; at the first
+// node of a chunk it does.
+template <int PER>
 struct Walk {
   const int64_t* ptr;
   int n_out, per;       // 32-bit state: the launcher checks that nodes and edges fit
@@ -541,7 +545,7 @@ struct Walk {
     const int d = chunk * per;
     p0 = at(d); p1 = at(d + 1); p2 = at(d + 2);
   }
-  __device__ Walk(const FusedArgs& a) : ptr(a.ptr), n_out((int)a.n_out), per(a.nodes_per_cta), chunk(blockIdx.x), d_in(0) { prime(); }
+  __device__ Walk(const FusedArgs& a) : ptr(a.ptr), n_out((int)a.n_out), per(PER ? PER : a.nodes_per_cta), chunk(blockIdx.x), d_in(0) { prime(); }
   // next node of this CTA: returns false at the end; d = node, e0 = its first edge, deg = its edge count
   __device__ bool next(int& d, int& e0, int& deg) {
     d = chunk * per + d_in;
@@ -562,7 +566,7 @@ struct Walk {
 
 }  // namespace segtc
 
-template <class S>
+template <class S, int PER>
 __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedArgs a) {
   using namespace segtc;
   using namespace tc;
@@ -605,7 +609,7 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
     // ---------------- producers: warp 0 requests rows 0-3 of every group, the harmonics and arms the barrier; warp 15
     // requests rows 4-7 (the issue of a bulk copy costs a few hundred cycles per request, so two warps share it) ----
     const int row0 = warp == 0 ? 0 : GE / 2;
-    Walk w(a);
+    Walk<PER> w(a);
     int d, e0, deg;
     int g = 0;                                       // edge groups issued
     // gather indices, one edge per lane, requested one group ahead: within a chunk the edges of consecutive nodes are
@@ -653,7 +657,7 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
     const int tile0 = warp == 1 ? 0 : 4;
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_tf32(16);
-      Walk w(a);
+      Walk<PER> w(a);
       int d, e0, deg, g = 0, nq = 0;
       bool ok = true;
       while (ok && !*ab && w.next(d, e0, deg)) {
@@ -691,7 +695,7 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
     int fo[8];                                               // offset of this lane's feature inside a row, per tile
 #pragma unroll
     for (int i = 0; i < 8; ++i) fo[i] = S::tc_mfeat(h, i) * C + c;
-    Walk w(a);
+    Walk<PER> w(a);
     int d, e0, deg, g = 0;
     bool ok = true;
     while (ok && !*ab && w.next(d, e0, deg)) {
@@ -737,7 +741,7 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
     // ---------------- contraction ----------------
     const int quarter = warp & 3;                            // warps 10-13 -> 2, 3, 0, 1: every quarter once
     const int L = quarter * 32 + lane, h = L >> 6, c = L & 63;
-    Walk w(a);
+    Walk<PER> w(a);
     int d, e0, deg, nq = 0;
     while (!*ab && w.next(d, e0, deg)) {
       float* o = a.out + (int64_t)d * (S::R * C) + c;
@@ -772,14 +776,16 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
 }
 
 // Nodes that a CTA of the persistent kernel takes at a time: at most 16, and sixteen rounds of the CTAs where there are that many
-// nodes, so that the last round weighs little (10k nodes in chunks of 16 were 4.2 rounds of 148 CTAs, i.e. five: 230 us for 200k edges,
-// 202 us in chunks of four; below 2400 nodes chunks of 16 leave SMs without any).
+// nodes, so that the last round weighs little.  Both segment sums of a training pass, 20 edges a node, l_max 3, 64 channels, in
+// chunks of 16 and so: 300 nodes 99 -> 27 us, 2000 nodes 106 -> 100 (below 2400 nodes chunks of 16 leave SMs without any), 8000 nodes 367 ->
+// 324 (3.4 rounds of 148 CTAs were four), 20k nodes 809 -> 780.  From 37,888 nodes on a chunk is 16 nodes again, a constant of the
+// kernel then: as an argument it costs 0.4 % (100k nodes: 3846 -> 3866 us).
 template <class S>
 int launch_segsum_tc(FusedArgs a, cudaStream_t s) {
   if constexpr (S::HAS_TC) {
-    a.nodes_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(16, a.n_out / ((int64_t)sm_count() * 16)));
+    a.nodes_per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(segtc::NODES_PER_CHUNK, a.n_out / ((int64_t)sm_count() * 16)));
     constexpr size_t bytes = segtc::OFF_SC + sizeof(float) * ((S::T + 3) & ~3) + 1024;
-    auto kern = tp_segsum_tc_kernel<S>;
+    auto kern = a.nodes_per_cta == segtc::NODES_PER_CHUNK ? tp_segsum_tc_kernel<S, segtc::NODES_PER_CHUNK> : tp_segsum_tc_kernel<S, 0>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     kern<<<(unsigned)std::min<int64_t>(ceil_div(a.n_out, a.nodes_per_cta), sm_count()), segtc::THREADS, bytes, s>>>(a);

@@ -172,3 +172,22 @@ def test_profiling_size_graph_prefix_against_oracle():
     for name, a, b in pairs:
         err = float((a.detach().double().cpu() - b.detach()).abs().max() / b.detach().abs().max())
         assert err < 1e-5, f"{name}: relative error {err:.2e}"
+
+
+@pytest.mark.parametrize("nodes", [1, 149, 4735, 4737, 37887, 37893])
+def test_chunks_of_the_segment_sum(nodes):
+    """Chunks of one node, of several and of the constant 16, each with a last chunk that is not whole: outputs of the first and last nodes
+    and of nodes about the middle against the oracle, and that no node is left out or summed twice."""
+    ir, c = "0e+1o+2e+3o", 64
+    g, src, dst, vec = _case(nodes, nodes, 5 * nodes)
+    layer = enn.SO3LinearGraph(ir, ir, ir, c, c, internal_weights=False, feature_mode="uv").to(DEV)
+    x, w = torch.randn(nodes, 16, c, generator=g), torch.randn(*layer.weight_shape, generator=g) / c ** 0.5
+    out = layer(x.to(DEV), enn.SphericalHarmonics(3)(vec.to(DEV)), EdgeGraph(src.to(DEV), dst.to(DEV), nodes), w.to(DEV)).cpu()
+    check_status()
+    picked = torch.unique(torch.cat([torch.arange(min(nodes, 20)), nodes // 2 + torch.arange(min(nodes // 2, 20)),
+                                     torch.arange(max(0, nodes - 20), nodes)]))
+    mine = torch.isin(dst, picked)
+    ref = otp.so3_linear_message_passing(x.double(), vec[mine].double(), src[mine], dst[mine], w.double(), ir, ir, ir, feature_mode="uv",
+                                         num_out_nodes=nodes)
+    assert float((out[picked].double() - ref[picked]).abs().max() / ref[picked].abs().max()) < 1e-5
+    assert torch.equal(out.flatten(1).abs().sum(1) > 0, torch.bincount(dst, minlength=nodes) > 0)
