@@ -28,7 +28,7 @@ namespace {
 constexpr int V = 4;                              // channels per thread
 
 // P: two values at a time in packed instructions (fma.rn.f32x2).  Fewer instructions, but the scalar operand needs a pair of its own:
-// 'uv' backward 279 -> 214 us (20,011 samples, l_max 3, 64 channels), 'uu' forward 55 -> 52 us (20,480 samples, bfloat16, weights per
+// 'uv' backward 279 -> 214 us (before its grid fitted the SMs; 20,011 samples, l_max 3, 64 channels), 'uu' forward 55 -> 52 us (20,480 samples, bfloat16, weights per
 // sample); 'uu' backward, which is at its register limit without, 107 -> 114 us, so that one does without.
 __device__ __forceinline__ unsigned long long two(float x, float y) {
   unsigned long long r;
@@ -542,7 +542,8 @@ __global__ void __launch_bounds__(128, 4) so3_uv_expand_kernel(PathArgs a) {
 // instruction caches hold (4 k instructions a sample at l_max 3), and walking through them takes a CTA some 65 k cycles whatever its
 // size, most of it waiting for instructions: what counts is the samples in flight.  x is therefore loaded a block at a time instead
 // of kept in columns of shared memory, which leaves room for three CTAs: 294 -> 279 us (20,011
-// samples, l_max 3, 64 channels); twelve warps in one CTA that keep together: 295 us.  Packed multiply-adds make the walk shorter: 214 us.
+// samples, l_max 3, 64 channels); twelve warps in one CTA that keep together: 295 us.  Packed multiply-adds make the walk shorter: 214 us,
+// and a grid of exactly the CTAs that fit: 182 us.
 template <int LO, int L1, int L2>
 __device__ __forceinline__ void uv_backward_path(float (&gx)[2 * L1 + 1][V], const float (&x)[2 * L1 + 1][V], RowStream& rs, const float* yr,
                                                  float* gyc, int threads, float scale) {
@@ -673,7 +674,10 @@ bool path_shape(PathMode mode, bool shared_gw, int64_t n, int c, int dtype, cons
     const PathSmem L(mode, shared_gw, dtype == EQT_F32 ? 4 : 2, threads, slots, t->d1, t->d_out, t->d2, t->num_weights,
                      backward ? t->num_bwd_blocks : t->num_fwd_blocks, t->num_paths, t->num_rows);
     if (L.total > PATH_SMEM_MAX) continue;
-    const int per_sm = std::max<int>(1, std::min<int>(512 / threads, (int)(PATH_SMEM_MAX / (L.total + 1024))));
+    // the gradients of the 'uv' rows take registers for three CTAs an SM: a grid of four leaves a quarter of them to a round of their
+    // own, and every walk costs the same (20,011 samples, 64 channels, four -> three: l_max 3 214 -> 182 us, l_max 2 90 -> 74, l_max 1 38 -> 29)
+    const int fit = (mode == UV_BACKWARD ? 384 : 512) / threads;
+    const int per_sm = std::max<int>(1, std::min<int>(fit, (int)(PATH_SMEM_MAX / (L.total + 1024))));
     s->threads = threads; s->slots = slots; s->smem = L.total;
     s->grid = (int)std::min<int64_t>(ceil_div(n, slots), (int64_t)sm_count() * per_sm);
     s->split = backward ? 1 : std::max(1, std::min(t->num_fwd_blocks, sm_count() / std::max(1, s->grid)));
