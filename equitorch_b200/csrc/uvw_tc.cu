@@ -610,7 +610,7 @@ extern "C" int eqt_uvw_contract(const eqt_uvw_role* roles, int32_t jobs, const f
 // stores it to tensor memory, where the MMA reads it; f arrives as [big | small] tiles of 32 samples, so that one MMA of 2 K
 // columns makes big * big and big * small, and one of K columns small * big.  An MMA waits for the one
 // before it into the same accumulator, so even and odd k-steps and the two kinds of MMA have accumulators of their own, folded into
-// float32 registers every 12 to 20 k-steps each (the adder of the tensor core truncates); and every instruction of the issuing
+// float32 registers every 16 to 24 k-steps each (the adder of the tensor core truncates); and every instruction of the issuing
 // thread counts, so the MMAs of a stage are straight-line code by the degree of f (one accumulator and a loop: 211 us at 2000 samples,
 // l_max 2, 32 channels; four: 201 us; without the loop 167 us; a third stage changes nothing).  The work - (path, channel group) x chunks of 32 samples -
 // is one line that is cut into equal costs, one range per SM; a range that ends inside a (path, channel group) leaves a partial sum,
@@ -626,8 +626,8 @@ constexpr int CHUNK = 32;                  // samples of a stage
 constexpr int W_STAGES = 2;
 constexpr int W_LOADERS = 4;
 constexpr int W_THREADS = (12 + W_LOADERS) * 32;
-constexpr int MAX_PIECES = 640;
-constexpr int MAX_CTAS = 192;
+constexpr int MAX_UNITS = 640;             // (path, channel group) and one CTA an SM
+constexpr int MAX_PIECES = 1024;
 
 // Rows of 32 samples of s and g in shared memory: the 16-byte chunks of a row are permuted so that eight neighbouring rows (a
 // phase of 16-byte reads) as well as rows 4 l + t for eight l (a store of the loaders) lie on different banks.
@@ -643,7 +643,7 @@ struct WLaunch {
   int64_t n;
   int ds, df, d_out, ci, ck, groups;
   int* status;
-  short cta[MAX_CTAS + 1];                 // pieces [cta[b], cta[b + 1]) of CTA b
+  short cta[MAX_PIECES + 1];               // pieces [cta[b], cta[b + 1]) of CTA b
   WPiece piece[MAX_PIECES];
 };
 
@@ -957,49 +957,175 @@ __global__ void __launch_bounds__(W_THREADS, 1) uvw_wgrad_kernel(const __grid_co
   if (abort_flag && tid == 0) atomicExch(p.status, 2);
 }
 
+// The same sums by float32 multiply-adds: a thread is a pair (i, j), with its Q in a register per component of f, K accumulators, and K
+// totals that take the accumulators every F_CHUNK samples, so that no chain of additions is long.  Operands arrive as they lie
+// in memory, a chunk ahead of their use.  Error of the norm against 64 bits, l_max 2, 32 channels, this | TF32 pairs | the two-step form:
+// 1 sample 0.6 | 1.0 | 0.6e-7, 200 samples 1.5 | 3.6 | 2.6e-7, 511 samples 1.6 | 4.1 | 4.0e-7.
+// Bound: multiply-adds and the broadcast reads of f (one of 16 bytes per two packed multiply-adds).  us, l_max 2, this | TF32 pairs: 511
+// samples, 32 channels 61 | 51, 16 channels 13 | 15; 2000 samples, 32 channels 212 | 170, 16 channels 35 | 41.  Two pairs a thread,
+// which halve those reads, spill: 227.
+constexpr int F_CHUNK = 16;
+constexpr int F_STAGES = 2;
+constexpr int f_ctas(int k) { return k > 16 ? 3 : 4; }                  // an SM; four with 32 accumulators spill
+__host__ __device__ constexpr int f_stage_bytes(int k, int cj) { return F_CHUNK * 5 * (COLS / cj + cj + k) * 4; }
+
+template <int J, int K> struct PairSums {
+  static constexpr int IQ = COLS / J;
+  const WLaunch& p;
+  unsigned char* smem;
+  int tid, i0;
+  Two total[K / 2];
+
+  template <int LO, int LS, int LF> __device__ __forceinline__ void run(const eqt_uvw_path* path, int chunk0, int chunk1) {
+    if constexpr (couples(LO, LS, LF)) {
+      constexpr int NO = 2 * LO + 1, NS = 2 * LS + 1, NF = 2 * LF + 1;
+      constexpr int SQ = NS * IQ / 4, GQ = NO * J / 4, FQ = NF * K / 4, PER = SQ + GQ + FQ;      // 16-byte pieces of a sample
+      const float* sp = p.s + (int64_t)__ldg(&path->offset_s) * p.ci + i0;
+      const float* gp = p.g + (int64_t)__ldg(&path->offset_o) * J;
+      const float* fp = p.f + (int64_t)__ldg(&path->offset_f) * K;
+      auto load = [&](int chunk) {               // samples past the batch are zero
+        if (chunk < chunk1) {
+          const uint32_t to = s32(smem + (chunk - chunk0) % F_STAGES * f_stage_bytes(K, J));
+          for (int t = tid; t < F_CHUNK * PER; t += COLS) {
+            const int u = t / PER, r = t - u * PER;
+            const int64_t n = (int64_t)chunk * F_CHUNK + u, m = min(n, p.n - 1);
+            const float* from = r < SQ ? sp + (m * p.ds + r / (IQ / 4)) * p.ci + r % (IQ / 4) * 4
+                                : r < SQ + GQ ? gp + m * p.d_out * J + (r - SQ) * 4 : fp + m * p.df * K + (r - SQ - GQ) * 4;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + t * 16), "l"(from), "r"(n < p.n ? 16 : 0) : "memory");
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      for (int c = 0; c < F_STAGES - 1; ++c) load(chunk0 + c);
+      const int i = tid / J, j = tid % J;
+      for (int chunk = chunk0; chunk < chunk1; ++chunk) {
+        load(chunk + F_STAGES - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(F_STAGES - 1) : "memory");
+        __syncthreads();
+        const float* at = reinterpret_cast<const float*>(smem + (chunk - chunk0) % F_STAGES * f_stage_bytes(K, J));
+        Two acc[K / 2];
+#pragma unroll
+        for (int m = 0; m < K / 2; ++m) acc[m] = two(0.f, 0.f);
+#pragma unroll 1
+        for (int u = 0; u < F_CHUNK; u += 2, at += 2 * PER * 4) {          // two samples side by side
+          Two s[NS][1], g[NO][1], q[NF][1];
+#pragma unroll
+          for (int b = 0; b < NS; ++b) s[b][0] = two(at[b * IQ + i], at[PER * 4 + b * IQ + i]);
+#pragma unroll
+          for (int a = 0; a < NO; ++a) g[a][0] = two(at[SQ * 4 + a * J + j], at[PER * 4 + SQ * 4 + a * J + j]);
+          CgTriple<LO, LS, LF>::template pair<1>(q, s, g);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = 0; c < NF; ++c) {
+              float x, y;
+              apart(q[c][0], x, y);
+              const Two qq = h ? two(y, y) : two(x, x);
+              const float4* f = reinterpret_cast<const float4*>(at + (h * PER + SQ + GQ) * 4 + c * K);
+#pragma unroll
+              for (int m = 0; m < K / 4; ++m) {
+                const float4 v = f[m];
+                acc[2 * m] = fma2(qq, two(v.x, v.y), acc[2 * m]);
+                acc[2 * m + 1] = fma2(qq, two(v.z, v.w), acc[2 * m + 1]);
+              }
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < K / 2; ++m) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(total[m].v) : "l"(acc[m].v));
+        __syncthreads();                         // the stage may be written again
+      }
+    }
+  }
+};
+
+template <int J, int K>
+__global__ void __launch_bounds__(COLS, f_ctas(K)) uvw_wgrad_f32_kernel(const __grid_constant__ WLaunch p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int p0 = p.cta[blockIdx.x], p1 = p.cta[blockIdx.x + 1];
+  for (int x = p0; x < p1; ++x) {
+    const WPiece pc = p.piece[x];
+    const eqt_uvw_path* path = p.paths + pc.unit / p.groups;
+    PairSums<J, K> w{p, smem_raw, (int)threadIdx.x, pc.unit % p.groups * (COLS / J)};
+#pragma unroll
+    for (int m = 0; m < K / 2; ++m) w.total[m] = two(0.f, 0.f);
+    switch (__ldg(&path->l_o) * 9 + __ldg(&path->l_s) * 3 + __ldg(&path->l_f)) {
+#define EQT_CASE(LO, LS, LF) case LO * 9 + LS * 3 + LF: w.template run<LO, LS, LF>(path, pc.chunk0, pc.chunk1); break;
+      EQT_CASE(0, 0, 0) EQT_CASE(0, 1, 1) EQT_CASE(0, 2, 2) EQT_CASE(1, 0, 1) EQT_CASE(1, 1, 0) EQT_CASE(1, 1, 1) EQT_CASE(1, 1, 2)
+      EQT_CASE(1, 2, 1) EQT_CASE(1, 2, 2) EQT_CASE(2, 0, 2) EQT_CASE(2, 1, 1) EQT_CASE(2, 1, 2) EQT_CASE(2, 2, 0) EQT_CASE(2, 2, 1)
+      EQT_CASE(2, 2, 2)
+#undef EQT_CASE
+    }
+    float sum[K];                                // columns in the order of the tensor-core kernel's
+#pragma unroll
+    for (int m = 0; m < K / 2; ++m) apart(w.total[m], sum[f_row(K, 2 * m)], sum[f_row(K, 2 * m + 1)]);
+    float* out = p.partial + ((int64_t)x * COLS + threadIdx.x) * K;
+#pragma unroll
+    for (int m = 0; m < K; m += 4) *reinterpret_cast<float4*>(out + m) = make_float4(sum[m], sum[m + 1], sum[m + 2], sum[m + 3]);
+  }
+}
+
 struct WSumLaunch {
   const float* partial;
   float* gw;                               // (paths, i, k, j) with the strides below
   const eqt_uvw_path* paths;
   int64_t si, sk, sj, sp;
   int ck, cj, groups, units;
-  short first[MAX_PIECES + 1];             // pieces of unit u: [first[u], first[u + 1])
+  short first[MAX_UNITS + 1];              // pieces of unit u: [first[u], first[u + 1])
 };
-__global__ void __launch_bounds__(256) uvw_wgrad_sum_kernel(const __grid_constant__ WSumLaunch p) {
-  const int quads = p.ck / 4, iq = COLS / p.cj;
-  const int64_t total = (int64_t)p.units * 128 * quads;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int row = (int)(t % 128), ch = (int)(t / 128 % quads), unit = (int)(t / 128 / quads);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int x = p.first[unit]; x < p.first[unit + 1]; ++x) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(p.partial + ((int64_t)x * 128 + row) * p.ck) + ch);
-      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-    }
-    const int q = unit / p.groups, i = unit % p.groups * iq + row / p.cj, j = row % p.cj;
-    const float scale = __ldg(&p.paths[q].scale);
-    float* to = p.gw + __ldg(&p.paths[q].weight) * p.sp + i * p.si + j * p.sj;
-    const float a[4] = {v.x, v.y, v.z, v.w};
+// gw of 32 pairs (i, j) of a unit: its pieces, each 32 K floats in a row, are dealt to lanes of 8 K threads and added up in 64 bits, the
+// lanes' sums in order; through shared memory, so that the writes run along j.
+__global__ void __launch_bounds__(1024) uvw_wgrad_sum_kernel(const __grid_constant__ WSumLaunch p) {
+  extern __shared__ double red[];                // 4 values of every thread (one lane: none)
+  __shared__ float tile[32][33];
+  const int tid = threadIdx.x, quads = p.ck / 4, per = 32 * quads, lanes = blockDim.x / per, lane = tid / per, e = tid % per;
+  const int unit = blockIdx.x / 4, row0 = blockIdx.x % 4 * 32, iq = COLS / p.cj;
+  double v[4] = {0., 0., 0., 0.};
+#pragma unroll 4
+  for (int t = p.first[unit] + lane; t < p.first[unit + 1]; t += lanes) {
+    const float4 u = __ldg(reinterpret_cast<const float4*>(p.partial) + ((int64_t)t * COLS + row0) * quads + e);
+    v[0] += u.x; v[1] += u.y; v[2] += u.z; v[3] += u.w;
+  }
+  if (lanes > 1) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) red[m * blockDim.x + tid] = v[m];
+    __syncthreads();
+  }
+  const int q = unit / p.groups;
+  if (lane == 0) {
+    const double scale = __ldg(&p.paths[q].scale);
 #pragma unroll
     for (int m = 0; m < 4; ++m) {                // column r of the accumulator: channel 4 (r % (K / 4)) + r / (K / 4)
-      const int r = ch * 4 + m;
-      to[(int64_t)(4 * (r % quads) + r / quads) * p.sk] = a[m] * scale;
+      for (int t = 1; t < lanes; ++t) v[m] += red[m * blockDim.x + t * per + e];
+      const int r = e % quads * 4 + m;
+      tile[4 * (r % quads) + r / quads][e / quads] = (float)(v[m] * scale);
     }
+  }
+  __syncthreads();
+  float* to = p.gw + __ldg(&p.paths[q].weight) * p.sp;
+  for (int t = tid; t < 32 * p.ck; t += blockDim.x) {
+    const int k = t / 32, row = row0 + t % 32, i = unit % p.groups * iq + row / p.cj, j = row % p.cj;
+    to[i * p.si + k * p.sk + j * p.sj] = tile[k][t % 32];
   }
 }
 
-// The line of (path, channel group, chunk), cut into ranges of equal cost.  Cost of a chunk: instructions of a row maker.
+// Float32 multiply-adds where TF32 pairs would be further from 64 bits than the two-step form was: below 512 samples, and with 16 output
+// channels, whose sums that form took on multiply-adds at any size (16 channels: 2.3e-7 against 3.4e-7 at 512 samples).  And where f
+// has 16 channels, whose MMAs are half as wide: 2000 samples, l_max 2, 32 x 16 -> 32 channels 152 us on tensor cores, 1.7e-7 instead of 4.5e-7.
+bool wgrad_f32(const eqt_uvw_role& r, int64_t n) { return n < 512 || r.cj == 16 || r.ck == 16; }
+
+// The line of (path, channel group, chunk), cut into ranges of equal cost.  Cost of a chunk: instructions of a thread that makes rows.
 int cut_wgrad(const eqt_uvw_role& r, const int32_t* degrees, int64_t n, WLaunch* L, WSumLaunch* S, int* ctas) {
-  const int64_t chunks = ceil_div(n, CHUNK);
+  const bool f32 = wgrad_f32(r, n);
+  const int64_t chunks = ceil_div(n, f32 ? F_CHUNK : CHUNK);
   const int groups = r.ci * r.cj / COLS, units = r.num_paths * groups;
-  if (chunks > 0x7fffffff) return -1;
+  if (chunks > 0x7fffffff || units + std::min<int64_t>(sm_count(), units * ceil_div(n, CHUNK)) > MAX_UNITS) return -1;
   auto cost = [&](int q) {
     const int no = 2 * degrees[3 * q] + 1, ns = 2 * degrees[3 * q + 1] + 1, nf = 2 * degrees[3 * q + 2] + 1;
-    return (int64_t)(16 + 20 * nf + 6 * no * ns);
+    return (int64_t)(f32 ? 8 * no * ns + 2 * (no + ns) + nf * (6 * r.ck / 4 + 4) : 16 + 20 * nf + 6 * no * ns);
   };
   int64_t total = 0;
   for (int q = 0; q < r.num_paths; ++q) total += cost(q) * groups * chunks;
-  const int want = (int)std::min<int64_t>(std::min(sm_count(), MAX_CTAS), units * chunks);
-  if (units + want > MAX_PIECES) return -1;
+  const int want = (int)std::min<int64_t>(std::min(sm_count() * (f32 ? f_ctas(r.ck) : 1), MAX_PIECES - units), units * chunks);
   int pieces = 0, cta = 0;
   int64_t before = 0;                      // cost of the units before the current one
   if (L) L->cta[0] = 0;
@@ -1028,6 +1154,17 @@ int cut_wgrad(const eqt_uvw_role& r, const int32_t* degrees, int64_t n, WLaunch*
     if (L) L->cta[cta + 1] = (short)pieces;
   if (ctas) *ctas = want;
   return pieces;
+}
+
+template <int J, int K> int launch_wgrad_tc(const WLaunch& L, int ctas, cudaStream_t st) {
+  if (int rc = allow_shared(uvw_wgrad_kernel<J, K>, 160 * 1024)) return rc;
+  uvw_wgrad_kernel<J, K><<<ctas, W_THREADS, (size_t)W_STAGES * WSmem(K, J).stage + 1024, st>>>(L);
+  return check_launch("uvw_wgrad_kernel");
+}
+template <int J, int K> int launch_wgrad_f32(const WLaunch& L, int ctas, cudaStream_t st) {
+  if (int rc = allow_shared(uvw_wgrad_f32_kernel<J, K>, 160 * 1024)) return rc;
+  uvw_wgrad_f32_kernel<J, K><<<ctas, COLS, F_STAGES * f_stage_bytes(K, J), st>>>(L);
+  return check_launch("uvw_wgrad_f32_kernel");
 }
 
 }  // namespace
@@ -1059,15 +1196,16 @@ extern "C" int eqt_uvw_wgrad(const eqt_uvw_role* role, const int32_t* degrees, c
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   L.s = s; L.f = f; L.g = g; L.partial = scratch; L.paths = r.paths; L.n = n;
   L.ds = r.ds; L.df = r.df; L.d_out = r.d_out; L.ci = r.ci; L.ck = r.ck; L.groups = r.ci * r.cj / COLS; L.status = status;
-  const size_t smem = (size_t)W_STAGES * WSmem(r.ck, r.cj).stage + 1024;
-  auto* kernel = r.cj == 32 ? (r.ck == 32 ? uvw_wgrad_kernel<32, 32> : uvw_wgrad_kernel<32, 16>)
-                            : (r.ck == 32 ? uvw_wgrad_kernel<16, 32> : uvw_wgrad_kernel<16, 16>);
-  if (int rc = allow_shared(kernel, 160 * 1024)) return rc;
-  kernel<<<ctas, W_THREADS, smem, st>>>(L);
-  if (int rc = check_launch("uvw_wgrad_kernel")) return rc;
+  const int rc = !wgrad_f32(r, n) ? launch_wgrad_tc<32, 32>(L, ctas, st)
+                 : r.cj == 32     ? (r.ck == 32 ? launch_wgrad_f32<32, 32>(L, ctas, st) : launch_wgrad_f32<32, 16>(L, ctas, st))
+                                  : (r.ck == 32 ? launch_wgrad_f32<16, 32>(L, ctas, st) : launch_wgrad_f32<16, 16>(L, ctas, st));
+  if (rc) return rc;
   S.partial = scratch; S.gw = gw; S.paths = r.paths;
   S.si = r.stride_i; S.sk = r.stride_k; S.sj = r.stride_j; S.sp = r.stride_p;
   S.ck = r.ck; S.cj = r.cj; S.groups = L.groups; S.units = r.num_paths * L.groups;
-  uvw_wgrad_sum_kernel<<<flat_grid((int64_t)S.units * 128 * (r.ck / 4), 256), 256, 0, st>>>(S);
+  const int per = 8 * r.ck;                      // about three pieces a lane
+  int lanes = 1;
+  while (2 * lanes * per <= 1024 && 3 * lanes * S.units < pieces) lanes *= 2;
+  uvw_wgrad_sum_kernel<<<(unsigned)(S.units * (COLS / 32)), per * lanes, lanes > 1 ? per * lanes * 32 : 0, st>>>(S);
   return check_launch("uvw_wgrad_sum_kernel");
 }
