@@ -79,7 +79,7 @@ class PathTableStruct(C.Structure):
 
 
 class UvwGroupStruct(C.Structure):
-    _fields_ = [("l", C.c_int32), ("offset", C.c_int32), ("count", C.c_int32)]
+    _fields_ = [("l", C.c_int32), ("offset", C.c_int32), ("count", C.c_int32), ("longest", C.c_int32)]
 
 
 class UvwRoleStruct(C.Structure):

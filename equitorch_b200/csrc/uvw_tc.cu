@@ -75,6 +75,7 @@ constexpr int MAX_GROUPS = 16;             // irreps of the contracted operand
 constexpr int MAX_SEGMENTS = 128;
 constexpr int CONTRACT_THREADS = 10 * 32;
 constexpr int B_STAGES = 2;
+constexpr int CHAIN = 160;                 // multiply-adds in a row into one output element (cut())
 
 __host__ __device__ constexpr bool couples(int a, int b, int c) { return a <= b + c && b <= a + c && c <= a + b; }
 // bytes of 128 rows split into big and small: two tiles of 128-byte rows, or [big | small] side by side in one
@@ -463,7 +464,7 @@ int check_role(const eqt_uvw_role& r) {
   int at = 0;
   for (int g = 0; g < r.num_groups; ++g) {
     const eqt_uvw_group& e = r.groups[g];
-    if (e.l < 0 || e.l > TRIPLE_MAX_L || e.count < 0 || e.offset < 0 || e.offset + 2 * e.l + 1 > r.df) return fail(EQT_ERR_BAD_ARGUMENT, "bad irrep %d", g);
+    if (e.l < 0 || e.l > TRIPLE_MAX_L || e.count < 0 || e.longest < (e.count > 0) || e.longest > e.count || e.offset < 0 || e.offset + 2 * e.l + 1 > r.df) return fail(EQT_ERR_BAD_ARGUMENT, "bad irrep %d", g);
     at += e.count;
   }
   return at == r.num_paths ? EQT_OK : fail(EQT_ERR_BAD_ARGUMENT, "the irreps list %d of %d paths", at, r.num_paths);
@@ -471,24 +472,31 @@ int check_role(const eqt_uvw_role& r) {
 
 // Channel groups of an irrep are dealt to CTAs so that the longest CTA is as short as the SMs allow: the smallest bound on the
 // accumulator slots of a CTA (components x paths x channel groups) whose CTAs fit one wave, or one CTA per irrep where
-// the sample tiles alone fill the chip.  Longest first.
+// the sample tiles alone fill the chip.  The multiply-adds into an output element are one chain, of which a CTA takes CHAIN at most (32
+// channels, l_max 2, error of the operand gradients against 64 bits: chains of 320 2.6e-7, of 160 2.1e-7, the two-step form 2.25e-7;
+// 20k samples 2840 -> 2980 us).  Longest first.  -1: one channel group alone is more than that, or too many CTAs a tile.
 int cut(const eqt_uvw_role* roles, int jobs, int64_t tiles, ContractLaunch* L, int (&slices)[2]) {
-  struct Item { int job, group, unit, quads; };
+  struct Item { int job, group, unit, quads, most; };        // most: channel groups of a CTA
   std::vector<Item> items;
   for (int j = 0; j < jobs; ++j)
-    for (int g = 0; g < roles[j].num_groups; ++g)
-      if (roles[j].groups[g].count)
-        items.push_back({j, g, roles[j].groups[g].count * (2 * roles[j].groups[g].l + 1), roles[j].ci * roles[j].cj / COLS});
+    for (int g = 0; g < roles[j].num_groups; ++g) {
+      const eqt_uvw_group& e = roles[j].groups[g];
+      if (!e.count) continue;
+      items.push_back({j, g, e.count * (2 * e.l + 1), roles[j].ci * roles[j].cj / COLS, CHAIN / (e.longest * (2 * e.l + 1) * (COLS / roles[j].cj))});
+      if (items.back().most < 1) return -1;
+    }
   const int64_t room = std::max<int64_t>((int64_t)items.size(), std::min<int64_t>(MAX_SEGMENTS, sm_count() / tiles));
-  if ((int64_t)items.size() > MAX_SEGMENTS) return -1;
   int bound = 0, worst = 0;
   for (const Item& i : items) { bound = std::max(bound, i.unit); worst = std::max(worst, i.unit * i.quads); }
-  auto per = [&](const Item& i, int b) { return std::max(1, std::min(i.quads, b / i.unit)); };
+  auto per = [&](const Item& i, int b) { return std::max(1, std::min({i.quads, i.most, b / i.unit})); };
   for (; bound < worst; ++bound) {
     int64_t need = 0;
     for (const Item& i : items) need += (i.quads + per(i, bound) - 1) / per(i, bound);
     if (need <= room) break;
   }
+  int64_t need = 0;
+  for (const Item& i : items) need += (i.quads + per(i, bound) - 1) / per(i, bound);
+  if (need > MAX_SEGMENTS) return -1;
   slices[0] = slices[1] = 0;
   int count = 0;
   std::vector<std::pair<int, Segment>> segs;

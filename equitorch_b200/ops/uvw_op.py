@@ -37,8 +37,9 @@ class _Role:
         self.table = np.array([(ls[w][o], ls[w][s], ls[w][f], start[o][paths[w][o]], start[s][paths[w][s]], start[f][paths[w][f]], w,
                                 scales[w] * exchanged_scale(ls[w], role)) for w in order], dtype=_PATH)
         self.degrees = (C.c_int32 * (3 * len(order)))(*(ls[w][a] for w in order for a in (o, s, f)))
+        outs = [[paths[w][o] for w in order if paths[w][f] == n] for n in range(len(degrees[f]))]
         self.groups = (_lib.UvwGroupStruct * len(degrees[f]))(
-            *(_lib.UvwGroupStruct(l, start[f][n], sum(paths[w][f] == n for w in order)) for n, l in enumerate(degrees[f])))
+            *(_lib.UvwGroupStruct(l, start[f][n], len(outs[n]), max(map(outs[n].count, outs[n]), default=0)) for n, l in enumerate(degrees[f])))
         self.axes = role
 
     def struct(self, channels: Tuple[int, int, int]) -> "_lib.UvwRoleStruct":
@@ -93,18 +94,19 @@ class UvwPlan:
 
 
 def uvw_contract(plan: UvwPlan, operands: Sequence[Optional[Tensor]], w: Tensor, roles) -> list:
-    """The products of ``roles`` (at most two; both run in one launch where their outputs have equally many channels), from
-    contiguous ``operands`` = (gradient of the output, first, second operand) and the weights."""
+    """The products of ``roles`` (at most two; both run in one launch where their outputs have equally many channels and one
+    launch has room for them), from contiguous ``operands`` = (gradient of the output, first, second operand) and the weights."""
     n = next(t for t in operands if t is not None).shape[0]
     channels = (w.shape[3], w.shape[1], w.shape[2])
-    if len(roles) == 2 and channels[roles[0][0]] != channels[roles[1][0]]:
-        return [uvw_contract(plan, operands, w, (r,))[0] for r in roles]
     structs, lib, dev = plan.structs(channels, roles), _lib.lib(), w.device
-    outs = [w.new_empty(n, plan.dims[r[0]], channels[r[0]]) for r in roles]
-    pointers = [(C.c_void_p * len(roles))(*ptrs) for ptrs in ([operands[r[1]].data_ptr() for r in roles],
-                                                             [operands[r[2]].data_ptr() for r in roles], [t.data_ptr() for t in outs])]
     with _lib.on_device(dev):
-        floats = int(lib.eqt_uvw_scratch_floats(structs, len(roles), n))
+        together = len(roles) == 1 or channels[roles[0][0]] == channels[roles[1][0]]
+        floats = int(lib.eqt_uvw_scratch_floats(structs, len(roles), n)) if together else -1
+        if floats < 0 and len(roles) == 2:
+            return [uvw_contract(plan, operands, w, (r,))[0] for r in roles]
+        outs = [w.new_empty(n, plan.dims[r[0]], channels[r[0]]) for r in roles]
+        pointers = [(C.c_void_p * len(roles))(*ptrs) for ptrs in ([operands[r[1]].data_ptr() for r in roles],
+                                                                 [operands[r[2]].data_ptr() for r in roles], [t.data_ptr() for t in outs])]
         scratch = torch.empty(max(floats, 0), dtype=torch.float32, device=dev)        # of this call: calls on other streams may overlap it
         _lib.check(lib.eqt_uvw_contract(structs, len(roles), *pointers, w.data_ptr(), scratch.data_ptr(), floats, n,
                                         status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_uvw_contract")

@@ -391,7 +391,8 @@ int eqt_so3_uu_backward(const eqt_path_table* table, const void* x, const void* 
  * irrep of f (`groups`, host memory, in the order of the list) and by output component inside; device memory.
  * eqt_uvw_wgrad: gw[p, i, k, j] = scale_p sum_n sum_(a, b, c) cg[a, b, c] s[n, b, i] f[n, c, k] g[n, a, j], every weight written;
  * `degrees` (host, 3 per path: out, s, f) in the order of the list.
- * Scratch: *_scratch_floats(); -1 = these sizes are not supported.  All operands 16-byte aligned.  Sums of the thread blocks
+ * Up to 160 multiply-adds of an output element are added up in a row, so roles are refused whose paths do not fit that 128 /
+ * cj channels at a time.  Scratch: *_scratch_floats(); -1 = these sizes are not supported.  All operands 16-byte aligned.  Sums of the thread blocks
  * are added in a fixed order.
  * replaces: TensorProductUVWDummy and its adjoints (equitorch/nn/functional/tensor_products.py:92-172).
  */
@@ -401,6 +402,7 @@ typedef struct eqt_uvw_path {
 } eqt_uvw_path;
 typedef struct eqt_uvw_group {
   int32_t l, offset, count;    /* irrep of f: degree, first component, paths                       */
+  int32_t longest;             /* the most of its paths that share an output irrep                 */
 } eqt_uvw_group;
 typedef struct eqt_uvw_role {
   const eqt_uvw_path* paths;   /* device                                                           */

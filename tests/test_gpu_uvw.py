@@ -47,13 +47,36 @@ def test_against_the_oracle(ir1, ir2, ir_out, n, c1, c2, c_out):
     ref = [t.to(where).double().requires_grad_(True) for t in (x1, x2, w)]
     want = [otp.tensor_product_dense(*ref, layer.irreps_in1, layer.irreps_in2, layer.irreps_out, feature_mode="uvw")]
     want += torch.autograd.grad(want[0], ref, cot.to(where).double())
-    # output and operand gradients: splits of both factors 2^-22 each and chains of at most 16 x 5 x 4 multiply-adds an accumulator;
-    # weights: chains of 80 multiply-adds below 512 samples and for 16 output channels (0.4 x 2^-24 x sqrt(80 / 2) and the roundings of the
+    # output and operand gradients: splits of both factors 2^-22 each and chains of at most 160 multiply-adds (0.4 x 2^-24 x sqrt(160 / 2): 2.1e-7
+    # where all are as long); weights: chains of 80 multiply-adds below 512 samples and for 16 output channels (0.4 x 2^-24 x sqrt(80 / 2) and the roundings of the
     # product of three: 2e-7), else truncation by the tensor core, up to 24 steps between two folds
     for k, (a, b) in enumerate(zip(got, want)):
-        assert _rel(a, b.cpu()) < (3e-7 if k < 3 else 2.5e-7 if n < 512 or c_out == 16 else 8e-7), k
+        assert _rel(a, b.cpu()) < (2.45e-7 if k < 3 else 2.5e-7 if n < 512 or c_out == 16 else 8e-7), k
     (only,) = torch.autograd.grad(layer(leaves[0].detach(), leaves[1], w.to(DEV)), [leaves[1]], cot.to(DEV))
     assert _rel(only, want[2].cpu()) < 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ir,c,taken", [("2x0e+2x1o+2x2e", 16, True), ("3x2e", 16, True), ("6x2e", 16, False)])
+def test_chains_of_many_paths(ir, c, taken):
+    """Several paths between the same irreps lengthen the sums of an output element: they are cut at 160 terms, and a layer whose paths do
+    not fit that for the channels of one accumulator runs the composed products."""
+    g = torch.Generator().manual_seed(5)
+    n = 2500
+    layer = enn.TensorProduct(ir, ir, ir, c, c, c, internal_weights=False, feature_mode="uvw").to(DEV)
+    x1, x2 = torch.randn(n, layer.irreps_in1_dim, c, generator=g), torch.randn(n, layer.irreps_in2_dim, c, generator=g)
+    w, cot = torch.randn(*layer.weight_shape, generator=g), torch.randn(n, layer.irreps_out_dim, c, generator=g)
+    leaves = [t.to(DEV).requires_grad_(True) for t in (x1, x2, w)]
+    out = layer(*leaves)
+    assert (type(out.grad_fn).__name__ == TensorProductUVW.__name__ + "Backward") == taken
+    got = [out, *torch.autograd.grad(out, leaves, cot.to(DEV))]
+    ref = [t.to(DEV).double().requires_grad_(True) for t in (x1, x2, w)]
+    want = [otp.tensor_product_dense(*ref, layer.irreps_in1, layer.irreps_in2, layer.irreps_out, feature_mode="uvw")]
+    want += torch.autograd.grad(want[0], ref, cot.to(DEV).double())
+    for a, b in zip(got[:3] if taken else got, want):
+        assert _rel(a, b.cpu()) < (2.45e-7 if taken else 5e-6)      # 5e-6: sums of 4096 terms and more in one float32 chain
+    if taken:
+        assert _rel(got[3], want[3].cpu()) < 2.5e-7
 
 
 @pytest.mark.gpu
