@@ -97,8 +97,9 @@ class TensorProductUVWDummy(Function):
 
 class TensorProductUVW(Function):
     """:func:`tensor_product_uvw` without an intermediate in memory (``plan``: the layer's tables on the device): the output and
-    both operand gradients are the same product with the roles of the operands exchanged.  A backward pass that is itself
-    differentiated is composed of the differentiable products, on the operands as they were given."""
+    both operand gradients are the same product with the roles of the operands exchanged.  Scratch stays below
+    ``UVW_INTERMEDIATE_LIMIT``.  A backward pass that is itself differentiated is composed of the differentiable products, on the
+    operands as they were given."""
 
     @staticmethod
     def forward(ctx, input1, input2, weight, plan, infos):
@@ -106,7 +107,7 @@ class TensorProductUVW(Function):
         ctx.save_for_backward(input1 if n2 or nw else None, input2 if n1 or nw else None, weight if n1 or n2 else None)
         ctx.plan, ctx.infos = plan, infos
         x1, x2, w = _dense(input1, input2, weight)
-        return _uvw.uvw_contract(plan, (None, x1, x2), w, (_uvw.FORWARD,))[0]
+        return _uvw.uvw_contract(plan, (None, x1, x2), w, (_uvw.FORWARD,), UVW_INTERMEDIATE_LIMIT)[0]
 
     @staticmethod
     def backward(ctx, grad):
@@ -116,7 +117,7 @@ class TensorProductUVW(Function):
             x1, x2, w, g = _dense(input1, input2, weight, grad)
             if all(t is None or t.data_ptr() % 16 == 0 for t in (x1, x2, w, g)):
                 roles = tuple(r for r, n in zip((_uvw.GRAD_1, _uvw.GRAD_2), need) if n)
-                grads = iter(_uvw.uvw_contract(ctx.plan, (g, x1, x2), w, roles) if roles else ())
+                grads = iter(_uvw.uvw_contract(ctx.plan, (g, x1, x2), w, roles, UVW_INTERMEDIATE_LIMIT) if roles else ())
                 gw = _uvw.uvw_wgrad(ctx.plan, x1, x2, g) if need[2] else None
                 return next(grads) if need[0] else None, next(grads) if need[1] else None, gw, None, None
         r1, r2 = _rot(ctx.infos)
@@ -131,8 +132,8 @@ class TensorProductUVW(Function):
         return g1, g2, gw, None, None
 
 
-#: largest per-call intermediate (N, num_Mij, C1, C2) of the 'uvw' product in bytes; larger batches are processed in
-#: slices of samples whose intermediate stays below it
+#: largest per-call intermediate (N, num_Mij, C1, C2) of the 'uvw' product, or scratch of the kernels without one, in bytes; larger
+#: batches are processed in slices of samples that stay below it
 UVW_INTERMEDIATE_LIMIT = 1 << 30
 
 

@@ -18,6 +18,7 @@ _PATH = np.dtype([("l_o", "<i4"), ("l_s", "<i4"), ("l_f", "<i4"), ("offset_o", "
                   ("weight", "<i4"), ("scale", "<f4")])
 # operands of the layer (0 = output, 1 = first, 2 = second operand) in the places (out, s, f) of a role
 FORWARD, GRAD_1, GRAD_2 = (0, 1, 2), (1, 2, 0), (2, 1, 0)
+_TILE = 128              # samples of a CTA
 
 
 def exchanged_scale(degrees: Sequence[int], role: Tuple[int, int, int]) -> float:
@@ -93,9 +94,11 @@ class UvwPlan:
         return self._fits.get(key, False) and (x1.data_ptr() | x2.data_ptr() | w.data_ptr()) % 16 == 0
 
 
-def uvw_contract(plan: UvwPlan, operands: Sequence[Optional[Tensor]], w: Tensor, roles) -> list:
+def uvw_contract(plan: UvwPlan, operands: Sequence[Optional[Tensor]], w: Tensor, roles, limit: int) -> list:
     """The products of ``roles`` (at most two; both run in one launch where their outputs have equally many channels and one
-    launch has room for them), from contiguous ``operands`` = (gradient of the output, first, second operand) and the weights."""
+    launch has room for them), from contiguous ``operands`` = (gradient of the output, first, second operand) and the weights.
+    Partial outputs and transposed operands take some 12 to 60 KB a sample; batches whose scratch would exceed ``limit`` bytes run in
+    slices of whole sample tiles."""
     n = next(t for t in operands if t is not None).shape[0]
     channels = (w.shape[3], w.shape[1], w.shape[2])
     structs, lib, dev = plan.structs(channels, roles), _lib.lib(), w.device
@@ -103,13 +106,18 @@ def uvw_contract(plan: UvwPlan, operands: Sequence[Optional[Tensor]], w: Tensor,
         together = len(roles) == 1 or channels[roles[0][0]] == channels[roles[1][0]]
         floats = int(lib.eqt_uvw_scratch_floats(structs, len(roles), n)) if together else -1
         if floats < 0 and len(roles) == 2:
-            return [uvw_contract(plan, operands, w, (r,))[0] for r in roles]
+            return [uvw_contract(plan, operands, w, (r,), limit)[0] for r in roles]
         outs = [w.new_empty(n, plan.dims[r[0]], channels[r[0]]) for r in roles]
-        pointers = [(C.c_void_p * len(roles))(*ptrs) for ptrs in ([operands[r[1]].data_ptr() for r in roles],
-                                                                 [operands[r[2]].data_ptr() for r in roles], [t.data_ptr() for t in outs])]
+        step = n
+        if 4 * floats > limit:
+            step = min(n, max(_TILE, n // -(-4 * floats // limit) // _TILE * _TILE))
+            floats = max(int(lib.eqt_uvw_scratch_floats(structs, len(roles), m)) for m in (step, (n - 1) % step + 1))
         scratch = torch.empty(max(floats, 0), dtype=torch.float32, device=dev)        # of this call: calls on other streams may overlap it
-        _lib.check(lib.eqt_uvw_contract(structs, len(roles), *pointers, w.data_ptr(), scratch.data_ptr(), floats, n,
-                                        status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_uvw_contract")
+        for a in range(0, n, step):
+            pointers = [(C.c_void_p * len(roles))(*(t[a:].data_ptr() for t in ts)) for ts in (
+                [operands[r[1]] for r in roles], [operands[r[2]] for r in roles], outs)]
+            _lib.check(lib.eqt_uvw_contract(structs, len(roles), *pointers, w.data_ptr(), scratch.data_ptr(), floats, min(step, n - a),
+                                            status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_uvw_contract")
     return outs
 
 

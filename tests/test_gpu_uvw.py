@@ -8,6 +8,7 @@ import torch
 
 from equitorch_b200 import nn as enn
 from equitorch_b200.constants import so3_clebsch_gordan
+from equitorch_b200.nn.functional import tensor_products as ftp
 from equitorch_b200.nn.functional.tensor_products import TensorProductUVW, tensor_product_uvw
 from equitorch_b200.ops.uvw_op import FORWARD, GRAD_1, GRAD_2, exchanged_scale
 from oracle import tensor_products as otp
@@ -92,3 +93,39 @@ def test_second_derivatives_are_those_of_the_composed_product():
         results.append([*first, *torch.autograd.grad(sum(t.square().sum() for t in first), leaves)])
     for a, b in zip(*results):
         assert _rel(a, b.cpu()) < 1e-5
+
+
+def _peak(call):
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    base = torch.cuda.memory_allocated()
+    result = call()
+    torch.cuda.synchronize()
+    return torch.cuda.max_memory_allocated() - base - sum(t.numel() * 4 for t in result), result
+
+
+@pytest.mark.gpu
+def test_scratch_stays_below_the_limit(monkeypatch):
+    """Batches whose partial outputs would exceed the limit run in slices of whole sample tiles: forward and backward below it (the packed
+    weights and the copies of the operands' gradients beside it), results as close to float64 as those of one call."""
+    g = torch.Generator(device=DEV).manual_seed(7)
+    ir, c, n = "2x0e+2x1o+2x2e", 16, 5003
+    layer = enn.TensorProduct(ir, ir, ir, c, c, c, internal_weights=False, feature_mode="uvw").to(DEV)
+    x1, x2, cot = (torch.randn(n, 18, c, generator=g, device=DEV) for _ in range(3))
+    w = torch.randn(*layer.weight_shape, generator=g, device=DEV)
+    leaves = [t.requires_grad_(True) for t in (x1, x2, w)]
+
+    def call():
+        out = layer(*leaves)
+        return [out, *torch.autograd.grad(out, leaves, cot)]
+    whole_peak, _ = _peak(call)
+    limit = 16 << 20
+    monkeypatch.setattr(ftp, "UVW_INTERMEDIATE_LIMIT", limit)
+    peak, got = _peak(call)
+    assert whole_peak > 2 * limit and peak < 1.5 * limit
+    ref = [t.detach().double().requires_grad_(True) for t in leaves]
+    want = [otp.tensor_product_dense(*ref, layer.irreps_in1, layer.irreps_in2, layer.irreps_out, feature_mode="uvw")]
+    want += torch.autograd.grad(want[0], ref, cot.double())
+    for a, b in zip(got, want):
+        assert _rel(a, b.cpu()) < 2.5e-7
+
