@@ -114,22 +114,44 @@ class TensorProductUVW(Function):
         input1, input2, weight = ctx.saved_tensors
         need = ctx.needs_input_grad[:3]
         if not torch.is_grad_enabled():
-            x1, x2, w, g = _dense(input1, input2, weight, grad)
-            if all(t is None or t.data_ptr() % 16 == 0 for t in (x1, x2, w, g)):
-                roles = tuple(r for r, n in zip((_uvw.GRAD_1, _uvw.GRAD_2), need) if n)
-                grads = iter(_uvw.uvw_contract(ctx.plan, (g, x1, x2), w, roles, UVW_INTERMEDIATE_LIMIT) if roles else ())
-                gw = _uvw.uvw_wgrad(ctx.plan, x1, x2, g) if need[2] else None
-                return next(grads) if need[0] else None, next(grads) if need[1] else None, gw, None, None
+            # the kernels read 16 bytes at a time: a gradient (or an operand that a hook brought back) elsewhere is copied
+            x1, x2, w, g = (t if t is None or t.data_ptr() % 16 == 0 else t.clone() for t in _dense(input1, input2, weight, grad))
+            roles = tuple(r for r, n in zip((_uvw.GRAD_1, _uvw.GRAD_2), need) if n)
+            grads = iter(_uvw.uvw_contract(ctx.plan, (g, x1, x2), w, roles, UVW_INTERMEDIATE_LIMIT) if roles else ())
+            gw = _uvw.uvw_wgrad(ctx.plan, x1, x2, g) if need[2] else None
+            return next(grads) if need[0] else None, next(grads) if need[1] else None, gw, None, None
         r1, r2 = _rot(ctx.infos)
         g1 = tensor_product_uvw(input2, grad, weight.permute(0, 2, 3, 1).contiguous(), *r1) if need[0] else None
         g2 = tensor_product_uvw(grad, input1, weight.permute(0, 3, 1, 2).contiguous(), *r2) if need[1] else None
-        gw = None
-        if need[2]:
-            f = ctx.infos[0]
-            inter = sparse_outer(input1, input2, *_mij(f, 0))
-            gw = sparse_outer(grad, inter.flatten(-2), *_m(f, 2), out_accumulated=True)
-            gw = gw.transpose(-1, -2).contiguous().unflatten(-2, inter.shape[-2:])
+        gw = TensorProductUVWWeight.apply(input1, input2, grad, ctx.infos) if need[2] else None
         return g1, g2, gw, None, None
+
+
+class TensorProductUVWWeight(Function):
+    """Gradient of :func:`tensor_product_uvw` with respect to weights shared by the batch, slice by slice over the samples.  It is
+    linear in each operand: its own derivatives are the product and its operand gradients with the cotangent as the weights."""
+
+    @staticmethod
+    def forward(ctx, input1, input2, grad, infos):
+        ctx.save_for_backward(input1, input2, grad)
+        ctx.infos = infos
+        f, gw = infos[0], None
+        step = _uvw_slice(input1, input2, f) or max(1, input1.shape[0])
+        for s in range(0, max(1, input1.shape[0]), step):
+            inter = sparse_outer(input1[s:s + step], input2[s:s + step], *_mij(f, 0))
+            part = sparse_outer(grad[s:s + step], inter.flatten(-2), *_m(f, 2), out_accumulated=True)
+            gw = part if gw is None else gw.add_(part)
+        return gw.transpose(-1, -2).contiguous().unflatten(-2, inter.shape[-2:])
+
+    @staticmethod
+    def backward(ctx, cotangent):
+        input1, input2, grad = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        r1, r2 = _rot(ctx.infos)
+        g1 = tensor_product_uvw(input2, grad, cotangent.permute(0, 2, 3, 1).contiguous(), *r1) if need[0] else None
+        g2 = tensor_product_uvw(grad, input1, cotangent.permute(0, 3, 1, 2).contiguous(), *r2) if need[1] else None
+        gg = tensor_product_uvw(input1, input2, cotangent.contiguous(), *ctx.infos) if need[2] else None
+        return g1, g2, gg, None
 
 
 #: largest per-call intermediate (N, num_Mij, C1, C2) of the 'uvw' product, or scratch of the kernels without one, in bytes; larger
@@ -184,13 +206,19 @@ class TensorProductUVWChunked(Function):
         return g1, g2, gw, None, None, None, None
 
 
+def _uvw_slice(input1, input2, info):
+    """Samples of a slice whose intermediate stays below the limit, ``None`` where the whole batch's does."""
+    per_sample = info.info_Mij_fwd.out_size * input1.shape[-1] * input2.shape[-1] * input1.element_size()
+    if per_sample * input1.shape[0] <= UVW_INTERMEDIATE_LIMIT:
+        return None
+    chunk = max(1, UVW_INTERMEDIATE_LIMIT // per_sample)
+    return chunk // 512 * 512 if chunk >= 512 else chunk           # whole tiles for the tensor-core paths
+
+
 def tensor_product_uvw(input1, input2, weight, tp_info_forward, tp_info_backward1=None, tp_info_backward2=None):
     if weight.ndim == 4 and input1.ndim == 3 and input2.ndim == 3 and input1.shape[0] == input2.shape[0]:
-        per_sample = (tp_info_forward.info_Mij_fwd.out_size * input1.shape[-1] * input2.shape[-1] * input1.element_size())
-        if per_sample * input1.shape[0] > UVW_INTERMEDIATE_LIMIT:
-            chunk = max(1, UVW_INTERMEDIATE_LIMIT // per_sample)
-            if chunk >= 512:
-                chunk = chunk // 512 * 512           # whole tiles for the tensor-core paths
+        chunk = _uvw_slice(input1, input2, tp_info_forward)
+        if chunk is not None:
             return TensorProductUVWChunked.apply(input1, input2, weight, tp_info_forward, tp_info_backward1,
                                                  tp_info_backward2, chunk)
     return TensorProductUVWDummy.apply(input1, input2, weight, tp_info_forward, tp_info_backward1, tp_info_backward2)[0]

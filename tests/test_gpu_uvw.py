@@ -129,3 +129,33 @@ def test_scratch_stays_below_the_limit(monkeypatch):
     for a, b in zip(got, want):
         assert _rel(a, b.cpu()) < 2.5e-7
 
+
+@pytest.mark.gpu
+def test_differentiable_weight_gradient_stays_below_the_limit(monkeypatch):
+    """A weight gradient that is to be differentiated again keeps no intermediate of the whole batch, and its derivatives are those of
+    the product; a gradient that does not lie on 16 bytes takes the same kernels as one that does."""
+    g = torch.Generator(device=DEV).manual_seed(9)
+    ir, c, n = "0e+1o+2e", 16, 4000
+    layer = enn.TensorProduct(ir, ir, ir, c, c, c, internal_weights=False, feature_mode="uvw").to(DEV)
+    leaves = [torch.randn(*s, generator=g, device=DEV).requires_grad_(True) for s in ((n, 9, c), (n, 9, c), layer.weight_shape)]
+    cot, v = torch.randn(n, 9, c, generator=g, device=DEV).requires_grad_(True), torch.randn(*layer.weight_shape, generator=g, device=DEV)
+    out = layer(*leaves)
+
+    def call():
+        return list(torch.autograd.grad(out, leaves[2:], cot, create_graph=True, retain_graph=True))
+    limit = 16 << 20                                        # the intermediate of the whole batch: 143 MB
+    monkeypatch.setattr(ftp, "UVW_INTERMEDIATE_LIMIT", limit)
+    peak, (gw,) = _peak(call)
+    assert peak < 3 * limit
+    got = [gw, *torch.autograd.grad(gw, [leaves[0], leaves[1], cot], v)]
+    ref = [t.detach().double().requires_grad_(True) for t in (*leaves, cot)]
+    dense = otp.tensor_product_dense(*ref[:3], layer.irreps_in1, layer.irreps_in2, layer.irreps_out, feature_mode="uvw")
+    (want,) = torch.autograd.grad(dense, ref[2:3], ref[3], create_graph=True)
+    for a, b in zip(got, [want, *torch.autograd.grad(want, [ref[0], ref[1], ref[3]], v.double())]):
+        assert _rel(a, b.cpu()) < 3e-6                     # sums of 256 terms and of 4000 samples in two steps
+
+    shifted = torch.empty(n * 9 * c + 1, device=DEV)[1:].view(n, 9, c).copy_(cot.detach())
+    assert shifted.data_ptr() % 16 == 4
+    for a, b in zip(torch.autograd.grad(out, leaves, shifted, retain_graph=True), torch.autograd.grad(out, leaves, cot.detach())):
+        assert torch.equal(a, b)
+
