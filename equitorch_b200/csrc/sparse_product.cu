@@ -783,6 +783,10 @@ extern "C" int eqt_sparse_product(const eqt_product_args* a, void* stream) {
   const bool empty = a->n == 0 || a->num_out == 0;
   if (!empty && (!a->in1 || !a->out || (a->op != EQT_OP_SCALE && !a->in2)))
     return fail(EQT_ERR_BAD_ARGUMENT, "NULL operand");
+  if (!a->index_out && a->num_out > a->out_size) return fail(EQT_ERR_BAD_ARGUMENT, "more rows than the output has");
+  if (!a->seg && !a->gather_index &&
+      ((!a->index1 && a->num_out > a->rows1) || (a->op != EQT_OP_SCALE && !a->index2 && a->num_out > a->rows2)))
+    return fail(EQT_ERR_BAD_ARGUMENT, "more entries than an operand without an index has rows");
   if (a->op == EQT_OP_SCALE && a->accumulated == 0 && a->shared1)
     return fail(EQT_ERR_BAD_ARGUMENT, "scale-segment needs a batched input");
   P p;

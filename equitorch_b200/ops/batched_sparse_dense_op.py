@@ -108,7 +108,14 @@ def sparse_product(op: int, input1: Tensor, input2: Optional[Tensor], scale=None
     elif index2 is not None:
         num_out = index2.shape[0]
     else:
-        num_out = rows1
+        # identity tables: the entries that both operands, the scale and the output have a row for (operands may have rows
+        # behind the last entry, which none reads)
+        named = [t.shape[0] for t in (scale, gather_index, index_out) if t is not None]
+        if index_out is None and out_size is not None:
+            named.append(out_size)
+        if not named and op != _lib.OP_SCALE and rows1 != rows2:
+            raise ValueError(f"operands of {rows1} and {rows2} rows, and nothing says which belong together")
+        num_out = min(rows1, *([] if op == _lib.OP_SCALE else [rows2]), *named)
     if out_size is None:
         out_size = num_out
 

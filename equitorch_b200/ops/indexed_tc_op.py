@@ -107,9 +107,9 @@ def vecmat_supported(x: Tensor, w: Tensor, gather_index, index_out, out_accumula
             and x.data_ptr() % 16 == 0)
 
 
-def _entries(index1, index2, seg, rows1: int) -> int:
+def _entries(index1, index2, seg, num_out: int) -> int:
     return (index1.shape[0] if index1 is not None else index2.shape[0] if index2 is not None
-            else rows1 if seg is None else -1)          # -1: as many as the last segment ends at, read with the plan
+            else num_out if seg is None else -1)          # -1: as many as the last segment ends at, read with the plan
 
 
 def vecmat_tc(x: Tensor, w: Tensor, scale, index1, index2, seg, num_out: int) -> Optional[Tensor]:
@@ -117,7 +117,7 @@ def vecmat_tc(x: Tensor, w: Tensor, scale, index1, index2, seg, num_out: int) ->
     dev = x.device
     n, rows1, cin = x.shape
     cout = w.shape[2]
-    entries = _entries(index1, index2, seg, rows1)
+    entries = _entries(index1, index2, seg, num_out)
     plan = _cached("vecmat", dev, (index1, seg), (entries, num_out, cin, cout),
                    lambda: VecmatPlan(index1, seg, entries, num_out, cin, cout, dev))
     if plan is None:
@@ -205,7 +205,7 @@ def outer_tc(a: Tensor, b: Tensor, scale, index1, index2, seg, num_w: int) -> Op
     dev = a.device
     n, rows1, c1 = a.shape
     rows2, c2 = b.shape[1], b.shape[2]
-    entries = _entries(index1, index2, seg, rows1)
+    entries = _entries(index1, index2, seg, num_w)
     plan = _cached("outer", dev, (scale, index1, index2, seg), (entries, num_w, c1, c2),
                    lambda: OuterPlan(scale, index1, index2, seg, entries, num_w, c1, c2, dev))
     if plan is None:

@@ -54,3 +54,17 @@ def test_cpu_tensors_are_rejected_loudly():
 def _import_error():
     from equitorch_b200._lib import EqtError
     return EqtError
+
+
+@pytest.mark.parametrize("sizes", [dict(num_out=16, out_size=1), dict(rows1=3, num_out=4, out_size=4), dict(rows2=1, num_out=2, out_size=2)])
+def test_sparse_product_refuses_more_entries_than_rows(sizes):
+    """Tables without an index: an entry is a row of both operands and of the output, and a row that one of them lacks is refused
+    before anything is launched."""
+    import torch
+
+    from equitorch_b200 import _lib
+    buffer = (ctypes.c_float * 64)()
+    at = ctypes.addressof(buffer)
+    args = dict(op=_lib.OP_OUTER, dtype=_lib.DTYPE_CODE[torch.float32], in1=at, in2=at, out=at, n=1, rows1=16, rows2=16, num_out=1, out_size=1, c1=1, c2=1)
+    rc = _lib.lib().eqt_sparse_product(ctypes.byref(_lib.ProductArgs(**{**args, **sizes})), None)
+    assert rc != 0 and b"rows" in _lib.lib().eqt_last_error()

@@ -140,3 +140,51 @@ def test_segment_sum_gradient(use_perm):
     torch.testing.assert_close(out.double().cpu(), want.detach(), rtol=1e-5, atol=1e-5)
     (gr,) = torch.autograd.grad(want, xr, cot.double())
     torch.testing.assert_close(gx.double().cpu(), gr, rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("n", [5, 700])
+@pytest.mark.parametrize("op", ["mul", "outer", "inner", "vecmat", "vecsca", "scale"])
+def test_identity_tables_with_operand_rows_that_no_entry_reads(op, n):
+    """No index at all: the entries are those that the output (or the scale) names, whatever rows the operands have behind them."""
+    g = torch.Generator().manual_seed(n)
+    rows, entries, c = 7, 3, 32
+    x = torch.randn(n, rows, c, generator=g)
+    y = {"mul": (n, entries, c), "outer": (n, entries, c), "inner": (n, rows, c), "vecmat": (entries, c, c), "vecsca": (n, 5)}.get(op)
+    y = None if y is None else torch.randn(*y, generator=g)
+    scale = torch.randn(entries, generator=g)
+    index = torch.arange(entries)
+    if op == "scale":
+        got = gops.sparse_product(gops._lib.OP_SCALE, x.to(DEV), None, scale.to(DEV))
+        want = x[:, :entries] * scale.view(1, -1, 1)
+    else:
+        got = getattr(gops, f"indexed_{op}_scale_gather")(x.to(DEV), y.to(DEV), scale.to(DEV), out_size=entries)
+        want = getattr(oops, f"indexed_{op}_scale_gather")(x.double(), y.double(), scale.double(), index, index)
+    assert got.shape == want.shape
+    torch.testing.assert_close(got.double().cpu(), want.double(), rtol=1e-5, atol=1e-4)
+    if y is not None and y.shape[0] == n and op != "inner":
+        with pytest.raises(ValueError, match="nothing says"):
+            getattr(gops, f"indexed_{op}_scale_gather")(x.to(DEV), y.to(DEV))
+
+
+@pytest.mark.parametrize("n", [40, 600])
+@pytest.mark.parametrize("mode,ir2,c", [("uvw", "0e", 16), ("uvw", "0e", 32), ("uuu", "0e", 16), ("uu", "0e", 32), ("uv", "0e", 32)])
+def test_layers_of_one_path_between_first_irreps(mode, ir2, c, n):
+    """One path between the first irreps of operands that have more of them: all tables of the forward product are identities."""
+    from equitorch_b200 import nn as enn
+    from oracle import tensor_products as otp
+    g = torch.Generator().manual_seed(c + n)
+    ir1 = "0e+1o+2e+3o"
+    kind = enn.TensorProduct if mode in ("uvw", "uuu") else enn.SO3Linear
+    channels = (c, c, c) if kind is enn.TensorProduct else (c, c)
+    layer = kind(ir1, ir2, "0e", *channels, internal_weights=False, feature_mode=mode).to(DEV)
+    x, w = torch.randn(n, 16, c, generator=g), torch.randn(*layer.weight_shape, generator=g) / c
+    y = torch.randn(n, 1, c, generator=g) if kind is enn.TensorProduct else torch.randn(n, 1, generator=g)
+    cot = torch.randn(n, 1, c, generator=g)
+    leaves = [t.to(DEV).requires_grad_(True) for t in (x, y, w)]
+    out = layer(*leaves)
+    ref = [t.double().requires_grad_(True) for t in (x, y, w)]
+    dense = otp.tensor_product_dense if kind is enn.TensorProduct else otp.so3_linear_dense
+    want = dense(*ref, ir1, ir2, "0e", feature_mode=mode)
+    for a, b in zip([out, *torch.autograd.grad(out, leaves, cot.to(DEV))], [want, *torch.autograd.grad(want, ref, cot.double())]):
+        assert a.shape == b.shape and float((a.double().cpu() - b).abs().max() / b.abs().max()) < 1e-5
+
