@@ -70,6 +70,7 @@ class UvwPlan:
         for n, r in enumerate(self.roles.values()):
             r.data_ptr = self.blob.data_ptr() + n * self.num_paths * _PATH.itemsize
         self._structs, self._fits = {}, {}
+        status_flag(self.device)          # now: a call under capture would take it from the graph's memory
 
     def structs(self, channels: Tuple[int, int, int], roles):
         key = (channels, roles)

@@ -137,3 +137,12 @@ def test_what_is_not_finite_stays_so(value, n):
         bad = set(torch.nonzero(~torch.isfinite(t).flatten(1).all(1)).flatten().tolist())
         assert bad == rows
     assert not torch.isfinite(gw).all()
+
+
+def test_a_plan_brings_its_flag(monkeypatch):
+    """The status flag outlives a captured graph, so it must not be made by a call inside one: the plan has it made."""
+    from equitorch_b200.ops import fused_tp_op
+    monkeypatch.setattr(fused_tp_op, "_status", {})
+    layer = _layer(c=16)
+    assert layer._path_plan(torch.device(DEV)).usable and torch.device(DEV) in fused_tp_op._status
+
