@@ -70,13 +70,6 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr) {
   return (uint64_t)((smem_byte_addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// MN-major, 128-byte swizzle with 32-byte atoms (layout type 1, the only swizzled layout tcgen05 takes
-// for 32-bit MN-major operands): 32 floats of M/N per 128-byte row, 4 reduction rows per 512-byte
-// group (stride byte offset), the next 32 floats of M/N `lbo` bytes further.
-__device__ __forceinline__ uint64_t umma_desc_mn32(uint32_t smem_byte_addr, uint32_t lbo_bytes) {
-  return (uint64_t)((smem_byte_addr & 0x3FFFF) >> 4) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16) |
-         ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)1 << 61);
-}
 // kind::tf32, D = f32, A and B K-major, M = 128, N = n
 __host__ __device__ inline uint32_t umma_idesc_tf32(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
@@ -111,7 +104,9 @@ __device__ __forceinline__ void umma_tf32_ta_lo(uint32_t d_tmem, uint32_t a_tmem
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], b, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI) : "memory");
 }
-// operands MN-major with 32-byte atoms (umma_desc_mn32): the low words carry the leading byte offset
+// Operands MN-major, 128-byte swizzle with 32-byte atoms (layout type 1, the only swizzled layout tcgen05 takes for 32-bit MN-major
+// operands): 32 floats of M/N per 128-byte row, 4 reduction rows per 512-byte group (stride byte offset), the next 32 floats of M/N
+// `lbo` bytes further.  The low words carry the leading byte offset.
 constexpr uint32_t UMMA_DESC_MN32_HI = (512 >> 4) | (1u << 14) | (1u << 29);
 __device__ __forceinline__ uint32_t umma_lo_mn32(uint32_t smem_byte_addr, uint32_t lbo_bytes) {
   return ((smem_byte_addr & 0x3FFFF) >> 4) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
