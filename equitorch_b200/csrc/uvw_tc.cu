@@ -1122,45 +1122,48 @@ __global__ void __launch_bounds__(1024) uvw_wgrad_sum_kernel(const __grid_consta
 bool wgrad_f32(const eqt_uvw_role& r, int64_t n) { return n < 512 || r.cj == 16 || r.ck == 16; }
 
 // The line of (path, channel group, chunk), cut into ranges of equal cost.  Cost of a chunk: instructions of a thread that makes rows.
+// Returns the number of pieces, or (without L) the most that there can be.
 int cut_wgrad(const eqt_uvw_role& r, const int32_t* degrees, int64_t n, WLaunch* L, WSumLaunch* S, int* ctas) {
   const bool f32 = wgrad_f32(r, n);
   const int64_t chunks = ceil_div(n, f32 ? F_CHUNK : CHUNK);
   const int groups = r.ci * r.cj / COLS, units = r.num_paths * groups;
   if (chunks > 0x7fffffff || units + std::min<int64_t>(sm_count(), units * ceil_div(n, CHUNK)) > MAX_UNITS) return -1;
+  const int want = (int)std::min<int64_t>(std::min(sm_count() * (f32 ? f_ctas(r.ck) : 1), MAX_PIECES - units), units * chunks);
+  if (!L) return units + want;
   auto cost = [&](int q) {
     const int no = 2 * degrees[3 * q] + 1, ns = 2 * degrees[3 * q + 1] + 1, nf = 2 * degrees[3 * q + 2] + 1;
     return (int64_t)(f32 ? 8 * no * ns + 2 * (no + ns) + nf * (6 * r.ck / 4 + 4) : 16 + 20 * nf + 6 * no * ns);
   };
   int64_t total = 0;
   for (int q = 0; q < r.num_paths; ++q) total += cost(q) * groups * chunks;
-  const int want = (int)std::min<int64_t>(std::min(sm_count() * (f32 ? f_ctas(r.ck) : 1), MAX_PIECES - units), units * chunks);
+  // the current CTA ends where its share of the total does (steps of total / want without a division each); the last one takes what is left
+  const int64_t share = total / want, rest = total % want;
+  int64_t end = share, carry = rest, before = 0;       // before: cost of the units before the current one
   int pieces = 0, cta = 0;
-  int64_t before = 0;                      // cost of the units before the current one
-  if (L) L->cta[0] = 0;
+  L->cta[0] = 0;
   for (int u = 0; u < units; ++u) {
-    if (S) S->first[u] = (short)pieces;
+    S->first[u] = (short)pieces;
     const int64_t c = cost(u / groups);
-    int64_t at = 0;
-    while (at < chunks) {
-      // the current CTA ends where its share of the total does; the last one takes what is left
-      const bool last = cta + 1 >= want;
-      const int64_t end = last ? total : total / want * (cta + 1) + total % want * (cta + 1) / want;
-      const int64_t upto = last ? chunks : std::min(chunks, (end - before + c / 2) / c);
+    for (int64_t at = 0; at < chunks;) {
+      const int64_t upto = cta + 1 >= want ? chunks : std::min(chunks, (end - before + c / 2) / c);
       if (upto <= at) {                    // nothing of this unit fits the current CTA any more
-        if (L) L->cta[cta + 1] = (short)pieces;
-        ++cta;
+        L->cta[++cta] = (short)pieces;
+        end += share;
+        carry += rest;
+        if (carry >= want) {
+          carry -= want;
+          ++end;
+        }
         continue;
       }
-      if (L) L->piece[pieces] = WPiece{u, (int)at, (int)upto};
-      ++pieces;
+      L->piece[pieces++] = WPiece{u, (int)at, (int)upto};
       at = upto;
     }
     before += c * chunks;
   }
-  if (S) S->first[units] = (short)pieces;
-  for (; cta < want; ++cta)
-    if (L) L->cta[cta + 1] = (short)pieces;
-  if (ctas) *ctas = want;
+  S->first[units] = (short)pieces;
+  while (cta < want) L->cta[++cta] = (short)pieces;
+  *ctas = want;
   return pieces;
 }
 

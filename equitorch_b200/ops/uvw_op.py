@@ -115,7 +115,7 @@ def uvw_contract(plan: UvwPlan, operands: Sequence[Optional[Tensor]], w: Tensor,
             floats = max(int(lib.eqt_uvw_scratch_floats(structs, len(roles), m)) for m in (step, (n - 1) % step + 1))
         scratch = torch.empty(max(floats, 0), dtype=torch.float32, device=dev)        # of this call: calls on other streams may overlap it
         for a in range(0, n, step):
-            pointers = [(C.c_void_p * len(roles))(*(t[a:].data_ptr() for t in ts)) for ts in (
+            pointers = [(C.c_void_p * len(roles))(*(t.data_ptr() + 4 * a * t.shape[1] * t.shape[2] for t in ts)) for ts in (
                 [operands[r[1]] for r in roles], [operands[r[2]] for r in roles], outs)]
             _lib.check(lib.eqt_uvw_contract(structs, len(roles), *pointers, w.data_ptr(), scratch.data_ptr(), floats, min(step, n - a),
                                             status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_uvw_contract")
