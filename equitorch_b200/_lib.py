@@ -104,6 +104,11 @@ SIGNATURES = {
                                         C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]),
     "eqt_tp_cg_inner": (C.c_int, [C.POINTER(TpTableStruct), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                   C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]),
+    "eqt_tp_cg_mix_scratch_floats": (C.c_int64, [C.c_uint64, C.c_int64, C.c_int32]),
+    "eqt_tp_cg_segment_mix": (C.c_int, [C.POINTER(TpTableStruct), C.c_uint64, *[C.c_void_p] * 10, C.c_int64, C.c_int64, C.c_int64,
+                                        C.c_int32, C.c_void_p]),
+    "eqt_tp_cg_inner_mix": (C.c_int, [C.POINTER(TpTableStruct), C.c_uint64, *[C.c_void_p] * 7, C.c_int64, C.c_int64, C.c_int32,
+                                      C.c_void_p]),
     "eqt_mix_tc": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_int32,
                              C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]),
     "eqt_mix_tc_transposed": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,

@@ -43,7 +43,8 @@ def _stale() -> bool:
     if not os.path.exists(LIB_PATH) or not os.path.exists(os.path.join(HERE, "generated", "tp_specs.inc")) \
             or not os.path.exists(os.path.join(HERE, "generated", "sh_specs.inc")) \
             or not os.path.exists(os.path.join(HERE, "generated", "path_specs.inc")) \
-            or not os.path.exists(os.path.join(HERE, "generated", "triple_specs.inc")):
+            or not os.path.exists(os.path.join(HERE, "generated", "triple_specs.inc")) \
+            or not os.path.exists(os.path.join(HERE, "generated", "walk_specs.inc")):
         return True
     built = os.path.getmtime(LIB_PATH)
     deps = sources() + glob.glob(os.path.join(HERE, "*.cuh")) + glob.glob(os.path.join(HERE, "*.inc")) + glob.glob(os.path.join(HERE, "*.py")) \
@@ -58,7 +59,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     from .gen_path_specs import generate as generate_paths, generate_triples
     from .gen_sh_specs import generate as generate_sh
     from .gen_tp_specs import generate
+    from .gen_walk_specs import generate as generate_walks
     generate()
+    generate_walks()
     generate_sh()
     generate_paths()
     generate_triples()

@@ -24,13 +24,15 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(HERE, "generated", "tp_specs.inc")
 
-# (irreps_out, irreps_in1, irreps_in2) of layers whose inner loops are unrolled at build time.
-# All role rotations (forward, gradient w.r.t. input1, gradient w.r.t. input2) are generated.
+# (irreps_out, irreps_in1, irreps_in2) of layers whose inner loops are unrolled at build time, here and in gen_walk_specs.py.
+# All role rotations (forward, gradient w.r.t. input1, gradient w.r.t. input2) are generated.  The kernels of this module take those
+# whose cells do not fit one lane's registers (``FOUR_WARPS``); the others run on one warp a node.
 REGISTRY = [
     ("0e+1o", "0e+1o", "0e+1o"),
     ("0e+1o+2e", "0e+1o+2e", "0e+1o+2e"),
     ("0e+1o+2e+3o", "0e+1o+2e+3o", "0e+1o+2e+3o"),
 ]
+FOUR_WARPS = REGISTRY[2:]
 
 
 class Structure(NamedTuple):
@@ -353,7 +355,7 @@ def collect() -> List[tuple]:
     from ..irreps import Irreps
     from ..tables import tp_infos
     seen, specs = set(), []
-    for o, a, b in REGISTRY:
+    for o, a, b in FOUR_WARPS:
         io, i1, i2 = Irreps(o), Irreps(a), Irreps(b)
         fwd, bwd1, bwd2, _ = tp_infos(io, i1, i2)
         # forward: feat = input1 (index1), y = input2.  gradient of input1: table of backward1, whose

@@ -9,7 +9,7 @@
 // respect to the harmonics.
 //
 // Two implementations of each:
-//  * "spec": for index structures unrolled at build time (generated/tp_specs.inc).  The sum over
+//  * "spec": for index structures unrolled at build time (generated/tp_specs.inc: l_max 3).  The sum over
 //    the edges of a node commutes with the CG contraction, so per edge only the dense outer
 //    product Q[m_y, m_feat] += y_e[m_y] x_e[m_feat] is accumulated (234 of the 256 cells are used
 //    at l_max = 3) and the 353-entry sparse contraction runs once per node.  One CTA walks a
@@ -21,10 +21,12 @@
 //    atomics: the edges of a node are consecutive.  The adjoint runs the same scheme backwards:
 //    H[cell] = sum_t scale[t] G_d[row(t)] once per node, then a dense dot product per edge.
 //  * "generic": table-driven, one thread per output element; any structure, any channel count.
+// What one warp can hold of a node on its own is in tp_walk.cu; walk_wanted() below says which sizes that is.
 #include <algorithm>
 #include <cstdlib>
 
 #include "tc_common.cuh"
+#include "tp_walk.cuh"
 
 namespace eqt {
 namespace specs {
@@ -366,8 +368,7 @@ __global__ void __launch_bounds__(128 * CG, CG == 1 ? 3 : 1) tp_segsum_spec_kern
 
 // Sum each of the N per-lane values over the 32 lanes and store the N totals.  The butterfly takes the largest power of two
 // of them at once and halves the number of live values at every step while there is more than one (16 values: 8 + 4 + 2 + 1 + 1
-// shuffles instead of 80; 9: 4 + 2 + 1 + 1 + 1 for eight and 5 for the ninth instead of 45).  l_max 2, 128 channels, 110k
-// edges: the adjoint went 293 -> 229 us.
+// shuffles instead of 80).
 template <int N>
 __device__ __forceinline__ void warp_reduce_to_smem(const float* v, float* dst, int lane) {
   constexpr int M = N >= 16 ? 16 : N >= 8 ? 8 : N >= 4 ? 4 : N >= 2 ? 2 : 1;
@@ -864,6 +865,22 @@ inline bool segsum_tc_wanted(const FusedArgs& a) {
          (reinterpret_cast<uintptr_t>(a.out) & 15u) == 0;
 }
 
+// One warp per node and 32 lanes of channels (tp_walk.cu) instead of the four warps per node above.  At l_max 1 and 2 and at 16
+// channels always: both segment sums / the adjoint of 20k nodes and 400k edges, 128 channels, l_max 2 1162 -> 614 / 751 -> 466 us, l_max 1
+// 497 -> 178 / 326 -> 114 us; 16 channels, 4000 nodes, 80k edges, l_max 3 1750 -> 110 / 2362 -> 74 us (table-driven before); 400 nodes,
+// 6000 edges, 32 channels, l_max 2 20.2 -> 18.3 / 13.1 -> 14.9 us.  At l_max 3 a node takes a warp's time of 120 cells an edge, which only
+// many nodes hide: 32 channels 600 nodes 35 -> 34 / 22 -> 19, 1000 nodes 24.5 -> 27.3 / 15.2 -> 16.8, 3000 nodes 170 -> 141 / 113 ->
+// 87 us.  128 channels leave room for eight warps an SM: 3000 nodes 540 -> 446 / 325 -> 303, 40k nodes 1416 -> 1739 / 889 -> 936 us.  64
+// channels: the adjoint ties (1800 nodes 91.5 -> 91.8, 20k nodes 702 -> 711 us), segment sums of few edges a node 202 -> 159 us.
+inline bool walk_wanted(uint64_t key, bool inner, const FusedArgs& a) {
+  if (((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.g)) & 15u) != 0 || a.n_out >= 0x7fffffffll ||
+      !walk_supported(key, false, inner, a.C)) return false;
+  if (a.DF < 16 || a.C == 16) return true;
+  if (a.C == 32) return a.n_out >= 10 * (int64_t)sm_count();
+  if (a.C == 64) return !inner && !segsum_tc_wanted(a);
+  return a.C != 128 || a.n_out <= 100 * (int64_t)sm_count();
+}
+
 template <class S>
 bool try_spec(uint64_t key, bool inner, const FusedArgs& a, cudaStream_t s, int& rc) {
   if (key != S::KEY || a.T != S::T || a.R != S::R || a.DF != S::DF || a.DY != S::DY) return false;
@@ -886,6 +903,12 @@ int run(bool inner, const eqt_tp_table* tab, FusedArgs a, cudaStream_t s) {
     per = std::min<int64_t>(per, std::max<int64_t>(1, 256 / avg_deg));
     a.nodes_per_cta = (int)per;
     int rc = EQT_OK;
+    if (walk_wanted(tab->structure_key, inner, a)) {
+      WalkArgs w{};
+      w.feat = a.feat; w.fidx = a.fidx; w.y = a.y; w.yidx = a.yidx; w.ptr = a.ptr; w.scale = a.scale; w.g = a.g; w.out = a.out;
+      w.n_out = a.n_out; w.n_edges = a.n_edges; w.C = a.C;
+      return inner ? walk_inner(tab->structure_key, w, s) : walk_segment_sum(tab->structure_key, w, s);
+    }
 #define EQT_TRY(SPEC) if (try_spec<specs::SPEC>(tab->structure_key, inner, a, s, rc)) return rc;
     EQT_FOR_EACH_SPEC(EQT_TRY)
 #undef EQT_TRY
@@ -941,4 +964,48 @@ extern "C" int eqt_tp_cg_inner(const eqt_tp_table* table, const float* feat, con
   a.feat = feat; a.fidx = feat_index; a.g = g; a.ptr = seg_ptr; a.enode = edge_node; a.yidx = y_index; a.out = grad_y;
   a.n_out = num_nodes; a.n_edges = num_edges; a.C = channels; a.status = status;
   return run(true, table, a, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int64_t eqt_tp_cg_mix_scratch_floats(uint64_t mix_key, int64_t num_out, int32_t channels) {
+  return num_out < 0 ? -1 : eqt::walk_scratch_floats(mix_key, num_out, channels);
+}
+
+extern "C" int eqt_tp_cg_segment_mix(const eqt_tp_table* table, uint64_t mix_key, const float* feat, const int64_t* feat_index, const float* y,
+                                     const int64_t* y_index, const int64_t* seg_ptr, const float* weight, const float* x, float* out,
+                                     float* grad_weight, float* scratch, int64_t scratch_floats, int64_t num_out, int64_t num_edges,
+                                     int32_t channels, void* stream) {
+  using namespace eqt;
+  FusedArgs t{};
+  if (int rc = fill(table, t)) return rc;
+  if (num_out < 0 || num_edges < 0 || num_edges >= 0x7fffffffll || num_out >= 0x7fffffffll || channels <= 0)
+    return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
+  const int64_t need = walk_scratch_floats(mix_key, num_out, channels);
+  if (need < 0) return fail(EQT_ERR_UNSUPPORTED, "no straight-line code for this structure and %d channels", channels);
+  if (!weight || (num_out > 0 && (!feat || !out || !seg_ptr)) || (num_edges > 0 && !y) || !x != !grad_weight)
+    return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  if (x && (!scratch || scratch_floats < need)) return fail(EQT_ERR_BAD_ARGUMENT, "scratch of %lld floats, %lld needed", (long long)scratch_floats, (long long)need);
+  if (((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15u) != 0)
+    return fail(EQT_ERR_UNSUPPORTED, "operands must lie on 16 bytes");
+  WalkArgs w{};
+  w.feat = feat; w.fidx = feat_index; w.y = y; w.yidx = y_index; w.ptr = seg_ptr; w.scale = t.scale; w.w = weight; w.x = x; w.out = out;
+  w.gw = grad_weight; w.scratch = scratch; w.n_out = num_out; w.n_edges = num_edges; w.C = channels;
+  return walk_segment_sum(mix_key, w, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int eqt_tp_cg_inner_mix(const eqt_tp_table* table, uint64_t mix_key, const float* feat, const int64_t* feat_index, const float* g,
+                                   const float* weight, const int64_t* seg_ptr, const int64_t* y_index, float* grad_y, int64_t num_nodes,
+                                   int64_t num_edges, int32_t channels, void* stream) {
+  using namespace eqt;
+  FusedArgs t{};
+  if (int rc = fill(table, t)) return rc;
+  if (num_nodes < 0 || num_edges < 0 || num_edges >= 0x7fffffffll || num_nodes >= 0x7fffffffll || channels <= 0)
+    return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
+  if (!walk_supported(mix_key, true, true, channels)) return fail(EQT_ERR_UNSUPPORTED, "no straight-line code for this structure and %d channels", channels);
+  if (num_edges == 0 || num_nodes == 0) return EQT_OK;
+  if (!feat || !g || !weight || !seg_ptr || !grad_y) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
+  if (((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(g)) & 15u) != 0) return fail(EQT_ERR_UNSUPPORTED, "operands must lie on 16 bytes");
+  WalkArgs w{};
+  w.feat = feat; w.fidx = feat_index; w.ptr = seg_ptr; w.yidx = y_index; w.scale = t.scale; w.g = g; w.w = weight; w.out = grad_y;
+  w.n_out = num_nodes; w.n_edges = num_edges; w.C = channels;
+  return walk_inner(mix_key, w, static_cast<cudaStream_t>(stream));
 }

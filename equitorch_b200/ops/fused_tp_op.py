@@ -7,7 +7,7 @@ selects the kernels unrolled at build time when the index structure is one of th
 from __future__ import annotations
 
 import ctypes as C
-from typing import Dict, Optional
+from typing import Dict, Optional, Tuple
 
 import numpy as np
 import torch
@@ -15,7 +15,10 @@ from torch import Tensor
 
 from .. import _lib
 from ..csrc.gen_tp_specs import outer_order, structure_from_info, structure_key
+from ..csrc.gen_walk_specs import mix_key, row_map
 from ..structs import SparseProductInfo
+
+INNER_CHANNELS = (16, 32, 64, 128)        # of the straight-line adjoints; the segment sums: 16 and multiples of 32
 
 _status: Dict[torch.device, Tensor] = {}
 
@@ -41,10 +44,15 @@ def check_status(device=None) -> None:
 
 
 class TpTable:
-    """Device copy of one CG table plus the C struct that points at it."""
+    """Device copy of one CG table plus the C struct that points at it.  ``mix``: table of the weight step on its rows, for the
+    kernels that mix them channel by channel without writing them."""
 
-    def __init__(self, info: SparseProductInfo, feat_is_input1: bool, d_feat: int, d_y: int, device):
+    def __init__(self, info: SparseProductInfo, feat_is_input1: bool, d_feat: int, d_y: int, device,
+                 mix: Optional[SparseProductInfo] = None):
         s = structure_from_info(info, feat_is_input1, d_feat, d_y)
+        rows = row_map(mix) if mix is not None else None
+        self.mix_key = mix_key(s, rows)
+        self.mix_size = (int(rows.comp.max()) + 1, int(rows.path.max()) + 1) if self.mix_key else (0, 0)     # components, paths
         rowptr = np.searchsorted(s.row, np.arange(s.num_rows + 1)).astype(np.int64)
         self.key = structure_key(s)
         self.scale = info.scale.detach().to(device=device, dtype=torch.float32).contiguous()
@@ -98,4 +106,55 @@ def cg_inner(table: TpTable, feat: Tensor, g: Tensor, feat_index: Optional[Tenso
             C.byref(table.struct), feat.data_ptr(), _lib.ptr(feat_index), g.data_ptr(), seg_ptr.data_ptr(),
             edge_node.data_ptr(), _lib.ptr(y_index), out.data_ptr(), g.shape[0], n_edges, feat.shape[2],
             status_flag(dev).data_ptr(), _lib.stream_ptr(dev)), "eqt_tp_cg_inner")
+    return out
+
+
+def _f32_aligned(t: Tensor, what: str) -> Tensor:
+    t = _f32(t, what)
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def mix_scratch(table: TpTable, num_out: int, channels: int) -> int:
+    """Floats of scratch for :func:`cg_segment_mix` with ``x``; -1 where no kernel takes the table or the channels."""
+    return int(_lib.lib().eqt_tp_cg_mix_scratch_floats(table.mix_key, num_out, channels)) if table.mix_key else -1
+
+
+def cg_segment_mix(table: TpTable, feat: Tensor, y: Tensor, feat_index: Tensor, y_index: Optional[Tensor], seg_ptr: Tensor,
+                   num_out: int, weight: Tensor, x: Optional[Tensor] = None) -> Tuple[Tensor, Optional[Tensor]]:
+    """``out[d, k] = sum of weight[path(r)] S[d, r]`` over the rows r of component k of :func:`cg_segment_sum`, which are not
+    written; with ``x`` also ``grad_weight[p] = sum of x[d, k(r)] S[d, r]`` over the nodes and the rows of path p."""
+    dev = _lib.require_cuda(feat, y, feat_index, y_index, seg_ptr, weight, x)
+    feat, y, weight = _f32_aligned(feat, "feat"), _f32(y, "y"), _f32(weight, "weight")
+    comps, paths = table.mix_size
+    c = feat.shape[2]
+    assert feat.ndim == 3 and feat.shape[1] == table.d_feat and y.shape[-1] == table.d_y and weight.shape == (paths, c)
+    out = torch.empty(num_out, comps, c, dtype=torch.float32, device=dev)
+    gw = scratch = None
+    floats = 0
+    if x is not None:
+        x = _f32_aligned(x, "x")
+        assert x.shape == out.shape
+        floats = mix_scratch(table, num_out, c)
+        gw, scratch = torch.empty_like(weight), torch.empty(max(floats, 0), dtype=torch.float32, device=dev)
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().eqt_tp_cg_segment_mix(
+            C.byref(table.struct), table.mix_key, feat.data_ptr(), feat_index.data_ptr(), y.data_ptr(), _lib.ptr(y_index),
+            seg_ptr.data_ptr(), weight.data_ptr(), _lib.ptr(x), out.data_ptr(), _lib.ptr(gw), _lib.ptr(scratch), floats,
+            num_out, feat_index.numel(), c, _lib.stream_ptr(dev)), "eqt_tp_cg_segment_mix")
+    return out, gw
+
+
+def cg_inner_mix(table: TpTable, feat: Tensor, g: Tensor, weight: Tensor, feat_index: Tensor, seg_ptr: Tensor,
+                 y_index: Optional[Tensor], num_y_rows: int) -> Tensor:
+    """:func:`cg_inner` for ``g'[d, r] = weight[path(r)] g[d, k(r)]``, which is not written."""
+    dev = _lib.require_cuda(feat, g, weight, feat_index, seg_ptr, y_index)
+    feat, g, weight = _f32_aligned(feat, "feat"), _f32_aligned(g, "g"), _f32(weight, "weight")
+    comps, paths = table.mix_size
+    c, n_edges = feat.shape[2], feat_index.numel()
+    assert g.shape == (seg_ptr.numel() - 1, comps, c) and weight.shape == (paths, c)
+    out = (torch.empty if num_y_rows == n_edges else torch.zeros)(num_y_rows, table.d_y, dtype=torch.float32, device=dev)
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().eqt_tp_cg_inner_mix(
+            C.byref(table.struct), table.mix_key, feat.data_ptr(), feat_index.data_ptr(), g.data_ptr(), weight.data_ptr(),
+            seg_ptr.data_ptr(), _lib.ptr(y_index), out.data_ptr(), g.shape[0], n_edges, c, _lib.stream_ptr(dev)), "eqt_tp_cg_inner_mix")
     return out

@@ -192,6 +192,26 @@ int eqt_tp_cg_inner(const eqt_tp_table* table, const float* feat, const int64_t*
                     int64_t num_nodes, int64_t num_edges, int32_t channels, int32_t* status, void* stream);
 
 /*
+ * The two steps above for a layer whose weights (paths, channels) act channel by channel, without the rows of the intermediate:
+ *   out[d, k, c] = sum_{r of component k} weight[path(r), c] * (row r of eqt_tp_cg_segment_sum)[d, c]
+ *   grad_weight[p, c] = sum_d sum_{r of path p} x[d, k(r), c] * (row r)[d, c]                    (where x is given)
+ *   grad_y as eqt_tp_cg_inner for g'[d, r, c] = weight[path(r), c] * g[d, k(r), c]
+ * out, x, g are (num_out, components, channels).  `mix_key` names the rows' components and paths together with the structure
+ * (gen_walk_specs.mix_key); eqt_tp_cg_mix_scratch_floats is the scratch that grad_weight needs, or -1 where no kernel was
+ * built for the key or the channels (16 or multiples of 32; the adjoint: 16, 32, 64, 128).  Operands lie on 16 bytes.
+ * replaces: the chain above with indexed_mul_scale_gather (equitorch/ops/batched_sparse_dense_op.py:277) behind it, as
+ *   tensor_product_1uu composes them (equitorch/nn/functional/linears.py:16-130), and its gradients.
+ */
+int64_t eqt_tp_cg_mix_scratch_floats(uint64_t mix_key, int64_t num_out, int32_t channels);
+int eqt_tp_cg_segment_mix(const eqt_tp_table* table, uint64_t mix_key, const float* feat, const int64_t* feat_index, const float* y,
+                          const int64_t* y_index, const int64_t* seg_ptr, const float* weight, const float* x, float* out,
+                          float* grad_weight, float* scratch, int64_t scratch_floats, int64_t num_out, int64_t num_edges,
+                          int32_t channels, void* stream);
+int eqt_tp_cg_inner_mix(const eqt_tp_table* table, uint64_t mix_key, const float* feat, const int64_t* feat_index, const float* g,
+                        const float* weight, const int64_t* seg_ptr, const int64_t* y_index, float* grad_y, int64_t num_nodes,
+                        int64_t num_edges, int32_t channels, void* stream);
+
+/*
  * Weight step of a layer with weights shared by all samples, on tensor cores (float32 in and out,
  * 3xTF32 split arithmetic, accumulation in float32):
  *   out[i, out_row0 + m, co] = sum_{p < paths} sum_ci s[i, in_row0 + m*paths + p, ci] * W_p[ci, co]

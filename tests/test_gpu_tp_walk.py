@@ -1,0 +1,105 @@
+"""Segment sums and adjoints with one warp a node: rows, rows mixed channel by channel, and the weights' gradient, against float64."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from equitorch_b200.irreps import Irreps
+from equitorch_b200.ops.fused_tp_op import (INNER_CHANNELS, TpTable, cg_inner, cg_inner_mix, cg_segment_mix, cg_segment_sum,
+                                            mix_scratch)
+from equitorch_b200.tables import tp_infos
+
+DEV = torch.device("cuda:0")
+# float32 sums of at most a few hundred terms: 1e-5 of the largest entry, the path's tolerance
+TOL = 1e-5
+
+
+def _tables(lmax, role):
+    ir = Irreps("+".join(f"{l}{'eo'[l % 2]}" for l in range(lmax + 1)))
+    fwd, bwd1, _, _ = tp_infos(ir, ir, ir)
+    info = fwd if role == "fwd" else bwd1
+    table = TpTable(info.info_Mij_fwd, role == "fwd", ir.dim, ir.dim, DEV, info.info_M_fwd)
+    row = torch.from_numpy(np.repeat(np.arange(table.num_rows), np.diff(table.row_ptr.cpu().numpy()))).to(DEV)
+    m = info.info_M_fwd
+    seg = m.seg_out.to(DEV)
+    comp = torch.repeat_interleave(torch.arange(m.out_size, device=DEV), seg[1:] - seg[:-1])
+    return ir.dim, table, row, comp, m.index2.to(DEV)
+
+
+def _close(got, want):
+    assert float((got.double() - want).abs().max()) <= TOL * max(float(want.abs().max()), 1e-30)
+
+
+# one node of one edge; fewer nodes than warps; degrees over a ring, a block of 32 indices and its remainders, empty nodes in front and behind
+DEGREES = {"one": [1], "few": [0, 3, 1, 0, 2, 5, 0], "blocks": [31, 32, 33, 0, 64, 65, 1, 4, 97], "many": None}
+
+
+@pytest.mark.parametrize("degrees", list(DEGREES))
+@pytest.mark.parametrize("c", [16, 32, 64, 96, 128])
+@pytest.mark.parametrize("lmax,role", [(1, "fwd"), (1, "bwd1"), (2, "fwd"), (2, "bwd1"), (3, "fwd"), (3, "bwd1")])
+def test_against_float64(lmax, role, c, degrees):
+    dim, table, row, comp, path = _tables(lmax, role)
+    g = torch.Generator().manual_seed(17 * lmax + c)
+    deg = torch.tensor(DEGREES[degrees]) if DEGREES[degrees] else torch.randint(0, 7, (5003,), generator=g)
+    n, e = deg.numel(), int(deg.sum())
+    ptr = torch.cat([torch.zeros(1, dtype=torch.int64), torch.cumsum(deg, 0)]).to(DEV)
+    fidx, yidx = torch.randint(0, 50, (e,), generator=g).to(DEV), torch.randperm(e, generator=g).to(DEV)
+    feat, y = torch.randn(50, dim, c, generator=g).to(DEV), torch.randn(e, dim, generator=g).to(DEV)
+    x, w = torch.randn(n, dim, c, generator=g).to(DEV), torch.randn(int(path.max()) + 1, c, generator=g).to(DEV)
+    grad = torch.randn(n, dim, c, generator=g).to(DEV)
+    node = torch.repeat_interleave(torch.arange(n, device=DEV), deg.to(DEV))
+
+    yd, sd = y.double()[yidx], table.scale.double()
+    rows = torch.zeros(n, table.num_rows, c, dtype=torch.float64, device=DEV)
+    gy = torch.zeros(e, dim, dtype=torch.float64, device=DEV)
+    big = w.double()[path] * grad.double()[:, comp]                      # (n, rows, c): gradient of the rows
+    for t0 in range(0, sd.numel(), 16):                                  # a few entries at a time: the terms of all would not fit
+        t = slice(t0, t0 + 16)
+        f = feat.double()[fidx][:, table.m_feat[t]] * sd[t, None]
+        term = f * yd[:, table.m_y[t], None]
+        rows.index_put_((node[:, None], row[None, t]), term, accumulate=True)
+        gy.index_add_(1, table.m_y[t], (f * big[node][:, row[t]]).sum(-1))
+    want = torch.zeros(n, dim, c, dtype=torch.float64, device=DEV).index_add_(1, comp, w.double()[path] * rows)
+    gw = torch.zeros(w.shape, dtype=torch.float64, device=DEV).index_add_(0, path, (x.double()[:, comp] * rows).sum(0))
+    want_gy = torch.zeros_like(gy)
+    want_gy[yidx] = gy
+
+    _close(cg_segment_sum(table, feat, y, fidx, yidx, ptr, n), rows)
+    out, none = cg_segment_mix(table, feat, y, fidx, yidx, ptr, n, w)
+    assert none is None
+    _close(out, want)
+    out, got_gw = cg_segment_mix(table, feat, y, fidx, yidx, ptr, n, w, x)
+    _close(out, want)
+    _close(got_gw, gw)
+    _close(cg_inner(table, feat, big.float(), fidx, ptr, node, yidx, e), want_gy)
+    if c in INNER_CHANNELS:
+        _close(cg_inner_mix(table, feat, grad, w, fidx, ptr, yidx, e), want_gy)
+
+
+@pytest.mark.parametrize("lmax,c", [(2, 16), (2, 64), (3, 16), (3, 32)])
+def test_values_that_are_not_finite_stay_at_their_nodes(lmax, c):
+    """Two edges share a warp at 16 channels, and a ring slot outlives its edge: neither may leak into other nodes."""
+    dim, table, _, _, path = _tables(lmax, "fwd")
+    g = torch.Generator().manual_seed(3)
+    n = 301
+    ptr = torch.arange(0, 3 * n + 1, 3, dtype=torch.int64, device=DEV)
+    feat, y = torch.randn(3 * n, dim, c, generator=g).to(DEV), torch.randn(3 * n, dim, generator=g).to(DEV)
+    w, grad = torch.randn(int(path.max()) + 1, c, generator=g).to(DEV), torch.randn(n, dim, c, generator=g).to(DEV)
+    fidx = torch.arange(3 * n, device=DEV)
+    feat[7], feat[450] = float("inf"), float("nan")
+    bad = torch.zeros(n, dtype=torch.bool, device=DEV)
+    bad[7 // 3] = bad[450 // 3] = True
+    for out in (cg_segment_sum(table, feat, y, fidx, None, ptr, n), cg_segment_mix(table, feat, y, fidx, None, ptr, n, w)[0]):
+        assert torch.isfinite(out[~bad]).all() and not torch.isfinite(out[bad]).all(dim=(1, 2)).any()
+    gy = cg_inner_mix(table, feat, grad, w, fidx, ptr, None, 3 * n)
+    finite = torch.isfinite(gy).all(dim=1)
+    assert not finite[7] and not finite[450] and int(finite.sum()) == 3 * n - 2
+
+
+def test_keys_without_kernels():
+    dim, table, _, _, _ = _tables(2, "fwd")
+    assert mix_scratch(table, 10, 64) > 0 and mix_scratch(table, 10, 24) == -1
+    odd = Irreps("0e+1e+1o+2e")
+    fwd = tp_infos(odd, Irreps("0e+1o+2e"), odd)[0]
+    assert mix_scratch(TpTable(fwd.info_Mij_fwd, True, odd.dim, 9, DEV, fwd.info_M_fwd), 10, 64) == -1
