@@ -341,7 +341,7 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
     }
     R.total = quads;
     if (int rc = launch_wgrad(B, smem, st)) return rc;
-    wgrad_reduce_batched_kernel<<<flat_grid(quads, 256), 256, 0, st>>>(R);
+    wgrad_reduce_batched_kernel<<<(unsigned)ceil_div(quads, 32), 32 * REDUCE_WARPS, 0, st>>>(R);
     if (int rc = check_launch("wgrad_reduce_batched_kernel")) return rc;
   }
   return EQT_OK;
@@ -514,9 +514,12 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
     if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
     return EQT_OK;
   }
-  auto* reduce = transposed ? outer_reduce_kernel<true> : outer_reduce_kernel<false>;
-  reduce<<<flat_grid((int64_t)num_w * c1 * c2 / 4, 256), 256, 0, st>>>(scratch, out, red_ptr, red_slot, red_scale, splits,
-                                                                      (int64_t)m_tiles * 128, num_w, c1, c2, columns);
+  const bool many = splits > REDUCE_WARPS;
+  auto* reduce = transposed ? (many ? outer_reduce_kernel<true, REDUCE_WARPS> : outer_reduce_kernel<true, 1>)
+                            : (many ? outer_reduce_kernel<false, REDUCE_WARPS> : outer_reduce_kernel<false, 1>);
+  const int64_t per_block = 32 * (many ? 1 : REDUCE_WARPS);
+  reduce<<<(unsigned)ceil_div((int64_t)num_w * c1 * c2 / 4, per_block), 32 * REDUCE_WARPS, 0, st>>>(
+      scratch, out, red_ptr, red_slot, red_scale, splits, (int64_t)m_tiles * 128, num_w, c1, c2, columns);
   return check_launch("outer_reduce_kernel");
 }
 
