@@ -519,16 +519,6 @@ constexpr size_t YS_BYTES = (size_t)NS * GE * 16 * 4;              // 2 KB
 constexpr size_t YB_BYTES = 2 * 2 * 2048;                          // [A slot][big, small] 16 rows x 128 B
 constexpr size_t OFF_YS = XS_BYTES, OFF_YB = OFF_YS + YS_BYTES, OFF_SC = OFF_YB + YB_BYTES;
 
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-        "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
-      : "memory");
-}
-
 constexpr int NODES_PER_CHUNK = 16;    // nodes that a CTA takes at a time, fewer on small graphs (launch_segsum_tc)
 
 // The node walk every role performs: nodes come in chunks of PER nodes (0: nodes_per_cta) dealt round-robin to the CTAs.  Inside a
@@ -714,16 +704,15 @@ __global__ void __launch_bounds__(segtc::THREADS, 1) tp_segsum_tc_kernel(FusedAr
 #pragma unroll
           for (int e = 0; e < GE; ++e) {
             const float x = e < cnt ? xr[e * ROWF + fo[i]] : 0.f;
-            const float hi = rn_tf32(x);
-            v[e] = hi;
-            v[8 + e] = x - hi;
+            v[e] = hi_tf32(x);
+            v[8 + e] = x - v[e];
           }
           tmem_st16(ta + i * 16, v);
         }
         {   // harmonics value (edge, component) -> the two B tiles (128-byte rows, 16-byte chunks swizzled by the row)
           const int ed = t128 >> 4, m = t128 & 15;
           const float yv = ed < cnt ? ys[(slot * GE + ed) * 16 + m] : 0.f;
-          const float hi = rn_tf32(yv);
+          const float hi = hi_tf32(yv);
           const uint32_t off = m * 128 + ((((uint32_t)ed >> 2) ^ (m & 7)) << 4) + (ed & 3) * 4;
           *reinterpret_cast<float*>(yb + G * 4096 + off) = hi;
           *reinterpret_cast<float*>(yb + G * 4096 + 2048 + off) = yv - hi;

@@ -85,11 +85,6 @@ __device__ __forceinline__ uint32_t split_at(int k, int r, int c, bool small) {
   const int chunk = k > 16 ? c : c + (small ? 4 : 0);
   return (k > 16 && small ? 128 * 128 : 0) + r * 128 + ((chunk ^ (r & 7)) << 4);
 }
-__device__ __forceinline__ void split4(const float4 v, float4& hi, float4& lo) {
-  hi = make_float4(rn_tf32(v.x), rn_tf32(v.y), rn_tf32(v.z), rn_tf32(v.w));
-  lo = make_float4(rn_tf32(v.x - hi.x), rn_tf32(v.y - hi.y), rn_tf32(v.z - hi.z), rn_tf32(v.w - hi.w));
-}
-
 struct ContractJob {
   const float* s;                  // (ds, ci, padded n): transposed, so that the samples of a warp are one run
   const float* f;                  // (n, df, ck)
@@ -332,7 +327,7 @@ __global__ void __launch_bounds__(CONTRACT_THREADS, 1) uvw_contract_kernel(const
       const int r = i / per_row, rest = i - r * per_row, c = rest / quads, ch = rest - c * quads;
       const int64_t n = tile * 128 + r;
       float4 hi, lo;
-      split4(n < p.n ? __ldg(reinterpret_cast<const float4*>(f + n * job.df * k) + rest) : make_float4(0.f, 0.f, 0.f, 0.f), hi, lo);
+      split_tf32(n < p.n ? __ldg(reinterpret_cast<const float4*>(f + n * job.df * k) + rest) : make_float4(0.f, 0.f, 0.f, 0.f), hi, lo);
       *reinterpret_cast<float4*>(base + c * a_bytes + split_at(k, r, ch, false)) = hi;
       *reinterpret_cast<float4*>(base + c * a_bytes + split_at(k, r, ch, true)) = lo;
     }
@@ -432,7 +427,7 @@ __global__ void __launch_bounds__(256) uvw_pack_kernel(const __grid_constant__ P
     const float scale = __ldg(&job.paths[q].scale);
     const float* w = p.w + __ldg(&job.paths[q].weight) * job.sp + i * job.si + j * job.sj + (int64_t)ch * 4 * job.sk;
     float4 hi, lo;
-    split4(make_float4(__ldg(w) * scale, __ldg(w + job.sk) * scale, __ldg(w + 2 * job.sk) * scale, __ldg(w + 3 * job.sk) * scale), hi, lo);
+    split_tf32(make_float4(__ldg(w) * scale, __ldg(w + job.sk) * scale, __ldg(w + 2 * job.sk) * scale, __ldg(w + 3 * job.sk) * scale), hi, lo);
     unsigned char* to = job.packed + image * split_bytes(job.ck);
     *reinterpret_cast<float4*>(to + split_at(job.ck, row, ch, false)) = hi;
     *reinterpret_cast<float4*>(to + split_at(job.ck, row, ch, true)) = lo;
@@ -729,8 +724,8 @@ template <int J> struct RowMaker {
               for (int e = 0; e < 4; e += 2) {       // the MMA drops what of the small part is past TF32
                 float x, y;
                 apart(q[h][c][e / 2], x, y);
-                v[h * 4 + e] = rn_tf32(x);
-                v[h * 4 + e + 1] = rn_tf32(y);
+                v[h * 4 + e] = hi_tf32(x);
+                v[h * 4 + e + 1] = hi_tf32(y);
                 apart(fma2(two(v[h * 4 + e], v[h * 4 + e + 1]), two(-1.f, -1.f), q[h][c][e / 2]), v[8 + h * 4 + e], v[8 + h * 4 + e + 1]);
               }
             tmem_put16(tmem + (uint32_t)(u * 80 + c * 16), v);
@@ -921,7 +916,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) uvw_wgrad_kernel(const __grid_co
           for (int c = 0; c < 5; ++c) {
             if (c >= nf) break;
             float4 hi, lo;
-            split4(fv[h][c], hi, lo);
+            split_tf32(fv[h][c], hi, lo);
             const float big[4] = {hi.x, hi.y, hi.z, hi.w}, small[4] = {lo.x, lo.y, lo.z, lo.w};
 #pragma unroll
             for (int m = 0; m < 4; ++m) {

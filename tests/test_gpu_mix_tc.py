@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from equitorch_b200 import nn as enn
 from equitorch_b200.irreps import Irreps
 from equitorch_b200.ops import batched_sparse_dense_op as gops
 from equitorch_b200.ops.fused_tp_op import check_status
@@ -94,3 +95,24 @@ def test_sums_run_in_the_order_of_the_channels(cout):
     got = mix_tc(s, w, plan)
     check_status()
     assert torch.count_nonzero(got) == 0
+
+
+@pytest.mark.parametrize("bits", [0x7fffffff, -1, 0x7fc00000, 0x7f800001, 0x7f800000])
+@pytest.mark.parametrize("c,cout", [(32, 32), (64, 64), (64, 128)])
+def test_values_that_are_not_finite_reach_what_they_enter(bits, c, cout):
+    """The pair of TF32 values of an operand is made in integer arithmetic, in which the largest NaNs wrap around."""
+    g = torch.Generator().manual_seed(5)
+    n = 700
+    layer = enn.IrrepsLinear("0e+1o", "0e+1o", c, cout, internal_weights=False).to(DEV)
+    x = torch.randn(n, 4, c, generator=g)
+    x.view(torch.int32)[13, 2, 3] = bits
+    w = torch.randn(*layer.weight_shape, generator=g)
+    xg, wg = x.to(DEV).requires_grad_(), w.to(DEV).requires_grad_()
+    out = layer(xg, wg)
+    (gw,) = torch.autograd.grad(out, wg, torch.randn(n, 4, cout, generator=g).to(DEV))
+    bad = torch.zeros(n, 4, cout, dtype=torch.bool, device=DEV)
+    bad[13, 2] = True
+    assert torch.equal(~torch.isfinite(out), bad)
+    worse = torch.zeros(gw.shape, dtype=torch.bool, device=DEV)
+    worse[1, 3] = True                                  # the row of 1o that the value is a factor of
+    assert torch.equal(~torch.isfinite(gw), worse)
