@@ -235,28 +235,57 @@ int launch_wgrad(const WgradBatch& b, size_t smem, cudaStream_t st) {
 
 // Launch shape of the weight-gradient GEMM of one block: reduction rows per tile, M tiles, node splits and the
 // floats of scratch the per-CTA partial sums need.  Returns an error code for blocks that do not fit.
-struct WgradShape { int npt, rows_pad, m_tiles, splits, stages, chunk_tiles; size_t stage_bytes; int64_t K, need; };
+struct WgradShape {
+  int npt, rows_pad, m_tiles, splits, stages, chunk_tiles, issuers, slots;
+  size_t smem;
+  int64_t K, tiles, need;
+  void split(int s, int cout) { splits = s; need = (int64_t)s * m_tiles * 128 * cout; }
+};
 int wgrad_shape(const eqt_mix_block& blk, int b, int64_t n, int cin, int cout, WgradShape* w) {
   if (blk.dim <= 0 || blk.dim > TILE_M || blk.paths <= 0) return fail(EQT_ERR_BAD_ARGUMENT, "bad block %d", b);
-  const int b_boxes = cout / 32;
-  const size_t budget = 220 * 1024 - 1024;
+  WgradTile tile;
+  if (!wgrad_tile(blk.dim, cout, &tile)) return fail(EQT_ERR_UNSUPPORTED, "irrep with %d components does not fit a reduction tile", blk.dim);
+  w->npt = tile.npt; w->rows_pad = tile.rows_pad; w->stages = tile.stages; w->smem = tile.smem;
+  w->issuers = tile.issuers; w->slots = tile.slots;
   w->K = (int64_t)blk.paths * cin;                               // M extent of this GEMM
   w->m_tiles = (int)ceil_div(w->K, 128);
-  // Reduction rows per tile: the most that leaves three stages in shared memory (with two, the TMA, split and MMA
-  // phases of the ring cannot overlap; smaller tiles pay more per-box issue cost per byte); whole nodes, padded with
-  // zero rows to a multiple of 8.
-  const size_t bytes_per_row = 2 * (size_t)(4 + b_boxes) * 128;
-  const int rows_target = std::max(8, (int)(budget / 3 / bytes_per_row) / 8 * 8);
-  w->npt = std::max(1, rows_target / blk.dim);
-  w->rows_pad = (w->npt * blk.dim + 7) / 8 * 8;
-  w->stage_bytes = bytes_per_row * (size_t)w->rows_pad;
-  w->stages = (int)std::min<size_t>(8, budget / w->stage_bytes);
-  if (w->stages < 2) return fail(EQT_ERR_UNSUPPORTED, "irrep with %d components does not fit a reduction tile", blk.dim);
-  w->chunk_tiles = std::max(1, 512 / w->rows_pad);
-  const int64_t tiles = ceil_div(n, w->npt);
-  w->splits = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count() / w->m_tiles));
-  w->need = (int64_t)w->splits * w->m_tiles * 128 * cout;
+  w->chunk_tiles = std::max(1, 320 / w->rows_pad);
+  w->tiles = ceil_div(n, w->npt);
+  w->split((int)std::max<int64_t>(1, std::min<int64_t>(w->tiles, sm_count() / w->m_tiles)), cout);
   return EQT_OK;
+}
+
+// Blocks of one launch share the SMs: another split for the block whose CTAs have the most tiles, while there are SMs.  A launch is then
+// one wave of CTAs with about as many tiles each, where every block on all SMs made a wave a block: each with its own fill and
+// drain, of one or two tiles a CTA on small batches (10k nodes, l_max 3, 64 channels 100.2 -> 82.0 us, 1000 nodes, l_max 2 22.3 -> 10.7).
+void wgrad_share(WgradShape* w, int count, int cout) {
+  int ctas = 0;
+  for (int b = 0; b < count; ++b) {
+    w[b].split(1, cout);
+    ctas += w[b].m_tiles;
+  }
+  for (;;) {
+    int most = 0;
+    for (int b = 1; b < count; ++b)
+      if (w[b].tiles * w[most].splits > w[most].tiles * w[b].splits) most = b;
+    if (ctas + w[most].m_tiles > sm_count() || w[most].splits >= w[most].tiles) return;
+    ctas += w[most].m_tiles;
+    w[most].split(w[most].splits + 1, cout);
+  }
+}
+
+// Splits of a product whose slices all have `tiles` tiles: as many waves of CTAs as leave the SMs least idle (32 slices: 4 splits are 128
+// CTAs, 9 are 288 of 296: 100k samples 712 -> 654 us), a wave's fill and drain counted as six tiles.
+int outer_splits(int64_t tiles, int m_tiles) {
+  const int sms = sm_count();
+  int best = 1;
+  double least = 1e300;
+  for (int waves = 1; waves <= 4; ++waves) {
+    const int64_t s = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)waves * sms / m_tiles));
+    const double cost = (double)ceil_div(s * m_tiles, sms) * (double)(ceil_div(tiles, s) + 6);
+    if (cost < least) { least = cost; best = (int)s; }
+  }
+  return best;
 }
 
 }  // namespace
@@ -268,13 +297,15 @@ extern "C" int64_t eqt_wgrad_tc_scratch_floats(int64_t n, int32_t cin, int32_t c
   if (n < 0 || cin <= 0 || cout <= 0 || cin % 32 || cout % 32 || num_blocks < 0 || (num_blocks && !blocks)) return -1;
   // the sum over the blocks: with that much scratch all blocks run in one launch; eqt_wgrad_tc also works with the
   // largest block's need alone (one launch per block then)
-  int64_t need = 0;
+  int64_t together = 0, alone = 0;
+  std::vector<WgradShape> shapes(num_blocks);
   for (int b = 0; b < num_blocks; ++b) {
-    WgradShape w{};
-    if (wgrad_shape(blocks[b], b, std::max<int64_t>(n, 1), cin, cout, &w)) return -1;
-    need += w.need;
+    if (wgrad_shape(blocks[b], b, std::max<int64_t>(n, 1), cin, cout, &shapes[b])) return -1;
+    alone = std::max(alone, shapes[b].need);
   }
-  return need;
+  for (int b0 = 0; b0 < num_blocks; b0 += WGRAD_MAX_BLOCKS) wgrad_share(&shapes[b0], std::min(WGRAD_MAX_BLOCKS, num_blocks - b0), cout);
+  for (const WgradShape& w : shapes) together += w.need;
+  return std::max(together, alone);
 }
 
 extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, float* scratch, int64_t scratch_floats,
@@ -294,18 +325,20 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
       return fail(EQT_ERR_BAD_ARGUMENT, "scratch too small: block %d needs %lld floats, %lld given", b,
                   (long long)shapes[b].need, (long long)scratch_floats);
   }
-  int64_t total_need = 0;
-  for (int b = 0; b < num_blocks; ++b) total_need += shapes[b].need;
   // With scratch for every block at once, up to WGRAD_MAX_BLOCKS blocks share a launch (and one reduction launch);
   // otherwise the blocks run one after the other and reuse the scratch.
+  std::vector<WgradShape> shared = shapes;
+  int64_t total_need = 0;
+  for (int b0 = 0; b0 < num_blocks; b0 += WGRAD_MAX_BLOCKS) wgrad_share(&shared[b0], std::min(WGRAD_MAX_BLOCKS, num_blocks - b0), cout);
+  for (const WgradShape& w : shared) total_need += w.need;
   const int per_launch = total_need <= scratch_floats ? WGRAD_MAX_BLOCKS : 1;
+  if (per_launch > 1) shapes = shared;
   for (int b0 = 0; b0 < num_blocks; b0 += per_launch) {
     const int count = std::min(per_launch, num_blocks - b0);
     WgradBatch B{};
     ReduceBatch R{};
     B.count = R.count = count;
     B.n = n; B.n_cols = R.cols = cout; B.status = status;
-    B.tmem_cols = 32;
     size_t smem = 0;
     int cta = 0;
     int64_t scratch_at = 0, quads = 0;
@@ -314,18 +347,16 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
       const WgradShape& w = shapes[b0 + q];
       WgradBlock& a = B.blk[q];
       a.dim = blk.dim; a.npt = w.npt; a.rows_pad = w.rows_pad; a.stages = w.stages; a.chunk_tiles = w.chunk_tiles;
-      a.issuers = w.rows_pad / 8 >= 2 ? 2 : 1;
       a.m_tiles = w.m_tiles; a.splits = w.splits; a.cta_begin = cta;
       a.partial = scratch + scratch_at;
       cta += w.splits * w.m_tiles;
-      while (B.tmem_cols < 2 * a.issuers * cout) B.tmem_cols <<= 1;
-      smem = std::max(smem, (size_t)w.stages * w.stage_bytes + 1024);
+      smem = std::max(smem, w.smem);
+      a.issuers = w.issuers; a.slots = w.slots;
       {
         cuuint64_t dims[3] = {(cuuint64_t)w.K, (cuuint64_t)blk.dim, (cuuint64_t)n};
         cuuint64_t strides[2] = {(cuuint64_t)w.K * 4, (cuuint64_t)rows * cin * 4};
-        cuuint32_t box[3] = {KB, (cuuint32_t)blk.dim, (cuuint32_t)w.npt};
-        if (int rc = make_map(&a.map_s, s + (int64_t)blk.in_row0 * cin, 3, dims, strides, box,
-                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return rc;
+        cuuint32_t box[3] = {128, (cuuint32_t)blk.dim, (cuuint32_t)w.npt};
+        if (int rc = make_map(&a.map_s, s + (int64_t)blk.in_row0 * cin, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return rc;
       }
       {
         cuuint64_t dims[3] = {(cuuint64_t)cout, (cuuint64_t)blk.dim, (cuuint64_t)n};
@@ -448,8 +479,9 @@ extern "C" int eqt_vecmat_tc(const float* x, const float* w, const int64_t* inde
 extern "C" int64_t eqt_outer_tc_scratch_floats(int64_t n, int32_t columns, int32_t m_tiles) {
   using namespace eqt;
   if (n < 0 || columns <= 0 || columns % 32 || m_tiles <= 0) return -1;
-  const int splits = std::max(1, sm_count() / m_tiles);
-  return (int64_t)splits * m_tiles * 128 * columns;
+  WgradTile tile;
+  if (columns > 128 || !wgrad_tile(1, columns, &tile)) return -1;
+  return (int64_t)outer_splits(std::max<int64_t>(1, ceil_div(n, tile.npt)), m_tiles) * m_tiles * 128 * columns;
 }
 
 extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* out, float* scratch, int64_t scratch_floats, int64_t n,
@@ -472,23 +504,17 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
   const int columns = group * c2;
   int splits = 1;
   if (n > 0 && m_tiles > 0) {
-    const int b_boxes = columns / 32;
-    const size_t budget = 220 * 1024 - 1024;
-    const size_t bytes_per_row = 2 * (size_t)(4 + b_boxes) * 128;
-    const int npt = std::max(8, (int)(budget / 3 / bytes_per_row) / 8 * 8);          // reduction rows per tile
+    WgradTile tile;
+    if (!wgrad_tile(1, columns, &tile)) return fail(EQT_ERR_UNSUPPORTED, "tile does not fit shared memory");
+    const int npt = tile.npt;                                                        // reduction rows per tile
     WgradBatch B{};
     B.count = 1; B.n = n; B.n_cols = columns; B.status = status;
     WgradBlock& a = B.blk[0];
-    a.dim = 1; a.npt = npt; a.rows_pad = npt;
-    const size_t stage_bytes = bytes_per_row * (size_t)npt;
-    a.stages = (int)std::min<size_t>(8, budget / stage_bytes);
-    a.issuers = npt / 8 >= 2 ? 2 : 1;
-    B.tmem_cols = 32;
-    while (B.tmem_cols < 2 * a.issuers * columns) B.tmem_cols <<= 1;
-    a.chunk_tiles = std::max(1, 256 / npt);        // samples between folds of the accumulators (512: error 1.6e-6 of the norm, 256: 9e-7, 1 % slower)
+    a.dim = 1; a.npt = npt; a.rows_pad = tile.rows_pad; a.stages = tile.stages; a.issuers = tile.issuers; a.slots = tile.slots;
+    a.chunk_tiles = std::max(1, 320 / npt);
     a.a_cols = a_cols; a.b_cols = b_cols; a.b_row_boxes = c2 / 32;
     const int64_t tiles = ceil_div(n, npt);
-    splits = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count() / m_tiles));
+    splits = outer_splits(tiles, m_tiles);
     const int64_t need = (int64_t)splits * m_tiles * 128 * columns;
     if (need > scratch_floats) return fail(EQT_ERR_BAD_ARGUMENT, "scratch too small: %lld floats needed", (long long)need);
     a.partial = scratch;
@@ -497,7 +523,7 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
       cuuint64_t dims[3] = {(cuuint64_t)rows1 * c1, 1, (cuuint64_t)n};
       cuuint64_t strides[2] = {(cuuint64_t)rows1 * c1 * 4, (cuuint64_t)rows1 * c1 * 4};
       cuuint32_t box[3] = {KB, 1, (cuuint32_t)npt};
-      if (int rc = make_map(&a.map_s, in1, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return rc;
+      if (int rc = make_map(&a.map_s, in1, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return rc;
     }
     {
       cuuint64_t dims[3] = {(cuuint64_t)rows2 * c2, 1, (cuuint64_t)n};
@@ -505,7 +531,7 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
       cuuint32_t box[3] = {KB, 1, (cuuint32_t)npt};
       if (int rc = make_map(&a.map_g, in2, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return rc;
     }
-    if (int rc = launch_wgrad(B, (size_t)a.stages * stage_bytes + 1024, st)) return rc;
+    if (int rc = launch_wgrad(B, tile.smem, st)) return rc;
   }
   // with no samples or no entries every unit list is read as empty only if m_tiles == 0; otherwise the partial sums
   // above were written by this call

@@ -116,3 +116,27 @@ def test_values_that_are_not_finite_reach_what_they_enter(bits, c, cout):
     worse = torch.zeros(gw.shape, dtype=torch.bool, device=DEV)
     worse[1, 3] = True                                  # the row of 1o that the value is a factor of
     assert torch.equal(~torch.isfinite(gw), worse)
+
+
+# one node; a tile of 40 rows and one more; fewer tiles than CTAs; chunks of eight tiles and their remainders.  Irreps that fill a tile of 40
+# rows, leave padding, or are longer than one (41: one node a tile; 65: one issuer and two slots at 64 columns)
+@pytest.mark.parametrize("irreps", ["0e+1o+2e+3o", "9o+10e", "20e+0e", "32e+1o"])
+@pytest.mark.parametrize("n,cin,cout", [(1, 32, 32), (40, 64, 64), (41, 32, 96), (333, 96, 64), (2600, 64, 128), (9001, 32, 64)])
+def test_wgrad_tc_at_the_edges_of_its_tiles(irreps, n, cin, cout):
+    if irreps == "32e+1o" and cout > 64:
+        pytest.skip("an irrep of 65 components does not fit beside more than 64 columns")
+    ir = Irreps(irreps)
+    fwd, _, _, paths = tp_infos(ir, ir, Irreps("0e"))
+    info = fwd.info_M_fwd.to(DEV)
+    plan = MixPlan(info, [i.dim for i in ir], DEV)
+    gen = torch.Generator().manual_seed(n + cout)
+    s = torch.randn(n, plan.rows, cin, generator=gen).to(DEV)
+    g = torch.randn(n, plan.comps, cout, generator=gen).to(DEV)
+    got = wgrad_tc(s, g, plan, paths)
+    check_status()
+    seg = info.seg_out.cpu() if info.seg_out is not None else torch.arange(info.out_size + 1)
+    comp_of_row = torch.repeat_interleave(torch.arange(info.out_size), seg[1:] - seg[:-1]).to(DEV)
+    want = torch.zeros(paths, cin, cout, dtype=torch.float64, device=DEV)
+    for r in range(plan.rows):
+        want[int(info.index2[r])] += s[:, r].double().T @ g[:, int(comp_of_row[r])].double()
+    assert float((got.double() - want).abs().max()) <= 8e-6 * float(want.abs().max())
