@@ -27,6 +27,7 @@
 // Every wait on an mbarrier is bounded; on expiry the kernel raises the status flag, stops
 // issuing work, frees its TMEM and returns.
 #include <algorithm>
+#include <initializer_list>
 #include <vector>
 
 #include "tc_common.cuh"
@@ -236,7 +237,7 @@ int launch_wgrad(const WgradBatch& b, size_t smem, cudaStream_t st) {
 // Launch shape of the weight-gradient GEMM of one block: reduction rows per tile, M tiles, node splits and the
 // floats of scratch the per-CTA partial sums need.  Returns an error code for blocks that do not fit.
 struct WgradShape {
-  int npt, rows_pad, m_tiles, splits, stages, chunk_tiles, issuers, slots;
+  int npt, rows_pad, m_tiles, splits, chunk_tiles, issuers;
   size_t smem;
   int64_t K, tiles, need;
   void split(int s, int cout) { splits = s; need = (int64_t)s * m_tiles * 128 * cout; }
@@ -245,8 +246,7 @@ int wgrad_shape(const eqt_mix_block& blk, int b, int64_t n, int cin, int cout, W
   if (blk.dim <= 0 || blk.dim > TILE_M || blk.paths <= 0) return fail(EQT_ERR_BAD_ARGUMENT, "bad block %d", b);
   WgradTile tile;
   if (!wgrad_tile(blk.dim, cout, &tile)) return fail(EQT_ERR_UNSUPPORTED, "irrep with %d components does not fit a reduction tile", blk.dim);
-  w->npt = tile.npt; w->rows_pad = tile.rows_pad; w->stages = tile.stages; w->smem = tile.smem;
-  w->issuers = tile.issuers; w->slots = tile.slots;
+  w->npt = tile.npt; w->rows_pad = tile.rows_pad; w->smem = tile.smem; w->issuers = tile.issuers;
   w->K = (int64_t)blk.paths * cin;                               // M extent of this GEMM
   w->m_tiles = (int)ceil_div(w->K, 128);
   w->chunk_tiles = std::max(1, 320 / w->rows_pad);
@@ -257,7 +257,7 @@ int wgrad_shape(const eqt_mix_block& blk, int b, int64_t n, int cin, int cout, W
 
 // Blocks of one launch share the SMs: another split for the block whose CTAs have the most tiles, while there are SMs.  A launch is then
 // one wave of CTAs with about as many tiles each, where every block on all SMs made a wave a block: each with its own fill and
-// drain, of one or two tiles a CTA on small batches (10k nodes, l_max 3, 64 channels 100.2 -> 82.0 us, 1000 nodes, l_max 2 22.3 -> 10.7).
+// drain, of one or two tiles a CTA on small batches (10k nodes, l_max 3, 64 channels 100 -> 82 us, 1000 nodes, l_max 2 22.3 -> 10.7).
 void wgrad_share(WgradShape* w, int count, int cout) {
   int ctas = 0;
   for (int b = 0; b < count; ++b) {
@@ -346,12 +346,12 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
       const eqt_mix_block& blk = blocks[b0 + q];
       const WgradShape& w = shapes[b0 + q];
       WgradBlock& a = B.blk[q];
-      a.dim = blk.dim; a.npt = w.npt; a.rows_pad = w.rows_pad; a.stages = w.stages; a.chunk_tiles = w.chunk_tiles;
+      a.dim = blk.dim; a.npt = w.npt; a.rows_pad = w.rows_pad; a.chunk_tiles = w.chunk_tiles;
       a.m_tiles = w.m_tiles; a.splits = w.splits; a.cta_begin = cta;
       a.partial = scratch + scratch_at;
       cta += w.splits * w.m_tiles;
       smem = std::max(smem, w.smem);
-      a.issuers = w.issuers; a.slots = w.slots;
+      a.issuers = w.issuers;
       {
         cuuint64_t dims[3] = {(cuuint64_t)w.K, (cuuint64_t)blk.dim, (cuuint64_t)n};
         cuuint64_t strides[2] = {(cuuint64_t)w.K * 4, (cuuint64_t)rows * cin * 4};
@@ -510,7 +510,7 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
     WgradBatch B{};
     B.count = 1; B.n = n; B.n_cols = columns; B.status = status;
     WgradBlock& a = B.blk[0];
-    a.dim = 1; a.npt = npt; a.rows_pad = tile.rows_pad; a.stages = tile.stages; a.issuers = tile.issuers; a.slots = tile.slots;
+    a.dim = 1; a.npt = npt; a.rows_pad = tile.rows_pad; a.issuers = tile.issuers;
     a.chunk_tiles = std::max(1, 320 / npt);
     a.a_cols = a_cols; a.b_cols = b_cols; a.b_row_boxes = c2 / 32;
     const int64_t tiles = ceil_div(n, npt);
