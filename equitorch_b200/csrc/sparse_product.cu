@@ -526,6 +526,73 @@ __global__ void __launch_bounds__(256) outer_acc_kernel(P p, int64_t chunk) {
     }
 }
 
+// The same for few channels (C1 and C2 multiples of four, up to 2048 products, 4096 for up to 1024 samples, float32): a team of (C1 / 4)
+// (C2 / 4) threads per sample, four by four products a thread, operands straight from global memory, of which tiles of 64 x 64 would use a
+// sixteenth at 16 x 16 channels.  Entries outside, samples inside, four of them in flight; the teams' sums meet in shared memory.  99 rows
+// into 23 outputs: 18k samples, 16 x 16 1980 -> 240 us; 20k samples, 24 x 24 2055 -> 530, 32 x 64 2124 -> 2104, 64 x 64 2151 -> 4239; 1000
+// samples, 64 x 64 103 -> 93; 252 entries into 41 outputs, 70k samples, 16 x 16 14.3 -> 1.9 ms.
+__global__ void __launch_bounds__(256) outer_acc_few_kernel(P p, int64_t chunk, int team, int teams) {
+  extern __shared__ __align__(16) float sums[];            // [teams][C1][C2]
+  const float* x = static_cast<const float*>(p.in1);
+  const float* y = static_cast<const float*>(p.in2);
+  float* out = static_cast<float*>(p.out);
+  const int c1 = (int)p.c1, c2 = (int)p.c2, q2 = c2 / 4, tid = threadIdx.x;
+  const int which = tid / team, place = tid % team, a0 = place / q2 * 4, b0 = place % q2 * 4;
+  const int64_t o = blockIdx.x, n0 = blockIdx.y * chunk, n1 = min(n0 + chunk, p.n);
+  if (which < teams) {
+    int64_t t0, t1;
+    seg_range(p, o, t0, t1);
+    float acc[4][4] = {};
+    for (int64_t t = t0; t < t1; ++t) {
+      const Entry e = entry(p, t);
+      const float s = scale_of<float>(p, e.tt);
+      const float* xt = x + e.r1 * c1 + a0;
+      const float* yt = y + e.r2 * c2 + b0;
+      float part[4][4] = {};
+      int64_t n = n0 + which;
+      for (; n + 3 * teams < n1; n += 4 * teams) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          a[u] = __ldg(reinterpret_cast<const float4*>(xt + (n + u * teams) * p.bs1));
+          b[u] = __ldg(reinterpret_cast<const float4*>(yt + (n + u * teams) * p.bs2));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float av[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, bv[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[i][j] = fmaf(av[i], bv[j], part[i][j]);
+        }
+      }
+      for (; n < n1; n += teams) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(xt + n * p.bs1)), b = __ldg(reinterpret_cast<const float4*>(yt + n * p.bs2));
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) part[i][j] = fmaf(av[i], bv[j], part[i][j]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(s, part[i][j], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float4*>(sums + (which * c1 + a0 + i) * c2 + b0) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  }
+  __syncthreads();
+  const int64_t orow = out_row(p, o);
+  for (int i = tid; i < c1 * c2; i += 256) {
+    float v = sums[i];
+    for (int w = 1; w < teams; ++w) v += sums[w * c1 * c2 + i];
+    atomicAdd(out + orow * c1 * c2 + i, v);
+  }
+}
+
+
 // ------------------------------------------------------------------------------------------
 // INNER: one warp per (sample, output row)
 // ------------------------------------------------------------------------------------------
@@ -629,6 +696,72 @@ __global__ void __launch_bounds__(256) vecmat_shared_w_kernel(P p) {
     }
   }
 }
+
+// The same for 16 or 32 output channels, where tiles of 64 would mostly be padding (C_in a multiple of four up to 64, float32): a
+// thread owns SPT samples and sixteen output channels; the weights of eight entries at a time, scaled, come from shared memory as
+// broadcasts, a sample's rows straight from global memory.  18k samples, 99 rows, 16 -> 16 channels, both products 432 -> 153 us; 70k
+// samples, 252 entries 3807 -> 901; 20k samples, 99 rows, 64 -> 32 878 -> 393 (64 -> 64 a sixteenth at a time: 53 -> 63 at 450 samples).
+template <int SPT>
+__global__ void __launch_bounds__(128) vecmat_few_kernel(P p) {
+  constexpr int ENTRIES = 8;
+  extern __shared__ __align__(16) float sw[];              // [ENTRIES][C_in][16]
+  __shared__ int64_t row[ENTRIES];
+  const float* x = static_cast<const float*>(p.in1);
+  const float* w = static_cast<const float*>(p.in2);
+  float* out = static_cast<float*>(p.out);
+  const int cin = (int)p.c1, cout = (int)p.c2, tiles = cout / 16, tid = threadIdx.x;
+  const int64_t o = blockIdx.y / tiles, co = blockIdx.y % tiles * 16;
+  const int64_t first = blockIdx.x * (int64_t)(128 * SPT) + tid;
+  int64_t t0, t1;
+  seg_range(p, o, t0, t1);
+  float acc[SPT][16] = {};
+  for (int64_t tb = t0; tb < t1; tb += ENTRIES) {
+    const int count = (int)min((int64_t)ENTRIES, t1 - tb);
+    __syncthreads();
+    for (int i = tid; i < count * cin * 16; i += 128) {
+      const int k = i / 16;
+      const Entry e = entry(p, tb + k / cin);
+      sw[i] = __ldg(w + (e.r2 * cin + k % cin) * cout + co + i % 16) * scale_of<float>(p, e.tt);
+    }
+    if (tid < count) row[tid] = entry(p, tb + tid).r1 * cin;
+    __syncthreads();
+    for (int t = 0; t < count; ++t) {
+      const float* xt = x + row[t];
+      for (int c = 0; c < cin; c += 4) {
+        float4 v[SPT];
+#pragma unroll
+        for (int s = 0; s < SPT; ++s)
+          v[s] = first + s * 128 < p.n ? __ldg(reinterpret_cast<const float4*>(xt + (first + s * 128) * p.bs1 + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float4* wk = reinterpret_cast<const float4*>(sw + (t * cin + c + k) * 16);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 f = wk[q];
+#pragma unroll
+            for (int s = 0; s < SPT; ++s) {
+              const float a = k == 0 ? v[s].x : k == 1 ? v[s].y : k == 2 ? v[s].z : v[s].w;
+              acc[s][4 * q] = fmaf(a, f.x, acc[s][4 * q]);
+              acc[s][4 * q + 1] = fmaf(a, f.y, acc[s][4 * q + 1]);
+              acc[s][4 * q + 2] = fmaf(a, f.z, acc[s][4 * q + 2]);
+              acc[s][4 * q + 3] = fmaf(a, f.w, acc[s][4 * q + 3]);
+            }
+          }
+        }
+      }
+    }
+  }
+  const int64_t orow = out_row(p, o);
+#pragma unroll
+  for (int s = 0; s < SPT; ++s) {
+    const int64_t n = first + s * 128;
+    if (n >= p.n) continue;
+    float4* to = reinterpret_cast<float4*>(out + (n * p.out_size + orow) * cout + co);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) to[q] = make_float4(acc[s][4 * q], acc[s][4 * q + 1], acc[s][4 * q + 2], acc[s][4 * q + 3]);
+  }
+}
+
 
 // Any other sharing pattern (per-sample matrices, shared vector, batch-summed output): one
 // thread per output element; the matrix is streamed once, so this form is bandwidth bound.
@@ -736,6 +869,15 @@ int launch(const eqt_product_args& a, P p, cudaStream_t s) {
     if (a.accumulated) {
       const int64_t tiles = ceil_div(p.c1, 64) * ceil_div(p.c2, 64);
       if (p.num_out > 65535) return fail(EQT_ERR_UNSUPPORTED, "accumulated outer: more than 65535 output rows");
+      if (std::is_same<T, float>::value && p.c1 % 4 == 0 && p.c2 % 4 == 0 && (p.c1 * p.c2 <= 2048 || (p.c1 * p.c2 <= 4096 && p.n <= 1024)) &&
+          aligned16(p.in1) && aligned16(p.in2)) {
+        const int team = (int)(p.c1 * p.c2 / 16), teams = std::min<int>(16, 256 / team);
+        int64_t chunks = std::min<int64_t>(ceil_div((int64_t)sm_count() * 8, p.num_out), ceil_div(p.n, 4 * teams));
+        chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, 65535));
+        const int64_t chunk = ceil_div(p.n, chunks);
+        outer_acc_few_kernel<<<dim3((unsigned)p.num_out, (unsigned)ceil_div(p.n, chunk)), 256, sizeof(float) * teams * p.c1 * p.c2, s>>>(p, chunk, team, teams);
+        return check_launch("outer_acc_few_kernel");
+      }
       int64_t chunks = ceil_div((int64_t)sm_count() * 4, tiles * p.num_out);
       chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, ceil_div(p.n, 32)));
       chunks = std::min<int64_t>(chunks, 65535);
@@ -761,6 +903,17 @@ int launch(const eqt_product_args& a, P p, cudaStream_t s) {
   }
   if (op == EQT_OP_VECMAT) {
     if (p.c2 == 0) return EQT_OK;
+    if (std::is_same<T, float>::value && a.shared2 && !a.shared1 && !a.accumulated && (p.c2 == 16 || p.c2 == 32) && p.c1 % 4 == 0 && p.c1 <= 64 &&
+        p.num_out * (p.c2 / 16) <= 65535 && aligned16(p.in1) && aligned16(p.out)) {
+      const size_t bytes = sizeof(float) * 8 * p.c1 * 16;
+      const unsigned rows = (unsigned)(p.num_out * (p.c2 / 16));
+      // the more samples a thread the fewer reads of the weights, as long as every SM has two blocks
+      const int64_t enough = 2 * (int64_t)sm_count();
+      if (ceil_div(p.n, 512) * rows >= enough) vecmat_few_kernel<4><<<dim3((unsigned)ceil_div(p.n, 512), rows), 128, bytes, s>>>(p);
+      else if (ceil_div(p.n, 256) * rows >= enough) vecmat_few_kernel<2><<<dim3((unsigned)ceil_div(p.n, 256), rows), 128, bytes, s>>>(p);
+      else vecmat_few_kernel<1><<<dim3((unsigned)ceil_div(p.n, 128), rows), 128, bytes, s>>>(p);
+      return check_launch("vecmat_few_kernel");
+    }
     if (a.shared2 && !a.shared1 && !a.accumulated && p.num_out <= 65535) {
       dim3 grid((unsigned)(ceil_div(p.n, 64) * ceil_div(p.c2, 64)), (unsigned)p.num_out);
       vecmat_shared_w_kernel<T><<<grid, 256, 0, s>>>(p);
