@@ -417,7 +417,8 @@ extern "C" int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64
   L.chunk_kb = group == 1 ? VM_SHORT_CHUNK_KB : VM_CHUNK_KB;
   L.acc_sets = (L.bigs + 1) * n_cols <= 128 ? 2 : 1;       // at least four A slots stay free (two at 128 columns)
   const int acc_cols = L.acc_sets * (L.bigs + 1) * n_cols;
-  L.stages = (int)std::min<size_t>(std::min<size_t>(8, (220 * 1024 - 1024 - EPI_PATCH_BYTES) / stage_bytes), (512 - acc_cols) / 64);
+  constexpr size_t patches = std::max(VecmatCfg<true>::PATCH_BYTES, VecmatCfg<false>::PATCH_BYTES);
+  L.stages = (int)std::min<size_t>(std::min<size_t>(8, (220 * 1024 - 1024 - patches) / stage_bytes), (512 - acc_cols) / 64);
   if (L.stages < 2) return fail(EQT_ERR_UNSUPPORTED, "tile too wide for the shared-memory ring");
   L.tmem_cols = 32;
   while (L.tmem_cols < acc_cols + 64 * L.stages) L.tmem_cols <<= 1;
@@ -460,11 +461,13 @@ extern "C" int eqt_vecmat_tc_grouped(const float* x, const float* w, const int64
                (size_t)b_bytes + (size_t)R.raw_stages * TILE_M * KB * 4 + 1024 + EPI_PATCH_BYTES, st>>>(R);
     return check_launch("vecmat_resident_kernel");
   }
-  auto* kernel = group == 1 && longest == 1 ? vecmat_tc_kernel<true> : vecmat_tc_kernel<false>;
+  const bool wide = group > 1;
+  auto* kernel = wide ? vecmat_tc_kernel<false, true> : longest == 1 ? vecmat_tc_kernel<true, false> : vecmat_tc_kernel<false, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   const unsigned grid = (unsigned)std::min<int64_t>(L.total_items, sm_count());
-  kernel<<<grid, TC_THREADS, (size_t)L.stages * stage_bytes + 1024 + EPI_PATCH_BYTES, st>>>(L);
+  kernel<<<grid, wide ? VecmatCfg<true>::THREADS : VecmatCfg<false>::THREADS,
+           (size_t)L.stages * stage_bytes + 1024 + (wide ? VecmatCfg<true>::PATCH_BYTES : VecmatCfg<false>::PATCH_BYTES), st>>>(L);
   return check_launch("vecmat_tc_kernel");
 }
 

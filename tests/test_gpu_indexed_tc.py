@@ -183,3 +183,23 @@ def test_calls_that_can_have_no_plan_take_the_table_driven_kernels():
     assert _rel(got, want) < 1e-5
     with torch.inference_mode():
         assert _rel(new()(x, w).clone(), want) < 1e-5
+
+
+@pytest.mark.parametrize("lmax,c", [(2, 32), (3, 64), (6, 32)])          # groups of 2 to 4 rows, some not full, of 64 to 128 columns
+@pytest.mark.parametrize("n", [512, 513, 4999])                           # whole tiles of 128 samples, one sample more, several items a CTA
+def test_rows_in_groups(lmax, c, n):
+    import copy
+    from equitorch_b200 import nn as enn
+    from equitorch_b200.irreps import Irreps
+    ir = Irreps((0, lmax))
+    layer = enn.SO2Linear(ir, ir, c, c, internal_weights=False, feature_mode="uv").to(DEV)
+    g = torch.Generator().manual_seed(n + lmax)
+    x, cot = (torch.randn(n, ir.dim, c, generator=g).to(DEV) for _ in range(2))
+    w = (torch.randn(*layer.weight_shape, generator=g) / c ** 0.5).to(DEV)
+    results = []
+    for module, dtype in ((layer, torch.float32), (copy.deepcopy(layer).double(), torch.float64)):
+        xs, ws = x.to(dtype).requires_grad_(), w.to(dtype).requires_grad_()
+        out = module(xs, ws)
+        results.append([out, *torch.autograd.grad(out, [xs, ws], cot.to(dtype))])
+    for got, want in zip(*results):
+        assert float((got.double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
