@@ -309,12 +309,26 @@ __global__ void __launch_bounds__(BR_THREADS) block_rotation_kernel(const float*
   }
 }
 
-// grad_M[n, i, j] = sum_c g[n, i, c] x[n, j, c] inside the blocks, zero outside.  A thread makes 4 x 4 entries of a block from
-// rows that are ceil(size / 4) apart (the lanes of a phase then read neighbouring rows, which a pitch of C + 4 floats puts on
-// different banks) with 16-byte loads along the channels, so that neither operand is transposed on the way in.  Results go to
-// an image of four samples whose zeros are written once, and the image leaves as one bulk copy.
-// 100k samples of l = 0..6, 32 channels: 1305 -> 539 us (4.1 TB/s).
-constexpr int BG_THREADS = 128;
+// Two float32 values multiplied and added by one instruction (fma.rn.f32x2), each rounded as fmaf rounds it.
+__device__ __forceinline__ void pair_fma(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r.x + r.y;
+}
+
+// grad_M[n, i, j] = sum_c g[n, i, c] x[n, j, c] inside the blocks, zero outside.  Two neighbouring lanes make 4 x 4 entries of a
+// block from rows that are ceil(size / 4) apart, one from the even and one from the odd groups of four channels, with 16-byte
+// loads along the channels, so that neither operand is transposed on the way in; they exchange halves of their sums at the
+// end.  Each lane begins with another group of channels: the lanes of a phase then read different banks although the rows are
+// not padded, and a pass copies one run of each operand without a division.  Results go to an image of four samples whose
+// zeros are written once, and the image leaves as one bulk copy.  Two lanes an item are twice the warps in the same shared
+// memory: with one, on padded rows, eight warps an SM waited for their own chains and for barriers (issue 45 %).
+// 40k samples, one lane / two: l = 0..6 of 32 channels 232 / 177 us (5.0 TB/s), l = 0..4 of 64 channels 211 / 124, l = 0..2 of 32
+// channels 45 / 35; a third pass in shared memory changes nothing (177, 124, 35).
+constexpr int BG_THREADS = 256;
 constexpr int BG_MAX_TILES = 512;
 struct GradTiles {
   int count;
@@ -325,74 +339,86 @@ __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const f
                                                                          int samples, int image_samples,
                                                                          const __grid_constant__ GradTiles tiles) {
   extern __shared__ __align__(16) float sm[];
-  __shared__ uint32_t tile[BG_MAX_TILES];       // indexed by lane
-  const int dd = dim * dim, pitch = c + 4, operand = dim * pitch, cg = c / 4, quads = dim * cg;
+  const int dd = dim * dim, features = dim * c, operand = samples * features, items = tiles.count;
   float* img = sm;                              // [image_samples][dim][dim]
-  float* stage = img + image_samples * dd;      // [2][samples][g, x][dim][pitch]
-  for (int i = threadIdx.x; i < tiles.count; i += blockDim.x) tile[i] = tiles.code[i];
+  float* stage = img + image_samples * dd;      // [2][g, x][samples][dim][c]
+  uint32_t* tile = reinterpret_cast<uint32_t*>(stage + 4 * operand);   // indexed by lane
+  for (int i = threadIdx.x; i < items; i += blockDim.x) tile[i] = tiles.code[i];
   for (int i = threadIdx.x; i < image_samples * dd; i += blockDim.x) img[i] = 0.f;
-  __syncthreads();
-  const int items = tiles.count;
-  auto fetch = [&](int64_t s0, int ns, int buf) {
-    for (int i = threadIdx.x; i < ns * quads; i += blockDim.x) {
-      const int s = i / quads, e = i - s * quads, r = e / cg, k = (e - r * cg) * 4;
-      float* to = stage + (buf * samples + s) * 2 * operand + r * pitch + k;
-      const int64_t from = (s0 + s) * dim * c + 4 * e;
-      cp_async16(to, g + from);
-      cp_async16(to + operand, x + from);
-    }
-  };
+  const int passes = image_samples / samples;   // per image
   const int64_t step = (int64_t)gridDim.x * image_samples;
-  int buf = 0;
-  int64_t base = (int64_t)blockIdx.x * image_samples;
-  if (base < n) fetch(base, (int)min((int64_t)samples, n - base), 0);
-  cp_async_commit();
-  for (; base < n; base += step) {
+  // the samples of one pass, and the pass after them: the next of the image or the first of the block's next image
+  auto fetch = [&](int64_t base, int pass, int buf) {
+    const int64_t s0 = base + pass * samples;
+    const int floats = (int)max((int64_t)0, min((int64_t)samples, n - s0)) * features;
+    float* to = stage + buf * 2 * operand;
+    for (int i = 4 * threadIdx.x; i < floats; i += 4 * blockDim.x) {
+      cp_async16(to + i, g + s0 * features + i);
+      cp_async16(to + operand + i, x + s0 * features + i);
+    }
+    cp_async_commit();
+  };
+  int64_t ahead = (int64_t)blockIdx.x * image_samples;
+  int ahead_pass = 0, buf = 0;
+  auto fetch_next = [&](int to) {
+    fetch(ahead, ahead_pass, to);
+    if (++ahead_pass == passes) ahead_pass = 0, ahead += step;
+  };
+  fetch_next(0);
+  const int lane = threadIdx.x & 31, half = lane & 1, cg = c / 4, groups = (cg + 1 - half) / 2;   // this lane's groups of channels
+  const int first = groups ? (threadIdx.x >> 1) % groups : 0;
+  for (int64_t base = (int64_t)blockIdx.x * image_samples; base < n; base += step) {
     const int total = (int)min((int64_t)image_samples, n - base);
-    image_release();
-    for (int part = 0; part < total; part += samples, buf ^= 1) {
-      const int ns = min(samples, total - part);
-      // the samples after these: in this group, or the first of the block's next group
-      const bool here = part + samples < total;
-      const int64_t next = here ? base + part + samples : base + step, end = here ? base + total : n;
-      if (next < end) fetch(next, (int)min((int64_t)samples, end - next), buf ^ 1);
-      cp_async_commit();
-      cp_async_wait<1>();
-      __syncthreads();
-      for (int i = threadIdx.x; i < ns * items; i += blockDim.x) {
-        const int s = i / items;
+    for (int pass = 0; pass < passes; ++pass) {
+      const int part = pass * samples, ns = min(samples, total - part);
+      if (pass == 0) image_release();
+      cp_async_wait<0>();
+      __syncthreads();                          // this pass has arrived; the place of the one before it is free
+      fetch_next(buf ^ 1);
+      for (int w = threadIdx.x - lane; w < 2 * ns * items; w += blockDim.x) {      // whole warps: the lanes exchange sums
+        const bool made = w + lane < 2 * ns * items;
+        const int i = made ? (w + lane) >> 1 : 0, s = i / items;
         const uint32_t code = tile[i - s * items];
         const int lo = code & 255, size = code >> 8 & 255, np = (size + 3) / 4, pa = code >> 16 & 255, qa = code >> 24;
-        const float* gp = stage + (buf * samples + s) * 2 * operand + lo * pitch;
+        const float* gp = stage + buf * 2 * operand + s * features + lo * c;
         const float* xp = gp + operand;
         int ro[4], co[4];                       // rows past the block read its last row and are not stored
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          ro[u] = min(pa + u * np, size - 1) * pitch;
-          co[u] = min(qa + u * np, size - 1) * pitch;
+          ro[u] = min(pa + u * np, size - 1) * c;
+          co[u] = min(qa + u * np, size - 1) * c;
         }
-        float acc[4][4] = {};
-        for (int k = 0; k < c; k += 4) {
-          float4 gv[4], xv[4];
+        uint64_t acc[4][4] = {};                // sums over even and odd channels
+        for (int k = 0, at = first; k < groups; ++k, at = at + 1 == groups ? 0 : at + 1) {
+          const int ch = 8 * at + 4 * half;
+          ulonglong2 gv[4], xv[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            gv[u] = *reinterpret_cast<const float4*>(gp + ro[u] + k);
-            xv[u] = *reinterpret_cast<const float4*>(xp + co[u] + k);
+            gv[u] = *reinterpret_cast<const ulonglong2*>(gp + ro[u] + ch);
+            xv[u] = *reinterpret_cast<const ulonglong2*>(xp + co[u] + ch);
           }
 #pragma unroll
           for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int w = 0; w < 4; ++w)
-              acc[u][w] = fmaf(gv[u].x, xv[w].x, fmaf(gv[u].y, xv[w].y, fmaf(gv[u].z, xv[w].z, fmaf(gv[u].w, xv[w].w, acc[u][w]))));
+            for (int v = 0; v < 4; ++v) {
+              pair_fma(acc[u][v], gv[u].x, xv[v].x);
+              pair_fma(acc[u][v], gv[u].y, xv[v].y);
+            }
         }
+        // the even lane keeps tile rows 0 and 1, the odd one 2 and 3
         float* o = img + (part + s) * dd + lo * dim + lo;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 2; ++u) {
+          const int row = pa + (u + 2 * half) * np;
 #pragma unroll
-          for (int w = 0; w < 4; ++w)
-            if (pa + u * np < size && qa + w * np < size) o[(pa + u * np) * dim + qa + w * np] = acc[u][w];
+          for (int v = 0; v < 4; ++v) {
+            const float low = pair_sum(acc[u][v]), high = pair_sum(acc[u + 2][v]);
+            const float sum = (half ? high : low) + __shfl_xor_sync(0xffffffffu, half ? low : high, 1);
+            if (made && row < size && qa + v * np < size) o[row * dim + qa + v * np] = sum;
+          }
+        }
       }
-      __syncthreads();
+      buf ^= 1;
     }
     image_store(gm + base * dd, img, (int64_t)total * dd);
   }
@@ -461,16 +487,16 @@ bool gradient_tiles(const int32_t* sizes, int blocks, GradTiles& t) {
   }
   return true;
 }
-// Samples per pass (a power of two, about one item per thread) and per image (a multiple of four and of the former); returns
+// Samples per pass (a power of two, about two threads an item) and per image (a multiple of four and of the former); returns
 // the shared memory, 0 where it does not fit.
 size_t gradient_samples(const GradTiles& t, int dim, int c, int* samples, int* image) {
   int s = 16;
-  while (s > 1 && s * t.count > BG_THREADS) s /= 2;
+  while (s > 1 && 2 * s * t.count > BG_THREADS) s /= 2;
   for (;; s /= 2) {
     *samples = s;
     *image = std::max(4, s);
-    const size_t bytes = sizeof(float) * ((size_t)*image * dim * dim + 4 * (size_t)s * dim * (c + 4));
-    if (bytes <= 100 * 1024 || (s == 1 && bytes <= SMEM_MOST)) return bytes;
+    const size_t bytes = sizeof(float) * ((size_t)*image * dim * dim + 4 * (size_t)s * dim * c + t.count);
+    if (bytes <= 112 * 1024 || (s == 1 && bytes <= SMEM_MOST)) return bytes;
     if (s == 1) return 0;
   }
 }
@@ -585,8 +611,9 @@ extern "C" int eqt_block_rotation_grad_matrix(const float* grad_out, const float
   gradient_tiles(block_sizes, num_blocks, g);
   const size_t bytes = gradient_samples(g, dim, channels, &samples, &image);
   unsigned grid = 1;
-  if (int rc = resident_grid(block_rotation_grad_kernel, BG_THREADS, bytes, ceil_div(n, image), &grid)) return rc;
-  block_rotation_grad_kernel<<<grid, BG_THREADS, bytes, static_cast<cudaStream_t>(stream)>>>(grad_out, x, grad_matrix, n, dim, channels,
+  const int threads = std::min(BG_THREADS, (2 * samples * g.count + 31) / 32 * 32);
+  if (int rc = resident_grid(block_rotation_grad_kernel, threads, bytes, ceil_div(n, image), &grid)) return rc;
+  block_rotation_grad_kernel<<<grid, threads, bytes, static_cast<cudaStream_t>(stream)>>>(grad_out, x, grad_matrix, n, dim, channels,
                                                                                             samples, image, g);
   return check_launch("block_rotation_grad_kernel");
 }

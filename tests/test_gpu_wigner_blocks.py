@@ -6,7 +6,7 @@ import torch
 
 from equitorch_b200 import nn as enn
 from equitorch_b200.irreps import Irreps
-from equitorch_b200.ops.wigner_op import block_diagonal
+from equitorch_b200.ops.wigner_op import block_diagonal, dense_rotation_grad_matrix
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -95,3 +95,18 @@ def test_features_at_an_odd_offset_take_the_general_kernel():
     x = store[1:].view(4, 9, 8)
     assert not block_diagonal(ir, x.device).takes(x)
     assert _err(enn.DenseWignerRotation(ir)(x, m), m.double() @ x.double()) < TOL
+
+
+@pytest.mark.parametrize("name,n,c", [("0e+1o+2e+3o+4e+5o+6e", 3001, 4), ("0e+1o+2e+3o+4e+5o+6e", 1303, 36), ("0e+1o+2e", 40003, 12),
+                                      ("9x5o", 701, 8), ("7o", 9002, 64)])
+def test_several_images_a_block(name, n, c):
+    """More samples than one round of blocks holds, the last image not full; entries outside the blocks stay zero.  A sum of
+    c products made in chains of at most c / 4 + 1 multiply-adds with two further additions differs from the exact one by at most
+    (c / 4 + 3) eps times the sum of the magnitudes."""
+    ir, gen = Irreps(name), torch.Generator().manual_seed(c)
+    mask = torch.block_diag(*[torch.ones(i.dim, i.dim) for i in ir]).to(DEV)
+    g, x = (torch.randn(n, ir.dim, c, generator=gen).to(DEV) for _ in range(2))
+    out = dense_rotation_grad_matrix(g, x, block_diagonal(ir, DEV))
+    exact = (g.double() @ x.double().mT) * mask
+    most = (g.double().abs() @ x.double().abs().mT) * mask
+    assert ((out - exact).abs() <= (c / 4 + 3) * 2.0 ** -24 * most).all()
