@@ -234,6 +234,21 @@ struct RowTiles {
   uint16_t at[BR_MAX_DIM], first[BR_MAX_DIM + 1];   // first shared float; first entry in the list of block entries
 };
 
+// Two float32 values multiplied and added by one instruction (fma.rn.f32x2), each rounded as fmaf rounds it.
+__device__ __forceinline__ void pair_fma(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r.x + r.y;
+}
+__device__ __forceinline__ uint64_t pair_of(float a) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+
 // out[n, i, c] = sum_j M[n, i, j] x[n, j, c] (transposed: M[n, j, i]) over the block of row i.  A thread makes four rows of
 // four channels: per contraction step one 16-byte load of features, one of four matrix entries (laid out [tile][j][row]) and
 // 16 multiply-adds.  The entries of the blocks are copied by a list made once per launch (a shared-memory pair of offsets per
@@ -309,14 +324,78 @@ __global__ void __launch_bounds__(BR_THREADS) block_rotation_kernel(const float*
   }
 }
 
-// Two float32 values multiplied and added by one instruction (fma.rn.f32x2), each rounded as fmaf rounds it.
-__device__ __forceinline__ void pair_fma(uint64_t& acc, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float pair_sum(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r.x + r.y;
+// The same product with the whole matrices copied, as one run per pass that begins at any float: where the blocks touch most
+// of the matrix's cache lines anyway, that costs no traffic and takes the list away.  A thread makes four rows of V times
+// four channels and keeps its tile and channels for the whole launch.
+template <int V>
+__global__ void __launch_bounds__(BR_THREADS) block_rotation_whole_kernel(const float* __restrict__ mat, const float* __restrict__ x,
+                                                                          float* __restrict__ out, int64_t n, int dim, int c,
+                                                                          int transposed, int samples,
+                                                                          const __grid_constant__ RowTiles tiles) {
+  extern __shared__ __align__(16) float sm[];                        // [2][3 + samples * dim * dim | samples * dim * c]
+  const int dd = dim * dim, features = dim * c, mat_room = (samples * dd + 6) & ~3, buffer = mat_room + samples * features;
+  const int cg = c / (4 * V), items = tiles.count * cg, sample = threadIdx.x / items, first = threadIdx.x - sample * items;
+  const int64_t step = (int64_t)gridDim.x * samples;
+  auto shift_of = [&](int64_t s0) { return (int)(reinterpret_cast<uintptr_t>(mat + s0 * dd) >> 2 & 3); };   // same place in 16 bytes
+  auto fetch = [&](int64_t s0, int buf) {
+    const int ns = (int)min((int64_t)samples, n - s0), floats = ns * dd, shift = shift_of(s0), head = min((4 - shift) & 3, floats);
+    const int tail = head + ((floats - head) & ~3);
+    const float* from = mat + s0 * dd;
+    float* to = sm + buf * buffer;
+    if ((int)threadIdx.x < head) cp_async4(to + shift + threadIdx.x, from + threadIdx.x);
+    if ((int)threadIdx.x < floats - tail) cp_async4(to + shift + tail + threadIdx.x, from + tail + threadIdx.x);
+    for (int i = head + 4 * threadIdx.x; i < tail; i += 4 * blockDim.x) cp_async16(to + shift + i, from + i);
+    to += mat_room;
+    from = x + s0 * features;
+    for (int i = 4 * threadIdx.x; i < ns * features; i += 4 * blockDim.x) cp_async16(to + i, from + i);
+  };
+  int64_t s0 = (int64_t)blockIdx.x * samples;
+  if (s0 < n) fetch(s0, 0);
+  cp_async_commit();
+  for (int buf = 0; s0 < n; s0 += step, buf ^= 1) {
+    if (s0 + step < n) fetch(s0 + step, buf ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    if (sample < (int)min((int64_t)samples, n - s0)) {
+      for (int item = first; item < items; item += blockDim.x) {     // one, or one sample and several items
+        const int t = item / cg, quad = (item - t * cg) * 4;
+        const int lo = tiles.lo[t], row = tiles.row[t], rows = tiles.rows[t], len = tiles.len[t];
+        // neighbouring tiles begin with different halves: the lanes of a phase then read different banks
+        const int half = c / 2, ch = V == 2 && (t & 1) ? quad + half : quad, other = V == 2 && (t & 1) ? quad : quad + half;
+        const int by_row = transposed ? 1 : dim, by_j = transposed ? dim : 1;
+        const float* mp = sm + buf * buffer + shift_of(s0) + sample * dd + row * by_row + lo * by_j;
+        const float* xp = sm + buf * buffer + mat_room + sample * features + lo * c;
+        int at[4];                                                   // rows that the tile does not have: its last, not stored
+#pragma unroll
+        for (int u = 0; u < 4; ++u) at[u] = min(u, rows - 1) * by_row;
+        uint64_t acc[4][2 * V] = {};
+#pragma unroll 2
+        for (int j = 0; j < len; ++j, xp += c, mp += by_j) {
+          uint64_t m[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) m[u] = pair_of(mp[at[u]]);
+#pragma unroll
+          for (int h = 0; h < V; ++h) {
+            const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(xp + (h ? other : ch));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              pair_fma(acc[u][2 * h], m[u], xv.x);
+              pair_fma(acc[u][2 * h + 1], m[u], xv.y);
+            }
+          }
+        }
+        float* o = out + (s0 + sample) * features + row * c;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < rows)
+#pragma unroll
+            for (int h = 0; h < V; ++h)
+              *reinterpret_cast<ulonglong2*>(o + u * c + (h ? other : ch)) = make_ulonglong2(acc[u][2 * h], acc[u][2 * h + 1]);
+      }
+    }
+    __syncthreads();
+  }
 }
 
 // grad_M[n, i, j] = sum_c g[n, i, c] x[n, j, c] inside the blocks, zero outside.  Two neighbouring lanes make 4 x 4 entries of a
@@ -477,6 +556,27 @@ int rotation_samples(const RowTiles& t, int dim, int c) {
   return rotation_bytes(t, dim, c, samples) <= SMEM_MOST ? samples : 0;
 }
 
+
+// Whole matrices where the rows of the blocks, in lines of 128 bytes, touch all of them (l = 0..5 and less; 81 % at l = 0..6, and
+// HBM reads that share of them).  40k samples, by list / whole: l = 0..4 of 64 channels 145 / 120 us, l = 0..3 of 32 67 / 53,
+// l = 0..2 of 32 54 / 38, l = 0..5 of 32 117 / 113, of 64 175 / 177; but l = 0..6 of 32 154 / 177, l = 0..7 of 32 186 / 218.
+bool rotation_whole(const int32_t* sizes, int blocks, int dim) {
+  int64_t touched = 124 * (int64_t)dim;
+  for (int b = 0; b < blocks; ++b) touched += 4 * (int64_t)sizes[b] * sizes[b];
+  return touched >= 4 * (int64_t)dim * dim;
+}
+// Channels of a thread: twice four where they divide so (l = 0..4 of 64 channels: 134 us with four, 119 so).
+int whole_quads(int c) { return c % 8 ? 1 : 2; }
+size_t whole_bytes(int dim, int c, int samples) {
+  return 2 * sizeof(float) * (((size_t)samples * dim * dim + 6) / 4 * 4 + (size_t)samples * dim * c);
+}
+// Samples per pass: one item per thread, or as many as leave three blocks per SM their shared memory; 0 if one does not fit.
+int whole_samples(const RowTiles& t, int dim, int c) {
+  int samples = std::max(1, std::min(16, BR_THREADS / std::max(1, t.count * (c / 4 / whole_quads(c)))));
+  while (samples > 1 && whole_bytes(dim, c, samples) > 72 * 1024) --samples;
+  return whole_bytes(dim, c, samples) <= SMEM_MOST ? samples : 0;
+}
+
 bool gradient_tiles(const int32_t* sizes, int blocks, GradTiles& t) {
   t.count = 0;
   for (int b = 0, start = 0; b < blocks; start += sizes[b++]) {
@@ -588,8 +688,16 @@ extern "C" int eqt_block_rotation(const float* matrix, const float* x, float* ou
   RowTiles t;
   int dim = 0;
   rotation_tiles(block_sizes, num_blocks, t, &dim);
-  const int samples = rotation_samples(t, dim, channels);
   unsigned grid = 1;
+  if (const int samples = rotation_whole(block_sizes, num_blocks, dim) ? whole_samples(t, dim, channels) : 0) {
+    const size_t bytes = whole_bytes(dim, channels, samples);
+    const auto kernel = whole_quads(channels) == 2 ? block_rotation_whole_kernel<2> : block_rotation_whole_kernel<1>;
+    const int items = samples * t.count * (channels / 4 / whole_quads(channels)), threads = std::min(BR_THREADS, (items + 31) / 32 * 32);
+    if (int rc = resident_grid(kernel, threads, bytes, ceil_div(n, samples), &grid)) return rc;
+    kernel<<<grid, threads, bytes, static_cast<cudaStream_t>(stream)>>>(matrix, x, out, n, dim, channels, transposed, samples, t);
+    return check_launch("block_rotation_whole_kernel");
+  }
+  const int samples = rotation_samples(t, dim, channels);
   const size_t bytes = rotation_bytes(t, dim, channels, samples);
   if (int rc = resident_grid(block_rotation_kernel, BR_THREADS, bytes, ceil_div(n, samples), &grid)) return rc;
   block_rotation_kernel<<<grid, BR_THREADS, bytes, static_cast<cudaStream_t>(stream)>>>(matrix, x, out, n, dim, channels, transposed,

@@ -6,7 +6,7 @@ import torch
 
 from equitorch_b200 import nn as enn
 from equitorch_b200.irreps import Irreps
-from equitorch_b200.ops.wigner_op import block_diagonal, dense_rotation_grad_matrix
+from equitorch_b200.ops.wigner_op import block_diagonal, dense_rotation, dense_rotation_grad_matrix
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -110,3 +110,19 @@ def test_several_images_a_block(name, n, c):
     exact = (g.double() @ x.double().mT) * mask
     most = (g.double().abs() @ x.double().abs().mT) * mask
     assert ((out - exact).abs() <= (c / 4 + 3) * 2.0 ** -24 * most).all()
+
+
+@pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 30011, 8), ("7o", 3003, 12), ("5x0e", 9001, 4), ("0e+1o+2e+3o+4e+5o", 2501, 64)])
+@pytest.mark.parametrize("skip", [0, 1, 3])
+def test_several_passes_of_whole_matrices(name, n, c, skip):
+    """More samples than one round of blocks holds, the matrices beginning at any float.  A chain of at most 15 multiply-adds
+    differs from the exact sum by at most 15 eps times the sum of the magnitudes."""
+    ir, gen = Irreps(name), torch.Generator().manual_seed(c)
+    mask = torch.block_diag(*[torch.ones(i.dim, i.dim) for i in ir]).to(DEV)
+    m = torch.randn(n * ir.dim ** 2 + skip, generator=gen).to(DEV)[skip:].view(n, ir.dim, ir.dim)
+    x = torch.randn(n, ir.dim, c, generator=gen).to(DEV)
+    for transposed in (False, True):
+        out = dense_rotation(m, x, transposed, block_diagonal(ir, DEV))
+        blocks = (m * mask).double()
+        blocks = blocks.mT if transposed else blocks
+        assert ((out - blocks @ x.double()).abs() <= 15 * 2.0 ** -24 * (blocks.abs() @ x.double().abs())).all()
