@@ -97,6 +97,25 @@ def test_values_that_are_not_finite_stay_at_their_nodes(lmax, c):
     assert not finite[7] and not finite[450] and int(finite.sum()) == 3 * n - 2
 
 
+def test_weight_gradient_of_many_nodes():
+    """A warp adds up rows in chains of sixteen nodes, whose sums are added up in 64 bits: at most 112 multiply-adds of random sign
+    at l_max 3, each rounded by at most half a unit of the partial sum, which is 2^-24 sqrt(112 / 6) of the result.  In one chain
+    over all its nodes, 90 here, the error was 3.6e-7."""
+    dim, table, row, comp, path = _tables(3, "fwd")
+    g, n, c = torch.Generator(device=DEV).manual_seed(1), 20_000, 128
+    e = 3 * n
+    ptr, node = torch.arange(0, e + 1, 3, device=DEV), torch.arange(n, device=DEV).repeat_interleave(3)
+    fidx = torch.randint(0, n, (e,), generator=g, device=DEV)
+    feat, x = (torch.randn(n, dim, c, generator=g, device=DEV) for _ in range(2))
+    y, w = torch.randn(e, dim, generator=g, device=DEV), torch.randn(int(path.max()) + 1, c, generator=g, device=DEV)
+    want = torch.zeros(w.shape, dtype=torch.float64, device=DEV)
+    for t in range(table.scale.numel()):
+        term = feat[fidx, table.m_feat[t]].double() * (y[:, table.m_y[t], None].double() * table.scale[t].double())
+        want[path[row[t]]] += (x[:, comp[row[t]]].double()[node] * term).sum(0)
+    _, got = cg_segment_mix(table, feat, y, fidx, None, ptr, n, w, x)
+    assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24 * (112 / 6) ** 0.5
+
+
 def test_keys_without_kernels():
     dim, table, _, _, _ = _tables(2, "fwd")
     assert mix_scratch(table, 10, 64) > 0 and mix_scratch(table, 10, 24) == -1
