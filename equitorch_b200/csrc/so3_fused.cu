@@ -863,7 +863,7 @@ inline bool segsum_tc_wanted(const FusedArgs& a) {
 // channels: the adjoint ties (1800 nodes 91.5 -> 91.8, 20k nodes 702 -> 711 us), segment sums of few edges a node 202 -> 159 us.
 inline bool walk_wanted(uint64_t key, bool inner, const FusedArgs& a) {
   if (((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.g)) & 15u) != 0 || a.n_out >= 0x7fffffffll ||
-      !walk_supported(key, false, inner, a.C)) return false;
+      !walk_supported(key, false, inner, a.C) || !walk_sizes(key, false, a.T, a.R, a.DF, a.DY)) return false;
   if (a.DF < 16 || a.C == 16) return true;
   if (a.C == 32) return a.n_out >= 10 * (int64_t)sm_count();
   if (a.C == 64) return !inner && !segsum_tc_wanted(a);
@@ -970,6 +970,7 @@ extern "C" int eqt_tp_cg_segment_mix(const eqt_tp_table* table, uint64_t mix_key
     return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
   const int64_t need = walk_scratch_floats(mix_key, num_out, channels);
   if (need < 0) return fail(EQT_ERR_UNSUPPORTED, "no straight-line code for this structure and %d channels", channels);
+  if (!walk_sizes(mix_key, true, t.T, t.R, t.DF, t.DY)) return fail(EQT_ERR_BAD_ARGUMENT, "the table's sizes are not those of its key");
   if (!weight || (num_out > 0 && (!feat || !out || !seg_ptr)) || (num_edges > 0 && !y) || !x != !grad_weight)
     return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   if (x && (!scratch || scratch_floats < need)) return fail(EQT_ERR_BAD_ARGUMENT, "scratch of %lld floats, %lld needed", (long long)scratch_floats, (long long)need);
@@ -990,6 +991,7 @@ extern "C" int eqt_tp_cg_inner_mix(const eqt_tp_table* table, uint64_t mix_key, 
   if (num_nodes < 0 || num_edges < 0 || num_edges >= 0x7fffffffll || num_nodes >= 0x7fffffffll || channels <= 0)
     return fail(EQT_ERR_BAD_ARGUMENT, "bad sizes");
   if (!walk_supported(mix_key, true, true, channels)) return fail(EQT_ERR_UNSUPPORTED, "no straight-line code for this structure and %d channels", channels);
+  if (!walk_sizes(mix_key, true, t.T, t.R, t.DF, t.DY)) return fail(EQT_ERR_BAD_ARGUMENT, "the table's sizes are not those of its key");
   if (num_edges == 0 || num_nodes == 0) return EQT_OK;
   if (!feat || !g || !weight || !seg_ptr || !grad_y) return fail(EQT_ERR_BAD_ARGUMENT, "NULL pointer");
   if (((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(g)) & 15u) != 0) return fail(EQT_ERR_UNSUPPORTED, "operands must lie on 16 bytes");

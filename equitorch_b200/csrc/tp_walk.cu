@@ -638,6 +638,14 @@ bool walk_supported(uint64_t key, bool with_weights, bool adjoint, int channels)
   return false;
 }
 
+bool walk_sizes(uint64_t key, bool with_weights, int entries, int rows, int d_feat, int d_y) {
+#define EQT_TRY(S) \
+  if (key && key == (with_weights ? S::MIX_KEY : S::KEY)) return entries == S::T && rows == S::R && d_feat == S::DF && d_y == S::DY;
+  EQT_FOR_EACH_WALK(EQT_TRY)
+#undef EQT_TRY
+  return false;
+}
+
 int64_t walk_scratch_floats(uint64_t mix_key, int64_t n_out, int channels) {
   if (!walk_supported(mix_key, true, false, channels)) return -1;
 #define EQT_TRY(S) \

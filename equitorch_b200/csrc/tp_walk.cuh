@@ -22,8 +22,10 @@ struct WalkArgs {
   int C;
 };
 
-// Whether the kernels take a structure (key of its table, or of its table and weight step where w is given).
+// Whether the kernels take a structure (key of its table, or of its table and weight step where w is given), and whether a table
+// has the sizes of the structure that it names: the kernels read rows and entries by the structure's own.
 bool walk_supported(uint64_t key, bool with_weights, bool adjoint, int channels);
+bool walk_sizes(uint64_t key, bool with_weights, int entries, int rows, int d_feat, int d_y);
 int64_t walk_scratch_floats(uint64_t mix_key, int64_t n_out, int channels);    // -1: not supported
 int walk_segment_sum(uint64_t key, const WalkArgs& a, cudaStream_t s);
 int walk_inner(uint64_t key, const WalkArgs& a, cudaStream_t s);

@@ -68,3 +68,18 @@ def test_sparse_product_refuses_more_entries_than_rows(sizes):
     args = dict(op=_lib.OP_OUTER, dtype=_lib.DTYPE_CODE[torch.float32], in1=at, in2=at, out=at, n=1, rows1=16, rows2=16, num_out=1, out_size=1, c1=1, c2=1)
     rc = _lib.lib().eqt_sparse_product(ctypes.byref(_lib.ProductArgs(**{**args, **sizes})), None)
     assert rc != 0 and b"rows" in _lib.lib().eqt_last_error()
+
+
+@pytest.mark.parametrize("wrong", ["num_entries", "num_rows", "d_feat", "d_y"])
+def test_kernels_of_a_structure_refuse_tables_of_other_sizes(wrong):
+    """They go by the sizes of the structure that the key names, so a table of fewer rows would be read past its end."""
+    from equitorch_b200 import _lib
+    from equitorch_b200.csrc.gen_walk_specs import collect, mix_key
+    structure, rows, _ = collect()[2]
+    table = _lib.TpTableStruct(scale=16, m_feat=16, m_y=16, row_ptr=16, num_entries=len(structure.row), num_rows=structure.num_rows,
+                               d_feat=structure.d_feat, d_y=structure.d_y)
+    setattr(table, wrong, getattr(table, wrong) - 1)
+    key, lib = mix_key(structure, rows), _lib.lib()
+    assert lib.eqt_tp_cg_segment_mix(ctypes.byref(table), key, 16, 16, 16, None, 16, 16, None, 16, None, None, 0, 4, 4, 32, None) == 1
+    assert lib.eqt_tp_cg_inner_mix(ctypes.byref(table), key, 16, 16, 16, 16, 16, None, 16, 4, 4, 32, None) == 1
+    assert b"sizes" in lib.eqt_last_error()

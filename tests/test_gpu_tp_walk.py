@@ -122,3 +122,18 @@ def test_keys_without_kernels():
     odd = Irreps("0e+1e+1o+2e")
     fwd = tp_infos(odd, Irreps("0e+1o+2e"), odd)[0]
     assert mix_scratch(TpTable(fwd.info_Mij_fwd, True, odd.dim, 9, DEV, fwd.info_M_fwd), 10, 64) == -1
+
+
+def test_tables_that_contradict_their_key_take_the_table_driven_kernels():
+    dim, table, _, _, _ = _tables(1, "fwd")
+    n, c = 50, 32
+    g = torch.Generator().manual_seed(2)
+    feat, y, grad = (torch.randn(*s, generator=g).to(DEV) for s in ((n, dim, c), (n, dim), (n, table.num_rows, c)))
+    fidx, ptr = torch.arange(n, device=DEV), torch.arange(n + 1, device=DEV)
+
+    def run():
+        return cg_segment_sum(table, feat, y, fidx, None, ptr, n), cg_inner(table, feat, grad, fidx, ptr, fidx, None, n)
+    want = run()
+    table.struct.structure_key = _tables(2, "fwd")[1].key
+    for got, expect in zip(run(), want):
+        _close(got, expect.double())
