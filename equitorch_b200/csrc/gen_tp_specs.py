@@ -26,13 +26,13 @@ OUT = os.path.join(HERE, "generated", "tp_specs.inc")
 
 # (irreps_out, irreps_in1, irreps_in2) of layers whose inner loops are unrolled at build time, here and in gen_walk_specs.py.
 # All role rotations (forward, gradient w.r.t. input1, gradient w.r.t. input2) are generated.  The kernels of this module take those
-# whose cells do not fit one lane's registers (``FOUR_WARPS``); the others run on one warp a node.
+# of ``FOUR_WARPS``: at l_max 1 one warp a node is the better kernel at every size.
 REGISTRY = [
     ("0e+1o", "0e+1o", "0e+1o"),
     ("0e+1o+2e", "0e+1o+2e", "0e+1o+2e"),
     ("0e+1o+2e+3o", "0e+1o+2e+3o", "0e+1o+2e+3o"),
 ]
-FOUR_WARPS = REGISTRY[2:]
+FOUR_WARPS = REGISTRY[1:]
 
 
 class Structure(NamedTuple):

@@ -9,7 +9,7 @@
 // respect to the harmonics.
 //
 // Two implementations of each:
-//  * "spec": for index structures unrolled at build time (generated/tp_specs.inc: l_max 3).  The sum over
+//  * "spec": for index structures unrolled at build time (generated/tp_specs.inc: l_max 2 and 3).  The sum over
 //    the edges of a node commutes with the CG contraction, so per edge only the dense outer
 //    product Q[m_y, m_feat] += y_e[m_y] x_e[m_feat] is accumulated (234 of the 256 cells are used
 //    at l_max = 3) and the 353-entry sparse contraction runs once per node.  One CTA walks a
@@ -854,20 +854,36 @@ inline bool segsum_tc_wanted(const FusedArgs& a) {
          (reinterpret_cast<uintptr_t>(a.out) & 15u) == 0;
 }
 
-// One warp per node and 32 lanes of channels (tp_walk.cu) instead of the four warps per node above.  At l_max 1 and 2 and at 16
-// channels always: both segment sums / the adjoint of 20k nodes and 400k edges, 128 channels, l_max 2 1162 -> 614 / 751 -> 466 us, l_max 1
-// 497 -> 178 / 326 -> 114 us; 16 channels, 4000 nodes, 80k edges, l_max 3 1750 -> 110 / 2362 -> 74 us (table-driven before); 400 nodes,
-// 6000 edges, 32 channels, l_max 2 20.2 -> 18.3 / 13.1 -> 14.9 us.  At l_max 3 a node takes a warp's time of 120 cells an edge, which only
-// many nodes hide: 32 channels 600 nodes 35 -> 34 / 22 -> 19, 1000 nodes 24.5 -> 27.3 / 15.2 -> 16.8, 3000 nodes 170 -> 141 / 113 ->
-// 87 us.  128 channels leave room for eight warps an SM: 3000 nodes 540 -> 446 / 325 -> 303, 40k nodes 1416 -> 1739 / 889 -> 936 us.  64
-// channels: the adjoint ties (1800 nodes 91.5 -> 91.8, 20k nodes 702 -> 711 us), segment sums of few edges a node 202 -> 159 us.
+// One warp per node and 32 lanes of channels (tp_walk.cu) instead of the four warps per node above.  l_max 1, 16 channels and channels
+// that are no 32, 64 or 128: always (20k nodes, 400k edges, 128 channels, l_max 1: both segment sums 497 -> 178 us, adjoint 326 -> 114).
+// l_max 2: the same at most sizes (1162 -> 614 / 751 -> 466); a graph of few nodes leaves a warp alone with an edge's chain of loads and
+// multiply-adds, which four warps share (four warps / one, us: adjoint of 100 nodes of 15 edges, 32 channels 9.4 / 10.8, 64 9.9 /
+// 10.8; 1000 nodes of 8, 32 channels 10.9 / 11.6, of 15 16.0 / 15.6; sums of 200 nodes of 3, 32 channels 3.9 / 4.2, of 15 the same).
+// l_max 3: 120 cells an edge and warp, which only many nodes hide.  32 channels: adjoint of 1000 nodes 15.2 / 16.8, of 3000 113 / 87.
+// 128: rounds of 1.5 nodes an SM are short of few nodes (sums of 20 edges, 100 nodes 15.5 / 17.8, 200 23.4 / 20.8, 300 29.0 / 31.0, 600
+// 53.2 / 49.2; 5000 of 8 176 / 149; 40k 1416 / 1739; adjoint of 300 nodes of 20 33.1 / 34.8, of 3, 400 nodes 14.2 / 12.3).  64: sums of
+// few edges a node, where the tensor-core kernel does not run (400 nodes 8.1 / 9.5, 2000 22.4 / 21.1, 8000 96 / 76, 20k 182 / 189, 60k 474 /
+// 585); the adjoint ties.  With few edges a node the rows that a sum writes decide, and past some 0.5 GB of them (1 to 2 GB at l_max 2) four
+// warps write them faster (128 channels: 9000 nodes of 4 200 / 185, 14.5k of 3 243 / 279, l_max 2, 60k of 2 275 / 304; 32: 60k of 3 257 / 278).
 inline bool walk_wanted(uint64_t key, bool inner, const FusedArgs& a) {
   if (((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.g)) & 15u) != 0 || a.n_out >= 0x7fffffffll ||
       !walk_supported(key, false, inner, a.C) || !walk_sizes(key, false, a.T, a.R, a.DF, a.DY)) return false;
-  if (a.DF < 16 || a.C == 16) return true;
-  if (a.C == 32) return a.n_out >= 10 * (int64_t)sm_count();
-  if (a.C == 64) return !inner && !segsum_tc_wanted(a);
-  return a.C != 128 || a.n_out <= 100 * (int64_t)sm_count();
+  if (a.DF < 9 || (a.C != 32 && a.C != 64 && a.C != 128)) return true;
+  const int64_t sms = sm_count(), n = a.n_out;
+  auto degree_below = [&](int edges) { return a.n_edges < edges * n; };
+  const bool rows_decide = a.DF < 16 ? degree_below(4) && n * a.C > (degree_below(3) ? 50000 : 100000) * sms
+                                     : degree_below(5) && n * a.C > 8200 * sms;
+  if (!inner && rows_decide) return false;
+  if (a.DF < 16) {
+    if (a.C == 128) return true;
+    if (!inner) return n > 3 * sms || !degree_below(6);
+    return n > 3 * sms ? a.C == 64 || n > 7 * sms || !degree_below(10) : a.C == 64 && n > 2 * sms && !degree_below(15);
+  }
+  if (a.C == 32) return n >= 10 * sms;
+  if (a.C == 64) return !inner && !segsum_tc_wanted(a) && n >= 10 * sms;
+  if (n > 100 * sms) return false;
+  if (inner) return 2 * n > 5 * sms || (n <= sms && !degree_below(8));
+  return n >= 4 * sms || (n > sms && 2 * n <= 3 * sms);
 }
 
 template <class S>

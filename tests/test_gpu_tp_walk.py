@@ -1,4 +1,5 @@
-"""Segment sums and adjoints with one warp a node: rows, rows mixed channel by channel, and the weights' gradient, against float64."""
+"""Segment sums and adjoints with one warp a node, or four where those are faster: rows, rows mixed channel by channel, and the
+weights' gradient, against float64."""
 import numpy as np
 import pytest
 import torch
@@ -75,6 +76,29 @@ def test_against_float64(lmax, role, c, degrees):
     _close(cg_inner(table, feat, big.float(), fidx, ptr, node, yidx, e), want_gy)
     if c in INNER_CHANNELS:
         _close(cg_inner_mix(table, feat, grad, w, fidx, ptr, yidx, e), want_gy)
+
+
+# sums that four warps a node make because the rows that they write decide; from 100 nodes an SM on also the adjoint at l_max 3, 128 channels
+@pytest.mark.parametrize("lmax,c,n", [(2, 128, 59_000), (3, 32, 38_500), (3, 64, 19_100), (3, 128, 14_900)])
+def test_large_graphs_of_few_edges(lmax, c, n):
+    dim, table, row, _, _ = _tables(lmax, "fwd")
+    g = torch.Generator(device=DEV).manual_seed(n)
+    e, some = 2 * n, torch.cat([torch.arange(200), torch.arange(n - 200, n)]).to(DEV)
+    ptr, node = torch.arange(0, e + 1, 2, device=DEV), torch.arange(n, device=DEV).repeat_interleave(2)
+    fidx = torch.randint(0, n, (e,), generator=g, device=DEV)
+    feat, y = torch.randn(n, dim, c, generator=g, device=DEV), torch.randn(e, dim, generator=g, device=DEV)
+    grad = torch.randn(n, table.num_rows, c, generator=g, device=DEV)
+    rows, gy = cg_segment_sum(table, feat, y, fidx, None, ptr, n), cg_inner(table, feat, grad, fidx, ptr, node, None, e)
+
+    edges = (2 * some[:, None] + torch.arange(2, device=DEV)).reshape(-1)
+    x, big = feat[fidx[edges]].double(), grad[node[edges]].double()
+    want, want_gy = torch.zeros(400, table.num_rows, c, dtype=torch.float64, device=DEV), torch.zeros(800, dim, dtype=torch.float64, device=DEV)
+    for t in range(table.scale.numel()):
+        f = x[:, table.m_feat[t]] * table.scale[t].double()
+        want[:, row[t]] += (f * y[edges, table.m_y[t], None].double()).view(400, 2, c).sum(1)
+        want_gy[:, table.m_y[t]] += (f * big[:, row[t]]).sum(-1)
+    _close(rows[some], want)
+    _close(gy[edges], want_gy)
 
 
 @pytest.mark.parametrize("lmax,c", [(2, 16), (2, 64), (3, 16), (3, 32)])
