@@ -123,10 +123,7 @@ class GraphTPPlan(MixTables):
             self._mixed[c] = c in INNER_CHANNELS and all(mix_scratch(t, 1, c) >= 0 for t in (self.fwd_table, self.bwd1_table))
         return (self._mixed[c] and node_x.shape == (graph.num_src, self.d_in1, c) and node_x.dtype == weight.dtype == torch.float32
                 and weight.shape == (self.fwd_table.mix_size[1], c) and graph.num_edges > 0
-                and max(graph.num_edges, graph.num_src, graph.num_dst) < 2 ** 31 - 1 and node_x.data_ptr() % 16 == 0
-                # sums of many edges on tensor cores pay for writing the rows: 20k nodes, l_max 3, 64 channels, a pass of 100k edges
-                # 1416 -> 755 us, of 400k edges 2039 -> 2144
-                and (c != 64 or self.d_in1 != 16 or graph.num_edges < 16 * graph.num_dst))
+                and max(graph.num_edges, graph.num_src, graph.num_dst) < 2 ** 31 - 1 and node_x.data_ptr() % 16 == 0)
 
 
 def _mix(s: Tensor, w: Tensor, info, mode: str, tc: "MixPlan | None" = None) -> Tensor:
@@ -186,37 +183,86 @@ class FusedGraphOps:
         return self.grad_x(state, grad) if need[0] else None, gy, gw
 
 
-class MixedGraphOps:
-    """The passes of a 'uu' layer where the kernels mix the rows: none of the intermediates exists, and the gradients with
-    respect to the features and the weights are one pass (the weights' gradient pairs its rows with the features)."""
+class ChannelwiseGraphOps(FusedGraphOps):
+    """The passes of a 'uu' layer where the kernels can mix the rows: a pass writes rows only where that is faster.
 
-    def __init__(self, graph: EdgeGraph, plan: GraphTPPlan):
-        self.graph, self.plan = graph, plan
+    Mixing saves writing and reading the rows, which counts with few edges a node; where the edges count, a pass without rows is
+    the slower one at l_max 3 (sums of 64 channels run on tensor cores, others on four warps a node), and the weights' gradient
+    costs a walk over all edges, shared with the features' gradient, unless the rows of the forward pass are kept.  The limits are
+    the crossings of both forms over 100 to 100k nodes of 2 to 60 edges.  l_max 3, us, with rows / mixed: forward pass of 30k nodes, 64
+    channels, of 8 edges 649 / 551, of 12 672 / 760; forward pass and the gradients of features and weights, 10k nodes, 128 channels, of 20 edges
+    1555 / 1460, of 30 2058 / 2099, of 60 3560 / 3965; forward pass and the weights' gradient alone, l_max 2, 32 channels, 10k nodes of 8
+    edges 56 / 57, of 15 70 / 85."""
+
+    def __init__(self, graph: EdgeGraph, plan: GraphTPPlan, channels: int, need_x: bool, need_weight: bool):
+        super().__init__(graph, plan, "uu")
+        nodes, edges, high = graph.num_dst, graph.num_edges, plan.d_in1 == 16
+        out, x, kept = self._rows_from(channels, nodes)
+        self.keeps = need_weight and (high and edges >= kept * nodes if need_x else self._kept_alone(channels))
+        self.out_rows = self.keeps or (high and edges >= out * nodes)
+        self.x_rows = high and edges >= x * graph.num_src
+        # four warps share the adjoint of a node in a small graph (300 nodes, 4 edges: l_max 2, 32 channels 8.6 / 9.1)
+        self.y_rows = nodes <= 400 and channels == (128 if plan.d_in1 == 4 else 32)
+
+    @staticmethod
+    def _rows_from(channels: int, nodes: int):
+        """Edges a node from which rows are written at l_max 3: in the forward pass, in the gradient of the features alone, and in
+        a forward pass that keeps them for the weights' gradient beside the features'."""
+        if channels == 16:       # few nodes leave SMs idle, and then edges cost little
+            return (60, 60, 60) if nodes < 450 else (25, 25, 45) if nodes < 1500 else (9, 10, 24)
+        # 128: from 100 nodes an SM on the sums' rows come from four warps a node, which gain less over a walk that mixes them
+        return {32: (16, 10, 18), 64: (11, 11, 13), 128: (16, 9, 24 if nodes < 14_800 else 45)}[channels]
+
+    def _kept_alone(self, channels: int) -> bool:
+        """Whether keeping the rows is faster than a walk for the weights' gradient alone: a matter of their bytes (L2 holds 126 MB)."""
+        nodes, edges = self.graph.num_dst, self.graph.num_edges
+        size = nodes * channels * self.plan.fwd_table.num_rows * 4
+        if self.plan.d_in1 == 16:
+            return size < 64e6 or edges >= (5 if channels in (32, 64) else 4) * nodes
+        return edges >= (3 if nodes >= 900 and size < 16e6 else 8 if 1e6 <= size < 48e6 else 13) * nodes
 
     def forward(self, node_x: Tensor, y: Tensor, weight: Tensor):
+        if self.out_rows:
+            out, state = super().forward(node_x, y, weight)
+            return out, state if self.keeps else (*state[:3], None)
         graph = self.graph
         with _profile.timed("cg_segment_sum[fwd]"):
             out, _ = cg_segment_mix(self.plan.fwd_table, node_x, y, graph.src_by_dst, graph.dst_order, graph.dst_ptr, graph.num_dst, weight)
         return out, (node_x, y, weight, None)
 
-    def backward(self, state, grad: Tensor, need):
+    def grad_y(self, state, grad: Tensor) -> Tensor:
+        if self.y_rows:
+            return super().grad_y(state, grad)
         node_x, y, weight, _ = state
-        graph, plan = self.graph, self.plan
-        gx = gy = gw = None
-        if need[1]:
-            with _profile.timed("cg_inner[grad_y]"):
-                gy = cg_inner_mix(plan.fwd_table, node_x, grad, weight, graph.src_by_dst, graph.dst_ptr, graph.dst_order, y.shape[0])
-        if need[0] or need[2]:
-            with _profile.timed("cg_segment_sum[grad_x]"):
-                gx, gw = cg_segment_mix(plan.bwd1_table, grad, y, graph.dst_by_src, graph.src_order, graph.src_ptr, graph.num_src,
-                                        weight, node_x if need[2] else None)
+        graph = self.graph
+        with _profile.timed("cg_inner[grad_y]"):
+            return cg_inner_mix(self.plan.fwd_table, node_x, grad, weight, graph.src_by_dst, graph.dst_ptr, graph.dst_order, y.shape[0])
+
+    def grad_x(self, state, grad: Tensor) -> Tensor:
+        return super().grad_x(state, grad) if self.x_rows else self._walk_sources(state, grad, False)[0]
+
+    def _walk_sources(self, state, grad: Tensor, with_weight: bool):
+        node_x, y, weight, _ = state
+        graph = self.graph
+        with _profile.timed("cg_segment_sum[grad_x]"):
+            return cg_segment_mix(self.plan.bwd1_table, grad, y, graph.dst_by_src, graph.src_order, graph.src_ptr, graph.num_src,
+                                  weight, node_x if with_weight else None)
+
+    def backward(self, state, grad: Tensor, need):
+        if not need[2] or self.keeps:
+            return super().backward(state, grad, need)
+        gy = self.grad_y(state, grad) if need[1] else None
+        gx, gw = self._walk_sources(state, grad, True)
         return gx if need[0] else None, gy, gw
 
 
 class SO3LinearGraphFunction(Function):
     @staticmethod
-    def forward(ctx, node_x: Tensor, y: Tensor, weight: Tensor, graph: EdgeGraph, plan: GraphTPPlan, mode: str):
-        ctx.ops = MixedGraphOps(graph, plan) if mode == "uu" and plan.mixed(graph, node_x, weight) else FusedGraphOps(graph, plan, mode)
+    def forward(ctx, node_x: Tensor, y: Tensor, weight: Tensor, graph: EdgeGraph, plan: GraphTPPlan, mode: str, with_grad: bool):
+        if mode == "uu" and plan.mixed(graph, node_x, weight):
+            ctx.ops = ChannelwiseGraphOps(graph, plan, node_x.shape[-1], with_grad and node_x.requires_grad, with_grad and weight.requires_grad)
+        else:
+            ctx.ops = FusedGraphOps(graph, plan, mode)
         out, state = ctx.ops.forward(node_x, y, weight)
         ctx.save_for_backward(*state)
         if _CHECK_EVERY_CALL:
@@ -230,7 +276,7 @@ class SO3LinearGraphFunction(Function):
         gx, gy, gw = ops.backward(state, grad.contiguous(), ctx.needs_input_grad)
         if _CHECK_EVERY_CALL:
             check_status(grad.device)
-        return gx, gy, gw, None, None, None
+        return gx, gy, gw, None, None, None, None
 
 
 def so3_linear_graph(node_x: Tensor, y: Tensor, weight: Tensor, graph: EdgeGraph, plan: GraphTPPlan,
@@ -239,4 +285,4 @@ def so3_linear_graph(node_x: Tensor, y: Tensor, weight: Tensor, graph: EdgeGraph
     ``y`` (E, D2) in the caller's edge order, shared ``weight``; returns (num_dst, Dout, Cout)."""
     if weight.ndim != (3 if feature_mode == "uv" else 2):
         raise ValueError("the fused graph layer needs weights shared by all edges")
-    return SO3LinearGraphFunction.apply(node_x, y, weight, graph, plan, feature_mode)
+    return SO3LinearGraphFunction.apply(node_x, y, weight, graph, plan, feature_mode, torch.is_grad_enabled())

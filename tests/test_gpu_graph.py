@@ -25,7 +25,8 @@ def _case(seed, nodes, edges, sort_dst=True, isolated=0):
 @pytest.mark.parametrize("irreps,lmax,c,mode", [
     ("0e+1o+2e+3o", 3, 64, "uv"), ("0e+1o+2e+3o", 3, 64, "uu"), ("0e+1o+2e+3o", 3, 32, "uv"),
     ("0e+1o+2e", 2, 64, "uv"), ("0e+1o", 1, 32, "uu"),
-    ("0e+1o+2e+3o", 3, 16, "uv"),          # channel count without unrolled kernel -> table-driven path
+    ("0e+1o+2e+3o", 3, 16, "uv"),
+    ("0e+1o+2e+3o", 3, 24, "uv"),          # channel count without unrolled kernel -> table-driven path
     ("0e+1e+1o+2e", 2, 64, "uv"),          # structure not in the registry -> table-driven path
 ])
 @pytest.mark.parametrize("sort_dst", [True, False])
@@ -53,6 +54,38 @@ def test_fused_graph_layer_matches_oracle(irreps, lmax, c, mode, sort_dst):
         err = float((a.detach().double().cpu() - b.detach()).abs().max() / b.detach().abs().max())
         assert err < 1e-5, f"{name}: relative error {err:.2e}"
     assert torch.count_nonzero(out[nodes - 5:]) == 0     # nodes without incoming edges
+
+
+# edges a node around the limits at which the passes of channel-wise layers write their rows or keep them, and below all of them; 405
+# nodes: the harmonics' gradient without rows at 32 channels
+@pytest.mark.parametrize("lmax,c,nodes,degree", [
+    (1, 32, 97, 3), (1, 128, 97, 14), (2, 16, 97, 6), (2, 32, 97, 9), (2, 32, 405, 3), (2, 128, 97, 5), (2, 128, 97, 14),
+    (3, 16, 97, 4), (3, 16, 97, 23), (3, 32, 405, 6), (3, 32, 97, 14), (3, 32, 97, 19), (3, 64, 97, 6), (3, 64, 97, 11), (3, 64, 97, 17),
+    (3, 128, 97, 4), (3, 128, 97, 15), (3, 128, 97, 23)])
+def test_channelwise_layers_with_any_of_the_gradients(lmax, c, nodes, degree):
+    ir, dim = "+".join(f"{l}{'eo'[l % 2]}" for l in range(lmax + 1)), (lmax + 1) ** 2
+    g, src, dst, vec = _case(lmax + c, nodes, nodes * degree, isolated=2)
+    x, cot = (torch.randn(nodes, dim, c, generator=g) for _ in range(2))
+    layer = enn.SO3LinearGraph(ir, ir, ir, c, c, internal_weights=False, feature_mode="uu").to(DEV)
+    w = torch.randn(*layer.weight_shape, generator=g)
+    xo, vo, wo = (t.double().requires_grad_(True) for t in (x, vec, w))
+    ref = otp.so3_linear_message_passing(xo, vo, src, dst, wo, ir, ir, ir, feature_mode="uu")
+    gref = torch.autograd.grad(ref, [xo, vo, wo], cot.double())
+    graph, harmonics = EdgeGraph(src.to(DEV), dst.to(DEV), nodes), enn.SphericalHarmonics(lmax)
+
+    def close(a, b):
+        return float((a.detach().double().cpu() - b.detach()).abs().max()) < 1e-5 * float(b.detach().abs().max())
+    for need in range(8):
+        ts = [t.to(DEV).requires_grad_(bool(need >> k & 1)) for k, t in enumerate((x, vec, w))]
+        out = layer(ts[0], harmonics(ts[1]), graph, ts[2])
+        assert close(out, ref), need
+        if need:
+            wanted = [k for k in range(3) if need >> k & 1]
+            for k, got in zip(wanted, torch.autograd.grad(out, [ts[k] for k in wanted], cot.to(DEV))):
+                assert close(got, gref[k]), (need, k)
+    with torch.no_grad():
+        assert close(layer(ts[0], harmonics(ts[1]), graph, ts[2]), ref)
+    check_status()
 
 
 def test_fused_graph_layer_equals_per_edge_layer_plus_scatter():
