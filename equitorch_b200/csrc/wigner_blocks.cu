@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(BR_THREADS) block_rotation_whole_kernel(const 
 // end.  Each lane begins with another group of channels: the lanes of a phase then read different banks although the rows are
 // not padded, and a pass copies one run of each operand without a division.  Results go to an image of four samples whose
 // zeros are written once, and the image leaves as one bulk copy.  Two lanes an item are twice the warps in the same shared
-// memory: with one, on padded rows, eight warps an SM waited for their own chains and for barriers (issue 45 %).
+// memory: with one, on padded rows, eight warps an SM waited for their own chains and for barriers (issue 45 %).  An odd number of
+// groups leaves the last to both lanes, two channels each (l = 0..6 of 36 channels, 40k samples 234 -> 207 us).
 // 40k samples, one lane / two: l = 0..6 of 32 channels 232 / 177 us (5.0 TB/s), l = 0..4 of 64 channels 211 / 124, l = 0..2 of 32
 // channels 45 / 35; a third pass in shared memory changes nothing (177, 124, 35).
 constexpr int BG_THREADS = 256;
@@ -413,6 +414,8 @@ struct GradTiles {
   int count;
   uint32_t code[BG_MAX_TILES];                  // first row of the block, its size, tile row, tile column: eight bits each
 };
+enum GradForm { EVEN_GROUPS, ODD_GROUPS, ONE_LANE };      // two lanes an item, with an even or odd number of channel groups; one
+template <GradForm FORM>
 __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const float* __restrict__ g, const float* __restrict__ x,
                                                                          float* __restrict__ gm, int64_t n, int dim, int c,
                                                                          int samples, int image_samples,
@@ -444,8 +447,9 @@ __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const f
     if (++ahead_pass == passes) ahead_pass = 0, ahead += step;
   };
   fetch_next(0);
-  const int lane = threadIdx.x & 31, half = lane & 1, cg = c / 4, groups = (cg + 1 - half) / 2;   // this lane's groups of channels
-  const int first = groups ? (threadIdx.x >> 1) % groups : 0;
+  constexpr int LANES = FORM == ONE_LANE ? 1 : 2;
+  const int lane = threadIdx.x & 31, half = FORM == ONE_LANE ? 0 : lane & 1, groups = c / (4 * LANES);     // this lane's groups of channels
+  const int first = FORM != ONE_LANE && groups ? (threadIdx.x >> 1) % groups : 0;
   for (int64_t base = (int64_t)blockIdx.x * image_samples; base < n; base += step) {
     const int total = (int)min((int64_t)image_samples, n - base);
     for (int pass = 0; pass < passes; ++pass) {
@@ -454,9 +458,9 @@ __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const f
       cp_async_wait<0>();
       __syncthreads();                          // this pass has arrived; the place of the one before it is free
       fetch_next(buf ^ 1);
-      for (int w = threadIdx.x - lane; w < 2 * ns * items; w += blockDim.x) {      // whole warps: the lanes exchange sums
-        const bool made = w + lane < 2 * ns * items;
-        const int i = made ? (w + lane) >> 1 : 0, s = i / items;
+      for (int w = threadIdx.x - lane; w < LANES * ns * items; w += blockDim.x) {  // whole warps: the lanes exchange sums
+        const bool made = w + lane < LANES * ns * items;
+        const int i = made ? (w + lane) / LANES : 0, s = i / items;
         const uint32_t code = tile[i - s * items];
         const int lo = code & 255, size = code >> 8 & 255, np = (size + 3) / 4, pa = code >> 16 & 255, qa = code >> 24;
         const float* gp = stage + buf * 2 * operand + s * features + lo * c;
@@ -469,7 +473,7 @@ __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const f
         }
         uint64_t acc[4][4] = {};                // sums over even and odd channels
         for (int k = 0, at = first; k < groups; ++k, at = at + 1 == groups ? 0 : at + 1) {
-          const int ch = 8 * at + 4 * half;
+          const int ch = 4 * LANES * at + 4 * half;
           ulonglong2 gv[4], xv[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
@@ -484,16 +488,36 @@ __global__ void __launch_bounds__(BG_THREADS) block_rotation_grad_kernel(const f
               pair_fma(acc[u][v], gv[u].y, xv[v].y);
             }
         }
-        // the even lane keeps tile rows 0 and 1, the odd one 2 and 3
+        if constexpr (FORM == ODD_GROUPS) {     // the last group: two channels each
+          const int ch = c - 4 + 2 * half;
+          uint64_t gv[4], xv[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            gv[u] = *reinterpret_cast<const uint64_t*>(gp + ro[u] + ch);
+            xv[u] = *reinterpret_cast<const uint64_t*>(xp + co[u] + ch);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) pair_fma(acc[u][v], gv[u], xv[v]);
+        }
         float* o = img + (part + s) * dd + lo * dim + lo;
+        if constexpr (FORM == ONE_LANE) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int row = pa + (u + 2 * half) * np;
+          for (int u = 0; u < 4; ++u)
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const float low = pair_sum(acc[u][v]), high = pair_sum(acc[u + 2][v]);
-            const float sum = (half ? high : low) + __shfl_xor_sync(0xffffffffu, half ? low : high, 1);
-            if (made && row < size && qa + v * np < size) o[row * dim + qa + v * np] = sum;
+            for (int v = 0; v < 4; ++v)
+              if (made && pa + u * np < size && qa + v * np < size) o[(pa + u * np) * dim + qa + v * np] = pair_sum(acc[u][v]);
+        } else {                                // the even lane keeps tile rows 0 and 1, the odd one 2 and 3
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int row = pa + (u + 2 * half) * np;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const float low = pair_sum(acc[u][v]), high = pair_sum(acc[u + 2][v]);
+              const float sum = (half ? high : low) + __shfl_xor_sync(0xffffffffu, half ? low : high, 1);
+              if (made && row < size && qa + v * np < size) o[row * dim + qa + v * np] = sum;
+            }
           }
         }
       }
@@ -719,9 +743,15 @@ extern "C" int eqt_block_rotation_grad_matrix(const float* grad_out, const float
   gradient_tiles(block_sizes, num_blocks, g);
   const size_t bytes = gradient_samples(g, dim, channels, &samples, &image);
   unsigned grid = 1;
-  const int threads = std::min(BG_THREADS, (2 * samples * g.count + 31) / 32 * 32);
-  if (int rc = resident_grid(block_rotation_grad_kernel, threads, bytes, ceil_div(n, image), &grid)) return rc;
-  block_rotation_grad_kernel<<<grid, threads, bytes, static_cast<cudaStream_t>(stream)>>>(grad_out, x, grad_matrix, n, dim, channels,
+  // few channels are soon multiplied, and then the exchange of sums costs more than the second lane saves, as long as the samples fill
+  // the SMs (40k samples, two lanes / one: l = 0..2 of 4 channels 12.7 / 7.8 us, l = 0..6 of 4 105 / 82, of 12 125 / 105; 300 samples 5.1 /
+  // 6.0; l = 0, 1 of 8 5.8 / 6.7)
+  const bool one = channels <= 12 && dim >= 9 && n >= 16 * (int64_t)sm_count();
+  const auto kernel = one ? block_rotation_grad_kernel<ONE_LANE>
+                          : channels % 8 ? block_rotation_grad_kernel<ODD_GROUPS> : block_rotation_grad_kernel<EVEN_GROUPS>;
+  const int threads = std::min(BG_THREADS, ((one ? 1 : 2) * samples * g.count + 31) / 32 * 32);
+  if (int rc = resident_grid(kernel, threads, bytes, ceil_div(n, image), &grid)) return rc;
+  kernel<<<grid, threads, bytes, static_cast<cudaStream_t>(stream)>>>(grad_out, x, grad_matrix, n, dim, channels,
                                                                                             samples, image, g);
   return check_launch("block_rotation_grad_kernel");
 }

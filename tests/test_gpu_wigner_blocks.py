@@ -98,18 +98,18 @@ def test_features_at_an_odd_offset_take_the_general_kernel():
 
 
 @pytest.mark.parametrize("name,n,c", [("0e+1o+2e+3o+4e+5o+6e", 3001, 4), ("0e+1o+2e+3o+4e+5o+6e", 1303, 36), ("0e+1o+2e", 40003, 12),
-                                      ("9x5o", 701, 8), ("7o", 9002, 64)])
+                                      ("9x5o", 701, 8), ("7o", 9002, 64), ("0e+1o+2e", 301, 12), ("0e+1o", 9001, 4)])
 def test_several_images_a_block(name, n, c):
-    """More samples than one round of blocks holds, the last image not full; entries outside the blocks stay zero.  A sum of
-    c products made in chains of at most c / 4 + 1 multiply-adds with two further additions differs from the exact one by at most
-    (c / 4 + 3) eps times the sum of the magnitudes."""
+    """More samples than one round of blocks holds, the last image not full, or few samples; entries outside the blocks stay zero.  A
+    sum of c products made in chains of at most c / 4 + 1 multiply-adds with two further additions differs from the exact one by at most
+    (c / 4 + 3) eps times the sum of the magnitudes; by one lane, up to 12 channels, in chains of c / 2 with one: (c / 2 + 1) eps."""
     ir, gen = Irreps(name), torch.Generator().manual_seed(c)
     mask = torch.block_diag(*[torch.ones(i.dim, i.dim) for i in ir]).to(DEV)
     g, x = (torch.randn(n, ir.dim, c, generator=gen).to(DEV) for _ in range(2))
     out = dense_rotation_grad_matrix(g, x, block_diagonal(ir, DEV))
     exact = (g.double() @ x.double().mT) * mask
     most = (g.double().abs() @ x.double().abs().mT) * mask
-    assert ((out - exact).abs() <= (c / 4 + 3) * 2.0 ** -24 * most).all()
+    assert ((out - exact).abs() <= max(c / 4 + 3, c / 2 + 1 if c <= 12 else 0) * 2.0 ** -24 * most).all()
 
 
 @pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 30011, 8), ("7o", 3003, 12), ("5x0e", 9001, 4), ("0e+1o+2e+3o+4e+5o", 2501, 64)])
