@@ -583,11 +583,18 @@ int rotation_samples(const RowTiles& t, int dim, int c) {
 
 // Whole matrices where the rows of the blocks, in lines of 128 bytes, touch all of them (l = 0..5 and less; 81 % at l = 0..6, and
 // HBM reads that share of them).  40k samples, by list / whole: l = 0..4 of 64 channels 145 / 120 us, l = 0..3 of 32 67 / 53,
-// l = 0..2 of 32 54 / 38, l = 0..5 of 32 117 / 113, of 64 175 / 177; but l = 0..6 of 32 154 / 177, l = 0..7 of 32 186 / 218.
+// l = 0..2 of 32 54 / 38, l = 0..5 of 32 117 / 113; but l = 0..6 of 32 154 / 177, l = 0..7 of 32 186 / 218.
 bool rotation_whole(const int32_t* sizes, int blocks, int dim) {
   int64_t touched = 124 * (int64_t)dim;
   for (int b = 0; b < blocks; ++b) touched += 4 * (int64_t)sizes[b] * sizes[b];
   return touched >= 4 * (int64_t)dim * dim;
+}
+// Not for operands far beyond L2 where a pass has one or two samples: a block then waits for what it copies, and the list leaves
+// room for more of them (l = 0..4 of 128 channels, 20k samples 99 / 96 us, 40k 190 / 193, 80k 371 / 392; l = 0..5 of 64, 20k 83 / 78, 40k 157 /
+// 161, 80k 306 / 326, of 192, 80k 758 / 847; l = 0..3 of 128, 80k 247 / 254; but l = 0..4 of 96, 80k 314 / 286).
+bool whole_too_slow(int samples, int dim, int c, int64_t n) {
+  const double bytes = 4. * n * ((double)dim * dim + 2. * dim * c);
+  return bytes > 0.8e9 && (samples == 1 || (samples == 2 && (c >= 128 || dim >= 36)));
 }
 // Channels of a thread: twice four where they divide so (l = 0..4 of 64 channels: 134 us with four, 119 so).
 int whole_quads(int c) { return c % 8 ? 1 : 2; }
@@ -713,7 +720,9 @@ extern "C" int eqt_block_rotation(const float* matrix, const float* x, float* ou
   int dim = 0;
   rotation_tiles(block_sizes, num_blocks, t, &dim);
   unsigned grid = 1;
-  if (const int samples = rotation_whole(block_sizes, num_blocks, dim) ? whole_samples(t, dim, channels) : 0) {
+  const int whole = rotation_whole(block_sizes, num_blocks, dim) ? whole_samples(t, dim, channels) : 0;
+  if (whole > 0 && !whole_too_slow(whole, dim, channels, n)) {
+    const int samples = whole;
     const size_t bytes = whole_bytes(dim, channels, samples);
     const auto kernel = whole_quads(channels) == 2 ? block_rotation_whole_kernel<2> : block_rotation_whole_kernel<1>;
     const int items = samples * t.count * (channels / 4 / whole_quads(channels)), threads = std::min(BR_THREADS, (items + 31) / 32 * 32);

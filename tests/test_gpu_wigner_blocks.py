@@ -112,7 +112,9 @@ def test_several_images_a_block(name, n, c):
     assert ((out - exact).abs() <= max(c / 4 + 3, c / 2 + 1 if c <= 12 else 0) * 2.0 ** -24 * most).all()
 
 
-@pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 30011, 8), ("7o", 3003, 12), ("5x0e", 9001, 4), ("0e+1o+2e+3o+4e+5o", 2501, 64)])
+# the last: operands of more than 0.8 GB, by the list of entries
+@pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 30011, 8), ("7o", 3003, 12), ("5x0e", 9001, 4), ("0e+1o+2e+3o+4e+5o", 2501, 64),
+                                      ("0e+1o+2e+3o+4e+5o", 34003, 64)])
 @pytest.mark.parametrize("skip", [0, 1, 3])
 def test_several_passes_of_whole_matrices(name, n, c, skip):
     """More samples than one round of blocks holds, the matrices beginning at any float.  A chain of at most 15 multiply-adds
