@@ -274,6 +274,12 @@ void wgrad_share(WgradShape* w, int count, int cout) {
   }
 }
 
+// Tile of the indexed form: no more rows than leave every SM a tile, but 48 (600 samples, 32 columns, 7 tiles of 96 rows 7.8 us, 13 of 48 6.5).
+bool outer_tile(int64_t n, int cols, int m_tiles, WgradTile* t) {
+  const int64_t rows = ceil_div(ceil_div(n * std::max(m_tiles, 1), sm_count()), 8) * 8;
+  return wgrad_tile(1, cols, t, (int)std::min<int64_t>(96, std::max<int64_t>(48, rows)));
+}
+
 // Splits of a product whose slices all have `tiles` tiles: as many waves of CTAs as leave the SMs least idle (32 slices: 4 splits are 128
 // CTAs, 9 are 288 of 296: 100k samples 712 -> 654 us), a wave's fill and drain counted as six tiles.
 int outer_splits(int64_t tiles, int m_tiles) {
@@ -483,7 +489,7 @@ extern "C" int64_t eqt_outer_tc_scratch_floats(int64_t n, int32_t columns, int32
   using namespace eqt;
   if (n < 0 || columns <= 0 || columns % 32 || m_tiles <= 0) return -1;
   WgradTile tile;
-  if (columns > 128 || !wgrad_tile(1, columns, &tile)) return -1;
+  if (columns > 128 || !outer_tile(n, columns, m_tiles, &tile)) return -1;
   return (int64_t)outer_splits(std::max<int64_t>(1, ceil_div(n, tile.npt)), m_tiles) * m_tiles * 128 * columns;
 }
 
@@ -508,7 +514,7 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
   int splits = 1;
   if (n > 0 && m_tiles > 0) {
     WgradTile tile;
-    if (!wgrad_tile(1, columns, &tile)) return fail(EQT_ERR_UNSUPPORTED, "tile does not fit shared memory");
+    if (!outer_tile(n, columns, m_tiles, &tile)) return fail(EQT_ERR_UNSUPPORTED, "tile does not fit shared memory");
     const int npt = tile.npt;                                                        // reduction rows per tile
     WgradBatch B{};
     B.count = 1; B.n = n; B.n_cols = columns; B.status = status;
@@ -544,8 +550,8 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
     return EQT_OK;
   }
   const bool many = splits > REDUCE_WARPS;
-  auto* reduce = transposed ? (many ? outer_reduce_kernel<true, REDUCE_WARPS> : outer_reduce_kernel<true, 1>)
-                            : (many ? outer_reduce_kernel<false, REDUCE_WARPS> : outer_reduce_kernel<false, 1>);
+  auto* reduce = transposed ? (many ? outer_reduce_kernel<true, REDUCE_WARPS, 2> : splits >= 4 ? outer_reduce_kernel<true, 1, 4> : outer_reduce_kernel<true, 1, 2>)
+                            : (many ? outer_reduce_kernel<false, REDUCE_WARPS, 2> : splits >= 4 ? outer_reduce_kernel<false, 1, 4> : outer_reduce_kernel<false, 1, 2>);
   const int64_t per_block = 32 * (many ? 1 : REDUCE_WARPS);
   reduce<<<(unsigned)ceil_div((int64_t)num_w * c1 * c2 / 4, per_block), 32 * REDUCE_WARPS, 0, st>>>(
       scratch, out, red_ptr, red_slot, red_scale, splits, (int64_t)m_tiles * 128, num_w, c1, c2, columns);
