@@ -258,20 +258,37 @@ int wgrad_shape(const eqt_mix_block& blk, int b, int64_t n, int cin, int cout, W
 // Blocks of one launch share the SMs: another split for the block whose CTAs have the most tiles, while there are SMs.  A launch is then
 // one wave of CTAs with about as many tiles each, where every block on all SMs made a wave a block: each with its own fill and
 // drain, of one or two tiles a CTA on small batches (10k nodes, l_max 3, 64 channels 100 -> 82 us, 1000 nodes, l_max 2 22.3 -> 10.7).
+// A wide layer has so many slices of M that its high degrees, with the fewest nodes a tile, would not get a second split in one wave and
+// run alone at its end: two to four waves where that makes CTAs more even than it costs, each wave's fill and drain counted as six tiles.
 void wgrad_share(WgradShape* w, int count, int cout) {
-  int ctas = 0;
+  const int sms = sm_count();
+  int ctas = 0, best[WGRAD_MAX_BLOCKS];
+  double even = 6;                                                  // tiles of a CTA if all were alike
   for (int b = 0; b < count; ++b) {
     w[b].split(1, cout);
     ctas += w[b].m_tiles;
+    even += (double)w[b].tiles * w[b].m_tiles / sms;
   }
-  for (;;) {
-    int most = 0;
-    for (int b = 1; b < count; ++b)
-      if (w[b].tiles * w[most].splits > w[most].tiles * w[b].splits) most = b;
-    if (ctas + w[most].m_tiles > sm_count() || w[most].splits >= w[most].tiles) return;
-    ctas += w[most].m_tiles;
-    w[most].split(w[most].splits + 1, cout);
+  double least = 1e300;
+  for (int waves = 1; waves <= 4; ++waves) {
+    int64_t longest = 0;
+    for (;;) {
+      int most = 0;
+      for (int b = 1; b < count; ++b)
+        if (w[b].tiles * w[most].splits > w[most].tiles * w[b].splits) most = b;
+      longest = ceil_div(w[most].tiles, w[most].splits);
+      if (ctas + w[most].m_tiles > waves * sms || w[most].splits >= w[most].tiles) break;
+      ctas += w[most].m_tiles;
+      w[most].split(w[most].splits + 1, cout);
+    }
+    const double cost = (double)ceil_div(ctas, sms) * (double)(longest + 6);
+    if (cost < 0.97 * least) {
+      least = cost;
+      for (int b = 0; b < count; ++b) best[b] = w[b].splits;
+    }
+    if (cost < 1.13 * even) break;
   }
+  for (int b = 0; b < count; ++b) w[b].split(best[b], cout);
 }
 
 // Tile of the indexed form: no more rows than leave every SM a tile, but 48 (600 samples, 32 columns, 7 tiles of 96 rows 7.8 us, 13 of 48 6.5).
