@@ -6,6 +6,7 @@
 // tensor-product layers do not go through these kernels but through the fused ones in
 // so3_fused.cu; these cover every flag combination of the operator API.
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <type_traits>
 
@@ -526,11 +527,11 @@ __global__ void __launch_bounds__(256) outer_acc_kernel(P p, int64_t chunk) {
     }
 }
 
-// The same for few channels (C1 and C2 multiples of four, up to 2048 products, 4096 for up to 1024 samples, float32): a team of (C1 / 4)
-// (C2 / 4) threads per sample, four by four products a thread, operands straight from global memory, of which tiles of 64 x 64 would use a
-// sixteenth at 16 x 16 channels.  Entries outside, samples inside, four of them in flight; the teams' sums meet in shared memory.  99 rows
-// into 23 outputs: 18k samples, 16 x 16 1980 -> 240 us; 20k samples, 24 x 24 2055 -> 530, 32 x 64 2124 -> 2104, 64 x 64 2151 -> 4239; 1000
-// samples, 64 x 64 103 -> 93; 252 entries into 41 outputs, 70k samples, 16 x 16 14.3 -> 1.9 ms.
+// The same for few channels (C1 and C2 multiples of four, float32; outer_few_wanted): a team of (C1 / 4) (C2 / 4) threads per sample, four
+// by four products a thread, operands straight from global memory, of which tiles of 64 x 64 would use a sixteenth at 16 x 16
+// channels.  Entries outside, samples inside, four of them in flight; the teams' sums meet in shared memory.  99 rows into 23 outputs,
+// 20k samples, 16 x 16 1909 -> 195 us, 24 x 24 1933 -> 389; 5000 samples, 48 x 40 528 -> 367; 252 entries into 41 outputs, 5000 samples, 16 x 16
+// 1096 -> 125.
 __global__ void __launch_bounds__(256) outer_acc_few_kernel(P p, int64_t chunk, int team, int teams) {
   extern __shared__ __align__(16) float sums[];            // [teams][C1][C2]
   const float* x = static_cast<const float*>(p.in1);
@@ -801,6 +802,27 @@ __global__ void __launch_bounds__(256) vecmat_direct_kernel(P p, int accumulated
 // ------------------------------------------------------------------------------------------
 inline bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
+// Chunks of samples for outer_acc_few_kernel, at most `most` of them: one sum after the other of k terms adds k to the square of the rounding
+// error (in units of 2^-24 and of half the result), which are here a thread's samples, the teams and the chunks' atomics, and
+// with the tiles of outer_acc_kernel `tiled` chunks and their samples.  No more chunks than keep the error below the tiles' (1000 samples,
+// one entry an output, 48 x 40 channels: tiles 1.5e-7, 125 chunks of two teams 2.1e-7).
+int64_t few_chunks(int64_t n, int teams, int64_t tiled, int64_t most) {
+  const double per_team = (double)n / teams, limit = 0.9 * ((double)tiled + (double)n / tiled) - teams, root = limit * limit - 4 * per_team;
+  const double chunks = limit > 0 && root >= 0 ? (limit + std::sqrt(root)) / 2 : std::sqrt(per_team);
+  return std::max<int64_t>(1, std::min<int64_t>({(int64_t)chunks, most, ceil_div(n, 4 * teams), 65535}));
+}
+
+// Whether teams are the faster kernel.  Up to 1024 products, or where tiles of 64 x 64 would be mostly padding, always.  One or two teams
+// a block are worth it for sums of several entries, where the tiles' indexing costs as much as their products (48 x 40, 23 rows into 9
+// outputs, 1000 samples 43 -> 35 us, 20k 438 -> 338), without sums only for few samples (4 rows, 1000 samples 23 -> 16, 20k 82 -> 100; segments
+// of one entry each, which the tables here never have, are taken for sums: 30 rows, 1000 samples 40 -> 47),
+// beyond 2048 products only for few in any case (64 x 64, 99 rows into 23 outputs, 200 samples 57 -> 41, 400 samples 68 -> 76).
+bool outer_few_wanted(const P& p, int64_t tiles) {
+  const int64_t products = p.c1 * p.c2;
+  if (products > 2048) return products <= 4096 && p.n <= 512 && p.n * p.num_out <= 4608;
+  return products <= 1024 || tiles > 1 || p.seg || p.n * p.num_out <= 8192;
+}
+
 template <typename T>
 int launch(const eqt_product_args& a, P p, cudaStream_t s) {
   const int op = a.op;
@@ -869,18 +891,17 @@ int launch(const eqt_product_args& a, P p, cudaStream_t s) {
     if (a.accumulated) {
       const int64_t tiles = ceil_div(p.c1, 64) * ceil_div(p.c2, 64);
       if (p.num_out > 65535) return fail(EQT_ERR_UNSUPPORTED, "accumulated outer: more than 65535 output rows");
-      if (std::is_same<T, float>::value && p.c1 % 4 == 0 && p.c2 % 4 == 0 && (p.c1 * p.c2 <= 2048 || (p.c1 * p.c2 <= 4096 && p.n <= 1024)) &&
+      int64_t chunks = ceil_div((int64_t)sm_count() * 4, tiles * p.num_out);
+      chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, ceil_div(p.n, 32)));
+      chunks = std::min<int64_t>(chunks, 65535);
+      if (std::is_same<T, float>::value && p.c1 % 4 == 0 && p.c2 % 4 == 0 && outer_few_wanted(p, tiles) &&
           aligned16(p.in1) && aligned16(p.in2)) {
         const int team = (int)(p.c1 * p.c2 / 16), teams = std::min<int>(16, 256 / team);
-        int64_t chunks = std::min<int64_t>(ceil_div((int64_t)sm_count() * 8, p.num_out), ceil_div(p.n, 4 * teams));
-        chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, 65535));
+        chunks = few_chunks(p.n, teams, chunks, ceil_div((int64_t)sm_count() * 8, p.num_out));
         const int64_t chunk = ceil_div(p.n, chunks);
         outer_acc_few_kernel<<<dim3((unsigned)p.num_out, (unsigned)ceil_div(p.n, chunk)), 256, sizeof(float) * teams * p.c1 * p.c2, s>>>(p, chunk, team, teams);
         return check_launch("outer_acc_few_kernel");
       }
-      int64_t chunks = ceil_div((int64_t)sm_count() * 4, tiles * p.num_out);
-      chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, ceil_div(p.n, 32)));
-      chunks = std::min<int64_t>(chunks, 65535);
       const int64_t chunk = ceil_div(p.n, chunks);
       dim3 grid((unsigned)tiles, (unsigned)p.num_out, (unsigned)ceil_div(p.n, chunk));
       outer_acc_kernel<T><<<grid, 256, 0, s>>>(p, chunk);

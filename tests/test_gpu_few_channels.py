@@ -51,3 +51,33 @@ def test_operands_off_sixteen_bytes(shift):
     got = indexed_outer_scale_gather(a, b, out_accumulated=True, out_size=rows)
     want = torch.einsum("nra,nrb->rab", a.double(), b.double())
     assert float((got.double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+# two and four samples a thread, the last block of both full of samples or not; 24 input channels keep 32 columns on these kernels
+@pytest.mark.parametrize("n", [2000, 4096, 4097, 5003])
+@pytest.mark.parametrize("c1,c2", [(16, 16), (24, 32)])
+def test_products_of_many_outputs(n, c1, c2):
+    g = torch.Generator().manual_seed(n + c2)
+    rows, out = 13, 40
+    a, w = torch.randn(n, rows, c1, generator=g).to(DEV), torch.randn(rows, c1, c2, generator=g).to(DEV)
+    i1, i2 = torch.randint(0, rows, (3 * out,), generator=g).to(DEV), torch.randint(0, rows, (3 * out,), generator=g).to(DEV)
+    scale = torch.randn(3 * out, generator=g).to(DEV)
+    seg = torch.arange(0, 3 * out + 1, 3, device=DEV)
+    got = indexed_vecmat_scale_gather(a, w, scale, i1, i2, seg, out_size=out)
+    want = torch.einsum("nta,tab->ntb", a.double()[:, i1] * scale.double()[:, None], w.double()[i2]).view(n, out, 3, c2).sum(2)
+    assert float((got.double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("n,c1,c2", [(450, 64, 64), (1000, 48, 40), (5000, 128, 16), (5000, 8, 128)])
+def test_sums_of_one_entry_keep_the_error_of_tiles(n, c1, c2):
+    """K additions one after the other of terms of random sign, each rounded by at most half a unit of the partial sum, are off by at
+    most 2^-24 sqrt(K / 6) of the norm of the result.  Tiles of 64 x 64 add up their samples and as many chunks as four blocks an SM are, of
+    at least 32 samples; the teams of few channels make no longer sums than that."""
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    rows = 4
+    chunks = min(-(-4 * sms // (rows * -(-c1 // 64) * -(-c2 // 64))), -(-n // 32))
+    g = torch.Generator().manual_seed(n)
+    a, b = torch.randn(n, rows, c1, generator=g).to(DEV), torch.randn(n, rows, c2, generator=g).to(DEV)
+    got = indexed_outer_scale_gather(a, b, out_accumulated=True, out_size=rows)
+    want = torch.einsum("nra,nrb->rab", a.double(), b.double())
+    assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24 * ((chunks + n / chunks) / 6) ** 0.5
