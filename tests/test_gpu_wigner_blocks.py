@@ -98,23 +98,33 @@ def test_features_at_an_odd_offset_take_the_general_kernel():
 
 
 @pytest.mark.parametrize("name,n,c", [("0e+1o+2e+3o+4e+5o+6e", 3001, 4), ("0e+1o+2e+3o+4e+5o+6e", 1303, 36), ("0e+1o+2e", 40003, 12),
-                                      ("9x5o", 701, 8), ("7o", 9002, 64), ("0e+1o+2e", 301, 12), ("0e+1o", 9001, 4)])
+                                      ("9x5o", 701, 8), ("7o", 9002, 64)])
 def test_several_images_a_block(name, n, c):
-    """More samples than one round of blocks holds, the last image not full, or few samples; entries outside the blocks stay zero.  A
-    sum of c products made in chains of at most c / 4 + 1 multiply-adds with two further additions differs from the exact one by at most
-    (c / 4 + 3) eps times the sum of the magnitudes; by one lane, up to 12 channels, in chains of c / 2 with one: (c / 2 + 1) eps."""
+    """More samples than one round of blocks holds, the last image not full; entries outside the blocks stay zero.  A sum of
+    c products made in chains of at most c / 4 + 1 multiply-adds with two further additions differs from the exact one by at most
+    (c / 4 + 3) eps times the sum of the magnitudes."""
     ir, gen = Irreps(name), torch.Generator().manual_seed(c)
     mask = torch.block_diag(*[torch.ones(i.dim, i.dim) for i in ir]).to(DEV)
     g, x = (torch.randn(n, ir.dim, c, generator=gen).to(DEV) for _ in range(2))
     out = dense_rotation_grad_matrix(g, x, block_diagonal(ir, DEV))
     exact = (g.double() @ x.double().mT) * mask
     most = (g.double().abs() @ x.double().abs().mT) * mask
-    assert ((out - exact).abs() <= max(c / 4 + 3, c / 2 + 1 if c <= 12 else 0) * 2.0 ** -24 * most).all()
+    assert ((out - exact).abs() <= (c / 4 + 3) * 2.0 ** -24 * most).all()
 
 
-# the last: operands of more than 0.8 GB, by the list of entries
-@pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 30011, 8), ("7o", 3003, 12), ("5x0e", 9001, 4), ("0e+1o+2e+3o+4e+5o", 2501, 64),
-                                      ("0e+1o+2e+3o+4e+5o", 34003, 64)])
+@pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 301, 12), ("0e+1o", 9001, 4), ("0e+1o+2e", 40003, 8)])
+def test_matrix_gradient_of_few_channels(name, n, c):
+    """Few samples, blocks too small for one lane an item, and one lane an item, whose chains of c / 2 multiply-adds meet in one addition."""
+    ir, gen = Irreps(name), torch.Generator().manual_seed(c)
+    mask = torch.block_diag(*[torch.ones(i.dim, i.dim) for i in ir]).to(DEV)
+    g, x = (torch.randn(n, ir.dim, c, generator=gen).to(DEV) for _ in range(2))
+    out = dense_rotation_grad_matrix(g, x, block_diagonal(ir, DEV))
+    exact = (g.double() @ x.double().mT) * mask
+    most = (g.double().abs() @ x.double().abs().mT) * mask
+    assert ((out - exact).abs() <= max(c / 4 + 3, c / 2 + 1) * 2.0 ** -24 * most).all()
+
+
+@pytest.mark.parametrize("name,n,c", [("0e+1o+2e", 30011, 8), ("7o", 3003, 12), ("5x0e", 9001, 4), ("0e+1o+2e+3o+4e+5o", 2501, 64)])
 @pytest.mark.parametrize("skip", [0, 1, 3])
 def test_several_passes_of_whole_matrices(name, n, c, skip):
     """More samples than one round of blocks holds, the matrices beginning at any float.  A chain of at most 15 multiply-adds
@@ -128,3 +138,8 @@ def test_several_passes_of_whole_matrices(name, n, c, skip):
         blocks = (m * mask).double()
         blocks = blocks.mT if transposed else blocks
         assert ((out - blocks @ x.double()).abs() <= 15 * 2.0 ** -24 * (blocks.abs() @ x.double().abs())).all()
+
+
+def test_operands_of_more_than_eight_hundred_megabytes_by_the_list():
+    for skip in (0, 1, 3):
+        test_several_passes_of_whole_matrices("0e+1o+2e+3o+4e+5o", 34003, 64, skip)
