@@ -237,19 +237,32 @@ int launch_wgrad(const WgradBatch& b, size_t smem, cudaStream_t st) {
 // Launch shape of the weight-gradient GEMM of one block: reduction rows per tile, M tiles, node splits and the
 // floats of scratch the per-CTA partial sums need.  Returns an error code for blocks that do not fit.
 struct WgradShape {
-  int npt, rows_pad, m_tiles, splits, chunk_tiles, issuers;
+  int npt, rows_pad, m_tiles, splits, issuers;
   size_t smem;
   int64_t K, tiles, need;
   void split(int s, int cout) { splits = s; need = (int64_t)s * m_tiles * 128 * cout; }
 };
-int wgrad_shape(const eqt_mix_block& blk, int b, int64_t n, int cin, int cout, WgradShape* w) {
+// Tiles of an accumulator before it is folded into registers: 320 terms.  A single issuer's accumulator has every tile of its CTA, and one of
+// few tiles folds them in thirds, which keeps its error at that of two issuers with half of them each (l = 0..4, 128 channels, 1500
+// nodes, six tiles: 7.0e-7 of the norm in one, 5.2e-7 with two issuers).
+int wgrad_chunk(int rows_pad, int issuers, int64_t tiles) {
+  const int64_t most = std::max(1, 320 / rows_pad);
+  return (int)(issuers == 1 ? std::min<int64_t>(most, ceil_div(tiles, 3)) : most);
+}
+
+// Rows of a tile: no more than leave every SM one, but 32.
+int wgrad_rows(const eqt_mix_block* blocks, int count, int64_t n, int cin) {
+  int64_t rows = 0;
+  for (int b = 0; b < count; ++b) rows += n * blocks[b].dim * ceil_div((int64_t)blocks[b].paths * cin, 128);
+  return (int)std::min<int64_t>(96, std::max<int64_t>(32, ceil_div(ceil_div(rows, sm_count()), 8) * 8));
+}
+int wgrad_shape(const eqt_mix_block& blk, int b, int64_t n, int cin, int cout, int rows, WgradShape* w) {
   if (blk.dim <= 0 || blk.dim > TILE_M || blk.paths <= 0) return fail(EQT_ERR_BAD_ARGUMENT, "bad block %d", b);
   WgradTile tile;
-  if (!wgrad_tile(blk.dim, cout, &tile)) return fail(EQT_ERR_UNSUPPORTED, "irrep with %d components does not fit a reduction tile", blk.dim);
+  if (!wgrad_tile(blk.dim, cout, &tile, rows) && !wgrad_tile(blk.dim, cout, &tile)) return fail(EQT_ERR_UNSUPPORTED, "irrep with %d components does not fit a reduction tile", blk.dim);
   w->npt = tile.npt; w->rows_pad = tile.rows_pad; w->smem = tile.smem; w->issuers = tile.issuers;
   w->K = (int64_t)blk.paths * cin;                               // M extent of this GEMM
   w->m_tiles = (int)ceil_div(w->K, 128);
-  w->chunk_tiles = std::max(1, 320 / w->rows_pad);
   w->tiles = ceil_div(n, w->npt);
   w->split((int)std::max<int64_t>(1, std::min<int64_t>(w->tiles, sm_count() / w->m_tiles)), cout);
   return EQT_OK;
@@ -322,8 +335,9 @@ extern "C" int64_t eqt_wgrad_tc_scratch_floats(int64_t n, int32_t cin, int32_t c
   // largest block's need alone (one launch per block then)
   int64_t together = 0, alone = 0;
   std::vector<WgradShape> shapes(num_blocks);
+  const int tile_rows = wgrad_rows(blocks, num_blocks, n, cin);
   for (int b = 0; b < num_blocks; ++b) {
-    if (wgrad_shape(blocks[b], b, std::max<int64_t>(n, 1), cin, cout, &shapes[b])) return -1;
+    if (wgrad_shape(blocks[b], b, std::max<int64_t>(n, 1), cin, cout, tile_rows, &shapes[b])) return -1;
     alone = std::max(alone, shapes[b].need);
   }
   for (int b0 = 0; b0 < num_blocks; b0 += WGRAD_MAX_BLOCKS) wgrad_share(&shapes[b0], std::min(WGRAD_MAX_BLOCKS, num_blocks - b0), cout);
@@ -342,8 +356,9 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // every block is checked before the first launch, so a refusal leaves gw_packed untouched
   std::vector<WgradShape> shapes(num_blocks);
+  const int tile_rows = wgrad_rows(blocks, num_blocks, n, cin);
   for (int b = 0; b < num_blocks; ++b) {
-    if (int rc = wgrad_shape(blocks[b], b, n, cin, cout, &shapes[b])) return rc;
+    if (int rc = wgrad_shape(blocks[b], b, n, cin, cout, tile_rows, &shapes[b])) return rc;
     if (shapes[b].need > scratch_floats)
       return fail(EQT_ERR_BAD_ARGUMENT, "scratch too small: block %d needs %lld floats, %lld given", b,
                   (long long)shapes[b].need, (long long)scratch_floats);
@@ -363,16 +378,17 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
     B.count = R.count = count;
     B.n = n; B.n_cols = R.cols = cout; B.status = status;
     size_t smem = 0;
-    int cta = 0;
+    int cta = 0, most_splits = 0;
     int64_t scratch_at = 0, quads = 0;
     for (int q = 0; q < count; ++q) {
       const eqt_mix_block& blk = blocks[b0 + q];
       const WgradShape& w = shapes[b0 + q];
       WgradBlock& a = B.blk[q];
-      a.dim = blk.dim; a.npt = w.npt; a.rows_pad = w.rows_pad; a.chunk_tiles = w.chunk_tiles;
+      a.dim = blk.dim; a.npt = w.npt; a.rows_pad = w.rows_pad; a.chunk_tiles = wgrad_chunk(w.rows_pad, w.issuers, ceil_div(w.tiles, w.splits));
       a.m_tiles = w.m_tiles; a.splits = w.splits; a.cta_begin = cta;
       a.partial = scratch + scratch_at;
       cta += w.splits * w.m_tiles;
+      most_splits = std::max(most_splits, w.splits);
       smem = std::max(smem, w.smem);
       a.issuers = w.issuers;
       {
@@ -395,7 +411,13 @@ extern "C" int eqt_wgrad_tc(const float* s, const float* g, float* gw_packed, fl
     }
     R.total = quads;
     if (int rc = launch_wgrad(B, smem, st)) return rc;
-    wgrad_reduce_batched_kernel<<<(unsigned)ceil_div(quads, 32), 32 * REDUCE_WARPS, 0, st>>>(R);
+    auto reduce = [&](auto* kernel, int warps) {
+      kernel<<<(unsigned)ceil_div(quads, 32 * (REDUCE_WARPS / warps)), 32 * REDUCE_WARPS, 0, st>>>(R);
+    };
+    if (most_splits == 1) reduce(wgrad_reduce_batched_kernel<1>, 1);
+    else if (most_splits == 2) reduce(wgrad_reduce_batched_kernel<2>, 2);
+    else if (most_splits <= 4) reduce(wgrad_reduce_batched_kernel<4>, 4);
+    else reduce(wgrad_reduce_batched_kernel<REDUCE_WARPS>, REDUCE_WARPS);
     if (int rc = check_launch("wgrad_reduce_batched_kernel")) return rc;
   }
   return EQT_OK;
@@ -537,10 +559,10 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
     B.count = 1; B.n = n; B.n_cols = columns; B.status = status;
     WgradBlock& a = B.blk[0];
     a.dim = 1; a.npt = npt; a.rows_pad = tile.rows_pad; a.issuers = tile.issuers;
-    a.chunk_tiles = std::max(1, 320 / npt);
     a.a_cols = a_cols; a.b_cols = b_cols; a.b_row_boxes = c2 / 32;
     const int64_t tiles = ceil_div(n, npt);
     splits = outer_splits(tiles, m_tiles);
+    a.chunk_tiles = wgrad_chunk(a.rows_pad, a.issuers, ceil_div(tiles, splits));
     const int64_t need = (int64_t)splits * m_tiles * 128 * columns;
     if (need > scratch_floats) return fail(EQT_ERR_BAD_ARGUMENT, "scratch too small: %lld floats needed", (long long)need);
     a.partial = scratch;
@@ -636,9 +658,10 @@ extern "C" int eqt_wgrad_tc_static(const float* s, const float* g, float* gw_pac
                 "eqt_wgrad_tc with a caller-provided scratch buffer", sm_count(), (int)cout,
                 (long long)kStaticScratchFloats);
   if (n > 0 && num_blocks > 0 && blocks && cin > 0 && cin % 32 == 0 && cout > 0 && cout % 32 == 0) {
+    const int tile_rows = wgrad_rows(blocks, num_blocks, n, cin);
     for (int b = 0; b < num_blocks; ++b) {   // the real need of every block, before anything is launched
       WgradShape w{};
-      if (int rc = wgrad_shape(blocks[b], b, n, cin, cout, &w)) return rc;
+      if (int rc = wgrad_shape(blocks[b], b, n, cin, cout, tile_rows, &w)) return rc;
       if (w.need > kStaticScratchFloats)
         return fail(EQT_ERR_UNSUPPORTED,
                     "eqt_wgrad_tc_static: block %d (%d paths x %d input channels) needs %lld floats of scratch, the "

@@ -140,3 +140,26 @@ def test_wgrad_tc_at_the_edges_of_its_tiles(irreps, n, cin, cout):
     for r in range(plan.rows):
         want[int(info.index2[r])] += s[:, r].double().T @ g[:, int(comp_of_row[r])].double()
     assert float((got.double() - want).abs().max()) <= 8e-6 * float(want.abs().max())
+
+
+# one, two, four and more splits of a block, whose sums one, two, four and eight warps add up; one issuer (more than 64 columns) with one to
+# six tiles a CTA, folded in thirds.  A part of K terms of random sign added by rounding halves, or by truncation in the tensor core, whose
+# steps of eight terms are off by up to a unit each, stays below 2^-24 (sqrt(K / 6) + K / 24); parts are at most 96 terms and the CTAs' sums
+# of K' parts add sqrt(K' / 6), here below 4; the operands' pairs of TF32 values leave 2^-22.
+@pytest.mark.parametrize("n", [1, 5, 20, 33, 60, 130, 1500])
+@pytest.mark.parametrize("irreps,cin,cout", [("3o", 64, 64), ("0e+1o+2e+3o+4e", 128, 128), ("3x1o", 32, 96)])
+def test_weight_gradient_of_few_nodes(irreps, cin, cout, n):
+    ir = Irreps(irreps)
+    fwd, _, _, paths = tp_infos(ir, Irreps("0e"), ir)
+    info = fwd.info_M_fwd.to(DEV)
+    plan = MixPlan(info, [i.dim for i in ir], DEV)
+    gen = torch.Generator().manual_seed(n)
+    s, g = torch.randn(n, plan.rows, cin, generator=gen).to(DEV), torch.randn(n, plan.comps, cout, generator=gen).to(DEV)
+    got = wgrad_tc(s, g, plan, paths)
+    check_status()
+    seg = info.seg_out.cpu() if info.seg_out is not None else torch.arange(info.out_size + 1)
+    comp_of_row = torch.repeat_interleave(torch.arange(info.out_size), seg[1:] - seg[:-1]).to(DEV)
+    path_of_row = info.index2 if info.index2 is not None else torch.arange(plan.rows, device=DEV)
+    per_row = torch.einsum("nri,nro->rio", s.double(), g.double()[:, comp_of_row])
+    want = torch.zeros(paths, cin, cout, dtype=torch.float64, device=DEV).index_add_(0, path_of_row, per_row)
+    assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24 * (4 + 4 + 4) + 2.0 ** -22
