@@ -588,12 +588,22 @@ extern "C" int eqt_outer_tc_grouped(const float* in1, const float* in2, float* o
     if (e != cudaSuccess) return fail(EQT_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
     return EQT_OK;
   }
-  const bool many = splits > REDUCE_WARPS;
-  auto* reduce = transposed ? (many ? outer_reduce_kernel<true, REDUCE_WARPS, 2> : splits >= 4 ? outer_reduce_kernel<true, 1, 4> : outer_reduce_kernel<true, 1, 2>)
-                            : (many ? outer_reduce_kernel<false, REDUCE_WARPS, 2> : splits >= 4 ? outer_reduce_kernel<false, 1, 4> : outer_reduce_kernel<false, 1, 2>);
-  const int64_t per_block = 32 * (many ? 1 : REDUCE_WARPS);
-  reduce<<<(unsigned)ceil_div((int64_t)num_w * c1 * c2 / 4, per_block), 32 * REDUCE_WARPS, 0, st>>>(
-      scratch, out, red_ptr, red_slot, red_scale, splits, (int64_t)m_tiles * 128, num_w, c1, c2, columns);
+  const auto reduce = [&](auto* kernel, int warps) {
+    kernel<<<(unsigned)ceil_div((int64_t)num_w * c1 * c2 / 4, 32 * (REDUCE_WARPS / warps)), 32 * REDUCE_WARPS, 0, st>>>(
+        scratch, out, red_ptr, red_slot, red_scale, splits, (int64_t)m_tiles * 128, num_w, c1, c2, columns);
+  };
+  // eight warps a result from nine splits on, fewer where the results alone fill the SMs (30 x 96 x 96 weights, 512 samples: the sum with eight
+  // warps 8.1 us, with two some 5; but 8 x 32 x 32, 4000 samples, both kernels 17.4 and 19.8)
+  const bool fill = (int64_t)num_w * c1 * c2 / 4 > 32 * 4 * (int64_t)sm_count();
+  const auto by_warps = [&](auto t) {
+    constexpr bool T = t();
+    if (splits > 8 && (!fill || splits >= 32)) reduce(outer_reduce_kernel<T, 8, 2>, 8);
+    else if (splits >= 16) reduce(outer_reduce_kernel<T, 4, 4>, 4);
+    else if (splits > 8) reduce(outer_reduce_kernel<T, 2, 4>, 2);
+    else if (splits >= 4) reduce(outer_reduce_kernel<T, 1, 4>, 1);
+    else reduce(outer_reduce_kernel<T, 1, 2>, 1);
+  };
+  if (transposed) by_warps(std::true_type{}); else by_warps(std::false_type{});
   return check_launch("outer_reduce_kernel");
 }
 
