@@ -13,7 +13,7 @@
 //
 // Precision: float32 results are required to 1e-5, which a single TF32 product (10 mantissa
 // bits) cannot give.  Each operand is split as x = big + small with big = x rounded to the 10
-// mantissa bits of TF32 and small = x - big (exact), and three
+// mantissa bits of TF32 and small = x - big rounded to as many (split_tf32), and three
 // kind::tf32 MMAs accumulate big*big + big*small + small*big in float32 in TMEM; the dropped
 // small*small term is below 2^-22 relative.  The weights are split once on the host side of the
 // call, the activations by four "splitter" warps between the TMA arrival and the MMA issue.
