@@ -863,16 +863,23 @@ inline bool segsum_tc_wanted(const FusedArgs& a) {
 // 128: rounds of 1.5 nodes an SM are short of few nodes (sums of 20 edges, 100 nodes 15.5 / 17.8, 200 23.4 / 20.8, 300 29.0 / 31.0, 600
 // 53.2 / 49.2; 5000 of 8 176 / 149; 40k 1416 / 1739; adjoint of 300 nodes of 20 33.1 / 34.8, of 3, 400 nodes 14.2 / 12.3).  64: sums of
 // few edges a node, where the tensor-core kernel does not run (400 nodes 8.1 / 9.5, 2000 22.4 / 21.1, 8000 96 / 76, 20k 182 / 189, 60k 474 /
-// 585); the adjoint ties.  With few edges a node the rows that a sum writes decide, and past some 0.5 GB of them (1 to 2 GB at l_max 2) four
-// warps write them faster (128 channels: 9000 nodes of 4 200 / 185, 14.5k of 3 243 / 279, l_max 2, 60k of 2 275 / 304; 32: 60k of 3 257 / 278).
+// 585); the adjoint ties.  With few edges a node the rows that a sum writes decide, and from a number of them on that falls with
+// the degree four warps write them faster (128 channels: 9000 nodes of 4 200 / 185, 14.5k of 3 243 / 279, l_max 2, 60k of 2 275 / 304; 32: 60k of 3 257 /
+// 278; one edge a node: l_max 2, 64 channels, 3200 nodes 14.3 / 9.3, 17.6k 38 / 42, 28k 57 / 66, l_max 3, 64, 5500 43.5 / 44.5, 9200 57 / 69,
+// 32, 7600 31 / 31, 14.7k 49 / 56; two: l_max 3, 32, 17k 70 / 71, 35k 121 / 140).
 inline bool walk_wanted(uint64_t key, bool inner, const FusedArgs& a) {
   if (((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.g)) & 15u) != 0 || a.n_out >= 0x7fffffffll ||
       !walk_supported(key, false, inner, a.C) || !walk_sizes(key, false, a.T, a.R, a.DF, a.DY)) return false;
   if (a.DF < 9 || (a.C != 32 && a.C != 64 && a.C != 128)) return true;
   const int64_t sms = sm_count(), n = a.n_out;
-  auto degree_below = [&](int edges) { return a.n_edges < edges * n; };
-  const bool rows_decide = a.DF < 16 ? degree_below(4) && n * a.C > (degree_below(3) ? 50000 : 100000) * sms
-                                     : degree_below(5) && n * a.C > 8200 * sms;
+  auto degree_below = [&](double edges) { return (double)a.n_edges < edges * (double)n; };
+  // floats of a component an SM from which the rows decide
+  int64_t rows_from = INT64_MAX;
+  if (a.DF < 16)
+    rows_from = degree_below(1.25) ? 7500 : degree_below(1.75) ? 15000 : degree_below(2.25) ? 24000 : degree_below(3) ? 50000 : degree_below(4) ? 100000 : rows_from;
+  else if (degree_below(5))
+    rows_from = a.C == 128 || !degree_below(3) ? 8200 : degree_below(1.25) ? 2000 : degree_below(1.75) ? 3000 : degree_below(2.25) ? 3800 : 6000;
+  const bool rows_decide = rows_from < INT64_MAX && n * a.C > rows_from * sms;
   if (!inner && rows_decide) return false;
   if (a.DF < 16) {
     if (a.C == 128) return true;
